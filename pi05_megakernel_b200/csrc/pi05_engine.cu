@@ -33,6 +33,7 @@
 #include "ptx_sm100.cuh"
 
 #include "pi05_common.cuh"
+#include "pi05_steps.h"
 using namespace pi05;
 
 // Four builds of the same device code (see pi05_chunk_kernel.cuh): the production kernel for one observation, the
@@ -155,6 +156,8 @@ struct pi05_engine {
                                  // which would serialise against every other stream of the GPU)
   bool in_flight = false;        // a launch has been issued since the last pi05_status
   bool can_cluster = false;      // the device takes the whole grid as clusters of two
+  bool graphs = true;            // the chunk may run as graphs of kernels (false: the static entry point, which allocates nothing)
+  StepGraphs steps;              // the chunk's kernels, captured for the bound tensors
   std::string config;
   std::string last_error;
 };
@@ -209,10 +212,12 @@ void build_layout(pi05_engine* h) {
   add("rope", B * T * (HD / 2) * 4);
   add("rope2", B * T * (HD / 2) * 4);
   add("x", B * T * ADIM * 4);
+  add("state", 256);
   add("h", B * T * W * 2);
   add("an_attn", B * AN_COPIES * T * W * 2);
   add("an_ffn", B * AN_COPIES * T * W * 2);
   add("qkv_acc", B * T * QKVW * 4);
+  add("q", B * T * QD * 2);
   add("k", B * T * HD * 2);
   add("v", B * T * HD * 2);
   add("attn", B * T * QD * 2);
@@ -220,6 +225,7 @@ void build_layout(pi05_engine* h) {
   add("d_acc", B * T * W * 4);
   add("act", B * T * FF * 2);
   add("att_part", (size_t)(MAX_KEY_GROUPS - 1) * NROW_CTAS * ATT_PART_FLOATS * 4);
+  add("part", steps_part_floats(h->sms, h->max_batch, h->max_prefix) * 4);
   if (h->tp_size > 1) {          // what the peers write into (see pi05_common.cuh)
     add("tp_recv", (size_t)2 * h->tp_size * TP_SLOT_FLOATS * 4);
     add("tp_flags", (size_t)2 * NROW_CTAS * TP_FLAG_STRIDE * 4);
@@ -506,6 +512,37 @@ void describe(pi05_engine* h) {
 
 bool valid_handle(pi05_handle_t h) { return h != nullptr; }
 
+// Whether a launch without debug controls runs as graphs of kernels (pi05_steps.cu).  The persistent kernel stays for
+// tensor parallel, for the static entry point, for debug controls, for callers that set one of its own tuning settings, and
+// for one observation with a short prefix (128 tokens: 5.42 against 5.63 ms; 968 tokens: 6.93 against 6.49).
+bool uses_graphs(const pi05_engine* h) {
+  pi05_tuning d;
+  default_tuning(&d);
+  d.poll_ns = h->tune.poll_ns;
+  return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0 && (h->batch > 1 || h->prefix > 384);
+}
+
+int build_graphs(pi05_engine* h, int n_steps, int n_layers) {
+  StepSetup s;
+  memset(&s, 0, sizeof s);
+  s.device = h->device; s.sms = h->sms; s.batch = h->batch; s.prefix = h->prefix;
+  s.in = h->inputs;
+  s.actions = (float*)h->actions;
+  s.status = region_ptr<unsigned int>(h, "ctrl");
+  s.state = region_ptr<int>(h, "state");
+  s.temb = region_ptr<float>(h, "temb"); s.hid = region_ptr<float>(h, "hid"); s.cond = region_ptr<float>(h, "cond");
+  s.mod = region_ptr<float>(h, "mod"); s.x = region_ptr<float>(h, "x"); s.part = region_ptr<float>(h, "part");
+  s.rope = region_ptr<uint32_t>(h, "rope");
+  s.h = region_ptr<__nv_bfloat16>(h, "h"); s.an = region_ptr<__nv_bfloat16>(h, "an_attn");
+  s.q = region_ptr<__nv_bfloat16>(h, "q"); s.k = region_ptr<__nv_bfloat16>(h, "k"); s.v = region_ptr<__nv_bfloat16>(h, "v");
+  s.attn = region_ptr<__nv_bfloat16>(h, "attn"); s.act = region_ptr<__nv_bfloat16>(h, "act");
+  s.maps = &h->maps;
+  s.page_table = region_ptr<int>(h, "page_table");
+  s.pages_per_obs = h->pages_per_obs; s.page_tokens = h->page_tokens;
+  s.wait_limit = h->wait_limit;
+  return steps_build(s, n_steps, n_layers, &h->steps, &h->last_error);
+}
+
 }  // namespace
 
 // =========================================================================================== C ABI
@@ -737,6 +774,9 @@ int pi05_bind_view(pi05_handle_t h, const void* const inputs[PI05_NUM_INPUTS], c
   e = cudaMemcpy(region_ptr<void>(h, "page_table"), kv->page_table, (size_t)batch * kv->pages_per_obs * sizeof(int),
                  cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail_cuda(h, "cudaMemcpy(page table)", e);
+  steps_free(&h->steps);
+  if (uses_graphs(h) && (rc = build_graphs(h, NS, NL))) return rc;
+  describe(h);
   e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceSynchronize", e);
   h->bound = true;
@@ -752,7 +792,10 @@ int pi05_debug(pi05_handle_t h, int max_stage, long long wait_limit_cycles, int 
   if (!valid_handle(h) || drop_event >= NEVENTS) return PI05_ERR_ARGUMENT;
   h->drop_event = drop_event < 0 ? -1 : drop_event;
   h->max_stage = max_stage < 0 ? 0x7fffffff : max_stage;
-  if (wait_limit_cycles > 0) h->wait_limit = wait_limit_cycles;
+  if (wait_limit_cycles > 0 && wait_limit_cycles != h->wait_limit) {
+    h->wait_limit = wait_limit_cycles;
+    h->steps.n_steps = 0;          // captured with the old limit: the next launch captures again
+  }
   return PI05_OK;
 }
 
@@ -762,6 +805,25 @@ int pi05_launch(pi05_handle_t h, int n_steps, int n_layers, void* stream, unsign
   if (n_steps < 1 || n_steps > NS || n_layers < 1 || n_layers > NL) return PI05_ERR_ARGUMENT;
   DeviceGuard guard(h->device);
   if (!guard.ok) return PI05_ERR_CUDA;
+  // stamps or a debug control wanted: the traced build of the persistent kernel
+  const bool debug = stamps != nullptr || h->max_stage != 0x7fffffff || h->drop_event >= 0;
+  if (!debug && uses_graphs(h)) {
+    if (h->steps.n_steps != n_steps || h->steps.n_layers != n_layers) {
+      if (h->in_flight) {          // the graphs that are about to be replaced may still be running
+        const cudaError_t e = cudaEventSynchronize(h->done);
+        if (e != cudaSuccess) return fail_cuda(h, "cudaEventSynchronize", e);
+      }
+      const int rc = build_graphs(h, n_steps, n_layers);
+      if (rc != PI05_OK) return rc;
+    }
+    cudaError_t e = steps_launch(h->steps, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail_cuda(h, "graph launch", e);
+    h->launches++;
+    e = cudaEventRecord(h->done, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail_cuda(h, "cudaEventRecord", e);
+    h->in_flight = true;
+    return PI05_OK;
+  }
   Params p;
   memset(&p, 0, sizeof p);
   p.maps = h->maps;
@@ -826,10 +888,8 @@ int pi05_launch(pi05_handle_t h, int n_steps, int n_layers, void* stream, unsign
   for (int s = 0; s < NS; ++s) p.t_steps[s] = (float)(1.0 + s * dt);
   p.dt = (float)dt;
   void* args[] = {&p};
-  // stamps or a debug control wanted: the traced build; otherwise the build without that code, specialised for
-  // one observation when there is only one, and with two or four observations side by side in every MMA when
-  // there are several (a weight stage in shared memory then serves all of them)
-  const bool debug = stamps != nullptr || h->max_stage != 0x7fffffff || h->drop_event >= 0;
+  // the traced build, or the build without that code: specialised for one observation when there is only one, and with
+  // two observations side by side in every MMA when the tuning asks for it
   const int gn = h->gn;
   if (debug && h->tp_size > 1) {
     h->last_error = "stamps and debug controls are not available in a tensor-parallel engine";
@@ -1032,6 +1092,8 @@ int pi05_destroy(pi05_handle_t h) {
   if (!valid_handle(h)) return PI05_ERR_ARGUMENT;
   if (h->done) {
     DeviceGuard guard(h->device);
+    if (h->in_flight) cudaEventSynchronize(h->done);     // the graphs must not go while they run
+    steps_free(&h->steps);
     cudaEventDestroy(h->done);
     if (h->side) cudaStreamDestroy(h->side);
     for (int r = 0; r < MAX_TP; ++r)
@@ -1093,6 +1155,7 @@ extern "C" int pi05_chunk_static(int device, const void* const inputs[PI05_NUM_I
       cudaError_t e = cudaGetSymbolAddress(&ptr, g_pi05_static_scratch);
       if (e != cudaSuccess || ptr == nullptr) { cudaGetLastError(); pi05_destroy(h); return PI05_ERR_CUDA; }
     }
+    h->graphs = false;             // instantiating a graph takes device memory
     slot.h = h;
     slot.scratch = ptr;
     slot.bound = false;

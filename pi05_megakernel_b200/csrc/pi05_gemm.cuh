@@ -1,0 +1,337 @@
+// The projections of the action chunk as tcgen05 GEMMs: out[tokens, N] = A[tokens, K] . W[N, K]^T with a fused epilogue.
+//
+// One CTA (or CTA pair, cta_group::2) works on output tiles of `rows` <= 128 tokens per CTA x BN features x a K range.  The
+// kernels of a chunk form one dependent chain of ~2-5 us each, so what matters is the time from the end of one to the first
+// MMA of the next:
+//   * weights do not depend on the chain, so a CTA fills its whole weight ring before it waits for the kernel before it
+//     (programmatic dependent launch);
+//   * a stage holds both operands of KS 64-k blocks behind one barrier, and its MMAs and the commit that frees it are one asm
+//     block: with a barrier and a commit per operand and 64-k block the issuing warp needed ~570 cycles for four MMAs that
+//     take the tensor core 160-200;
+//   * the tile's tokens are balanced (rows = ceil(tokens / tiles)) and only those rows are copied; the MMA still reads 128
+//     rows, the ones beyond the tile are whatever shared memory holds and end in accumulator lanes nobody reads;
+//   * K is split over several CTAs where whole-K tiles would leave SMs without work; every split stores its FP32 partial
+//     sums to a slice of its own and the residual kernel adds the slices (atomics made the end of the kernel ~1 us later);
+//   * results go through shared memory, so that a warp's stores cover whole lines (a thread per row stores 16 bytes to 32
+//     different lines, which the LSU takes one at a time: 2 us at 128 features per thread);
+//   * with more tiles than CTAs the launch is persistent with two accumulators, so that a tile's epilogue runs under the
+//     next tile's MMAs.
+#pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <stdint.h>
+
+#include "pi05_common.cuh"
+#include "ptx_sm100.cuh"
+
+namespace gemm {
+using namespace pi05;
+
+constexpr int THREADS_G = 320;     // warp 0 producer, warp 1 MMA issuer, warps 2..9 epilogue (two per TMEM lane quadrant)
+constexpr int EPI_THREADS = 256;
+constexpr int BK = 64;             // k per stage (one 128-byte swizzle row)
+constexpr int MAX_STAGES = 16;
+
+enum { EPI_QKV = 0, EPI_GEGLU = 1, EPI_PART = 2 };
+
+struct Args {
+  CUtensorMap a;                   // activations [tokens, K], box {64, rows}
+  CUtensorMap b0, b1, b2;          // weights, box {64, BN / 2}.  QKV: wq, wk, wv; GEGLU: gate, up; PART: b0
+  int tokens, rows, m_groups, splits, kblocks, units, layer, stages, a_stride, bufs, off_out;   // kblocks: 64-k blocks per unit
+  unsigned int* status;
+  long long limit;
+  __nv_bfloat16 *q, *k, *v;        // EPI_QKV: [tokens, 2048], [tokens, 256], [tokens, 256]
+  const uint32_t* rope;            // [tokens][128]: cos BF16 | sin BF16 << 16
+  __nv_bfloat16* act;              // EPI_GEGLU: [tokens, 4096]
+  float* part;                     // EPI_PART: [splits][tokens, 1024]
+};
+
+__device__ __forceinline__ float rb(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+__device__ __forceinline__ float lo16(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float hi16(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// 0.5 x (1 + tanh z) = x / (1 + exp(-2 z)) with z = 0.79788 (x + 0.044715 x^3): one exponential and one division, no
+// cancellation for negative x.  The constants carry the factor -2 log2 e.
+__device__ __forceinline__ float gelu_tanh(float x) {
+  const float e = ptx::ex2_approx(x * fmaf(x * x, -0.10294324f, -2.3022082f));
+  return __fdividef(x, 1.0f + e);
+}
+
+// Row bytes of a tile's results in the staging buffer (0: small tiles store directly), and its row stride.
+template <int EPI, int BN>
+__host__ __device__ constexpr int out_bytes() {
+  return EPI == EPI_PART ? (BN >= 64 ? BN * 4 : 0) : EPI == EPI_GEGLU ? (BN >= 128 ? BN : 0) : (BN >= 64 ? BN * 2 : 0);
+}
+
+// This thread's token row of the accumulator (TMEM lanes of its warp, BN columns from t0); `half` is the half of the columns
+// (of each half of the tile for QKV and GEGLU) that its warp handles.  `out` is the row's place in the staging buffer.
+// Eight columns at a time in loops that stay loops: an instruction that runs once costs several cycles to fetch.
+template <int EPI, int BN>
+__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int token, bool live, int half, uint32_t out) {
+  constexpr bool STAGED = out_bytes<EPI, BN>() > 0;
+  const int tok = live ? token : 0;
+  if constexpr (EPI == EPI_PART) {
+    uint32_t src = t0 + half * (BN / 2), dst = out + half * (BN / 2) * 4;
+    uint4* g = reinterpret_cast<uint4*>(p.part + ((size_t)split * p.tokens + tok) * W + nt * BN + half * (BN / 2));
+#pragma unroll 1
+    for (int c = 0; c < BN / 2; c += 16) {
+      uint32_t r[16];
+      ptx::tmem_ld_32x16(src + c, r);
+      ptx::tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (STAGED) ptx::st_shared_v4(dst + (c + 4 * j) * 4, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        else if (live) g[c / 4 + j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+      }
+    }
+  } else {
+    // QKV and GEGLU need columns c and c + BN / 2 of the tile together (rotary partner, gate with up)
+    constexpr int PER = HD / BN;                            // QKV: tiles per head
+    const int head = nt / PER, dim0 = (nt % PER) * (BN / 2);
+    const uint4* cs4 = reinterpret_cast<const uint4*>(p.rope + (size_t)tok * 128 + dim0);
+    __nv_bfloat16* g = EPI == EPI_GEGLU ? p.act + (size_t)tok * FF + nt * (BN / 2)
+                       : (head < NQH ? p.q + (size_t)tok * QD + head * HD : (head == NQH ? p.k : p.v) + (size_t)tok * HD) + dim0;
+#pragma unroll 1
+    for (int c = half * (BN / 4); c < (half + 1) * (BN / 4); c += 8) {
+      uint32_t r1[8], r2[8], o1[4], o2[4];
+      ptx::tmem_ld_32x8(t0 + c, r1);
+      ptx::tmem_ld_32x8(t0 + BN / 2 + c, r2);
+      uint4 wa, wb;
+      if (EPI == EPI_QKV) { wa = __ldg(cs4 + c / 4); wb = __ldg(cs4 + c / 4 + 1); }
+      ptx::tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t x = pack2(__uint_as_float(r1[2 * j]), __uint_as_float(r1[2 * j + 1]));
+        const uint32_t y = pack2(__uint_as_float(r2[2 * j]), __uint_as_float(r2[2 * j + 1]));
+        if (EPI == EPI_GEGLU) {
+          const uint32_t z = pack2(gelu_tanh(lo16(x)), gelu_tanh(hi16(x)));
+          o1[j] = pack2(lo16(z) * lo16(y), hi16(z) * hi16(y));
+        } else {
+          // RoPE (reference/pi05.py:218-229 on BF16 tensors): x cos + rotate_half(x) sin, every product and the sum rounded
+          // to BF16; dim d pairs with dim d + 128.  A table word holds cos | sin << 16 of one dim.
+          const uint32_t w0 = j == 0 ? wa.x : j == 1 ? wa.z : j == 2 ? wb.x : wb.z, w1 = j == 0 ? wa.y : j == 1 ? wa.w : j == 2 ? wb.y : wb.w;
+          const uint32_t cw = __byte_perm(w0, w1, 0x5410), sw = __byte_perm(w0, w1, 0x7632);
+          const __nv_bfloat162 co = *reinterpret_cast<const __nv_bfloat162*>(&cw), si = *reinterpret_cast<const __nv_bfloat162*>(&sw);
+          const __nv_bfloat162 xv = *reinterpret_cast<const __nv_bfloat162*>(&x), yv = *reinterpret_cast<const __nv_bfloat162*>(&y);
+          const __nv_bfloat162 a = __hadd2_rn(__hmul2_rn(xv, co), __hmul2_rn(__hneg2(yv), si));
+          const __nv_bfloat162 b = __hadd2_rn(__hmul2_rn(yv, co), __hmul2_rn(xv, si));
+          o1[j] = head <= NQH ? *reinterpret_cast<const uint32_t*>(&a) : x;
+          o2[j] = head <= NQH ? *reinterpret_cast<const uint32_t*>(&b) : y;
+        }
+      }
+      if (STAGED) ptx::st_shared_v4(out + c * 2, o1[0], o1[1], o1[2], o1[3]);
+      else if (live) *reinterpret_cast<uint4*>(g + c) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+      if (EPI == EPI_QKV) {
+        if (STAGED) ptx::st_shared_v4(out + (BN / 2 + c) * 2, o2[0], o2[1], o2[2], o2[3]);
+        else if (live) *reinterpret_cast<uint4*>(g + 128 + c) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+      }
+    }
+  }
+}
+
+// One staged row to its place in memory, as bulk copies out of shared memory.
+template <int EPI, int BN>
+__device__ __forceinline__ void copy_row(const Args& p, uint32_t src, int nt, int split, int token) {
+  if (EPI == EPI_PART) {
+    ptx::bulk_store(p.part + ((size_t)split * p.tokens + token) * W + nt * BN, src, BN * 4);
+  } else if (EPI == EPI_GEGLU) {
+    ptx::bulk_store(p.act + (size_t)token * FF + nt * (BN / 2), src, BN);
+  } else {
+    constexpr int PER = HD / BN;
+    const int head = nt / PER;
+    __nv_bfloat16* dst = (head < NQH ? p.q + (size_t)token * QD + head * HD : (head == NQH ? p.k : p.v) + (size_t)token * HD) +
+                         (nt % PER) * (BN / 2);
+    ptx::bulk_store(dst, src, BN);
+    ptx::bulk_store(dst + 128, src + BN, BN);
+  }
+}
+
+// KS: 64-k blocks per stage.
+template <int EPI, int BN, bool PAIR, int KS>
+__global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__ Args p) {
+  constexpr int WR = PAIR ? BN / 2 : BN;                  // weight rows this CTA loads per 64-k block
+  constexpr int W_BYTES = WR * 128, HALF = (BN / 2) * 128, OUT = out_bytes<EPI, BN>();
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t bars[2 * MAX_STAGES + 4];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
+  const int unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, ustep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  // a stage: KS activation blocks, then KS weight blocks
+  const uint32_t ring = ptx::smem_u32(smem), a_stride = p.a_stride, w_off = KS * a_stride, st_stride = w_off + KS * W_BYTES;
+  const uint32_t full = ptx::smem_u32(bars), empty = full + 8 * MAX_STAGES, t_full = empty + 8 * MAX_STAGES, t_empty = t_full + 16;
+  const bool leader = ptx::elect_one();
+  const int nst = p.kblocks / KS, stages = p.stages;      // stages per unit, stages in the ring
+  const int tcols = p.bufs * (BN < 32 ? 32 : BN);
+
+  if (tid == 0) {
+    // a stage is full when both producers' arrivals (weights, activations) and every byte of both have come
+    for (int i = 0; i < stages; ++i) { ptx::mbar_init(full + 8 * i, 2); ptx::mbar_init(empty + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { ptx::mbar_init(t_full + 8 * i, 1); ptx::mbar_init(t_empty + 8 * i, PAIR ? 2 * EPI_THREADS : EPI_THREADS); }
+    ptx::fence_mbar_init();
+    ptx::fence_proxy_async_shared();
+  }
+  __syncwarp();
+  if (PAIR) ptx::cluster_sync();           // the even CTA's barriers exist before the odd CTA's copies count on them
+
+  // tile of a unit: groups of tokens fastest (neighbours share weights), then K split, then features
+  auto locate = [&](int unit, int& mt, int& split, int& nt) {
+    const int rest = unit / p.m_groups, mg = unit - rest * p.m_groups;
+    nt = rest / p.splits;
+    split = rest - nt * p.splits;
+    mt = PAIR ? 2 * mg + (int)rank : mg;
+  };
+  const CUtensorMap *m0 = &p.b0, *m1 = &p.b0;
+  int r0 = 0, r1 = 0;
+  auto weight_rows = [&](int nt) {
+    if (EPI == EPI_QKV) {                  // tile = BN / 2 dims of a head and their rotary partners
+      constexpr int PER = HD / BN;
+      const int head = nt / PER, d0 = (nt % PER) * (BN / 2);
+      m0 = m1 = head < NQH ? &p.b0 : head == NQH ? &p.b1 : &p.b2;
+      r0 = head < NQH ? p.layer * QD + head * HD + d0 : p.layer * HD + d0;
+      r1 = r0 + 128;
+    } else if (EPI == EPI_GEGLU) {
+      m1 = &p.b1;
+      r0 = r1 = p.layer * FF + nt * (BN / 2);
+    } else {
+      r0 = p.layer * W + nt * BN;
+      r1 = r0 + BN / 2;
+    }
+  };
+  auto load_w = [&](int kc, uint32_t slot) {
+    const uint32_t dst = ring + slot * st_stride + w_off;
+    const uint32_t bar = PAIR ? ptx::map_to_rank(full + 8 * slot, 0) : full + 8 * slot;
+    if (!PAIR || rank == 0) ptx::mbar_expect_tx(full + 8 * slot, (PAIR ? 2 : 1) * KS * W_BYTES);
+#pragma unroll
+    for (int h = 0; h < KS; ++h) {
+      if (PAIR) {
+        ptx::tma_load_2d_pair(dst + h * W_BYTES, rank ? m1 : m0, bar, kc + h * BK, rank ? r1 : r0);
+      } else {
+        ptx::tma_load_2d(dst + h * W_BYTES, m0, bar, kc + h * BK, r0);
+        ptx::tma_load_2d(dst + h * W_BYTES + HALF, m1, bar, kc + h * BK, r1);
+      }
+    }
+  };
+  int ahead = 0;                           // weight stages of the first unit requested before the dependency is waited for
+  if (warp == 0) {
+    int mt, split, nt;
+    locate(unit0, mt, split, nt);
+    weight_rows(nt);
+    ahead = stages < nst ? stages : nst;
+    if (leader) {
+      for (int i = 0; i < ahead; ++i) load_w((split * nst + i) * KS * BK, i);
+      ptx::prefetch_tensormap(&p.a);
+    }
+  } else if (warp == 1) {
+    if (PAIR) { ptx::tmem_alloc_pair(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish_pair(); }
+    else { ptx::tmem_alloc(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish(); }
+    ptx::grid_dep_launch();                // after the allocation: a later kernel cannot take the columns first
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = s_tmem;
+  ptx::grid_dep_wait();
+
+  if (warp == 0) {
+    // ---- producer
+    const uint32_t a_bytes = (uint32_t)p.rows * 128 * KS;
+    uint32_t slot = 0, par = 1;
+    bool ok = true;
+    for (int unit = unit0; ok && unit < p.units; unit += ustep) {
+      int mt, split, nt;
+      locate(unit, mt, split, nt);
+      weight_rows(nt);
+      for (int i = 0; i < nst; ++i) {
+        const int kc = (split * nst + i) * KS * BK;
+        const bool have_w = unit == unit0 && i < ahead;
+        if (!have_w && !(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1))) break;
+        if (leader) {
+          const uint32_t dst = ring + slot * st_stride, bar = PAIR ? ptx::map_to_rank(full + 8 * slot, 0) : full + 8 * slot;
+          if (!PAIR || rank == 0) ptx::mbar_expect_tx(full + 8 * slot, (PAIR ? 2 : 1) * a_bytes);
+#pragma unroll
+          for (int h = 0; h < KS; ++h) {
+            if (PAIR) ptx::tma_load_2d_pair(dst + h * a_stride, &p.a, bar, kc + h * BK, mt * p.rows);
+            else ptx::tma_load_2d(dst + h * a_stride, &p.a, bar, kc + h * BK, mt * p.rows);
+          }
+          if (!have_w) load_w(kc, slot);
+        }
+        if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer (of a pair: the even CTA only)
+    if (!PAIR || rank == 0) {
+      const uint32_t idesc = ptx::umma_idesc_bf16(PAIR ? 256 : 128, BN);
+      const uint64_t adesc0 = ptx::umma_smem_desc(ring), bdesc0 = ptx::umma_smem_desc(ring + w_off);
+      uint32_t slot = 0, par = 0, it = 0;
+      bool ok = true;
+      for (int unit = unit0; ok && unit < p.units; unit += ustep, ++it) {
+        const uint32_t buf = it & 1;
+        if (!(ok = ptx::wait_bar(p.status, p.limit, t_empty + 8 * buf, ((it >> 1) & 1) ^ 1, 6))) break;
+        ptx::tc_fence_after();
+        const uint32_t d = tmem + buf * BN;
+        uint32_t acc = 0;
+        for (int i = 0; i < nst; ++i) {
+          if (!(ok = ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, 3))) break;
+          const uint64_t off = (uint64_t)((slot * st_stride) >> 4);
+          if (leader)
+            ptx::umma_bf16_stage<PAIR, KS>(d, adesc0 + off, bdesc0 + off, idesc, acc, empty + 8 * slot, a_stride >> 4, W_BYTES >> 4);
+          acc = 1;
+          if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; }
+        }
+        if (ok && leader) {
+          if (PAIR) ptx::umma_commit_pair(t_full + 8 * buf);
+          else ptx::umma_commit(t_full + 8 * buf);
+        }
+      }
+    }
+  } else {
+    // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) ..; thread = token row of the tile, half of its columns.  A wait that
+    // gives up does not end the loop: the other epilogue warps count on this one at their barriers
+    const int quad = warp & 3, row = quad * 32 + lane, half = warp >= 6 ? 1 : 0;
+    const uint32_t release = PAIR ? ptx::map_to_rank(t_empty, 0) : 0u;
+    const uint32_t stage = ptx::smem_u32(smem) + p.off_out, out = stage + row * (OUT + 16);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int unit = unit0; unit < p.units; unit += ustep, ++it) {
+      const uint32_t buf = it & 1;
+      int mt, split, nt;
+      locate(unit, mt, split, nt);
+      const int token = mt * p.rows + row;
+      ok &= ptx::wait_bar(p.status, p.limit, t_full + 8 * buf, (it >> 1) & 1, 5);
+      ptx::tc_fence_after();
+      if (OUT > 0 && it > 0) {             // the tile before has left the staging rows of this quadrant
+        ptx::bulk_wait_read();
+        ptx::named_bar_sync(1 + quad, 64);
+      }
+      if (quad * 32 < p.rows)
+        epilogue_row<EPI, BN>(p, tmem + buf * BN + ((uint32_t)(quad * 32) << 16), nt, split, token, ok && row < p.rows && token < p.tokens, half, out);
+      ptx::tc_fence_before();
+      if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);
+      else ptx::mbar_arrive(t_empty + 8 * buf);
+      if constexpr (OUT > 0) {
+        // both warps of the quadrant have written their halves of its 32 rows; each sends 16 of them off
+        ptx::fence_proxy_async_shared();
+        ptx::named_bar_sync(1 + quad, 64);
+        const int r16 = quad * 32 + half * 16 + lane, tok16 = mt * p.rows + r16;
+        if (ok && lane < 16 && r16 < p.rows && tok16 < p.tokens) copy_row<EPI, BN>(p, stage + r16 * (OUT + 16), nt, split, tok16);
+        ptx::bulk_commit();
+      }
+    }
+    if (OUT > 0) ptx::bulk_wait_read();
+  }
+  __syncthreads();
+  if (PAIR) ptx::cluster_sync();           // neither CTA leaves (or frees tensor memory) while the other may still use it
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    if (PAIR) ptx::tmem_dealloc_pair(tmem, tcols);
+    else ptx::tmem_dealloc(tmem, tcols);
+  }
+}
+
+}  // namespace gemm

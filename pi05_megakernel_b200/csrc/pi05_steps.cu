@@ -1,0 +1,742 @@
+// The action chunk as a chain of kernels, one set per layer pass, replayed from CUDA graphs.
+//
+// A layer pass is seven kernels - QKV projection (+ RoPE), attention, O projection, gated residual + adaRMS, gate / up
+// projection (+ GeGLU), down projection, gated residual + adaRMS - and an Euler step is 18 of them, the last residual being
+// the step tail.  The step's kernels are captured once per binding; the Euler step index lives in device memory, so the
+// same graph is launched ten times.  Every kernel is launched with programmatic stream serialisation: its CTAs become
+// resident, set up and request their weights (or cached keys) while the kernel before it runs, and wait for it only
+// before they touch what it wrote.  Measured on B200, a hop along such a chain (last store to first load) costs 1.25 us
+// against 1.75-2.3 us for a device-scope counter of a persistent kernel, and every stage may use all SMs.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#include <algorithm>
+#include <string>
+#include <utility>
+
+#include "../../include/pi05_b200.h"
+#include "pi05_attention.cuh"
+#include "pi05_gemm.cuh"
+#include "pi05_steps.h"
+
+namespace pi05 {
+namespace {
+
+using gemm::hi16;
+using gemm::lo16;
+using gemm::pack2;
+using gemm::rb;
+
+// ------------------------------------------------------------------------------------------- prologue
+struct TableArgs {
+  float t_steps[NS];
+  float* temb;
+  uint32_t* rope;
+  const uint8_t* mask;
+  int* state;
+  int prefix;
+};
+
+// Time embedding (FP64, reference/pi05.py:232-237), RoPE tables of the suffix positions (reference/pi05.py:218-229, they
+// start at the observation's number of valid prefix tokens) and the step counter.  blockIdx.y = observation.
+__global__ void __launch_bounds__(256) tables_kernel(const TableArgs p) {
+  const int b = blockIdx.y, tid = threadIdx.x, gtid = blockIdx.x * 256 + tid, gn = gridDim.x * 256;
+  __shared__ int s_cnt;
+  if (tid == 0) s_cnt = 0;
+  __syncthreads();
+  int n = 0;
+  for (int i = tid; i < p.prefix; i += 256) n += p.mask[(size_t)b * p.prefix + i] ? 1 : 0;
+  for (int sh = 16; sh; sh >>= 1) n += __shfl_xor_sync(0xffffffffu, n, sh);
+  if ((tid & 31) == 0 && n) atomicAdd(&s_cnt, n);
+  __syncthreads();
+  const int nvalid = s_cnt;
+  for (int i = gtid; i < T * (HD / 2); i += gn) {
+    const int t = i / (HD / 2), j = i % (HD / 2);
+    const float e = (float)(2 * j) / (float)HD;
+    const float inv = 1.0f / (float)pow(10000.0, (double)e);
+    const float phase = (float)(nvalid + t) * inv;
+    p.rope[(size_t)b * T * (HD / 2) + i] = pack2((float)cos((double)phase), (float)sin((double)phase));
+  }
+  if (b == 0) {
+    for (int i = gtid; i < NS * W; i += gn) {
+      const int s = i / W, j = i % W, f = j % (W / 2);
+      const double step = 1.0 / (W / 2 - 1);
+      const double frac = f < (W / 4) ? step * f : 1.0 - step * (W / 2 - 1 - f);
+      const double period = 4e-3 * pow(4.0 / 4e-3, frac);
+      const double phase = (double)p.t_steps[s] * (1.0 / period * 2 * 3.141592653589793);
+      p.temb[i] = (float)(j < W / 2 ? sin(phase) : cos(phase));
+    }
+    if (gtid < 2) p.state[gtid] = 0;
+  }
+}
+
+struct MatArgs {
+  const float* in;                           // [10][1024]
+  const float *w[3], *b[3];                  // modulation: attention norms, feed-forward norms, final norm
+  float* out;
+};
+
+// One layer of the time MLP for the ten time steps at once: out[s][row] = silu(W[row][:] . in[s][:] + bias[row]).  A warp
+// per row; the whole row is requested before the kernel before this one has finished.
+__global__ void __launch_bounds__(256) time_mlp_kernel(const MatArgs p) {
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  ptx::grid_dep_launch();
+  float4 w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = ptx::ldg_stream_f4(p.w[0] + (size_t)row * W + j * 128 + lane * 4);
+  const float bias = __ldg(p.b[0] + row);
+  ptx::grid_dep_wait();
+  float mine = 0.f;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    float a = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(p.in + s * W) + j * 32 + lane);
+      a = fmaf(w[j].x, v.x, a); a = fmaf(w[j].y, v.y, a); a = fmaf(w[j].z, v.z, a); a = fmaf(w[j].w, v.w, a);
+    }
+    for (int sh = 16; sh; sh >>= 1) a += __shfl_xor_sync(0xffffffffu, a, sh);
+    if (lane == s) mine = a;
+  }
+  if (lane < NS) {
+    const float y = mine + bias;
+    p.out[(size_t)lane * W + row] = y / (1.0f + expf(-y));
+  }
+}
+
+// The 37 modulation layers for the ten time steps at once: out[s][row] = W[row][:] . in[s][:] + bias[row]; the 474 MB of FP32
+// weights are streamed from HBM exactly once.  A warp takes four rows; lane l covers k = 4 l .. 4 l + 3 of every 128, the
+// ten vectors lie in shared memory, products are accumulated in packed FP32 pairs.
+__global__ void __launch_bounds__(256, 2) modulation_kernel(const MatArgs p) {
+  constexpr int R = 4;
+  __shared__ float4 c[NS][W / 4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  ptx::grid_dep_launch();
+  const int nrows = NNORM * MODW;
+  const float* wrow = nullptr;
+  const float* bias = nullptr;
+  auto locate = [&](int row0) {
+    const int n = row0 / MODW, j = row0 - n * MODW, which = n == NNORM - 1 ? 2 : (n & 1);
+    const size_t r = which == 2 ? (size_t)j : (size_t)(n >> 1) * MODW + j;
+    wrow = p.w[which] + r * W;
+    bias = p.b[which] + r;
+  };
+  int row0 = (blockIdx.x * 8 + warp) * R;
+  float4 w[2][R];
+  if (row0 < nrows) {
+    locate(row0);
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[0][r] = ptx::ldg_stream_f4(wrow + (size_t)r * W + lane * 4);
+  }
+  ptx::grid_dep_wait();
+  for (int i = tid; i < NS * W / 4; i += 256) (&c[0][0])[i] = __ldcg(reinterpret_cast<const float4*>(p.in) + i);
+  __syncthreads();
+  for (; row0 < nrows; row0 += gridDim.x * 8 * R) {
+    float2 acc[R][NS];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int s = 0; s < NS; ++s) acc[r][s] = make_float2(0.f, 0.f);
+    const float* wcur = wrow;
+    const float* bcur = bias;
+    const int next = row0 + gridDim.x * 8 * R;
+    if (next < nrows) locate(next);
+#pragma unroll
+    for (int j = 0; j < W / 128; ++j) {
+      // the loads of the next 128 columns (or of the next rows) are issued before this block's products
+      if (j + 1 < W / 128) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[(j + 1) & 1][r] = ptx::ldg_stream_f4(wcur + (size_t)r * W + (j + 1) * 128 + lane * 4);
+      } else if (next < nrows) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[0][r] = ptx::ldg_stream_f4(wrow + (size_t)r * W + lane * 4);
+      }
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const float4 v = c[s][j * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float4 a = w[j & 1][r];
+          acc[r][s] = ptx::fma2(make_float2(a.x, a.y), make_float2(v.x, v.y), acc[r][s]);
+          acc[r][s] = ptx::fma2(make_float2(a.z, a.w), make_float2(v.z, v.w), acc[r][s]);
+        }
+      }
+    }
+    // 40 sums over the 32 lanes: fold the lanes' halves together while halving the number of values each lane keeps
+    float v[40];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int s = 0; s < NS; ++s) v[r * NS + s] = acc[r][s].x + acc[r][s].y;
+#pragma unroll
+    for (int i = 0; i < 20; ++i) {
+      const float keep = lane & 16 ? v[i + 20] : v[i], send = lane & 16 ? v[i] : v[i + 20];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 10; ++i) {
+      const float keep = lane & 8 ? v[i + 10] : v[i], send = lane & 8 ? v[i] : v[i + 10];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const float keep = lane & 4 ? v[i + 5] : v[i], send = lane & 4 ? v[i] : v[i + 5];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 2);
+      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 1);
+    }
+    if ((lane & 3) == 0) {
+      const int base = (lane & 16 ? 20 : 0) + (lane & 8 ? 10 : 0) + (lane & 4 ? 5 : 0);
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int r = (base + i) / NS, s = (base + i) % NS;
+        p.out[(size_t)s * NNORM * MODW + row0 + r] = v[i] + __ldg(bcur + r);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------- row kernels
+struct NormArgs {
+  const float* part;                         // [splits][tokens][1024] partial sums of the projection before
+  __nv_bfloat16 *h, *out;
+  const float* mod;
+  const int* state;
+  int gate_norm, next_norm;
+};
+
+// h += bf16(bf16(sum of the parts) * bf16(gate)); out = adaRMS(h) with the next norm's scale and shift
+// (reference/pi05.py:240-279).  One token per block, four columns per thread (every load of a warp covers whole lines).
+template <int S>
+__global__ void __launch_bounds__(256) residual_norm_kernel(const NormArgs p) {
+  __shared__ float red[8];
+  const int c0 = threadIdx.x * 4;
+  ptx::grid_dep_launch();
+  // the modulation was finished before this graph was launched, and the step counter only moves at the end of a step
+  const float* mod_s = p.mod + (size_t)__ldcg(p.state) * NNORM * MODW;
+  const float4 g = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)p.gate_norm * MODW + 2 * W + c0));
+  const float4 sc = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)p.next_norm * MODW + c0));
+  const float4 sh = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)p.next_norm * MODW + W + c0));
+  const float gate[4] = {g.x, g.y, g.z, g.w}, scale[4] = {sc.x, sc.y, sc.z, sc.w}, shift[4] = {sh.x, sh.y, sh.z, sh.w};
+  const size_t at = (size_t)blockIdx.x * W + c0, slice = (size_t)gridDim.x * W / 4;
+  ptx::grid_dep_wait();
+  const float4* a4 = reinterpret_cast<const float4*>(p.part + at);
+  float4 a[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) a[s] = __ldcg(a4 + s * slice);
+  const uint2 hv = __ldcg(reinterpret_cast<const uint2*>(p.h + at));
+#pragma unroll
+  for (int s = 1; s < S; ++s) { a[0].x += a[s].x; a[0].y += a[s].y; a[0].z += a[s].z; a[0].w += a[s].w; }
+  const float av[4] = {a[0].x, a[0].y, a[0].z, a[0].w}, hw[4] = {lo16(hv.x), hi16(hv.x), lo16(hv.y), hi16(hv.y)};
+  float v[4], ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    v[e] = rb(hw[e] + rb(rb(av[e]) * rb(gate[e])));
+    ss += v[e] * v[e];
+  }
+  *reinterpret_cast<uint2*>(p.h + at) = make_uint2(pack2(v[0], v[1]), pack2(v[2], v[3]));
+  for (int d = 16; d; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+  const float rs = 1.0f / sqrtf(ss * (1.0f / W) + EPS);
+  float o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) o[e] = __fadd_rn(__fmul_rn(__fmul_rn(v[e], rs), __fadd_rn(1.0f, scale[e])), shift[e]);
+  *reinterpret_cast<uint2*>(p.out + at) = make_uint2(pack2(o[0], o[1]), pack2(o[2], o[3]));
+}
+
+struct TailArgs {
+  const float* part;
+  __nv_bfloat16 *h, *out;
+  const float* mod;
+  int* state;
+  const float *noise, *ain_w, *ain_b, *aout_w, *aout_b;
+  float *x, *actions;
+  const unsigned int* status;
+  float dt;
+  int gate_norm, n_steps, tokens, splits;
+};
+
+constexpr int TAIL_THREADS = 256;
+constexpr int TAIL_SMEM = W * ADIM * 4 + W * 4;
+
+// The end of an Euler step (INIT: the beginning of the first): residual of the last layer, final adaRMS, action_out, Euler
+// update, and - unless it was the last step - action_in and the first layer's norm for the next step (reference/pi05.py:282-309).
+// A block works through tokens blockIdx.x, + gridDim.x, ...; action_in's weights wait in shared memory and action_out's in
+// registers, both requested before the kernel before this one has finished.
+template <bool INIT>
+__global__ void __launch_bounds__(TAIL_THREADS, 1) tail_kernel(const TailArgs p) {
+  extern __shared__ __align__(16) float s_dyn[];
+  float4* s_in = reinterpret_cast<float4*>(s_dyn);          // [1024 rows][8 pieces], piece c of row r at c ^ (r & 7)
+  float* s_row = s_dyn + W * ADIM;                          // [1024]
+  __shared__ float red[8], s_x[ADIM];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = tid * 4;
+  ptx::grid_dep_launch();
+  const int step = INIT ? -1 : __ldcg(p.state);
+  const bool last = !INIT && step + 1 == p.n_steps;
+  float4 wo[4][8];                                          // action_out rows 4 warp .. 4 warp + 3, columns 4 lane + 128 j
+  if (!INIT) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) wo[r][j] = __ldg(reinterpret_cast<const float4*>(p.aout_w + (size_t)(warp * 4 + r) * W) + lane + 32 * j);
+  }
+  if (!last)
+    for (int i = tid; i < W * 8; i += TAIL_THREADS) s_in[(i & ~7) | ((i & 7) ^ ((i >> 3) & 7))] = __ldg(reinterpret_cast<const float4*>(p.ain_w) + i);
+  auto block_sum = [&](float v) {
+    for (int sh = 16; sh; sh >>= 1) v += __shfl_xor_sync(0xffffffffu, v, sh);
+    __syncthreads();
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += red[i];
+    return s;
+  };
+  ptx::grid_dep_wait();
+  for (int t = blockIdx.x; t < p.tokens; t += gridDim.x) {
+    if (!INIT) {
+      const size_t at = (size_t)t * W + c0;
+      const float* mod_s = p.mod + (size_t)step * NNORM * MODW;
+      const float4 g = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)p.gate_norm * MODW + 2 * W + c0));
+      const float4 sc = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)(NNORM - 1) * MODW + c0));
+      const float4 sh = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)(NNORM - 1) * MODW + W + c0));
+      const uint2 hv = __ldcg(reinterpret_cast<const uint2*>(p.h + at));
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+      for (int s = 0; s < p.splits; ++s) {
+        const float4 b = __ldcg(reinterpret_cast<const float4*>(p.part + ((size_t)s * p.tokens) * W + at));
+        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+      }
+      float v[4];
+      v[0] = rb(lo16(hv.x) + rb(rb(a.x) * rb(g.x)));
+      v[1] = rb(hi16(hv.x) + rb(rb(a.y) * rb(g.y)));
+      v[2] = rb(lo16(hv.y) + rb(rb(a.z) * rb(g.z)));
+      v[3] = rb(hi16(hv.y) + rb(rb(a.w) * rb(g.w)));
+      const float rs = 1.0f / sqrtf(block_sum((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3])) * (1.0f / W) + EPS);
+      const float sca[4] = {sc.x, sc.y, sc.z, sc.w}, sha[4] = {sh.x, sh.y, sh.z, sh.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        s_row[c0 + e] = rb(__fadd_rn(__fmul_rn(__fmul_rn(v[e], rs), __fadd_rn(1.0f, sca[e])), sha[e]));
+      __syncthreads();
+      float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 n = reinterpret_cast<const float4*>(s_row)[lane + 32 * j];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          dot[r] = fmaf(wo[r][j].x, n.x, dot[r]); dot[r] = fmaf(wo[r][j].y, n.y, dot[r]);
+          dot[r] = fmaf(wo[r][j].z, n.z, dot[r]); dot[r] = fmaf(wo[r][j].w, n.w, dot[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        for (int sh2 = 16; sh2; sh2 >>= 1) dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], sh2);
+      if (lane < 4) {
+        const int a4 = warp * 4 + lane;
+        const float d = lane == 0 ? dot[0] : lane == 1 ? dot[1] : lane == 2 ? dot[2] : dot[3];
+        const float xn = __fadd_rn(p.x[(size_t)t * ADIM + a4], __fmul_rn(p.dt, d + __ldg(p.aout_b + a4)));
+        p.x[(size_t)t * ADIM + a4] = xn;
+        s_x[a4] = xn;
+        // a chunk in which a bounded wait gave up must not be mistaken for a result
+        if (last) p.actions[(size_t)t * ADIM + a4] = ptx::ld_relaxed(p.status) != 0u ? __int_as_float(0x7fc00000) : xn;
+      }
+    } else if (tid < ADIM) {
+      const float xv = __ldg(p.noise + (size_t)t * ADIM + tid);
+      p.x[(size_t)t * ADIM + tid] = xv;
+      s_x[tid] = xv;
+    }
+    __syncthreads();
+    if (last) continue;
+    // h = bf16(Win x + b) and the next norm, columns tid, tid + 256, ..
+    const float* mod_n = p.mod + (size_t)(step + 1) * NNORM * MODW;
+    float y[4], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int col = tid + TAIL_THREADS * e;
+      float a = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float4 w4 = s_in[col * 8 + (k ^ (col & 7))];
+        a = fmaf(w4.x, s_x[4 * k], a); a = fmaf(w4.y, s_x[4 * k + 1], a);
+        a = fmaf(w4.z, s_x[4 * k + 2], a); a = fmaf(w4.w, s_x[4 * k + 3], a);
+      }
+      y[e] = rb(a + __ldg(p.ain_b + col));
+      ss += y[e] * y[e];
+      p.h[(size_t)t * W + col] = __float2bfloat16_rn(y[e]);
+    }
+    const float rs = 1.0f / sqrtf(block_sum(ss) * (1.0f / W) + EPS);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int col = tid + TAIL_THREADS * e;
+      p.out[(size_t)t * W + col] = __float2bfloat16_rn(
+          __fadd_rn(__fmul_rn(__fmul_rn(y[e], rs), __fadd_rn(1.0f, __ldcg(mod_n + col))), __ldcg(mod_n + W + col)));
+    }
+  }
+  if (!INIT) {
+    // the last block to finish moves the step counter: every block has read it by then
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      if (atomicAdd(p.state + 1, 1) == (int)gridDim.x - 1) {
+        p.state[1] = 0;
+        p.state[0] = step + 1;
+      }
+    }
+  }
+}
+
+// =========================================================================================== host side
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encoder() {
+  static EncodeTiledFn fn = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
+        qres != cudaDriverEntryPointSuccess)
+      ptr = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(ptr);
+  }();
+  return fn;
+}
+
+// {inner = K, rows} BF16 row-major, box {64 k, box_rows}, 128-byte swizzle; rows beyond `rows` read as zeros.
+bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) return false;
+  cuuint64_t dims[2] = {inner, rows};
+  cuuint64_t strides[1] = {inner * 2};
+  cuuint32_t box[2] = {64, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[n].val.programmaticStreamSerializationAllowed = 1;
+  ++n;
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = at; cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// How one projection of `tokens` x n features over k is cut.
+struct GemmPlan {
+  bool pair;
+  int bn, ks, splits, m_tiles, rows, units, grid, stages, a_stride, bufs, off_out, smem;
+};
+
+// One CTA per tile up to 128 tokens; from two tiles of tokens on CTA pairs, which load half of the tile's weight rows each.
+// BN: the smallest one built, so the most CTAs, that does not give more tiles than SMs; K of the projections whose sums meet
+// in the residual kernel is split in powers of two down to eight 64-k blocks per CTA.  Rings: the whole K range of both
+// operands where it fits, else as many stages of both as do.
+GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi) {
+  GemmPlan g;
+  g.m_tiles = (tokens + 127) / 128;
+  g.pair = g.m_tiles >= 2;
+  if (g.pair) g.m_tiles = (g.m_tiles + 1) / 2 * 2;
+  g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
+  static const int qkv1[] = {32, 0}, qkv2[] = {32, 64, 128, 0}, gu1[] = {64, 0}, gu2[] = {128, 256, 0}, part1[] = {32, 64, 0},
+                   part2[] = {64, 128, 0};
+  const int* c = epi == gemm::EPI_QKV ? (g.pair ? qkv2 : qkv1) : epi == gemm::EPI_GEGLU ? (g.pair ? gu2 : gu1) : (g.pair ? part2 : part1);
+  const int kb = k / gemm::BK;
+  for (; *c; ++c) {
+    g.bn = *c;
+    g.splits = 1;
+    const int tiles = g.m_tiles * (n / g.bn);
+    if (epi == gemm::EPI_PART) {
+      while (tiles * g.splits * 2 <= sms && kb / (g.splits * 2) >= 8) g.splits *= 2;
+      if (tiles <= sms && kb / g.splits <= 8) break;
+    } else if (tiles <= sms) {
+      break;
+    }
+  }
+  const int ctas = g.m_tiles * (n / g.bn) * g.splits;
+  g.units = g.pair ? ctas / 2 : ctas;
+  g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
+  g.bufs = g.grid < ctas ? 2 : 1;
+  g.a_stride = (g.rows + 7) / 8 * 1024;
+  const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128;
+  g.ks = g.bn <= 128 ? 2 : 1;
+  // results staged for the copy to memory: in the ring when the CTA has one tile (its operands are consumed by then)
+  const int out_row = epi == gemm::EPI_PART ? (g.bn >= 64 ? g.bn * 4 : 0) : epi == gemm::EPI_GEGLU ? (g.bn >= 128 ? g.bn : 0) : (g.bn >= 64 ? g.bn * 2 : 0);
+  const int out = out_row ? 128 * (out_row + 16) : 0;
+  const int budget = 220 * 1024 - (g.bufs > 1 ? out : 0), stage = g.ks * (g.a_stride + w_bytes);
+  g.stages = std::min({gemm::MAX_STAGES, budget / stage, g.bufs > 1 ? gemm::MAX_STAGES : kb / g.splits / g.ks});
+  g.off_out = g.bufs > 1 ? g.stages * stage : 0;
+  // the MMA reads 128 rows from the last activation block on
+  g.smem = std::max({g.stages * stage, (g.stages - 1) * stage + (g.ks - 1) * g.a_stride + 128 * 128, g.off_out + out}) + 1024;
+  return g;
+}
+
+// How the attention of `batch` observations is cut: tiles of 5 tokens (40 query rows, three key / value stages) for a few
+// observations, where the time of one CTA counts, of 13 (104 rows) for more, where the keys that all CTAs read together do; the
+// keys of a tile over as many CTAs of a cluster as leaves each what its stages hold, as long as the CTAs fit the SMs.
+struct AttnPlan { int tok_tile, tiles, splits; };
+
+AttnPlan plan_attention(int sms, int batch, int prefix) {
+  AttnPlan a;
+  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1, per_cta = batch <= 3 ? 3 : 4;
+  a.tok_tile = batch <= 3 ? 5 : 13;
+  a.tiles = (T + a.tok_tile - 1) / a.tok_tile;
+  a.splits = 1;
+  while (a.splits < 8 && (chunks + a.splits - 1) / a.splits > per_cta && batch * a.tiles * a.splits * 2 <= sms) a.splits *= 2;
+  return a;
+}
+
+typedef void (*GemmKernel)(const gemm::Args);
+
+GemmKernel gemm_kernel_for(int epi, const GemmPlan& g) {
+  using namespace gemm;
+  if (epi == EPI_QKV) {
+    if (!g.pair) return gemm_kernel<EPI_QKV, 32, false, 2>;
+    return g.bn == 32 ? gemm_kernel<EPI_QKV, 32, true, 2> : g.bn == 64 ? gemm_kernel<EPI_QKV, 64, true, 2> : gemm_kernel<EPI_QKV, 128, true, 2>;
+  }
+  if (epi == EPI_GEGLU) {
+    if (!g.pair) return gemm_kernel<EPI_GEGLU, 64, false, 2>;
+    return g.bn == 128 ? gemm_kernel<EPI_GEGLU, 128, true, 2> : gemm_kernel<EPI_GEGLU, 256, true, 1>;
+  }
+  if (!g.pair) return g.bn == 32 ? gemm_kernel<EPI_PART, 32, false, 2> : gemm_kernel<EPI_PART, 64, false, 2>;
+  return g.bn == 64 ? gemm_kernel<EPI_PART, 64, true, 2> : gemm_kernel<EPI_PART, 128, true, 2>;
+}
+
+typedef void (*NormKernel)(const NormArgs);
+NormKernel norm_kernel_for(int splits) {
+  return splits == 1 ? residual_norm_kernel<1> : splits == 2 ? residual_norm_kernel<2> : splits == 4 ? residual_norm_kernel<4> : residual_norm_kernel<8>;
+}
+
+// Shared-memory opt-in of every kernel of the chain, once per device.
+cudaError_t opt_in(int device) {
+  static bool done[64] = {};
+  if (device < 64 && done[device]) return cudaSuccess;
+  using namespace gemm;
+  struct { const void* kernel; int smem; } all[] = {
+      {(const void*)gemm_kernel<EPI_QKV, 32, false, 2>, 1}, {(const void*)gemm_kernel<EPI_QKV, 32, true, 2>, 1},
+      {(const void*)gemm_kernel<EPI_QKV, 64, true, 2>, 1}, {(const void*)gemm_kernel<EPI_QKV, 128, true, 2>, 1},
+      {(const void*)gemm_kernel<EPI_GEGLU, 64, false, 2>, 1}, {(const void*)gemm_kernel<EPI_GEGLU, 128, true, 2>, 1},
+      {(const void*)gemm_kernel<EPI_GEGLU, 256, true, 1>, 1}, {(const void*)gemm_kernel<EPI_PART, 32, false, 2>, 1},
+      {(const void*)gemm_kernel<EPI_PART, 64, false, 2>, 1}, {(const void*)gemm_kernel<EPI_PART, 64, true, 2>, 1},
+      {(const void*)gemm_kernel<EPI_PART, 128, true, 2>, 1}, {(const void*)attn::attention_kernel, 225 * 1024},
+      {(const void*)tail_kernel<false>, TAIL_SMEM}, {(const void*)tail_kernel<true>, TAIL_SMEM},
+      {(const void*)residual_norm_kernel<1>, 0}, {(const void*)residual_norm_kernel<2>, 0},
+      {(const void*)residual_norm_kernel<4>, 0}, {(const void*)residual_norm_kernel<8>, 0},
+      {(const void*)modulation_kernel, 0}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
+  for (const auto& k : all) {
+    cudaError_t e = cudaSuccess;
+    if (k.smem) e = cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem == 1 ? 222 * 1024 : k.smem);
+    // one split of L1 and shared memory for all of them: an SM that has to change it drains first, which would keep a
+    // kernel's CTAs from becoming resident beside the ones of the kernel before
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+  }
+  if (device < 64) done[device] = true;
+  return cudaSuccess;
+}
+
+struct Capture {
+  const StepSetup& s;
+  int n_steps, n_layers, kernels = 0;
+  cudaStream_t stream = nullptr;
+  cudaError_t e = cudaSuccess;
+  std::string what;
+  GemmPlan pq, po, pg, pd;
+
+  Capture(const StepSetup& setup, int steps, int layers) : s(setup), n_steps(steps), n_layers(layers) {
+    const int tokens = T * s.batch;
+    pq = plan_gemm(s.sms, tokens, QKVW, W, gemm::EPI_QKV);
+    po = plan_gemm(s.sms, tokens, W, QD, gemm::EPI_PART);
+    pg = plan_gemm(s.sms, tokens, 2 * FF, W, gemm::EPI_GEGLU);
+    pd = plan_gemm(s.sms, tokens, W, FF, gemm::EPI_PART);
+  }
+
+  template <typename... P, typename... A>
+  void put(void (*kernel)(P...), int grid, int block, size_t smem, int cluster, A&&... args) {
+    if (e != cudaSuccess) return;
+    e = launch(kernel, grid, block, smem, stream, cluster, std::forward<A>(args)...);
+    ++kernels;
+  }
+
+  TailArgs tail_args() const {
+    TailArgs t;
+    memset(&t, 0, sizeof t);
+    t.part = s.part; t.h = s.h; t.out = s.an; t.mod = s.mod; t.state = s.state;
+    t.noise = (const float*)s.in[21];
+    t.ain_w = (const float*)s.in[0]; t.ain_b = (const float*)s.in[1];
+    t.aout_w = (const float*)s.in[6]; t.aout_b = (const float*)s.in[7];
+    t.x = s.x; t.actions = s.actions; t.status = s.status; t.dt = (float)(-1.0 / NS);
+    t.gate_norm = 2 * (n_layers - 1) + 1; t.n_steps = n_steps; t.tokens = T * s.batch; t.splits = pd.splits;
+    return t;
+  }
+
+  void prologue() {
+    TableArgs t;
+    const double dt = -1.0 / NS;
+    for (int i = 0; i < NS; ++i) t.t_steps[i] = (float)(1.0 + i * dt);
+    t.temb = s.temb; t.rope = s.rope; t.mask = (const uint8_t*)s.in[24]; t.state = s.state; t.prefix = s.prefix;
+    tables_kernel<<<dim3(std::max(8, s.sms / s.batch), s.batch), 256, 0, stream>>>(t);
+    e = cudaGetLastError();
+    ++kernels;
+    MatArgs m;
+    memset(&m, 0, sizeof m);
+    m.in = s.temb; m.w[0] = (const float*)s.in[2]; m.b[0] = (const float*)s.in[3]; m.out = s.hid;
+    put(time_mlp_kernel, W / 8, 256, 0, 1, m);
+    m.in = s.hid; m.w[0] = (const float*)s.in[4]; m.b[0] = (const float*)s.in[5]; m.out = s.cond;
+    put(time_mlp_kernel, W / 8, 256, 0, 1, m);
+    m.in = s.cond; m.out = s.mod;
+    m.w[0] = (const float*)s.in[15]; m.b[0] = (const float*)s.in[16];
+    m.w[1] = (const float*)s.in[17]; m.b[1] = (const float*)s.in[18];
+    m.w[2] = (const float*)s.in[19]; m.b[2] = (const float*)s.in[20];
+    put(modulation_kernel, 2 * s.sms, 256, 0, 1, m);
+    put(tail_kernel<true>, std::min(T * s.batch, s.sms), TAIL_THREADS, TAIL_SMEM, 1, tail_args());
+  }
+
+  void project(int epi, const GemmPlan& g, const CUtensorMap& a, const CUtensorMap* b0, const CUtensorMap* b1, const CUtensorMap* b2,
+               int k, int layer) {
+    gemm::Args p;
+    memset(&p, 0, sizeof p);
+    p.a = a; p.b0 = *b0;
+    if (b1) p.b1 = *b1;
+    if (b2) p.b2 = *b2;
+    p.tokens = T * s.batch; p.rows = g.rows; p.m_groups = g.pair ? g.m_tiles / 2 : g.m_tiles; p.splits = g.splits;
+    p.kblocks = k / gemm::BK / g.splits; p.units = g.units; p.layer = layer; p.stages = g.stages; p.a_stride = g.a_stride;
+    p.bufs = g.bufs; p.off_out = g.off_out; p.status = s.status; p.limit = s.wait_limit;
+    p.q = s.q; p.k = s.k; p.v = s.v; p.rope = s.rope; p.act = s.act; p.part = s.part;
+    put(gemm_kernel_for(epi, g), g.grid, gemm::THREADS_G, g.smem, g.pair ? 2 : 1, p);
+  }
+
+  void step() {
+    const int tokens = T * s.batch;
+    CUtensorMap a_qkv, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;
+    attn::Args ap;
+    memset(&ap, 0, sizeof ap);
+    const AttnPlan pa = plan_attention(s.sms, s.batch, s.prefix);
+    ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits; ap.stages = attn::stages_for(pa.tok_tile * NQH);
+    ap.merge = s.part;
+    const uint64_t L = NL, M = tokens;
+    if (!(map_2d(&a_qkv, s.an, W, M, pq.rows) && map_2d(&a_o, s.attn, QD, M, po.rows) && map_2d(&a_gu, s.an, W, M, pg.rows) &&
+          map_2d(&a_dn, s.act, FF, M, pd.rows) && map_2d(&wq, s.in[8], W, L * QD, pq.bn / 2) &&
+          map_2d(&wk, s.in[9], W, L * HD, pq.bn / 2) && map_2d(&wv, s.in[10], W, L * HD, pq.bn / 2) &&
+          map_2d(&wo, s.in[11], QD, L * W, po.bn / 2) && map_2d(&wg, s.in[12], W, L * FF, pg.bn / 2) &&
+          map_2d(&wu, s.in[13], W, L * FF, pg.bn / 2) && map_2d(&wd, s.in[14], FF, L * W, pd.bn / 2) &&
+          map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH))) {
+      e = cudaErrorUnknown;
+      what = "cuTensorMapEncodeTiled failed";
+      return;
+    }
+    ap.pk = s.maps->pk; ap.pk_tail = s.maps->pk_tail; ap.pv = s.maps->pv; ap.pv_tail = s.maps->pv_tail;
+    ap.sk = s.maps->sk; ap.sv = s.maps->sv;
+    ap.page_table = s.page_table; ap.pages_per_obs = s.pages_per_obs; ap.page_tokens = s.page_tokens;
+    ap.valid = (const uint8_t*)s.in[24]; ap.out = s.attn; ap.prefix = s.prefix; ap.suffix = T; ap.obs_tokens = T;
+    ap.early = 1; ap.status = s.status; ap.limit = s.wait_limit;
+    NormArgs n;
+    n.part = s.part; n.h = s.h; n.out = s.an; n.mod = s.mod; n.state = s.state;
+    for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
+      project(gemm::EPI_QKV, pq, a_qkv, &wq, &wk, &wv, W, l);
+      ap.layer = l;
+      put(attn::attention_kernel, s.batch * ap.tiles * ap.splits, attn::THREADS, attn::smem_for(ap.tok_tile * NQH), ap.splits, ap);
+      project(gemm::EPI_PART, po, a_o, &wo, nullptr, nullptr, QD, l);
+      n.gate_norm = 2 * l; n.next_norm = 2 * l + 1;
+      put(norm_kernel_for(po.splits), tokens, 256, 0, 1, n);
+      project(gemm::EPI_GEGLU, pg, a_gu, &wg, &wu, nullptr, W, l);
+      project(gemm::EPI_PART, pd, a_dn, &wd, nullptr, nullptr, FF, l);
+      if (l + 1 < n_layers) {
+        n.gate_norm = 2 * l + 1; n.next_norm = 2 * l + 2;
+        put(norm_kernel_for(pd.splits), tokens, 256, 0, 1, n);
+      }
+    }
+    put(tail_kernel<false>, std::min(tokens, s.sms), TAIL_THREADS, TAIL_SMEM, 1, tail_args());
+  }
+
+  // Captures what `body` launches into an executable graph.
+  template <typename F>
+  cudaGraphExec_t graph(F body) {
+    if (e != cudaSuccess) return nullptr;
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t x = nullptr;
+    kernels = 0;
+    e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return nullptr;
+    body();
+    const cudaError_t end = cudaStreamEndCapture(stream, &g);
+    if (e == cudaSuccess) e = end;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&x, g, 0);
+    if (e == cudaSuccess) e = cudaGraphUpload(x, stream);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess && x) { cudaGraphExecDestroy(x); x = nullptr; }
+    return x;
+  }
+};
+
+}  // namespace
+
+size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
+  size_t most = 0;
+  for (int b = 1; b <= max_batch; ++b) {
+    for (int k : {QD, FF}) most = std::max(most, (size_t)plan_gemm(sms, T * b, W, k, gemm::EPI_PART).splits * T * b * W);
+    const AttnPlan a = plan_attention(sms, b, max_prefix);          // splits grow with the prefix
+    if (a.splits > 1) most = std::max(most, (size_t)b * a.tiles * a.splits * attn::MERGE_COLS * a.tok_tile * NQH);
+  }
+  return most;
+}
+
+int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, std::string* error) {
+  steps_free(g);
+  Capture c(s, n_steps, n_layers);
+  c.e = opt_in(s.device);
+  if (c.e == cudaSuccess) c.e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+  g->prologue = c.graph([&] { c.prologue(); });
+  g->kernels_prologue = c.kernels;
+  g->step = c.graph([&] { c.step(); });
+  g->kernels_step = c.kernels;
+  if (c.stream) {
+    const cudaError_t done = cudaStreamSynchronize(c.stream);
+    if (c.e == cudaSuccess) c.e = done;
+    cudaStreamDestroy(c.stream);
+  }
+  if (c.e != cudaSuccess) {
+    *error = "capture of the chunk's kernels: " + (c.what.empty() ? std::string(cudaGetErrorString(c.e)) : c.what);
+    cudaGetLastError();
+    steps_free(g);
+    return PI05_ERR_CUDA;
+  }
+  g->n_steps = n_steps;
+  g->n_layers = n_layers;
+  return PI05_OK;
+}
+
+cudaError_t steps_launch(const StepGraphs& g, cudaStream_t stream) {
+  cudaError_t e = cudaGraphLaunch(g.prologue, stream);
+  for (int s = 0; s < g.n_steps && e == cudaSuccess; ++s) e = cudaGraphLaunch(g.step, stream);
+  return e;
+}
+
+void steps_free(StepGraphs* g) {
+  if (g->prologue) cudaGraphExecDestroy(g->prologue);
+  if (g->step) cudaGraphExecDestroy(g->step);
+  *g = StepGraphs();
+}
+
+}  // namespace pi05

@@ -1,0 +1,42 @@
+// The action chunk as a chain of kernels replayed from CUDA graphs (pi05_steps.cu): what the engine hands over at bind.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <string>
+
+#include "pi05_common.cuh"
+
+namespace pi05 {
+
+struct StepSetup {
+  int device, sms, batch, prefix;
+  const void* const* in;                     // the 25 inputs
+  float* actions;
+  unsigned int* status;
+  int* state;                                // {Euler step, finished blocks of the step tail}
+  float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions (steps_part_floats)
+  uint32_t* rope;
+  __nv_bfloat16 *h, *an, *q, *k, *v, *attn, *act;
+  const TMaps* maps;                         // prefix and suffix key / value maps
+  const int* page_table;
+  int pages_per_obs, page_tokens;
+  long long wait_limit;
+};
+
+struct StepGraphs {
+  cudaGraphExec_t prologue = nullptr, step = nullptr;
+  int n_steps = 0, n_layers = 0;             // what the graphs were captured for
+  int kernels_prologue = 0, kernels_step = 0;
+};
+
+// FP32 words of partial sums that up to `max_batch` observations with up to `max_prefix` prefix tokens need.
+size_t steps_part_floats(int sms, int max_batch, int max_prefix);
+// Captures and instantiates the graphs for (n_steps, n_layers); frees what `g` held.
+int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, std::string* error);
+// Enqueues one chunk.
+cudaError_t steps_launch(const StepGraphs& g, cudaStream_t stream);
+void steps_free(StepGraphs* g);
+
+}  // namespace pi05

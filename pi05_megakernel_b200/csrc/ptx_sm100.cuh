@@ -1,6 +1,6 @@
 // Thin inline-PTX wrappers for sm_100a: mbarrier, TMA (cp.async.bulk.tensor), tcgen05 MMA / TMEM,
 // proxy fences, device-scope release/acquire, warp MMA (mma.sync) and ldmatrix for the attention stage.
-// No wrapper here uses cluster multicast in any form: every CTA is its own cluster (cta_group::1).
+// No load here uses cluster multicast in any form.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -106,6 +106,13 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// Untiled bulk copy shared memory -> global (same alignment), as part of the thread's current bulk group; the wait returns
+// when the groups committed so far have read their shared memory.
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1,
                                                  uint64_t policy) {
   asm volatile(
@@ -136,6 +143,18 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two FP32 fused multiply-adds in one instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long ra, rb, rc, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rd) : "l"(ra), "l"(rb), "l"(rc));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
 }
 
 // ----------------------------------------------------------------------------- programmatic dependent launch
@@ -176,6 +195,13 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
 __device__ __forceinline__ uint32_t umma_idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// The same for an operand that is MN-major (its rows run along K): 64 M / N elements per 128-byte swizzled row, eight K
+// rows per 1024-byte group, the next 64 M / N elements `segment` bytes further; the instruction descriptor of a B operand
+// in this layout carries UMMA_B_MN_MAJOR.
+__device__ __forceinline__ uint64_t umma_smem_desc_mn(uint32_t saddr, uint32_t segment) {
+  return (uint64_t)((saddr >> 4) & 0x3fffu) | ((uint64_t)(segment >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+constexpr uint32_t UMMA_B_MN_MAJOR = 1u << 16;
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -207,6 +233,55 @@ __device__ __forceinline__ void umma_bf16_stage8(uint32_t d_tmem, uint64_t adesc
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n}"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(commit_bar),
         "n"((unsigned long long)A_ATOM), "n"((unsigned long long)B_ATOM) : "memory");
+}
+// Four K = 16 MMAs, `astep` / `bstep` descriptor units (16 bytes) apart.
+__device__ __forceinline__ void umma_bf16_k64(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate, uint64_t astep, uint64_t bstep) {
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b64 a1, a2, a3, b1, b2, b3;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "add.u64 a1, %1, %5;\n add.u64 a2, a1, %5;\n add.u64 a3, a2, %5;\n"
+      "add.u64 b1, %2, %6;\n add.u64 b2, b1, %6;\n add.u64 b3, b2, %6;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "l"(astep), "l"(bstep) : "memory");
+}
+// One pipeline stage of KS 64-k blocks in one piece: 4 KS MMAs of K = 16 (32-byte steps inside the 128-byte swizzle rows of
+// a block, blocks `ablock` / `bblock` descriptor units apart) and the commit that frees the stage, on one CTA or on a pair
+// (whose commit arrives in both CTAs).
+template <bool PAIR, int KS>
+__device__ __forceinline__ void umma_bf16_stage(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                                uint32_t commit_bar, uint64_t ablock, uint64_t bblock) {
+#define PI05_UMMA4(G, A0, B0, P0)                                                       \
+  "add.u64 a1, " A0 ", 2;\n add.u64 a2, " A0 ", 4;\n add.u64 a3, " A0 ", 6;\n"          \
+  "add.u64 b1, " B0 ", 2;\n add.u64 b2, " B0 ", 4;\n add.u64 b3, " B0 ", 6;\n"          \
+  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], " A0 ", " B0 ", %3, " P0 ";\n"           \
+  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], a1, b1, %3, 1;\n"                       \
+  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], a2, b2, %3, 1;\n"                       \
+  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], a3, b3, %3, 1;\n"
+#define PI05_UMMA_HEAD "{\n.reg .pred p;\n.reg .b64 a1, a2, a3, b1, b2, b3, a4, b4;\nsetp.ne.b32 p, %4, 0;\n"
+#define PI05_UMMA_NEXT "add.u64 a4, %1, %6;\n add.u64 b4, %2, %7;\n"
+#define PI05_UMMA_COMMIT1 "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n}"
+#define PI05_UMMA_COMMIT2 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], %8;\n}"
+#define PI05_UMMA_ARGS ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(commit_bar), "l"(ablock), "l"(bblock)
+  if constexpr (PAIR && KS == 1)
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "%1", "%2", "p") PI05_UMMA_COMMIT2 PI05_UMMA_ARGS, "h"((unsigned short)3) : "memory");
+  else if constexpr (PAIR)
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "%1", "%2", "p") PI05_UMMA_NEXT PI05_UMMA4("2", "a4", "b4", "1") PI05_UMMA_COMMIT2
+                 PI05_UMMA_ARGS, "h"((unsigned short)3) : "memory");
+  else if constexpr (KS == 1)
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "%1", "%2", "p") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS : "memory");
+  else
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "%1", "%2", "p") PI05_UMMA_NEXT PI05_UMMA4("1", "a4", "b4", "1") PI05_UMMA_COMMIT1
+                 PI05_UMMA_ARGS : "memory");
+#undef PI05_UMMA4
+#undef PI05_UMMA_HEAD
+#undef PI05_UMMA_NEXT
+#undef PI05_UMMA_COMMIT1
+#undef PI05_UMMA_COMMIT2
+#undef PI05_UMMA_ARGS
 }
 // One lane of a converged warp (always the same one), for instructions that a single thread must issue while the
 // loop around them stays warp-uniform.
@@ -254,6 +329,11 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_32x2(uint32_t taddr, uint32_t (&r)[2]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
@@ -303,6 +383,33 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap,
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+
+// Bounded wait on an mbarrier of this CTA, by a whole converged warp: a wait that runs out records (kind, block) in the
+// status words once, and every later wait returns.  The vote keeps the result warp-uniform and the warp converged, which
+// the .aligned tcgen05 instructions behind a wait rely on.  The waiting itself is one function per kernel: the code of a
+// kernel that runs for a few microseconds is fetched once, and what it does not repeat it pays for.
+static __device__ __noinline__ bool wait_bar_slow(unsigned int* status, long long limit, uint32_t bar, uint32_t parity, int kind) {
+  const long long t0 = clock64();
+  for (unsigned i = 0;; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 63u) == 63u) {
+      bool stop = ld_relaxed(status) != 0u;
+      if (!stop && clock64() - t0 > limit) {
+        if (atomicCAS(status, 0u, (unsigned)kind) == 0u) status[1] = blockIdx.x << 16;
+        stop = true;
+      }
+      if (__any_sync(0xffffffffu, stop)) break;
+    }
+  }
+  // copies and MMAs that this CTA has in flight finish within microseconds: let them land before it tears itself down
+  const long long t1 = clock64();
+  while (clock64() - t1 < 200000) __nanosleep(1000);
+  return false;
+}
+__device__ __forceinline__ bool wait_bar(unsigned int* status, long long limit, uint32_t bar, uint32_t parity, int kind) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return wait_bar_slow(status, limit, bar, parity, kind);
 }
 
 // ----------------------------------------------------------------------------- warp MMA + ldmatrix (attention)
