@@ -8,10 +8,11 @@ import subprocess
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = [os.path.join(HERE, "csrc", "pi05_engine.cu"), os.path.join(HERE, "csrc", "pi05_prefill.cu"),
-           os.path.join(HERE, "csrc", "pi05_steps.cu")]
+           os.path.join(HERE, "csrc", "pi05_steps.cu"), os.path.join(HERE, "csrc", "pi05_ops.cu")]
 HEADERS = [os.path.join(HERE, "csrc", "ptx_sm100.cuh"), os.path.join(HERE, "csrc", "pi05_common.cuh"),
            os.path.join(HERE, "csrc", "pi05_chunk_kernel.cuh"), os.path.join(HERE, "csrc", "pi05_attention.cuh"),
            os.path.join(HERE, "csrc", "pi05_gemm.cuh"), os.path.join(HERE, "csrc", "pi05_steps.h"),
+           os.path.join(HERE, "csrc", "pi05_ops.h"),
            os.path.join(os.path.dirname(HERE), "include", "pi05_b200.h")]
 LIB = os.path.join(HERE, "libpi05_b200.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -1,5 +1,6 @@
-// Attention on the tcgen05 tensor cores, used by the action chunk (50 suffix tokens over a prefix cache): several query
-// tokens x 8 heads share the one KV head, so a tile of up to 128 query rows is one MMA operand.
+// Attention on the tcgen05 tensor cores, used by the action chunk (50 suffix tokens over a prefix cache) and by the prefix
+// prefill (every token over every token): several query tokens x 8 heads share the one KV head, so a tile of up to 128 query
+// rows is one MMA operand.
 //
 //   * One CTA = one tile of `tok_tile` query tokens against a contiguous share of the keys, in chunks of 64.  A cluster of
 //     `splits` CTAs shares the keys of a tile and merges through distributed shared memory (below).
@@ -34,7 +35,6 @@ namespace attn {
 constexpr int HD = 256, NQH = 8, KCH = 64, THREADS = 320;
 constexpr int K_BYTES = KCH * HD * 2;                         // four 64-dim segments of [64 keys x 128 B]
 constexpr int MAX_STG = 3;                                    // key / value stages
-constexpr int OUT_ROW = HD * 2 + 16;                          // staging of results: BF16 rows
 constexpr int MERGE_COLS = HD + 2;                            // FP32 columns of a part: the accumulator, maximum, sum
 constexpr int SMEM_LIMIT = 226 * 1024;                        // dynamic shared memory without the alignment slack
 constexpr int TM_O = 0, TM_S = 256, TM_COLS = 512;            // TMEM columns: O [128 x 256], two S buffers [128 x 64]
@@ -47,11 +47,10 @@ __host__ __device__ constexpr int stages_for(int rows) {
 }
 __host__ __device__ constexpr int smem_for(int rows) { return 6 * rows * 128 + 2 * stages_for(rows) * K_BYTES + 1024; }
 static_assert(stages_for(128) == 2 && smem_for(128) + 2048 <= 227 * 1024 && stages_for(40) == 3, "attention shared memory");
-static_assert(2 * 2 * K_BYTES >= 128 * OUT_ROW, "the staging fits the key / value stages");
-
 struct Args {
   CUtensorMap q;                           // [tokens x 8 rows, 256 dims], box {64, 8 x tok_tile}
   CUtensorMap pk, pk_tail, pv, pv_tail;    // prefix keys / values {64 dims, page tokens, 4, layers, pages}, box {64, 64, 4, 1, 1}
+  CUtensorMap o;                           // the output as [observations][rows per observation][256], box {64, rows, 1}
   CUtensorMap sk, sv;                      // suffix keys / values {64, tokens, 4, observations}, box {64, 64, 4, 1}
   const int* page_table;                   // [observation][pages_per_obs], or null: page = observation
   const uint8_t* valid;                    // [observation][prefix]
@@ -71,7 +70,8 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 __device__ __forceinline__ float lo16(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi16(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
-static __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_constant__ Args p) {
+template <int = 0>   // a template, so that only the file that launches it holds its code
+__global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_constant__ Args p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // barriers: q, k_full[3], k_empty[3], v_full[3], v_empty[3], s_full[2], s_empty[2], p_full[2], p_empty[2], o_full
@@ -317,33 +317,42 @@ static __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __gr
   if (warp >= 2) l += s_sum[half ^ 1][row];               // both halves of the row's sum
   __syncthreads();
 
-  // ---- O / l -> BF16: row = token_local * 8 + head, so the tile's rows are one contiguous block of [tokens, 2048].  Through
-  // shared memory (the key / value stages are consumed), so that a warp's stores cover whole lines
+  // ---- O / l -> BF16: row = token_local * 8 + head, so the tile's rows are one contiguous block of [tokens, 2048].  They leave
+  // through shared memory by tiled copies (which clip what lies beyond the observation's tokens)
   const int left = p.obs_tokens - tile * p.tok_tile, out_rows = (left < p.tok_tile ? left : p.tok_tile) * NQH;
   uint4* base = reinterpret_cast<uint4*>(p.out + (size_t)(ob * p.obs_tokens + tile * p.tok_tile) * NQH * HD);
   const int c_half = half * (HD / 2);
   if (p.splits == 1) {
+    const uint32_t stage = q_base;                        // four swizzled 64-dim blocks, over Q (every MMA has completed)
     if (busy) {
       const float il = 1.0f / l;
-      const uint32_t dst = k_base + row * OUT_ROW + c_half * 2;
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD / 2; c0 += 32) {
-        uint32_t r[32];
-        ptx::tmem_ld_32x32(trow + TM_O + c_half + c0, r);
+      for (int c0 = 0; c0 < HD / 2; c0 += 16) {
+        uint32_t r[16];
+        ptx::tmem_ld_32x16(trow + TM_O + c_half + c0, r);
         ptx::tmem_wait_ld();
+        const int ch = (c_half + c0) >> 3;                // 16-byte piece of the row
+        const uint32_t line = stage + (ch >> 3) * blk + row * 128;
+        if (row < rows)
 #pragma unroll
-        for (int j = 0; j < 32; j += 8)
-          ptx::st_shared_v4(dst + (c0 + j) * 2, pack2(__uint_as_float(r[j]) * il, __uint_as_float(r[j + 1]) * il),
-                            pack2(__uint_as_float(r[j + 2]) * il, __uint_as_float(r[j + 3]) * il),
-                            pack2(__uint_as_float(r[j + 4]) * il, __uint_as_float(r[j + 5]) * il),
-                            pack2(__uint_as_float(r[j + 6]) * il, __uint_as_float(r[j + 7]) * il));
+          for (int j = 0; j < 2; ++j)
+            ptx::st_shared_v4(line + ((((uint32_t)ch + j) & 7) ^ (row & 7)) * 16,
+                              pack2(__uint_as_float(r[8 * j]) * il, __uint_as_float(r[8 * j + 1]) * il),
+                              pack2(__uint_as_float(r[8 * j + 2]) * il, __uint_as_float(r[8 * j + 3]) * il),
+                              pack2(__uint_as_float(r[8 * j + 4]) * il, __uint_as_float(r[8 * j + 5]) * il),
+                              pack2(__uint_as_float(r[8 * j + 6]) * il, __uint_as_float(r[8 * j + 7]) * il));
+        __syncwarp();
       }
       ptx::tc_fence_before();
+      ptx::fence_proxy_async_shared();
     }
     __syncthreads();
+    if (tid == 64 && ok) {
 #pragma unroll 1
-    for (int i = tid; i < out_rows * (HD / 8); i += THREADS)
-      base[i] = *reinterpret_cast<const uint4*>(smem + off_k + (i >> 5) * OUT_ROW + (i & 31) * 16);
+      for (int kb = 0; kb < 4; ++kb) ptx::tma_store_3d(&p.o, stage + kb * blk, kb * 64, tile * rows, ob);
+      ptx::bulk_commit();
+      ptx::bulk_wait_read();
+    }
   } else {
     const size_t pstride = (size_t)MERGE_COLS * rows;
     float* parts = p.merge + (size_t)unit * p.splits * pstride;

@@ -1,8 +1,9 @@
-// The projections of the action chunk as tcgen05 GEMMs: out[tokens, N] = A[tokens, K] . W[N, K]^T with a fused epilogue.
+// The projections of the action chunk and of the prefix prefill as tcgen05 GEMMs: out[tokens, N] = A[tokens, K] . W[N, K]^T with
+// a fused epilogue.
 //
 // One CTA (or CTA pair, cta_group::2) works on output tiles of `rows` <= 128 tokens per CTA x BN features x a K range.  The
-// kernels of a chunk form one dependent chain of ~2-5 us each, so what matters is the time from the end of one to the first
-// MMA of the next:
+// kernels of a chunk (and of a short prefill) form one dependent chain of ~2-5 us each, so what matters is the time from the
+// end of one to the first MMA of the next:
 //   * weights do not depend on the chain, so a CTA fills its whole weight ring before it waits for the kernel before it
 //     (programmatic dependent launch);
 //   * a stage holds both operands of KS 64-k blocks behind one barrier, and its MMAs and the commit that frees it are one asm
@@ -12,8 +13,12 @@
 //     rows, the ones beyond the tile are whatever shared memory holds and end in accumulator lanes nobody reads;
 //   * K is split over several CTAs where whole-K tiles would leave SMs without work; every split stores its FP32 partial
 //     sums to a slice of its own and the residual kernel adds the slices (atomics made the end of the kernel ~1 us later);
-//   * results go through shared memory, so that a warp's stores cover whole lines (a thread per row stores 16 bytes to 32
-//     different lines, which the LSU takes one at a time: 2 us at 128 features per thread);
+//   * results of all but the smallest tiles leave through shared memory by tiled copies (a thread per row stores 16 bytes to
+//     32 different lines, which the LSU takes one at a time: 2 us at 128 features per thread; a bulk copy per row: 1.5 us);
+//   * SK ("stream-K"): tiles x 64-k blocks, taken as one sequence, are cut into one contiguous, equal range per CTA, so that a
+//     long K with few tiles keeps every SM busy for the same time.  A range that begins inside a tile (a contributor's) leaves
+//     its partial sums in the slot of its CTA, one that begins with a tile (the owner's) in the slot of the tile; the residual
+//     kernel adds them.  Nobody waits for anybody;
 //   * with more tiles than CTAs the launch is persistent with two accumulators, so that a tile's epilogue runs under the
 //     next tile's MMAs.
 #pragma once
@@ -37,13 +42,16 @@ enum { EPI_QKV = 0, EPI_GEGLU = 1, EPI_PART = 2 };
 struct Args {
   CUtensorMap a;                   // activations [tokens, K], box {64, rows}
   CUtensorMap b0, b1, b2;          // weights, box {64, BN / 2}.  QKV: wq, wk, wv; GEGLU: gate, up; PART: b0
+  CUtensorMap o0, o1, o2;          // staged results, box {128 or 64 bytes, rows}.  QKV: q, k, v; GEGLU: act; PART: part (3-D)
   int tokens, rows, m_groups, splits, kblocks, units, layer, stages, a_stride, bufs, off_out;   // kblocks: 64-k blocks per unit
+  int width;                       // GEGLU: MLP width; PART: features of the output (rows of a layer's weights)
+  int unit0;                       // first unit of the launch (QKV of a last layer: keys and values only)
   unsigned int* status;
   long long limit;
   __nv_bfloat16 *q, *k, *v;        // EPI_QKV: [tokens, 2048], [tokens, 256], [tokens, 256]
   const uint32_t* rope;            // [tokens][128]: cos BF16 | sin BF16 << 16
-  __nv_bfloat16* act;              // EPI_GEGLU: [tokens, 4096]
-  float* part;                     // EPI_PART: [splits][tokens, 1024]
+  __nv_bfloat16* act;              // EPI_GEGLU: [tokens, width]
+  float* part;                     // EPI_PART: [splits][tokens, width]; SK: [slots][128][BN]
 };
 
 __device__ __forceinline__ float rb(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
@@ -60,30 +68,43 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return __fdividef(x, 1.0f + e);
 }
 
-// Row bytes of a tile's results in the staging buffer (0: small tiles store directly), and its row stride.
+// Staging of a tile's results: boxes of 128 rows x BOX bytes (swizzled as the tiled copy expects), COUNT of them; 0: the tile
+// is small and its rows are stored directly.  PART: 32 FP32 columns a box; GEGLU and QKV: 64 BF16 (QKV of 64
+// features: 32, each half of the tile a box).
 template <int EPI, int BN>
-__host__ __device__ constexpr int out_bytes() {
-  return EPI == EPI_PART ? (BN >= 64 ? BN * 4 : 0) : EPI == EPI_GEGLU ? (BN >= 128 ? BN : 0) : (BN >= 64 ? BN * 2 : 0);
-}
+struct Staging {
+  static constexpr int COUNT = EPI == EPI_PART ? (BN >= 64 ? BN / 32 : 0) : EPI == EPI_GEGLU ? BN / 128 : (BN == 256 ? 4 : BN >= 64 ? 2 : 0);
+  static constexpr int BOX = EPI == EPI_QKV && BN == 64 ? 64 : 128;
+  static constexpr int BYTES = COUNT * 128 * BOX;
+  // 16-byte piece `c` (counted over the whole row of BN results) of row `row`
+  static __device__ __forceinline__ uint32_t at(int row, int c) {
+    constexpr int PER = BOX / 16;
+    const uint32_t sw = BOX == 128 ? (row & 7) : ((row >> 1) & 3);
+    return (uint32_t)(c / PER) * (128 * BOX) + row * BOX + (((c % PER) ^ sw) << 4);
+  }
+};
 
 // This thread's token row of the accumulator (TMEM lanes of its warp, BN columns from t0); `half` is the half of the columns
-// (of each half of the tile for QKV and GEGLU) that its warp handles.  `out` is the row's place in the staging buffer.
+// (of each half of the tile for QKV and GEGLU) that its warp handles.  `out` is the staging buffer; PART fills `boxes` boxes of
+// it from column 32 box0 on.
 // Eight columns at a time in loops that stay loops: an instruction that runs once costs several cycles to fetch.
 template <int EPI, int BN>
-__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int token, bool live, int half, uint32_t out) {
-  constexpr bool STAGED = out_bytes<EPI, BN>() > 0;
+__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int row, int token, bool live, int half, uint32_t out,
+                                             int box0, int boxes) {
+  using St = Staging<EPI, BN>;
+  constexpr bool STAGED = St::COUNT > 0;
   const int tok = live ? token : 0;
   if constexpr (EPI == EPI_PART) {
-    uint32_t src = t0 + half * (BN / 2), dst = out + half * (BN / 2) * 4;
-    uint4* g = reinterpret_cast<uint4*>(p.part + ((size_t)split * p.tokens + tok) * W + nt * BN + half * (BN / 2));
+    const int cols = STAGED ? boxes * 16 : BN / 2, c0 = (STAGED ? box0 * 32 : 0) + half * cols;
+    uint4* g = reinterpret_cast<uint4*>(p.part + ((size_t)split * p.tokens + tok) * p.width + nt * BN + c0);
 #pragma unroll 1
-    for (int c = 0; c < BN / 2; c += 16) {
+    for (int c = 0; c < cols; c += 16) {
       uint32_t r[16];
-      ptx::tmem_ld_32x16(src + c, r);
+      ptx::tmem_ld_32x16(t0 + c0 + c, r);
       ptx::tmem_wait_ld();
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (STAGED) ptx::st_shared_v4(dst + (c + 4 * j) * 4, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        if (STAGED) ptx::st_shared_v4(out + St::at(row, (half * cols + c) / 4 + j), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         else if (live) g[c / 4 + j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
       }
     }
@@ -92,7 +113,7 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
     constexpr int PER = HD / BN;                            // QKV: tiles per head
     const int head = nt / PER, dim0 = (nt % PER) * (BN / 2);
     const uint4* cs4 = reinterpret_cast<const uint4*>(p.rope + (size_t)tok * 128 + dim0);
-    __nv_bfloat16* g = EPI == EPI_GEGLU ? p.act + (size_t)tok * FF + nt * (BN / 2)
+    __nv_bfloat16* g = EPI == EPI_GEGLU ? p.act + (size_t)tok * p.width + nt * (BN / 2)
                        : (head < NQH ? p.q + (size_t)tok * QD + head * HD : (head == NQH ? p.k : p.v) + (size_t)tok * HD) + dim0;
 #pragma unroll 1
     for (int c = half * (BN / 4); c < (half + 1) * (BN / 4); c += 8) {
@@ -122,50 +143,61 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
           o2[j] = head <= NQH ? *reinterpret_cast<const uint32_t*>(&b) : y;
         }
       }
-      if (STAGED) ptx::st_shared_v4(out + c * 2, o1[0], o1[1], o1[2], o1[3]);
+      if (STAGED) ptx::st_shared_v4(out + St::at(row, c / 8), o1[0], o1[1], o1[2], o1[3]);
       else if (live) *reinterpret_cast<uint4*>(g + c) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
       if (EPI == EPI_QKV) {
-        if (STAGED) ptx::st_shared_v4(out + (BN / 2 + c) * 2, o2[0], o2[1], o2[2], o2[3]);
+        if (STAGED) ptx::st_shared_v4(out + St::at(row, (BN / 2 + c) / 8), o2[0], o2[1], o2[2], o2[3]);
         else if (live) *reinterpret_cast<uint4*>(g + 128 + c) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
       }
     }
   }
 }
 
-// One staged row to its place in memory, as bulk copies out of shared memory.
-template <int EPI, int BN>
-__device__ __forceinline__ void copy_row(const Args& p, uint32_t src, int nt, int split, int token) {
-  if (EPI == EPI_PART) {
-    ptx::bulk_store(p.part + ((size_t)split * p.tokens + token) * W + nt * BN, src, BN * 4);
-  } else if (EPI == EPI_GEGLU) {
-    ptx::bulk_store(p.act + (size_t)token * FF + nt * (BN / 2), src, BN);
+// The staged tile (PART: boxes box0 .. box0 + boxes - 1 of it) to its place in memory: one thread, a tiled copy per box (rows
+// beyond the tokens are clipped).
+template <int EPI, int BN, bool SK>
+__device__ __forceinline__ void copy_out(const Args& p, uint32_t stage, int nt, int split, int token0, int box0, int boxes) {
+  using St = Staging<EPI, BN>;
+  if constexpr (EPI == EPI_PART) {
+#pragma unroll 1
+    for (int b = 0; b < boxes; ++b)
+      ptx::tma_store_3d(&p.o0, stage + b * 128 * St::BOX, (SK ? 0 : nt * BN) + (box0 + b) * 32, SK ? 0 : token0, split);
+  } else if constexpr (EPI == EPI_GEGLU) {
+#pragma unroll
+    for (int b = 0; b < St::COUNT; ++b) ptx::tma_store_2d(&p.o0, stage + b * 128 * St::BOX, nt * (BN / 2) + b * 64, token0);
   } else {
-    constexpr int PER = HD / BN;
-    const int head = nt / PER;
-    __nv_bfloat16* dst = (head < NQH ? p.q + (size_t)token * QD + head * HD : (head == NQH ? p.k : p.v) + (size_t)token * HD) +
-                         (nt % PER) * (BN / 2);
-    ptx::bulk_store(dst, src, BN);
-    ptx::bulk_store(dst + 128, src + BN, BN);
+    constexpr int PER = HD / BN, HB = St::COUNT / 2;
+    const int head = nt / PER, c0 = (head < NQH ? head * HD : 0) + (nt % PER) * (BN / 2);
+    const CUtensorMap* m = head < NQH ? &p.o0 : head == NQH ? &p.o1 : &p.o2;
+#pragma unroll
+    for (int b = 0; b < St::COUNT; ++b)
+      ptx::tma_store_2d(m, stage + b * 128 * St::BOX, c0 + (b / (HB ? HB : 1)) * 128 + (b % (HB ? HB : 1)) * 64, token0);
   }
 }
 
+// The contiguous ranges of (tile, 64-k block) units of a stream-K launch, in which a tile's blocks are neighbours.
+struct Segments {
+  __host__ __device__ static long long begin(int tiles, int kblocks, int cta, int ctas) { return (long long)tiles * kblocks * cta / ctas; }
+};
+
 // KS: 64-k blocks per stage.
-template <int EPI, int BN, bool PAIR, int KS>
+template <int EPI, int BN, bool PAIR, int KS, bool SK>
 __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__ Args p) {
+  static_assert(!SK || (EPI == EPI_PART && BN == 256 && !PAIR && KS == 1), "stream-K: partial sums of 128 x 256 tiles");
   constexpr int WR = PAIR ? BN / 2 : BN;                  // weight rows this CTA loads per 64-k block
-  constexpr int W_BYTES = WR * 128, HALF = (BN / 2) * 128, OUT = out_bytes<EPI, BN>();
+  constexpr int W_BYTES = WR * 128, HALF = (BN / 2) * 128, OUT = Staging<EPI, BN>::BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t bars[2 * MAX_STAGES + 4];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
-  const int unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, ustep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const int ustep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x, unit0 = p.unit0 + (PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x);
   // a stage: KS activation blocks, then KS weight blocks
   const uint32_t ring = ptx::smem_u32(smem), a_stride = p.a_stride, w_off = KS * a_stride, st_stride = w_off + KS * W_BYTES;
   const uint32_t full = ptx::smem_u32(bars), empty = full + 8 * MAX_STAGES, t_full = empty + 8 * MAX_STAGES, t_empty = t_full + 16;
   const bool leader = ptx::elect_one();
-  const int nst = p.kblocks / KS, stages = p.stages;      // stages per unit, stages in the ring
+  const int stages = p.stages;
   const int tcols = p.bufs * (BN < 32 ? 32 : BN);
 
   if (tid == 0) {
@@ -178,12 +210,31 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
   __syncwarp();
   if (PAIR) ptx::cluster_sync();           // the even CTA's barriers exist before the odd CTA's copies count on them
 
-  // tile of a unit: groups of tokens fastest (neighbours share weights), then K split, then features
-  auto locate = [&](int unit, int& mt, int& split, int& nt) {
-    const int rest = unit / p.m_groups, mg = unit - rest * p.m_groups;
-    nt = rest / p.splits;
-    split = rest - nt * p.splits;
-    mt = PAIR ? 2 * mg + (int)rank : mg;
+  // The CTA's work, unit after unit: tile (mt, nt), slice of the partial sums, first stage and number of stages of its K range.
+  // Regular: groups of tokens fastest (neighbours share weights), then K split, then features.
+  struct Work { int mt, nt, split, st0, nst; };
+  auto first = [&]() -> long long { return SK ? Segments::begin(p.units, p.kblocks, blockIdx.x, gridDim.x) : unit0; };
+  const long long last = SK ? Segments::begin(p.units, p.kblocks, blockIdx.x + 1, gridDim.x) : p.unit0 + p.units;
+  auto take = [&](long long& at, Work& w) -> bool {
+    if (at >= last) return false;
+    if (SK) {
+      const int tile = (int)(at / p.kblocks);
+      w.st0 = (int)(at - (long long)tile * p.kblocks);
+      w.nst = (int)(last - at < p.kblocks - w.st0 ? last - at : p.kblocks - w.st0);
+      w.nt = tile / p.m_groups;
+      w.mt = tile - w.nt * p.m_groups;
+      w.split = w.st0 ? (int)blockIdx.x : (int)gridDim.x + tile;      // slot of the partial sums
+      at += w.nst;
+    } else {
+      const int unit = (int)at, rest = unit / p.m_groups, mg = unit - rest * p.m_groups;
+      w.nt = rest / p.splits;
+      w.split = rest - w.nt * p.splits;
+      w.mt = PAIR ? 2 * mg + (int)rank : mg;
+      w.nst = p.kblocks / KS;
+      w.st0 = w.split * w.nst;
+      at += ustep;
+    }
+    return true;
   };
   const CUtensorMap *m0 = &p.b0, *m1 = &p.b0;
   int r0 = 0, r1 = 0;
@@ -196,9 +247,9 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       r1 = r0 + 128;
     } else if (EPI == EPI_GEGLU) {
       m1 = &p.b1;
-      r0 = r1 = p.layer * FF + nt * (BN / 2);
+      r0 = r1 = p.layer * p.width + nt * (BN / 2);
     } else {
-      r0 = p.layer * W + nt * BN;
+      r0 = p.layer * p.width + nt * BN;
       r1 = r0 + BN / 2;
     }
   };
@@ -218,12 +269,13 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
   };
   int ahead = 0;                           // weight stages of the first unit requested before the dependency is waited for
   if (warp == 0) {
-    int mt, split, nt;
-    locate(unit0, mt, split, nt);
-    weight_rows(nt);
-    ahead = stages < nst ? stages : nst;
+    long long at = first();
+    Work w;
+    take(at, w);
+    weight_rows(w.nt);
+    ahead = stages < w.nst ? stages : w.nst;
     if (leader) {
-      for (int i = 0; i < ahead; ++i) load_w((split * nst + i) * KS * BK, i);
+      for (int i = 0; i < ahead; ++i) load_w((w.st0 + i) * KS * BK, i);
       ptx::prefetch_tensormap(&p.a);
     }
   } else if (warp == 1) {
@@ -242,21 +294,21 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     const uint32_t a_bytes = (uint32_t)p.rows * 128 * KS;
     uint32_t slot = 0, par = 1;
     bool ok = true;
-    for (int unit = unit0; ok && unit < p.units; unit += ustep) {
-      int mt, split, nt;
-      locate(unit, mt, split, nt);
-      weight_rows(nt);
-      for (int i = 0; i < nst; ++i) {
-        const int kc = (split * nst + i) * KS * BK;
-        const bool have_w = unit == unit0 && i < ahead;
+    long long at = first();
+    Work w;
+    for (int it = 0; ok && take(at, w); ++it) {
+      weight_rows(w.nt);
+      for (int i = 0; i < w.nst; ++i) {
+        const int kc = (w.st0 + i) * KS * BK;
+        const bool have_w = it == 0 && i < ahead;
         if (!have_w && !(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1))) break;
         if (leader) {
           const uint32_t dst = ring + slot * st_stride, bar = PAIR ? ptx::map_to_rank(full + 8 * slot, 0) : full + 8 * slot;
           if (!PAIR || rank == 0) ptx::mbar_expect_tx(full + 8 * slot, (PAIR ? 2 : 1) * a_bytes);
 #pragma unroll
           for (int h = 0; h < KS; ++h) {
-            if (PAIR) ptx::tma_load_2d_pair(dst + h * a_stride, &p.a, bar, kc + h * BK, mt * p.rows);
-            else ptx::tma_load_2d(dst + h * a_stride, &p.a, bar, kc + h * BK, mt * p.rows);
+            if (PAIR) ptx::tma_load_2d_pair(dst + h * a_stride, &p.a, bar, kc + h * BK, w.mt * p.rows);
+            else ptx::tma_load_2d(dst + h * a_stride, &p.a, bar, kc + h * BK, w.mt * p.rows);
           }
           if (!have_w) load_w(kc, slot);
         }
@@ -270,13 +322,15 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       const uint64_t adesc0 = ptx::umma_smem_desc(ring), bdesc0 = ptx::umma_smem_desc(ring + w_off);
       uint32_t slot = 0, par = 0, it = 0;
       bool ok = true;
-      for (int unit = unit0; ok && unit < p.units; unit += ustep, ++it) {
+      long long at = first();
+      Work w;
+      for (; ok && take(at, w); ++it) {
         const uint32_t buf = it & 1;
         if (!(ok = ptx::wait_bar(p.status, p.limit, t_empty + 8 * buf, ((it >> 1) & 1) ^ 1, 6))) break;
         ptx::tc_fence_after();
         const uint32_t d = tmem + buf * BN;
         uint32_t acc = 0;
-        for (int i = 0; i < nst; ++i) {
+        for (int i = 0; i < w.nst; ++i) {
           if (!(ok = ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, 3))) break;
           const uint64_t off = (uint64_t)((slot * st_stride) >> 4);
           if (leader)
@@ -295,35 +349,42 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     // gives up does not end the loop: the other epilogue warps count on this one at their barriers
     const int quad = warp & 3, row = quad * 32 + lane, half = warp >= 6 ? 1 : 0;
     const uint32_t release = PAIR ? ptx::map_to_rank(t_empty, 0) : 0u;
-    const uint32_t stage = ptx::smem_u32(smem) + p.off_out, out = stage + row * (OUT + 16);
+    const uint32_t stage = ptx::smem_u32(smem) + p.off_out;
+    constexpr int BOXES = SK ? 2 : Staging<EPI, BN>::COUNT;          // boxes staged at a time
     uint32_t it = 0;
     bool ok = true;
-    for (int unit = unit0; unit < p.units; unit += ustep, ++it) {
+    long long at = first();
+    Work w;
+    for (; take(at, w); ++it) {
       const uint32_t buf = it & 1;
-      int mt, split, nt;
-      locate(unit, mt, split, nt);
-      const int token = mt * p.rows + row;
+      const int token = w.mt * p.rows + row;
       ok &= ptx::wait_bar(p.status, p.limit, t_full + 8 * buf, (it >> 1) & 1, 5);
       ptx::tc_fence_after();
-      if (OUT > 0 && it > 0) {             // the tile before has left the staging rows of this quadrant
-        ptx::bulk_wait_read();
-        ptx::named_bar_sync(1 + quad, 64);
-      }
-      if (quad * 32 < p.rows)
-        epilogue_row<EPI, BN>(p, tmem + buf * BN + ((uint32_t)(quad * 32) << 16), nt, split, token, ok && row < p.rows && token < p.tokens, half, out);
-      ptx::tc_fence_before();
-      if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);
-      else ptx::mbar_arrive(t_empty + 8 * buf);
-      if constexpr (OUT > 0) {
-        // both warps of the quadrant have written their halves of its 32 rows; each sends 16 of them off
-        ptx::fence_proxy_async_shared();
-        ptx::named_bar_sync(1 + quad, 64);
-        const int r16 = quad * 32 + half * 16 + lane, tok16 = mt * p.rows + r16;
-        if (ok && lane < 16 && r16 < p.rows && tok16 < p.tokens) copy_row<EPI, BN>(p, stage + r16 * (OUT + 16), nt, split, tok16);
-        ptx::bulk_commit();
+#pragma unroll 1
+      for (int box0 = 0; box0 < (SK ? Staging<EPI, BN>::COUNT : 1); box0 += SK ? BOXES : 1) {
+        if (OUT > 0 && (it > 0 || box0 > 0)) {                       // what was staged before has left the buffer
+          if (tid == 64) ptx::bulk_wait_read();
+          ptx::named_bar_sync(1, EPI_THREADS);
+        }
+        if (quad * 32 < p.rows)
+          epilogue_row<EPI, BN>(p, tmem + buf * BN + ((uint32_t)(quad * 32) << 16), w.nt, w.split, row, token,
+                                ok && row < p.rows && token < p.tokens, half, stage, box0, BOXES);
+        if (!SK || box0 + BOXES >= Staging<EPI, BN>::COUNT) {        // the accumulator has been read
+          ptx::tc_fence_before();
+          if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);
+          else ptx::mbar_arrive(t_empty + 8 * buf);
+        }
+        if constexpr (OUT > 0) {
+          ptx::fence_proxy_async_shared();
+          ptx::named_bar_sync(1, EPI_THREADS);
+          if (tid == 64) {
+            if (ok) copy_out<EPI, BN, SK>(p, stage, w.nt, w.split, w.mt * p.rows, box0, BOXES);
+            ptx::bulk_commit();
+          }
+        }
       }
     }
-    if (OUT > 0) ptx::bulk_wait_read();
+    if (OUT > 0 && tid == 64) ptx::bulk_wait_read();
   }
   __syncthreads();
   if (PAIR) ptx::cluster_sync();           // neither CTA leaves (or frees tensor memory) while the other may still use it

@@ -1,0 +1,201 @@
+// Host side of the tcgen05 projections and attention: tensor maps, how a projection is cut, launches.
+#include "pi05_ops.h"
+
+#include <algorithm>
+
+namespace pi05 {
+namespace {
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encoder() {
+  static EncodeTiledFn fn = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
+        qres != cudaDriverEntryPointSuccess)
+      ptr = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(ptr);
+  }();
+  return fn;
+}
+
+// Bytes of the staging buffer of a tile's results (gemm::Staging).
+int staging_bytes(int epi, int bn) {
+  using namespace gemm;
+  if (epi == EPI_PART) return bn == 32 ? 0 : bn == 64 ? Staging<EPI_PART, 64>::BYTES : bn == 128 ? Staging<EPI_PART, 128>::BYTES : Staging<EPI_PART, 256>::BYTES;
+  if (epi == EPI_GEGLU) return bn == 64 ? 0 : bn == 128 ? Staging<EPI_GEGLU, 128>::BYTES : Staging<EPI_GEGLU, 256>::BYTES;
+  return bn == 32 ? 0 : bn == 64 ? Staging<EPI_QKV, 64>::BYTES : bn == 128 ? Staging<EPI_QKV, 128>::BYTES : Staging<EPI_QKV, 256>::BYTES;
+}
+
+typedef void (*GemmKernel)(const gemm::Args);
+struct Cut { int epi, bn, ks; bool pair, sk; GemmKernel kernel; };
+
+// Every cut that is built.
+const Cut kCuts[] = {
+    {gemm::EPI_QKV, 32, 2, false, false, gemm::gemm_kernel<gemm::EPI_QKV, 32, false, 2, false>},
+    {gemm::EPI_QKV, 128, 2, false, false, gemm::gemm_kernel<gemm::EPI_QKV, 128, false, 2, false>},
+    {gemm::EPI_QKV, 32, 2, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 32, true, 2, false>},
+    {gemm::EPI_QKV, 64, 2, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 64, true, 2, false>},
+    {gemm::EPI_QKV, 128, 2, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 128, true, 2, false>},
+    {gemm::EPI_QKV, 256, 1, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 256, true, 1, false>},
+    {gemm::EPI_GEGLU, 64, 2, false, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 64, false, 2, false>},
+    {gemm::EPI_GEGLU, 128, 2, false, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 128, false, 2, false>},
+    {gemm::EPI_GEGLU, 256, 1, false, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 256, false, 1, false>},
+    {gemm::EPI_GEGLU, 128, 2, true, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 128, true, 2, false>},
+    {gemm::EPI_GEGLU, 256, 1, true, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 256, true, 1, false>},
+    {gemm::EPI_PART, 32, 2, false, false, gemm::gemm_kernel<gemm::EPI_PART, 32, false, 2, false>},
+    {gemm::EPI_PART, 64, 2, false, false, gemm::gemm_kernel<gemm::EPI_PART, 64, false, 2, false>},
+    {gemm::EPI_PART, 64, 2, true, false, gemm::gemm_kernel<gemm::EPI_PART, 64, true, 2, false>},
+    {gemm::EPI_PART, 128, 2, true, false, gemm::gemm_kernel<gemm::EPI_PART, 128, true, 2, false>},
+    {gemm::EPI_PART, 256, 1, true, false, gemm::gemm_kernel<gemm::EPI_PART, 256, true, 1, false>},
+    {gemm::EPI_PART, 256, 1, false, true, gemm::gemm_kernel<gemm::EPI_PART, 256, false, 1, true>},
+};
+
+// Ring, staging and shared memory of a cut whose tile, grid and accumulators are decided.
+void lay_out(GemmPlan* g, int epi, int stages_wanted) {
+  const int w_bytes = (g->pair ? g->bn / 2 : g->bn) * 128, stage = g->ks * (g->a_stride + w_bytes);
+  // results are staged in the ring when the CTA has one tile (its operands are consumed by then), else behind it
+  const bool behind = g->bufs > 1;
+  const int out = g->sk ? 2 * 16384 : staging_bytes(epi, g->bn), budget = 220 * 1024 - (behind ? out : 0);
+  g->stages = std::min({gemm::MAX_STAGES, budget / stage, stages_wanted});
+  g->off_out = behind ? g->stages * stage : 0;
+  // the MMA reads 128 rows from the last activation block on
+  g->smem = std::max({g->stages * stage, (g->stages - 1) * stage + (g->ks - 1) * g->a_stride + 128 * 128, g->off_out + out}) + 1024;
+}
+
+}  // namespace
+
+bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) return false;
+  cuuint64_t dims[2] = {inner, rows};
+  cuuint64_t strides[1] = {inner * 2};
+  cuuint32_t box[2] = {64, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool map_out(CUtensorMap* m, const void* base, bool f32, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_bytes, uint32_t box_rows) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) return false;
+  const uint32_t es = f32 ? 4 : 2;
+  cuuint64_t dims[3] = {d0, d1, d2}, strides[2] = {d0 * es, d0 * d1 * es};
+  cuuint32_t box[3] = {box_bytes / es, box_rows, 1}, estr[3] = {1, 1, 1};
+  return enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d2 ? 3 : 2, const_cast<void*>(base), dims, strides,
+             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) return false;
+  cuuint64_t dims[5] = {64, tokens, 4, layers, 1};
+  cuuint64_t strides[4] = {256 * 2, 64 * 2, tokens * 256 * 2, layers * tokens * 256 * 2};
+  cuuint32_t box[5] = {64, 64, 4, 1, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The cheapest of the cuts that are built, by a model of the launch's time in SM cycles: rounds x 64-k blocks x the slower of the
+// MMAs (measured per M128 / M256 K16 instruction: 47 cycles up to N = 32, 50 / 65 / 129 at 64 / 128 / 256) and the operands' way
+// into shared memory (~67 B per cycle and SM), not less than the weights' way from HBM (3.3 KB per cycle), plus what every
+// launch pays, an epilogue that grows with the tile, and the way of partial sums through L2 (~2 KB per cycle).  Pairs of CTAs
+// (256 tokens) load half of the tile's weight rows each.  K of the projections whose sums meet in the residual kernel is split
+// in powers of two, down to four 64-k blocks.
+GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
+  GemmPlan best = {};
+  double best_cost = 1e30;
+  for (const Cut& c : kCuts)
+    for (int splits = 1; c.epi == epi && !c.sk && splits <= (epi == gemm::EPI_PART ? 8 : 1); splits *= 2) {
+      GemmPlan g = {};
+      g.pair = c.pair; g.bn = c.bn; g.ks = c.ks; g.splits = splits;
+      g.kblocks = k / gemm::BK / splits;
+      g.m_tiles = (tokens + 127) / 128;
+      if ((g.pair && g.m_tiles < 2) || (pairs >= 0 && (int)g.pair != pairs)) continue;
+      if (g.pair) g.m_tiles = (g.m_tiles + 1) / 2 * 2;
+      if (g.kblocks < 4) continue;
+      g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
+      g.a_stride = (g.rows + 7) / 8 * 1024;
+      const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128, ctas = g.m_tiles * (n / g.bn) * splits, rounds = (ctas + sms - 1) / sms;
+      const double mma = 4 * (g.bn <= 32 ? 47 : g.bn == 64 ? 50 : g.bn == 128 ? 65 : 129), ingest = (g.rows * 128 + w_bytes) / 67.0;
+      const double cost = std::max(rounds * g.kblocks * std::max(mma, ingest), (double)n * k * 2 / 3300) + 2000 +
+                          g.bn * (epi == gemm::EPI_GEGLU ? 12 : 8) + (splits > 1 ? std::max(150.0 * splits, splits * (double)tokens * n * 4 / 2000) : 0);
+      if (cost >= best_cost) continue;
+      g.units = g.pair ? ctas / 2 : ctas;
+      g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
+      g.bufs = g.grid < ctas ? 2 : 1;
+      lay_out(&g, epi, g.bufs > 1 ? gemm::MAX_STAGES : g.kblocks / g.ks);
+      best = g;
+      best_cost = cost;
+    }
+  return best;
+}
+
+GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k) {
+  GemmPlan g = {};
+  g.sk = true; g.bn = 256; g.ks = 1; g.splits = 1; g.bufs = 2;
+  g.kblocks = k / gemm::BK;
+  g.m_tiles = (tokens + 127) / 128;
+  g.rows = g.m_tiles > 1 ? 128 : tokens;
+  g.a_stride = (g.rows + 7) / 8 * 1024;
+  g.units = g.m_tiles * (n / g.bn);
+  const long long work = (long long)g.units * g.kblocks;
+  g.grid = work < sms ? (int)work : sms;
+  lay_out(&g, gemm::EPI_PART, gemm::MAX_STAGES);
+  return g;
+}
+
+cudaError_t launch_gemm(const GemmPlan& g, int epi, gemm::Args& p, cudaStream_t stream) {
+  const Cut* cut = nullptr;
+  for (const Cut& c : kCuts)
+    if (c.epi == epi && c.bn == g.bn && c.pair == g.pair && c.sk == g.sk) cut = &c;
+  if (!cut) return cudaErrorInvalidValue;
+  p.rows = g.rows; p.m_groups = g.pair ? g.m_tiles / 2 : g.m_tiles; p.splits = g.splits; p.kblocks = g.kblocks;
+  p.stages = g.stages; p.a_stride = g.a_stride; p.bufs = g.bufs; p.off_out = g.off_out;
+  p.units = g.units - p.unit0;
+  const uint64_t M = p.tokens;
+  bool ok = true;
+  if (g.sk) ok = map_out(&p.o0, p.part, true, g.bn, 128, g.grid + g.units, 128, g.rows);
+  else if (staging_bytes(epi, g.bn) && epi == gemm::EPI_PART) ok = map_out(&p.o0, p.part, true, p.width, M, g.splits, 128, g.rows);
+  else if (staging_bytes(epi, g.bn) && epi == gemm::EPI_GEGLU) ok = map_out(&p.o0, p.act, false, p.width, M, 0, 128, g.rows);
+  else if (staging_bytes(epi, g.bn)) {
+    const int box = g.bn == 64 ? 64 : 128;
+    ok = map_out(&p.o0, p.q, false, QD, M, 0, box, g.rows) && map_out(&p.o1, p.k, false, HD, M, 0, box, g.rows) &&
+         map_out(&p.o2, p.v, false, HD, M, 0, box, g.rows);
+  }
+  if (!ok) return cudaErrorInvalidValue;
+  const int ctas = g.pair ? 2 * p.units : p.units, grid = g.sk || g.grid < ctas ? g.grid : ctas;
+  return launch_chained(cut->kernel, grid, gemm::THREADS_G, g.smem, stream, g.pair ? 2 : 1, p);
+}
+
+cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream) {
+  const int rows = p.tok_tile * NQH;
+  p.stages = attn::stages_for(rows);
+  return launch_chained(attn::attention_kernel<0>, observations * p.tiles * p.splits, attn::THREADS, attn::smem_for(rows), stream, p.splits, p);
+}
+
+cudaError_t chain_opt_in(const void* kernel, int smem) {
+  cudaError_t e = cudaSuccess;
+  if (smem) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  return e;
+}
+
+cudaError_t ops_opt_in(int device) {
+  static bool done[64] = {};
+  if (device < 64 && done[device]) return cudaSuccess;
+  cudaError_t e = chain_opt_in((const void*)attn::attention_kernel<0>, 225 * 1024);
+  for (const Cut& c : kCuts)
+    if (e == cudaSuccess) e = chain_opt_in((const void*)c.kernel, 222 * 1024);
+  if (e == cudaSuccess && device < 64) done[device] = true;
+  return e;
+}
+
+}  // namespace pi05

@@ -1,0 +1,62 @@
+// Host side of the tcgen05 projections and attention (pi05_ops.cu): tensor maps, how a projection is cut, launches.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <string.h>
+
+#include <utility>
+
+#include "pi05_attention.cuh"
+#include "pi05_gemm.cuh"
+
+namespace pi05 {
+
+// Launch with programmatic stream serialisation (the kernel may become resident and set up while the one before it in the
+// stream runs) and, with `cluster` > 1, as clusters of that many CTAs.
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[n].val.programmaticStreamSerializationAllowed = 1;
+  ++n;
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = at; cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// {inner = K, rows} BF16 row-major, box {64 k, box_rows}, 128-byte swizzle; rows beyond `rows` read as zeros.
+bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows);
+// A dense tensor of two (d2 = 0) or three dimensions, innermost first, of BF16 or FP32 elements, box {box_bytes, box_rows, 1} with
+// the swizzle of that many bytes: the destination of a tiled store.
+bool map_out(CUtensorMap* m, const void* base, bool f32, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_bytes, uint32_t box_rows);
+// Keys or values as the attention's tiled copies read them: {64 dims, tokens, 4 segments, layers, 1} of a dense [layers][tokens][256].
+bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers);
+
+// How one projection of `tokens` x n features over k is cut.
+struct GemmPlan {
+  bool pair, sk;
+  int bn, ks, splits, m_tiles, rows, units, grid, stages, a_stride, bufs, off_out, smem, kblocks;
+};
+// pairs: 1 / 0 leaves only cuts on CTA pairs / on single CTAs, -1 all.
+GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs = -1);
+// The stream-K cut of a projection with partial sums: 128 x 256 tiles, one equal range of 64-k blocks per CTA.
+GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k);
+// Fills in what the plan decides and the destination maps, and launches.  `width` and the pointers have to be set.
+cudaError_t launch_gemm(const GemmPlan& g, int epi, gemm::Args& p, cudaStream_t stream);
+cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream);
+// Shared-memory opt-in of the kernels behind the two calls above, once per device.
+cudaError_t ops_opt_in(int device);
+// One split of L1 and shared memory for all kernels of a chain: an SM that has to change it drains first, which would keep a
+// kernel's CTAs from becoming resident beside the ones of the kernel before.
+cudaError_t chain_opt_in(const void* kernel, int smem);
+
+}  // namespace pi05

@@ -16,11 +16,9 @@
 
 #include <algorithm>
 #include <string>
-#include <utility>
 
 #include "../../include/pi05_b200.h"
-#include "pi05_attention.cuh"
-#include "pi05_gemm.cuh"
+#include "pi05_ops.h"
 #include "pi05_steps.h"
 
 namespace pi05 {
@@ -395,103 +393,6 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) tail_kernel(const TailArgs p)
 }
 
 // =========================================================================================== host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encoder() {
-  static EncodeTiledFn fn = [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      ptr = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(ptr);
-  }();
-  return fn;
-}
-
-// {inner = K, rows} BF16 row-major, box {64 k, box_rows}, 128-byte swizzle; rows beyond `rows` read as zeros.
-bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
-  EncodeTiledFn enc = encoder();
-  if (!enc) return false;
-  cuuint64_t dims[2] = {inner, rows};
-  cuuint64_t strides[1] = {inner * 2};
-  cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <typename... Params, typename... Args>
-cudaError_t launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute at[2];
-  int n = 0;
-  at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[n].val.programmaticStreamSerializationAllowed = 1;
-  ++n;
-  if (cluster > 1) {
-    at[n].id = cudaLaunchAttributeClusterDimension;
-    at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
-    ++n;
-  }
-  cfg.attrs = at; cfg.numAttrs = n;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
-// How one projection of `tokens` x n features over k is cut.
-struct GemmPlan {
-  bool pair;
-  int bn, ks, splits, m_tiles, rows, units, grid, stages, a_stride, bufs, off_out, smem;
-};
-
-// One CTA per tile up to 128 tokens; from two tiles of tokens on CTA pairs, which load half of the tile's weight rows each.
-// BN: the smallest one built, so the most CTAs, that does not give more tiles than SMs; K of the projections whose sums meet
-// in the residual kernel is split in powers of two down to eight 64-k blocks per CTA.  Rings: the whole K range of both
-// operands where it fits, else as many stages of both as do.
-GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi) {
-  GemmPlan g;
-  g.m_tiles = (tokens + 127) / 128;
-  g.pair = g.m_tiles >= 2;
-  if (g.pair) g.m_tiles = (g.m_tiles + 1) / 2 * 2;
-  g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
-  static const int qkv1[] = {32, 0}, qkv2[] = {32, 64, 128, 0}, gu1[] = {64, 0}, gu2[] = {128, 256, 0}, part1[] = {32, 64, 0},
-                   part2[] = {64, 128, 0};
-  const int* c = epi == gemm::EPI_QKV ? (g.pair ? qkv2 : qkv1) : epi == gemm::EPI_GEGLU ? (g.pair ? gu2 : gu1) : (g.pair ? part2 : part1);
-  const int kb = k / gemm::BK;
-  for (; *c; ++c) {
-    g.bn = *c;
-    g.splits = 1;
-    const int tiles = g.m_tiles * (n / g.bn);
-    if (epi == gemm::EPI_PART) {
-      while (tiles * g.splits * 2 <= sms && kb / (g.splits * 2) >= 8) g.splits *= 2;
-      if (tiles <= sms && kb / g.splits <= 8) break;
-    } else if (tiles <= sms) {
-      break;
-    }
-  }
-  const int ctas = g.m_tiles * (n / g.bn) * g.splits;
-  g.units = g.pair ? ctas / 2 : ctas;
-  g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
-  g.bufs = g.grid < ctas ? 2 : 1;
-  g.a_stride = (g.rows + 7) / 8 * 1024;
-  const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128;
-  g.ks = g.bn <= 128 ? 2 : 1;
-  // results staged for the copy to memory: in the ring when the CTA has one tile (its operands are consumed by then)
-  const int out_row = epi == gemm::EPI_PART ? (g.bn >= 64 ? g.bn * 4 : 0) : epi == gemm::EPI_GEGLU ? (g.bn >= 128 ? g.bn : 0) : (g.bn >= 64 ? g.bn * 2 : 0);
-  const int out = out_row ? 128 * (out_row + 16) : 0;
-  const int budget = 220 * 1024 - (g.bufs > 1 ? out : 0), stage = g.ks * (g.a_stride + w_bytes);
-  g.stages = std::min({gemm::MAX_STAGES, budget / stage, g.bufs > 1 ? gemm::MAX_STAGES : kb / g.splits / g.ks});
-  g.off_out = g.bufs > 1 ? g.stages * stage : 0;
-  // the MMA reads 128 rows from the last activation block on
-  g.smem = std::max({g.stages * stage, (g.stages - 1) * stage + (g.ks - 1) * g.a_stride + 128 * 128, g.off_out + out}) + 1024;
-  return g;
-}
-
 // How the attention of `batch` observations is cut: tiles of 5 tokens (40 query rows, three key / value stages) for a few
 // observations, where the time of one CTA counts, of 13 (104 rows) for more, where the keys that all CTAs read together do; the
 // keys of a tile over as many CTAs of a cluster as leaves each what its stages hold, as long as the CTAs fit the SMs.
@@ -499,7 +400,8 @@ struct AttnPlan { int tok_tile, tiles, splits; };
 
 AttnPlan plan_attention(int sms, int batch, int prefix) {
   AttnPlan a;
-  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1, per_cta = batch <= 3 ? 3 : 4;
+  // (a merge costs about as much as eight chunks of a CTA of 104 rows, or as two of one that finds all its chunks resident)
+  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1, per_cta = batch <= 3 ? 4 : 8;
   a.tok_tile = batch <= 3 ? 5 : 13;
   a.tiles = (T + a.tok_tile - 1) / a.tok_tile;
   a.splits = 1;
@@ -507,53 +409,25 @@ AttnPlan plan_attention(int sms, int batch, int prefix) {
   return a;
 }
 
-typedef void (*GemmKernel)(const gemm::Args);
-
-GemmKernel gemm_kernel_for(int epi, const GemmPlan& g) {
-  using namespace gemm;
-  if (epi == EPI_QKV) {
-    if (!g.pair) return gemm_kernel<EPI_QKV, 32, false, 2>;
-    return g.bn == 32 ? gemm_kernel<EPI_QKV, 32, true, 2> : g.bn == 64 ? gemm_kernel<EPI_QKV, 64, true, 2> : gemm_kernel<EPI_QKV, 128, true, 2>;
-  }
-  if (epi == EPI_GEGLU) {
-    if (!g.pair) return gemm_kernel<EPI_GEGLU, 64, false, 2>;
-    return g.bn == 128 ? gemm_kernel<EPI_GEGLU, 128, true, 2> : gemm_kernel<EPI_GEGLU, 256, true, 1>;
-  }
-  if (!g.pair) return g.bn == 32 ? gemm_kernel<EPI_PART, 32, false, 2> : gemm_kernel<EPI_PART, 64, false, 2>;
-  return g.bn == 64 ? gemm_kernel<EPI_PART, 64, true, 2> : gemm_kernel<EPI_PART, 128, true, 2>;
-}
-
 typedef void (*NormKernel)(const NormArgs);
 NormKernel norm_kernel_for(int splits) {
   return splits == 1 ? residual_norm_kernel<1> : splits == 2 ? residual_norm_kernel<2> : splits == 4 ? residual_norm_kernel<4> : residual_norm_kernel<8>;
 }
 
-// Shared-memory opt-in of every kernel of the chain, once per device.
+// Launch settings of the chain's own kernels, once per device.
 cudaError_t opt_in(int device) {
   static bool done[64] = {};
   if (device < 64 && done[device]) return cudaSuccess;
-  using namespace gemm;
   struct { const void* kernel; int smem; } all[] = {
-      {(const void*)gemm_kernel<EPI_QKV, 32, false, 2>, 1}, {(const void*)gemm_kernel<EPI_QKV, 32, true, 2>, 1},
-      {(const void*)gemm_kernel<EPI_QKV, 64, true, 2>, 1}, {(const void*)gemm_kernel<EPI_QKV, 128, true, 2>, 1},
-      {(const void*)gemm_kernel<EPI_GEGLU, 64, false, 2>, 1}, {(const void*)gemm_kernel<EPI_GEGLU, 128, true, 2>, 1},
-      {(const void*)gemm_kernel<EPI_GEGLU, 256, true, 1>, 1}, {(const void*)gemm_kernel<EPI_PART, 32, false, 2>, 1},
-      {(const void*)gemm_kernel<EPI_PART, 64, false, 2>, 1}, {(const void*)gemm_kernel<EPI_PART, 64, true, 2>, 1},
-      {(const void*)gemm_kernel<EPI_PART, 128, true, 2>, 1}, {(const void*)attn::attention_kernel, 225 * 1024},
       {(const void*)tail_kernel<false>, TAIL_SMEM}, {(const void*)tail_kernel<true>, TAIL_SMEM},
       {(const void*)residual_norm_kernel<1>, 0}, {(const void*)residual_norm_kernel<2>, 0},
       {(const void*)residual_norm_kernel<4>, 0}, {(const void*)residual_norm_kernel<8>, 0},
       {(const void*)modulation_kernel, 0}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
-  for (const auto& k : all) {
-    cudaError_t e = cudaSuccess;
-    if (k.smem) e = cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem == 1 ? 222 * 1024 : k.smem);
-    // one split of L1 and shared memory for all of them: an SM that has to change it drains first, which would keep a
-    // kernel's CTAs from becoming resident beside the ones of the kernel before
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-  }
-  if (device < 64) done[device] = true;
-  return cudaSuccess;
+  cudaError_t e = ops_opt_in(device);
+  for (const auto& k : all)
+    if (e == cudaSuccess) e = chain_opt_in(k.kernel, k.smem);
+  if (e == cudaSuccess && device < 64) done[device] = true;
+  return e;
 }
 
 struct Capture {
@@ -575,7 +449,7 @@ struct Capture {
   template <typename... P, typename... A>
   void put(void (*kernel)(P...), int grid, int block, size_t smem, int cluster, A&&... args) {
     if (e != cudaSuccess) return;
-    e = launch(kernel, grid, block, smem, stream, cluster, std::forward<A>(args)...);
+    e = launch_chained(kernel, grid, block, smem, stream, cluster, std::forward<A>(args)...);
     ++kernels;
   }
 
@@ -614,17 +488,17 @@ struct Capture {
   }
 
   void project(int epi, const GemmPlan& g, const CUtensorMap& a, const CUtensorMap* b0, const CUtensorMap* b1, const CUtensorMap* b2,
-               int k, int layer) {
+               int width, int layer) {
+    if (e != cudaSuccess) return;
     gemm::Args p;
     memset(&p, 0, sizeof p);
     p.a = a; p.b0 = *b0;
     if (b1) p.b1 = *b1;
     if (b2) p.b2 = *b2;
-    p.tokens = T * s.batch; p.rows = g.rows; p.m_groups = g.pair ? g.m_tiles / 2 : g.m_tiles; p.splits = g.splits;
-    p.kblocks = k / gemm::BK / g.splits; p.units = g.units; p.layer = layer; p.stages = g.stages; p.a_stride = g.a_stride;
-    p.bufs = g.bufs; p.off_out = g.off_out; p.status = s.status; p.limit = s.wait_limit;
+    p.tokens = T * s.batch; p.layer = layer; p.width = width; p.status = s.status; p.limit = s.wait_limit;
     p.q = s.q; p.k = s.k; p.v = s.v; p.rope = s.rope; p.act = s.act; p.part = s.part;
-    put(gemm_kernel_for(epi, g), g.grid, gemm::THREADS_G, g.smem, g.pair ? 2 : 1, p);
+    e = launch_gemm(g, epi, p, stream);
+    ++kernels;
   }
 
   void step() {
@@ -633,7 +507,7 @@ struct Capture {
     attn::Args ap;
     memset(&ap, 0, sizeof ap);
     const AttnPlan pa = plan_attention(s.sms, s.batch, s.prefix);
-    ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits; ap.stages = attn::stages_for(pa.tok_tile * NQH);
+    ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits;
     ap.merge = s.part;
     const uint64_t L = NL, M = tokens;
     if (!(map_2d(&a_qkv, s.an, W, M, pq.rows) && map_2d(&a_o, s.attn, QD, M, po.rows) && map_2d(&a_gu, s.an, W, M, pg.rows) &&
@@ -641,7 +515,8 @@ struct Capture {
           map_2d(&wk, s.in[9], W, L * HD, pq.bn / 2) && map_2d(&wv, s.in[10], W, L * HD, pq.bn / 2) &&
           map_2d(&wo, s.in[11], QD, L * W, po.bn / 2) && map_2d(&wg, s.in[12], W, L * FF, pg.bn / 2) &&
           map_2d(&wu, s.in[13], W, L * FF, pg.bn / 2) && map_2d(&wd, s.in[14], FF, L * W, pd.bn / 2) &&
-          map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH))) {
+          map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH) &&
+          map_out(&ap.o, s.attn, false, HD, (uint64_t)T * NQH, s.batch, 128, ap.tok_tile * NQH))) {
       e = cudaErrorUnknown;
       what = "cuTensorMapEncodeTiled failed";
       return;
@@ -654,14 +529,14 @@ struct Capture {
     NormArgs n;
     n.part = s.part; n.h = s.h; n.out = s.an; n.mod = s.mod; n.state = s.state;
     for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
-      project(gemm::EPI_QKV, pq, a_qkv, &wq, &wk, &wv, W, l);
+      project(gemm::EPI_QKV, pq, a_qkv, &wq, &wk, &wv, 0, l);
       ap.layer = l;
-      put(attn::attention_kernel, s.batch * ap.tiles * ap.splits, attn::THREADS, attn::smem_for(ap.tok_tile * NQH), ap.splits, ap);
-      project(gemm::EPI_PART, po, a_o, &wo, nullptr, nullptr, QD, l);
+      if (e == cudaSuccess) { e = launch_attention(ap, s.batch, stream); ++kernels; }
+      project(gemm::EPI_PART, po, a_o, &wo, nullptr, nullptr, W, l);
       n.gate_norm = 2 * l; n.next_norm = 2 * l + 1;
       put(norm_kernel_for(po.splits), tokens, 256, 0, 1, n);
-      project(gemm::EPI_GEGLU, pg, a_gu, &wg, &wu, nullptr, W, l);
-      project(gemm::EPI_PART, pd, a_dn, &wd, nullptr, nullptr, FF, l);
+      project(gemm::EPI_GEGLU, pg, a_gu, &wg, &wu, nullptr, FF, l);
+      project(gemm::EPI_PART, pd, a_dn, &wd, nullptr, nullptr, W, l);
       if (l + 1 < n_layers) {
         n.gate_norm = 2 * l + 1; n.next_norm = 2 * l + 2;
         put(norm_kernel_for(pd.splits), tokens, 256, 0, 1, n);

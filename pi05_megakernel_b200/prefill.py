@@ -69,8 +69,10 @@ class Pi05Prefill:
                 or valid.device != self.device:
             raise ValueError(f"embeddings and valid must be contiguous and live on {self.device}")
         shape = (self.geo.layers, tokens, self.geo.kv_heads, self.geo.head_dim)
-        k, v = out if out is not None else (torch.zeros(shape, dtype=torch.bfloat16, device=self.device),
-                                            torch.zeros(shape, dtype=torch.bfloat16, device=self.device))
+        # a run over all layers writes every element; a shorter one leaves the later layers at zero
+        make = torch.empty if layers in (None, self.geo.layers) else torch.zeros
+        k, v = out if out is not None else (make(shape, dtype=torch.bfloat16, device=self.device),
+                                            make(shape, dtype=torch.bfloat16, device=self.device))
         stream = torch.cuda.current_stream(self.device).cuda_stream
         self._check(self.lib.pi05_prefill_run(self.handle, embeddings.data_ptr(), valid.data_ptr(), tokens, k.data_ptr(),
                                               v.data_ptr(), self.geo.layers if layers is None else layers, stream))
