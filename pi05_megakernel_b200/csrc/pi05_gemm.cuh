@@ -7,12 +7,17 @@
 //   * weights do not depend on the chain, so a CTA fills its whole weight ring before it waits for the kernel before it
 //     (programmatic dependent launch);
 //   * a stage holds both operands of KS 64-k blocks behind one barrier, and its MMAs and the commit that frees it are one asm
-//     block: with a barrier and a commit per operand and 64-k block the issuing warp needed ~570 cycles for four MMAs that
-//     take the tensor core 160-200;
-//   * the tile's tokens are balanced (rows = ceil(tokens / tiles)) and only those rows are copied; the MMA still reads 128
-//     rows, the ones beyond the tile are whatever shared memory holds and end in accumulator lanes nobody reads;
-//   * K is split over several CTAs where whole-K tiles would leave SMs without work; every split stores its FP32 partial
-//     sums to a slice of its own and the residual kernel adds the slices (atomics made the end of the kernel ~1 us later);
+//     block.  Weights and activations have a producer warp each, and a copy brings all KS blocks of an operand;
+//   * what a stage takes is the way of its operands through shared memory (128 B per cycle: 4 KB of activations and 1-2 KB of
+//     weights read per MMA, and the copies that write them): an MMA reads 128 rows of activations however few are valid.  A
+//     tile of up to 64 rows is an MMA of 64: at 50 tokens a stage of 128 k x 64 features takes 0.27 us instead of 0.38, a layer
+//     pass 28.3 us instead of 30.2;
+//   * the tile's tokens are balanced (rows = ceil(tokens / tiles)) and only those rows are copied; the MMA still reads 64
+//     or 128 rows, the ones beyond the tile are whatever shared memory holds and end in accumulator lanes nobody reads;
+//   * K is split over several CTAs where whole-K tiles would leave SMs without work.  Every split stores its FP32 partial
+//     sums to a slice of its own and a row kernel adds the slices (atomics made the end of the kernel ~1 us later; folding the
+//     row kernel's normalisation into the projections around it and adding the splits within a cluster made a layer pass
+//     slower, since the row kernel is what the weights of the next projection arrive under);
 //   * results of all but the smallest tiles leave through shared memory by tiled copies (a thread per row stores 16 bytes to
 //     32 different lines, which the LSU takes one at a time: 2 us at 128 features per thread; a bulk copy per row: 1.5 us);
 //   * SK ("stream-K"): tiles x 64-k blocks, taken as one sequence, are cut into one contiguous, equal range per CTA, so that a
@@ -32,18 +37,18 @@
 namespace gemm {
 using namespace pi05;
 
-constexpr int THREADS_G = 320;     // warp 0 producer, warp 1 MMA issuer, warps 2..9 epilogue (two per TMEM lane quadrant)
+constexpr int THREADS_G = 352;     // warp 0 weight producer, warp 1 MMA issuer, warps 2..9 epilogue (two per TMEM lane quadrant), warp 10
+                                   // activation producer
 constexpr int EPI_THREADS = 256;
 constexpr int BK = 64;             // k per stage (one 128-byte swizzle row)
 constexpr int MAX_STAGES = 16;
 
 enum { EPI_QKV = 0, EPI_GEGLU = 1, EPI_PART = 2 };
-
 struct Args {
-  CUtensorMap a;                   // activations [tokens, K], box {64, rows}
-  CUtensorMap b0, b1, b2;          // weights, box {64, BN / 2}.  QKV: wq, wk, wv; GEGLU: gate, up; PART: b0
+  CUtensorMap a;                   // activations as {64 k, rows, K / 64}, box {64, arows, KS}
+  CUtensorMap b0, b1, b2;          // weights likewise, box {64, rows of a load, 64-k blocks of a load}.  QKV: wq, wk, wv; GEGLU: gate, up
   CUtensorMap o0, o1, o2;          // staged results, box {128 or 64 bytes, rows}.  QKV: q, k, v; GEGLU: act; PART: part (3-D)
-  int tokens, rows, m_groups, splits, kblocks, units, layer, stages, a_stride, bufs, off_out;   // kblocks: 64-k blocks per unit
+  int tokens, rows, arows, m_groups, splits, kblocks, units, layer, stages, bufs, off_out;   // kblocks: 64-k blocks per unit
   int width;                       // GEGLU: MLP width; PART: features of the output (rows of a layer's weights)
   int unit0;                       // first unit of the launch (QKV of a last layer: keys and values only)
   unsigned int* status;
@@ -89,7 +94,7 @@ struct Staging {
 // it from column 32 box0 on.
 // Eight columns at a time in loops that stay loops: an instruction that runs once costs several cycles to fetch.
 template <int EPI, int BN>
-__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int row, int token, bool live, int half, uint32_t out,
+__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int row, int token, bool live, bool mine, int half, uint32_t out,
                                              int box0, int boxes) {
   using St = Staging<EPI, BN>;
   constexpr bool STAGED = St::COUNT > 0;
@@ -104,7 +109,7 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
       ptx::tmem_wait_ld();
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (STAGED) ptx::st_shared_v4(out + St::at(row, (half * cols + c) / 4 + j), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, (half * cols + c) / 4 + j), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]); }
         else if (live) g[c / 4 + j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
       }
     }
@@ -143,10 +148,10 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
           o2[j] = head <= NQH ? *reinterpret_cast<const uint32_t*>(&b) : y;
         }
       }
-      if (STAGED) ptx::st_shared_v4(out + St::at(row, c / 8), o1[0], o1[1], o1[2], o1[3]);
+      if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, c / 8), o1[0], o1[1], o1[2], o1[3]); }
       else if (live) *reinterpret_cast<uint4*>(g + c) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
       if (EPI == EPI_QKV) {
-        if (STAGED) ptx::st_shared_v4(out + St::at(row, (BN / 2 + c) / 8), o2[0], o2[1], o2[2], o2[3]);
+        if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, (BN / 2 + c) / 8), o2[0], o2[1], o2[2], o2[3]); }
         else if (live) *reinterpret_cast<uint4*>(g + 128 + c) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
       }
     }
@@ -185,16 +190,18 @@ template <int EPI, int BN, bool PAIR, int KS, bool SK>
 __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__ Args p) {
   static_assert(!SK || (EPI == EPI_PART && BN == 256 && !PAIR && KS == 1), "stream-K: partial sums of 128 x 256 tiles");
   constexpr int WR = PAIR ? BN / 2 : BN;                  // weight rows this CTA loads per 64-k block
+  constexpr bool TWO = !PAIR && (EPI == EPI_QKV || EPI == EPI_GEGLU);      // .. from two places, block by block
   constexpr int W_BYTES = WR * 128, HALF = (BN / 2) * 128, OUT = Staging<EPI, BN>::BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t bars[2 * MAX_STAGES + 4];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
-  const int ustep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x, unit0 = p.unit0 + (PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x);
+  const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;                // pair: the even CTA issues
+  const int per_unit = PAIR ? 2 : 1;
+  const int ustep = (int)gridDim.x / per_unit, unit0 = p.unit0 + (int)blockIdx.x / per_unit;
   // a stage: KS activation blocks, then KS weight blocks
-  const uint32_t ring = ptx::smem_u32(smem), a_stride = p.a_stride, w_off = KS * a_stride, st_stride = w_off + KS * W_BYTES;
+  const uint32_t a_stride = (uint32_t)p.arows * 128, w_off = KS * a_stride, st_stride = w_off + KS * W_BYTES, ring = ptx::smem_u32(smem);
   const uint32_t full = ptx::smem_u32(bars), empty = full + 8 * MAX_STAGES, t_full = empty + 8 * MAX_STAGES, t_empty = t_full + 16;
   const bool leader = ptx::elect_one();
   const int stages = p.stages;
@@ -208,7 +215,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     ptx::fence_proxy_async_shared();
   }
   __syncwarp();
-  if (PAIR) ptx::cluster_sync();           // the even CTA's barriers exist before the odd CTA's copies count on them
+  if (PAIR) ptx::cluster_sync();           // every CTA's barriers exist before another's copies count on them
 
   // The CTA's work, unit after unit: tile (mt, nt), slice of the partial sums, first stage and number of stages of its K range.
   // Regular: groups of tokens fastest (neighbours share weights), then K split, then features.
@@ -226,7 +233,8 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       w.split = w.st0 ? (int)blockIdx.x : (int)gridDim.x + tile;      // slot of the partial sums
       at += w.nst;
     } else {
-      const int unit = (int)at, rest = unit / p.m_groups, mg = unit - rest * p.m_groups;
+      const int unit = (int)at;
+      const int rest = unit / p.m_groups, mg = unit - rest * p.m_groups;
       w.nt = rest / p.splits;
       w.split = rest - w.nt * p.splits;
       w.mt = PAIR ? 2 * mg + (int)rank : mg;
@@ -236,91 +244,91 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     }
     return true;
   };
-  const CUtensorMap *m0 = &p.b0, *m1 = &p.b0;
-  int r0 = 0, r1 = 0;
-  auto weight_rows = [&](int nt) {
-    if (EPI == EPI_QKV) {                  // tile = BN / 2 dims of a head and their rotary partners
-      constexpr int PER = HD / BN;
-      const int head = nt / PER, d0 = (nt % PER) * (BN / 2);
-      m0 = m1 = head < NQH ? &p.b0 : head == NQH ? &p.b1 : &p.b2;
-      r0 = head < NQH ? p.layer * QD + head * HD + d0 : p.layer * HD + d0;
-      r1 = r0 + 128;
-    } else if (EPI == EPI_GEGLU) {
-      m1 = &p.b1;
-      r0 = r1 = p.layer * p.width + nt * (BN / 2);
-    } else {
-      r0 = p.layer * p.width + nt * BN;
-      r1 = r0 + BN / 2;
-    }
-  };
-  auto load_w = [&](int kc, uint32_t slot) {
-    const uint32_t dst = ring + slot * st_stride + w_off;
-    const uint32_t bar = PAIR ? ptx::map_to_rank(full + 8 * slot, 0) : full + 8 * slot;
-    if (!PAIR || rank == 0) ptx::mbar_expect_tx(full + 8 * slot, (PAIR ? 2 : 1) * KS * W_BYTES);
-#pragma unroll
-    for (int h = 0; h < KS; ++h) {
-      if (PAIR) {
-        ptx::tma_load_2d_pair(dst + h * W_BYTES, rank ? m1 : m0, bar, kc + h * BK, rank ? r1 : r0);
-      } else {
-        ptx::tma_load_2d(dst + h * W_BYTES, m0, bar, kc + h * BK, r0);
-        ptx::tma_load_2d(dst + h * W_BYTES + HALF, m1, bar, kc + h * BK, r1);
-      }
-    }
-  };
-  int ahead = 0;                           // weight stages of the first unit requested before the dependency is waited for
   if (warp == 0) {
-    long long at = first();
-    Work w;
-    take(at, w);
-    weight_rows(w.nt);
-    ahead = stages < w.nst ? stages : w.nst;
-    if (leader) {
-      for (int i = 0; i < ahead; ++i) load_w((w.st0 + i) * KS * BK, i);
-      ptx::prefetch_tensormap(&p.a);
-    }
-  } else if (warp == 1) {
-    if (PAIR) { ptx::tmem_alloc_pair(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish_pair(); }
-    else { ptx::tmem_alloc(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish(); }
-    ptx::grid_dep_launch();                // after the allocation: a later kernel cannot take the columns first
-  }
-  ptx::tc_fence_before();
-  __syncthreads();
-  ptx::tc_fence_after();
-  const uint32_t tmem = s_tmem;
-  ptx::grid_dep_wait();
-
-  if (warp == 0) {
-    // ---- producer
-    const uint32_t a_bytes = (uint32_t)p.rows * 128 * KS;
+    // ---- weight producer: does not wait for the kernel before this one, nor does anybody wait for it but the MMAs
+    ptx::bar_arrive(6, THREADS_G);
+    const uint32_t bytes = (PAIR ? 2 : 1) * KS * W_BYTES;
     uint32_t slot = 0, par = 1;
     bool ok = true;
     long long at = first();
     Work w;
-    for (int it = 0; ok && take(at, w); ++it) {
-      weight_rows(w.nt);
+    while (ok && take(at, w)) {
+      const CUtensorMap *m0 = &p.b0, *m1 = &p.b0;
+      int r0, r1;
+      if (EPI == EPI_QKV) {                // tile = BN / 2 dims of a head and their rotary partners
+        constexpr int PER = HD / BN;
+        const int head = w.nt / PER, d0 = (w.nt % PER) * (BN / 2);
+        m0 = m1 = head < NQH ? &p.b0 : head == NQH ? &p.b1 : &p.b2;
+        r0 = head < NQH ? p.layer * QD + head * HD + d0 : p.layer * HD + d0;
+        r1 = r0 + 128;
+      } else if (EPI == EPI_GEGLU) {
+        m1 = &p.b1;
+        r0 = r1 = p.layer * p.width + w.nt * (BN / 2);
+      } else {
+        r0 = p.layer * p.width + w.nt * BN;
+        r1 = r0 + BN / 2;
+      }
+      if (PAIR && rank) { m0 = m1; r0 = r1; }
       for (int i = 0; i < w.nst; ++i) {
-        const int kc = (w.st0 + i) * KS * BK;
-        const bool have_w = it == 0 && i < ahead;
-        if (!have_w && !(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1))) break;
+        const int kb = (w.st0 + i) * KS;
+        if (!(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 2))) break;
         if (leader) {
-          const uint32_t dst = ring + slot * st_stride, bar = PAIR ? ptx::map_to_rank(full + 8 * slot, 0) : full + 8 * slot;
-          if (!PAIR || rank == 0) ptx::mbar_expect_tx(full + 8 * slot, (PAIR ? 2 : 1) * a_bytes);
+          const uint32_t dst = ring + slot * st_stride + w_off;
+          if (rank == 0) ptx::mbar_expect_tx(full + 8 * slot, bytes);
+          if (PAIR) {
+            ptx::tma_load_3d_pair(dst, m0, ptx::map_to_rank(full + 8 * slot, 0), 0, r0, kb);
+          } else if (TWO) {
 #pragma unroll
-          for (int h = 0; h < KS; ++h) {
-            if (PAIR) ptx::tma_load_2d_pair(dst + h * a_stride, &p.a, bar, kc + h * BK, w.mt * p.rows);
-            else ptx::tma_load_2d(dst + h * a_stride, &p.a, bar, kc + h * BK, w.mt * p.rows);
+            for (int h = 0; h < KS; ++h) {
+              ptx::tma_load_3d(dst + h * W_BYTES, m0, full + 8 * slot, 0, r0, kb + h);
+              ptx::tma_load_3d(dst + h * W_BYTES + HALF, m1, full + 8 * slot, 0, r1, kb + h);
+            }
+          } else {
+            ptx::tma_load_3d(dst, m0, full + 8 * slot, 0, r0, kb);
           }
-          if (!have_w) load_w(kc, slot);
         }
         if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; }
       }
     }
+  } else {
+    if (warp == 1) {
+      if (PAIR) { ptx::tmem_alloc_pair(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish_pair(); }
+      else { ptx::tmem_alloc(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish(); }
+      ptx::grid_dep_launch();              // after the allocation: a later kernel cannot take the columns first
+    } else if (warp == 10 && leader) {
+      ptx::prefetch_tensormap(&p.a);
+    }
+    ptx::tc_fence_before();
+    ptx::named_bar_sync(6, THREADS_G);     // the barriers are initialised, the tensor memory is allocated
+    ptx::tc_fence_after();
+  }
+  const uint32_t tmem = s_tmem;
+
+  if (warp == 10) {
+    // ---- activation producer
+    ptx::grid_dep_wait();
+    const uint32_t bytes = (PAIR ? 2 : 1) * KS * a_stride;
+    uint32_t slot = 0, par = 1;
+    bool ok = true;
+    long long at = first();
+    Work w;
+    while (ok && take(at, w))
+      for (int i = 0; i < w.nst; ++i) {
+        if (!(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1))) break;
+        if (leader) {
+          const uint32_t dst = ring + slot * st_stride;
+          if (rank == 0) ptx::mbar_expect_tx(full + 8 * slot, bytes);
+          if (PAIR) ptx::tma_load_3d_pair(dst, &p.a, ptx::map_to_rank(full + 8 * slot, 0), 0, w.mt * p.rows, (w.st0 + i) * KS);
+          else ptx::tma_load_3d(dst, &p.a, full + 8 * slot, 0, w.mt * p.rows, (w.st0 + i) * KS);
+        }
+        if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; }
+      }
   } else if (warp == 1) {
     // ---- MMA issuer (of a pair: the even CTA only)
-    if (!PAIR || rank == 0) {
-      const uint32_t idesc = ptx::umma_idesc_bf16(PAIR ? 256 : 128, BN);
-      const uint64_t adesc0 = ptx::umma_smem_desc(ring), bdesc0 = ptx::umma_smem_desc(ring + w_off);
-      uint32_t slot = 0, par = 0, it = 0;
+    if (rank == 0) {
+      const uint32_t idesc = ptx::umma_idesc_bf16(PAIR ? 256 : p.rows <= 64 ? 64 : 128, BN);
+      const uint32_t adesc0 = (uint32_t)ptx::umma_smem_desc(ring), bdesc0 = (uint32_t)ptx::umma_smem_desc(ring + w_off);
+      uint32_t slot = 0, par = 0, it = 0, off = 0;
       bool ok = true;
       long long at = first();
       Work w;
@@ -330,46 +338,49 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
         ptx::tc_fence_after();
         const uint32_t d = tmem + buf * BN;
         uint32_t acc = 0;
+#pragma unroll 1
         for (int i = 0; i < w.nst; ++i) {
           if (!(ok = ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, 3))) break;
-          const uint64_t off = (uint64_t)((slot * st_stride) >> 4);
-          if (leader)
-            ptx::umma_bf16_stage<PAIR, KS>(d, adesc0 + off, bdesc0 + off, idesc, acc, empty + 8 * slot, a_stride >> 4, W_BYTES >> 4);
+          const uint32_t cur = off, bar = empty + 8 * slot;
+          off += st_stride >> 4;
+          if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; off = 0; }
+          ptx::umma_bf16_stage<PAIR, KS>(d, adesc0 + cur, bdesc0 + cur, idesc, acc, bar, a_stride >> 4, W_BYTES >> 4, leader ? 1u : 0u);
           acc = 1;
-          if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; }
         }
         if (ok && leader) {
-          if (PAIR) ptx::umma_commit_pair(t_full + 8 * buf);
+          if (PAIR) ptx::umma_commit_pair(t_full + 8 * buf, 3);
           else ptx::umma_commit(t_full + 8 * buf);
         }
       }
     }
-  } else {
+  } else if (warp >= 2) {
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) ..; thread = token row of the tile, half of its columns.  A wait that
     // gives up does not end the loop: the other epilogue warps count on this one at their barriers
-    const int quad = warp & 3, row = quad * 32 + lane, half = warp >= 6 ? 1 : 0;
+    // (a tile of up to 64 rows is an MMA of 64, whose rows lie in the first 16 lanes of every warp)
+    const bool m64 = !PAIR && p.rows <= 64;
+    const int quad = warp & 3, qrow = m64 ? quad * 16 : quad * 32, row = qrow + lane, half = warp >= 6 ? 1 : 0;
     const uint32_t release = PAIR ? ptx::map_to_rank(t_empty, 0) : 0u;
-    const uint32_t stage = ptx::smem_u32(smem) + p.off_out;
-    constexpr int BOXES = SK ? 2 : Staging<EPI, BN>::COUNT;          // boxes staged at a time
     uint32_t it = 0;
     bool ok = true;
     long long at = first();
     Work w;
+    const uint32_t stage = ptx::smem_u32(smem) + p.off_out;
+    constexpr int BOXES = SK ? 2 : Staging<EPI, BN>::COUNT;          // boxes staged at a time
     for (; take(at, w); ++it) {
       const uint32_t buf = it & 1;
       const int token = w.mt * p.rows + row;
       ok &= ptx::wait_bar(p.status, p.limit, t_full + 8 * buf, (it >> 1) & 1, 5);
       ptx::tc_fence_after();
+      const uint32_t t0 = tmem + buf * BN + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
       for (int box0 = 0; box0 < (SK ? Staging<EPI, BN>::COUNT : 1); box0 += SK ? BOXES : 1) {
         if (OUT > 0 && (it > 0 || box0 > 0)) {                       // what was staged before has left the buffer
           if (tid == 64) ptx::bulk_wait_read();
           ptx::named_bar_sync(1, EPI_THREADS);
         }
-        if (quad * 32 < p.rows)
-          epilogue_row<EPI, BN>(p, tmem + buf * BN + ((uint32_t)(quad * 32) << 16), w.nt, w.split, row, token,
-                                ok && row < p.rows && token < p.tokens, half, stage, box0, BOXES);
-        if (!SK || box0 + BOXES >= Staging<EPI, BN>::COUNT) {        // the accumulator has been read
+        if (qrow < p.rows)
+          epilogue_row<EPI, BN>(p, t0, w.nt, w.split, row, token, ok && row < p.rows && token < p.tokens && (!m64 || lane < 16), !m64 || lane < 16, half, stage, box0, BOXES);
+        if (!SK || box0 + BOXES >= Staging<EPI, BN>::COUNT) {   // the accumulator has been read
           ptx::tc_fence_before();
           if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);
           else ptx::mbar_arrive(t_empty + 8 * buf);
@@ -387,7 +398,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     if (OUT > 0 && tid == 64) ptx::bulk_wait_read();
   }
   __syncthreads();
-  if (PAIR) ptx::cluster_sync();           // neither CTA leaves (or frees tensor memory) while the other may still use it
+  if (PAIR) ptx::cluster_sync();           // neither CTA leaves (or frees tensor memory) while the other may still use what is in it
   if (warp == 1) {
     ptx::tc_fence_after();
     if (PAIR) ptx::tmem_dealloc_pair(tmem, tcols);

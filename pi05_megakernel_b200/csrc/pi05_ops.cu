@@ -34,39 +34,47 @@ typedef void (*GemmKernel)(const gemm::Args);
 struct Cut { int epi, bn, ks; bool pair, sk; GemmKernel kernel; };
 
 // Every cut that is built.
+#define CUT(E, BN, PAIR, KS, SK) {gemm::E, BN, KS, PAIR, SK, gemm::gemm_kernel<gemm::E, BN, PAIR, KS, SK>}
 const Cut kCuts[] = {
-    {gemm::EPI_QKV, 32, 2, false, false, gemm::gemm_kernel<gemm::EPI_QKV, 32, false, 2, false>},
-    {gemm::EPI_QKV, 128, 2, false, false, gemm::gemm_kernel<gemm::EPI_QKV, 128, false, 2, false>},
-    {gemm::EPI_QKV, 32, 2, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 32, true, 2, false>},
-    {gemm::EPI_QKV, 64, 2, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 64, true, 2, false>},
-    {gemm::EPI_QKV, 128, 2, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 128, true, 2, false>},
-    {gemm::EPI_QKV, 256, 1, true, false, gemm::gemm_kernel<gemm::EPI_QKV, 256, true, 1, false>},
-    {gemm::EPI_GEGLU, 64, 2, false, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 64, false, 2, false>},
-    {gemm::EPI_GEGLU, 128, 2, false, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 128, false, 2, false>},
-    {gemm::EPI_GEGLU, 256, 1, false, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 256, false, 1, false>},
-    {gemm::EPI_GEGLU, 128, 2, true, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 128, true, 2, false>},
-    {gemm::EPI_GEGLU, 256, 1, true, false, gemm::gemm_kernel<gemm::EPI_GEGLU, 256, true, 1, false>},
-    {gemm::EPI_PART, 32, 2, false, false, gemm::gemm_kernel<gemm::EPI_PART, 32, false, 2, false>},
-    {gemm::EPI_PART, 64, 2, false, false, gemm::gemm_kernel<gemm::EPI_PART, 64, false, 2, false>},
-    {gemm::EPI_PART, 64, 2, true, false, gemm::gemm_kernel<gemm::EPI_PART, 64, true, 2, false>},
-    {gemm::EPI_PART, 128, 2, true, false, gemm::gemm_kernel<gemm::EPI_PART, 128, true, 2, false>},
-    {gemm::EPI_PART, 256, 1, true, false, gemm::gemm_kernel<gemm::EPI_PART, 256, true, 1, false>},
-    {gemm::EPI_PART, 256, 1, false, true, gemm::gemm_kernel<gemm::EPI_PART, 256, false, 1, true>},
+    CUT(EPI_QKV, 32, false, 2, false), CUT(EPI_QKV, 128, false, 2, false), CUT(EPI_QKV, 64,true, 2, false),
+    CUT(EPI_QKV, 128,true, 2, false), CUT(EPI_QKV, 256,true, 1, false),
+    CUT(EPI_GEGLU, 64, false, 2, false), CUT(EPI_GEGLU, 128, false, 2, false), CUT(EPI_GEGLU, 256, false, 1, false),
+    CUT(EPI_GEGLU, 128,true, 2, false), CUT(EPI_GEGLU, 256,true, 1, false),
+    CUT(EPI_PART, 32, false, 2, false), CUT(EPI_PART, 64, false, 2, false), CUT(EPI_PART, 64,true, 2, false),
+    CUT(EPI_PART, 128,true, 2, false), CUT(EPI_PART, 256,true, 1, false), CUT(EPI_PART, 256, false, 1, true),
 };
+#undef CUT
 
-// Ring, staging and shared memory of a cut whose tile, grid and accumulators are decided.
-void lay_out(GemmPlan* g, int epi, int stages_wanted) {
-  const int w_bytes = (g->pair ? g->bn / 2 : g->bn) * 128, stage = g->ks * (g->a_stride + w_bytes);
+// Loads, ring, staging and shared memory of a cut whose tile, grid and accumulators are decided.
+void lay_out(GemmPlan* g, int stages_wanted) {
+  const bool two = !g->pair && (g->epi == gemm::EPI_QKV || g->epi == gemm::EPI_GEGLU);
+  g->w_rows = g->pair || two ? g->bn / 2 : g->bn;
+  g->w_kb = two ? 1 : g->ks;
+  const int w_bytes = (g->pair ? g->bn / 2 : g->bn) * 128, stage = g->ks * (g->arows * 128 + w_bytes);
   // results are staged in the ring when the CTA has one tile (its operands are consumed by then), else behind it
   const bool behind = g->bufs > 1;
-  const int out = g->sk ? 2 * 16384 : staging_bytes(epi, g->bn), budget = 220 * 1024 - (behind ? out : 0);
+  const int out = g->sk ? 2 * 16384 : staging_bytes(g->epi, g->bn);
+  const int budget = 218 * 1024 - (behind ? out : 0);
   g->stages = std::min({gemm::MAX_STAGES, budget / stage, stages_wanted});
-  g->off_out = behind ? g->stages * stage : 0;
+  const int ring = g->stages * stage;
+  g->off_out = behind ? ring : 0;
   // the MMA reads 128 rows from the last activation block on
-  g->smem = std::max({g->stages * stage, (g->stages - 1) * stage + (g->ks - 1) * g->a_stride + 128 * 128, g->off_out + out}) + 1024;
+  g->smem = std::max({ring, (g->stages - 1) * stage + (g->ks - 1) * g->arows * 128 + 128 * 128, g->off_out + out}) + 1024;
 }
 
 }  // namespace
+
+bool map_k(CUtensorMap* m, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t blocks) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) return false;
+  cuuint64_t dims[3] = {64, rows, k / 64};
+  cuuint64_t strides[2] = {k * 2, 128};
+  cuuint32_t box[3] = {64, box_rows, blocks};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
   EncodeTiledFn enc = encoder();
@@ -104,7 +112,8 @@ bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers) 
 }
 
 // The cheapest of the cuts that are built, by a model of the launch's time in SM cycles: rounds x 64-k blocks x the slower of the
-// MMAs (measured per M128 / M256 K16 instruction: 47 cycles up to N = 32, 50 / 65 / 129 at 64 / 128 / 256) and the operands' way
+// MMAs (measured per M128 / M256 K16 instruction: 47 cycles up to N = 32, 50 / 65 / 129 at 64 / 128 / 256; M64:
+// 39 and 41 up to N = 64) and the operands' way
 // into shared memory (~67 B per cycle and SM), not less than the weights' way from HBM (3.3 KB per cycle), plus what every
 // launch pays, an epilogue that grows with the tile, and the way of partial sums through L2 (~2 KB per cycle).  Pairs of CTAs
 // (256 tokens) load half of the tile's weight rows each.  K of the projections whose sums meet in the residual kernel is split
@@ -115,23 +124,24 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
   for (const Cut& c : kCuts)
     for (int splits = 1; c.epi == epi && !c.sk && splits <= (epi == gemm::EPI_PART ? 8 : 1); splits *= 2) {
       GemmPlan g = {};
-      g.pair = c.pair; g.bn = c.bn; g.ks = c.ks; g.splits = splits;
+      g.epi = epi; g.pair = c.pair; g.bn = c.bn; g.ks = c.ks; g.splits = splits;
       g.kblocks = k / gemm::BK / splits;
       g.m_tiles = (tokens + 127) / 128;
       if ((g.pair && g.m_tiles < 2) || (pairs >= 0 && (int)g.pair != pairs)) continue;
       if (g.pair) g.m_tiles = (g.m_tiles + 1) / 2 * 2;
       if (g.kblocks < 4) continue;
       g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
-      g.a_stride = (g.rows + 7) / 8 * 1024;
+      g.arows = (g.rows + 7) / 8 * 8;
       const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128, ctas = g.m_tiles * (n / g.bn) * splits, rounds = (ctas + sms - 1) / sms;
-      const double mma = 4 * (g.bn <= 32 ? 47 : g.bn == 64 ? 50 : g.bn == 128 ? 65 : 129), ingest = (g.rows * 128 + w_bytes) / 67.0;
-      const double cost = std::max(rounds * g.kblocks * std::max(mma, ingest), (double)n * k * 2 / 3300) + 2000 +
-                          g.bn * (epi == gemm::EPI_GEGLU ? 12 : 8) + (splits > 1 ? std::max(150.0 * splits, splits * (double)tokens * n * 4 / 2000) : 0);
+      const bool m64 = !g.pair && g.rows <= 64;
+      const double mma = 4 * (g.bn <= 32 ? (m64 ? 39 : 47) : g.bn == 64 ? (m64 ? 41 : 50) : g.bn == 128 ? 65 : 129), ingest = (g.arows * 128 + w_bytes) / 67.0;
+      double cost = std::max(rounds * g.kblocks * std::max(mma, ingest), (double)n * k * 2 / 3300) + 2000 + g.bn * (epi == gemm::EPI_GEGLU ? 12 : 8);
+      if (epi == gemm::EPI_PART && splits > 1) cost += std::max(150.0 * splits, splits * (double)tokens * n * 4 / 2000);
       if (cost >= best_cost) continue;
       g.units = g.pair ? ctas / 2 : ctas;
       g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
       g.bufs = g.grid < ctas ? 2 : 1;
-      lay_out(&g, epi, g.bufs > 1 ? gemm::MAX_STAGES : g.kblocks / g.ks);
+      lay_out(&g, g.bufs > 1 ? gemm::MAX_STAGES : g.kblocks / g.ks);
       best = g;
       best_cost = cost;
     }
@@ -140,32 +150,34 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
 
 GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k) {
   GemmPlan g = {};
-  g.sk = true; g.bn = 256; g.ks = 1; g.splits = 1; g.bufs = 2;
+  g.epi = gemm::EPI_PART; g.sk = true; g.bn = 256; g.ks = 1; g.splits = 1; g.bufs = 2;
   g.kblocks = k / gemm::BK;
   g.m_tiles = (tokens + 127) / 128;
   g.rows = g.m_tiles > 1 ? 128 : tokens;
-  g.a_stride = (g.rows + 7) / 8 * 1024;
+  g.arows = (g.rows + 7) / 8 * 8;
   g.units = g.m_tiles * (n / g.bn);
   const long long work = (long long)g.units * g.kblocks;
   g.grid = work < sms ? (int)work : sms;
-  lay_out(&g, gemm::EPI_PART, gemm::MAX_STAGES);
+  lay_out(&g, gemm::MAX_STAGES);
   return g;
 }
 
-cudaError_t launch_gemm(const GemmPlan& g, int epi, gemm::Args& p, cudaStream_t stream) {
+cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream) {
   const Cut* cut = nullptr;
   for (const Cut& c : kCuts)
-    if (c.epi == epi && c.bn == g.bn && c.pair == g.pair && c.sk == g.sk) cut = &c;
+    if (c.epi == g.epi && c.bn == g.bn && c.pair == g.pair && c.sk == g.sk) cut = &c;
   if (!cut) return cudaErrorInvalidValue;
-  p.rows = g.rows; p.m_groups = g.pair ? g.m_tiles / 2 : g.m_tiles; p.splits = g.splits; p.kblocks = g.kblocks;
-  p.stages = g.stages; p.a_stride = g.a_stride; p.bufs = g.bufs; p.off_out = g.off_out;
+  p.rows = g.rows; p.arows = g.arows;
+  p.m_groups = g.pair ? g.m_tiles / 2 : g.m_tiles; p.splits = g.splits; p.kblocks = g.kblocks;
+  p.stages = g.stages; p.bufs = g.bufs; p.off_out = g.off_out;
   p.units = g.units - p.unit0;
   const uint64_t M = p.tokens;
-  bool ok = true;
-  if (g.sk) ok = map_out(&p.o0, p.part, true, g.bn, 128, g.grid + g.units, 128, g.rows);
-  else if (staging_bytes(epi, g.bn) && epi == gemm::EPI_PART) ok = map_out(&p.o0, p.part, true, p.width, M, g.splits, 128, g.rows);
-  else if (staging_bytes(epi, g.bn) && epi == gemm::EPI_GEGLU) ok = map_out(&p.o0, p.act, false, p.width, M, 0, 128, g.rows);
-  else if (staging_bytes(epi, g.bn)) {
+  bool ok =true;
+  if (g.sk) ok = map_out(&p.o0, p.part,true, g.bn, 128, g.grid + g.units, 128, g.rows);
+  else if (!staging_bytes(g.epi, g.bn)) ok =true;
+  else if (g.epi == gemm::EPI_PART) ok = map_out(&p.o0, p.part,true, p.width, M, g.splits, 128, g.rows);
+  else if (g.epi == gemm::EPI_GEGLU) ok = map_out(&p.o0, p.act, false, p.width, M, 0, 128, g.rows);
+  else {
     const int box = g.bn == 64 ? 64 : 128;
     ok = map_out(&p.o0, p.q, false, QD, M, 0, box, g.rows) && map_out(&p.o1, p.k, false, HD, M, 0, box, g.rows) &&
          map_out(&p.o2, p.v, false, HD, M, 0, box, g.rows);

@@ -33,7 +33,10 @@ cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// {inner = K, rows} BF16 row-major, box {64 k, box_rows}, 128-byte swizzle; rows beyond `rows` read as zeros.
+// An operand [rows, K] BF16 row-major as {64 k, rows, K / 64}, box {64, box_rows, blocks}, 128-byte swizzle: one copy brings
+// `blocks` 64-k blocks of box_rows rows.  Rows beyond `rows` read as zeros.
+bool map_k(CUtensorMap* m, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t blocks);
+// {inner, rows} BF16 row-major, box {64, box_rows}, 128-byte swizzle.
 bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows);
 // A dense tensor of two (d2 = 0) or three dimensions, innermost first, of BF16 or FP32 elements, box {box_bytes, box_rows, 1} with
 // the swizzle of that many bytes: the destination of a tiled store.
@@ -43,15 +46,17 @@ bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers);
 
 // How one projection of `tokens` x n features over k is cut.
 struct GemmPlan {
+  int epi;            // gemm::EPI_*
   bool pair, sk;
-  int bn, ks, splits, m_tiles, rows, units, grid, stages, a_stride, bufs, off_out, smem, kblocks;
+  int bn, ks, splits, m_tiles, rows, arows, units, grid, stages, bufs, off_out, smem, kblocks;
+  int w_rows, w_kb;   // rows and 64-k blocks of one weight copy (the box of the weights' maps)
 };
 // pairs: 1 / 0 leaves only cuts on CTA pairs / on single CTAs, -1 all.
 GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs = -1);
 // The stream-K cut of a projection with partial sums: 128 x 256 tiles, one equal range of 64-k blocks per CTA.
 GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k);
 // Fills in what the plan decides and the destination maps, and launches.  `width` and the pointers have to be set.
-cudaError_t launch_gemm(const GemmPlan& g, int epi, gemm::Args& p, cudaStream_t stream);
+cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream);
 cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream);
 // Shared-memory opt-in of the kernels behind the two calls above, once per device.
 cudaError_t ops_opt_in(int device);

@@ -312,12 +312,14 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
   attn::Args ap;
   memset(&ap, 0, sizeof ap);
   const uint64_t L = pf::LAYERS;
-  const bool ok = map_2d(&a_qkv, nrm, pf::H, P, pl.qkv.rows) && map_2d(&a_o, mixed, QD, P, pl.o.rows) &&
-                  map_2d(&a_gu, nrm, pf::H, P, pl.gu.rows) && map_2d(&a_dn, act, pf::FFN, P, pl.down.rows) &&
-                  map_2d(&wq, w[LQ], pf::H, L * QD, pl.qkv.bn / 2) && map_2d(&wk, w[LK], pf::H, L * HD, pl.qkv.bn / 2) &&
-                  map_2d(&wv, w[LV], pf::H, L * HD, pl.qkv.bn / 2) && map_2d(&wo, w[LO], QD, L * pf::H, pl.o.bn / 2) &&
-                  map_2d(&wg, w[LG], pf::H, L * pf::FFN, pl.gu.bn / 2) && map_2d(&wu, w[LU], pf::H, L * pf::FFN, pl.gu.bn / 2) &&
-                  map_2d(&wd, w[LD], pf::FFN, L * pf::H, pl.down.bn / 2) && map_kv(&ap.pk, K, P, L) && map_kv(&ap.pv, V, P, L) &&
+  auto act_map = [&](CUtensorMap* m, const void* base, int k, const GemmPlan& g) { return map_k(m, base, k, P, g.arows, g.ks); };
+  auto weight_map = [&](CUtensorMap* m, int which, int k, int rows, const GemmPlan& g) { return map_k(m, w[which], k, L * rows, g.w_rows, g.w_kb); };
+  const bool ok = act_map(&a_qkv, nrm, pf::H, pl.qkv) && act_map(&a_o, mixed, QD, pl.o) && act_map(&a_gu, nrm, pf::H, pl.gu) &&
+                  act_map(&a_dn, act, pf::FFN, pl.down) && weight_map(&wq, LQ, pf::H, QD, pl.qkv) && weight_map(&wk, LK, pf::H, HD, pl.qkv) &&
+                  weight_map(&wv, LV, pf::H, HD, pl.qkv) && weight_map(&wo, LO, QD, pf::H, pl.o) && weight_map(&wg, LG, pf::H, pf::FFN, pl.gu) &&
+                  weight_map(&wu, LU, pf::H, pf::FFN, pl.gu) && weight_map(&wd, LD, pf::FFN, pf::H, pl.down) &&
+                  map_kv(&ap.pk, K, P, L) &&
+                  map_kv(&ap.pv, V, P, L) &&
                   map_2d(&ap.q, q, HD, (uint64_t)P * NQH, pl.tok_tile * NQH) &&
                   map_out(&ap.o, mixed, false, HD, (uint64_t)P * NQH, 1, 128, pl.tok_tile * NQH);
   if (!ok) { h->last_error = "cuTensorMapEncodeTiled failed"; return PI05_ERR_CUDA; }
@@ -327,7 +329,7 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
   ap.tok_tile = pl.tok_tile; ap.tiles = (P + pl.tok_tile - 1) / pl.tok_tile; ap.splits = 1;
   ap.status = status; ap.limit = h->wait_limit;
 
-  auto project = [&](int epi, const GemmPlan& g, const CUtensorMap& a, const CUtensorMap& b0, const CUtensorMap* b1, const CUtensorMap* b2,
+  auto project = [&](const GemmPlan& g, const CUtensorMap& a, const CUtensorMap& b0, const CUtensorMap* b1, const CUtensorMap* b2,
                      int width, int layer, int unit0 = 0) {
     if (e != cudaSuccess) return;
     gemm::Args p;
@@ -337,7 +339,7 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
     if (b2) p.b2 = *b2;
     p.tokens = P; p.layer = layer; p.width = width; p.unit0 = unit0; p.status = status; p.limit = h->wait_limit;
     p.q = q; p.k = K + (size_t)layer * P * HD; p.v = V + (size_t)layer * P * HD; p.rope = rope; p.act = act; p.part = part;
-    e = launch_gemm(g, epi, p, stream);
+    e = launch_gemm(g, p, stream);
   };
   pf::NormArgs n;
   memset(&n, 0, sizeof n);
@@ -360,16 +362,16 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
   norm(pf::norm_kernel<0>, static_cast<const __nv_bfloat16*>(embeddings), w[LN1]);
   for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
     if (l + 1 == n_layers) {                      // keys and values only: the tiles behind the eight query heads
-      project(gemm::EPI_QKV, pl.qkv, a_qkv, wq, &wk, &wv, 0, l, pl.qkv.units / (NQH + 2) * NQH);
+      project(pl.qkv, a_qkv, wq, &wk, &wv, 0, l, pl.qkv.units / (NQH + 2) * NQH);
       break;
     }
-    project(gemm::EPI_QKV, pl.qkv, a_qkv, wq, &wk, &wv, 0, l);
+    project(pl.qkv, a_qkv, wq, &wk, &wv, 0, l);
     ap.layer = l;
     if (e == cudaSuccess) e = launch_attention(ap, 1, stream);
-    project(gemm::EPI_PART, pl.o, a_o, wo, nullptr, nullptr, pf::H, l);
+    project(pl.o, a_o, wo, nullptr, nullptr, pf::H, l);
     norm(pf::norm_kernel_for(pl.o.splits), x, w[LN2] + (size_t)l * pf::H);
-    project(gemm::EPI_GEGLU, pl.gu, a_gu, wg, &wu, nullptr, pf::FFN, l);
-    project(gemm::EPI_PART, pl.down, a_dn, wd, nullptr, nullptr, pf::H, l);
+    project(pl.gu, a_gu, wg, &wu, nullptr, pf::FFN, l);
+    project(pl.down, a_dn, wd, nullptr, nullptr, pf::H, l);
     norm(pl.sk_down ? pf::norm_kernel<-1> : pf::norm_kernel_for(pl.down.splits), x, w[LN1] + (size_t)(l + 1) * pf::H);
   }
   if (e == cudaSuccess) e = cudaGetLastError();

@@ -87,6 +87,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
 // 4-D tiled load (innermost coordinate first).
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1, int c2, int c3) {
   asm volatile(
@@ -254,32 +259,31 @@ __device__ __forceinline__ void umma_bf16_k64(uint32_t d_tmem, uint64_t adesc, u
 }
 // One pipeline stage of KS 64-k blocks in one piece: 4 KS MMAs of K = 16 (32-byte steps inside the 128-byte swizzle rows of
 // a block, blocks `ablock` / `bblock` descriptor units apart) and the commit that frees the stage, on one CTA or on a pair
-// (whose commit arrives in both CTAs).
+// (whose commit arrives in both CTAs).  `alo`, `blo`: lower words of the descriptors; the upper word is the same for all.
+constexpr uint32_t UMMA_DESC_HI = 64u | (1u << 14) | (2u << 29);
 template <bool PAIR, int KS>
-__device__ __forceinline__ void umma_bf16_stage(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
-                                                uint32_t commit_bar, uint64_t ablock, uint64_t bblock) {
-#define PI05_UMMA4(G, A0, B0, P0)                                                       \
-  "add.u64 a1, " A0 ", 2;\n add.u64 a2, " A0 ", 4;\n add.u64 a3, " A0 ", 6;\n"          \
-  "add.u64 b1, " B0 ", 2;\n add.u64 b2, " B0 ", 4;\n add.u64 b3, " B0 ", 6;\n"          \
-  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], " A0 ", " B0 ", %3, " P0 ";\n"           \
-  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], a1, b1, %3, 1;\n"                       \
-  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], a2, b2, %3, 1;\n"                       \
-  "tcgen05.mma.cta_group::" G ".kind::f16 [%0], a3, b3, %3, 1;\n"
-#define PI05_UMMA_HEAD "{\n.reg .pred p;\n.reg .b64 a1, a2, a3, b1, b2, b3, a4, b4;\nsetp.ne.b32 p, %4, 0;\n"
-#define PI05_UMMA_NEXT "add.u64 a4, %1, %6;\n add.u64 b4, %2, %7;\n"
-#define PI05_UMMA_COMMIT1 "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n}"
-#define PI05_UMMA_COMMIT2 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], %8;\n}"
-#define PI05_UMMA_ARGS ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(commit_bar), "l"(ablock), "l"(bblock)
+__device__ __forceinline__ void umma_bf16_stage(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc, uint32_t accumulate,
+                                                uint32_t commit_bar, uint32_t ablock, uint32_t bblock, uint32_t on) {
+#define PI05_UMMA1(G, AO, BO, P0)                                              \
+  "add.u32 al, a0, " AO ";\n add.u32 bl, b0, " BO ";\n"                        \
+  "mov.b64 da, {al, %8};\n mov.b64 db, {bl, %8};\n"                            \
+  "@q tcgen05.mma.cta_group::" G ".kind::f16 [%0], da, db, %3, " P0 ";\n"
+#define PI05_UMMA4(G, P0) PI05_UMMA1(G, "0", "0", P0) PI05_UMMA1(G, "2", "2", "t") PI05_UMMA1(G, "4", "4", "t") PI05_UMMA1(G, "6", "6", "t")
+#define PI05_UMMA_HEAD "{\n.reg .pred p, q, t;\n.reg .b32 a0, b0, al, bl;\n.reg .b64 da, db;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %9, 0;\n" \
+                       "setp.eq.b32 t, 0, 0;\nmov.b32 a0, %1;\nmov.b32 b0, %2;\n"
+#define PI05_UMMA_NEXT "add.u32 a0, a0, %6;\n add.u32 b0, b0, %7;\n"
+#define PI05_UMMA_COMMIT1 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n}"
+#define PI05_UMMA_COMMIT2 ".reg .b16 m;\nmov.b16 m, 3;\n@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], m;\n}"
+#define PI05_UMMA_ARGS ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(commit_bar), "r"(ablock), "r"(bblock), "n"(UMMA_DESC_HI), "r"(on) : "memory"
   if constexpr (PAIR && KS == 1)
-    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "%1", "%2", "p") PI05_UMMA_COMMIT2 PI05_UMMA_ARGS, "h"((unsigned short)3) : "memory");
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "p") PI05_UMMA_COMMIT2 PI05_UMMA_ARGS);
   else if constexpr (PAIR)
-    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "%1", "%2", "p") PI05_UMMA_NEXT PI05_UMMA4("2", "a4", "b4", "1") PI05_UMMA_COMMIT2
-                 PI05_UMMA_ARGS, "h"((unsigned short)3) : "memory");
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "p") PI05_UMMA_NEXT PI05_UMMA4("2", "t") PI05_UMMA_COMMIT2 PI05_UMMA_ARGS);
   else if constexpr (KS == 1)
-    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "%1", "%2", "p") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS : "memory");
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "p") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS);
   else
-    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "%1", "%2", "p") PI05_UMMA_NEXT PI05_UMMA4("1", "a4", "b4", "1") PI05_UMMA_COMMIT1
-                 PI05_UMMA_ARGS : "memory");
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "p") PI05_UMMA_NEXT PI05_UMMA4("1", "t") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS);
+#undef PI05_UMMA1
 #undef PI05_UMMA4
 #undef PI05_UMMA_HEAD
 #undef PI05_UMMA_NEXT
@@ -311,7 +315,14 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
       : "r"(taddr) : "memory");
 }
 
-// The store that mirrors tmem_ld_32x32, and the wait that orders it before later tcgen05 loads of the same thread.
+// The store that mirrors tmem_ld_32x16, and the wait that orders it before later tcgen05 loads of the same thread.
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -359,6 +370,8 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The shared::cluster address of `saddr` (an address in this CTA's shared memory) in the CTA of rank `rank`.
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -378,15 +391,23 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // Tiled load into this CTA's shared memory whose bytes count on an mbarrier of the pair's even CTA (`cluster_bar`).
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, uint32_t cluster_bar, int c0, int c1) {
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* tmap, uint32_t cluster_bar, int c0, int c1, int c2) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(tmap), "r"(cluster_bar), "r"(c0), "r"(c1) : "memory");
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(tmap), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-// Arrive on the barrier at this offset in both CTAs of the pair when every tcgen05 op issued so far has completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+// Arrive on the barrier at this offset in both CTAs of the pair (`mask`: their ranks in the cluster) when every tcgen05 op issued
+// so far has completed.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, unsigned short mask) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"((unsigned short)3) : "memory");
+               ::"r"(bar), "h"(mask) : "memory");
+}
+
+// Bulk copy from this CTA's shared memory into another's of the cluster (both 16-byte aligned, addresses from map_to_rank),
+// completion on an mbarrier there.
+__device__ __forceinline__ void bulk_copy_cluster(uint32_t cluster_dst, uint32_t src, uint32_t bytes, uint32_t cluster_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(cluster_dst), "r"(src), "r"(bytes), "r"(cluster_bar) : "memory");
 }
 
 // Bounded wait on an mbarrier of this CTA, by a whole converged warp: a wait that runs out records (kind, block) in the
@@ -451,6 +472,16 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// The same barrier with the disjunction of a predicate over its threads.
+__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
+  int r;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\nbarrier.cta.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
+               : "=r"(r) : "r"(id), "r"(nthreads), "r"(pred ? 1 : 0) : "memory");
+  return r != 0;
 }
 // Streaming 16-byte load that does not allocate in L1.
 __device__ __forceinline__ float4 ldg_stream_f4(const float* p) {
