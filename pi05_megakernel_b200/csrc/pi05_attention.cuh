@@ -1,28 +1,30 @@
 // Attention on the tcgen05 tensor cores, used by the action chunk (50 suffix tokens over a prefix cache) and by the prefix
-// prefill (every token over every token): several query tokens x 8 heads share the one KV head, so a tile of up to 128 query
-// rows is one MMA operand.
+// prefill (every token over every token): the 8 heads of several query tokens share the one KV head, so a tile of N = 8 x tokens
+// query rows is one MMA operand.
 //
-//   * One CTA = one tile of `tok_tile` query tokens against a contiguous share of the keys, in chunks of 64.  A cluster of
-//     `splits` CTAs shares the keys of a tile and merges through distributed shared memory (below).
-//   * Warp 0 streams Q, the key chunks and the value chunks with TMA (the 256 dims of a token as four 64-dim segments of
-//     128-byte swizzled rows); warp 1 issues S = Q K^T of chunk i + 1 before O += P V of chunk i; warps 2..9 are the
-//     softmax threads, two per query row, each with half of the chunk's keys and half of the output's dims.  V is the
-//     K-dimension operand as it lies in memory (rows = keys): the MMA takes it as an MN-major B operand, so nothing is
-//     ever transposed.
-//   * The keys are passed over once.  The exponent's reference is the maximum of the first chunk; the accumulator is only
-//     rescaled when a later chunk exceeds it by more than RESCALE (nats), so that almost no chunk pays for it.  Numerator
-//     and denominator always use the same reference, hence the result does not depend on when it moves.
+//   * Everything is computed transposed: S^T = K Q^T (128 keys x N), O^T = V^T P (2 x 128 dims x N).  What bounds a CTA is
+//     shared memory (128 B per cycle: operands read by the MMAs and copies written), and an MMA reads 128 rows of its A operand
+//     whatever is valid.  With the keys, and the dims of V, as A those rows are always full, and the few query rows are
+//     B, which may be as narrow as it is: 128 keys cost 1.2 us with 16 query rows and 1.7 us with 112, against 2.3 us for
+//     up to 128 rows the other way round.
+//   * One CTA = one tile of query tokens against a contiguous share of the keys, in chunks of 128 (the suffix is a chunk of its
+//     own; a chunk of up to 64 valid keys skips the other half of V).  `splits` CTAs of a cluster share the keys of a tile
+//     and merge through global memory (below).
+//   * Warp 0 streams Q and the keys and values with TMA into a ring of 32 KB units, in the order in which the MMAs consume them:
+//     K (dims 0-127, dims 128-255) of chunk i + 1, V (keys 0-63, keys 64-127) of chunk i, ..; warp 1 issues S^T of chunk i + 1
+//     before O^T of chunk i; warps 2..9 are the softmax threads: thread = one key and half of the query rows.  V and P are
+//     taken as they lie, as MN-major operands: nothing is ever transposed in memory.
+//   * The keys are passed over once, and after the first chunk without looking for their maximum: the exponent's reference of a
+//     row is its maximum over the first chunk, and only when a probability of a later chunk comes out above 2^RESCALE is the
+//     reference moved, the accumulator rescaled and the chunk done again.  Numerator and denominator always use the same
+//     reference, hence the result does not depend on when it moves.
 //   * Scores are rounded to BF16 before the scale 1 / 16, and probabilities before P V, as the reference's BF16 matmuls
 //     round (reference/pi05.py:184-188, 254-265).
-//   * The key and value chunks of the cached prefix do not depend on the kernel before this one: with `early` the first
-//     ones are requested before the grid dependency is waited for.
-//   * Shared memory is cut by the tile's rows (only those of Q and P are stored; the MMAs read 128 rows, the ones beyond are
-//     whatever follows and end in accumulator lanes nobody reads): small tiles leave room for three key / value stages, all
-//     that a CTA of a short or well split prefix ever needs, so that nothing of it waits for a stage to be freed.
-//   * Merge of a cluster: each CTA stores its accumulator and (max, sum) per row to global memory, column by column so that a
-//     warp's 32 rows are one line; after a cluster barrier every rank adds its 256 / splits columns of all `splits` parts,
-//     each scaled by exp(m - M) / L.  (The same exchange through distributed shared memory ran at 8-14 B/clk per SM in
-//     either direction and took 6-7 us.)
+//   * The cached prefix does not depend on the kernel before this one: with `early` as much of it as the ring holds is requested
+//     before the grid dependency is waited for.
+//   * Merge of a cluster: each CTA stores its accumulator [row][256] and (reference, sum) per row to global memory; after a
+//     cluster barrier every rank adds N / splits rows of all parts, each scaled by exp(m - M) / L.  (The same exchange through
+//     distributed shared memory, by ld / st.shared::cluster or by bulk copies, ran at 6-14 B/clk per SM.)
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -32,32 +34,34 @@
 
 namespace attn {
 
-constexpr int HD = 256, NQH = 8, KCH = 64, THREADS = 320;
-constexpr int K_BYTES = KCH * HD * 2;                         // four 64-dim segments of [64 keys x 128 B]
-constexpr int MAX_STG = 3;                                    // key / value stages
-constexpr int MERGE_COLS = HD + 2;                            // FP32 columns of a part: the accumulator, maximum, sum
-constexpr int SMEM_LIMIT = 226 * 1024;                        // dynamic shared memory without the alignment slack
-constexpr int TM_O = 0, TM_S = 256, TM_COLS = 512;            // TMEM columns: O [128 x 256], two S buffers [128 x 64]
-constexpr int MASK_WORDS = 130;                               // validity bits of up to 4096 prefix tokens + the suffix
-constexpr float RESCALE = 5.0f;
-// Shared memory of a tile of `rows` query rows: Q as four 64-dim blocks [rows x 128 B], two P buffers [rows x 64 keys], then
-// the key and the value stages.
-__host__ __device__ constexpr int stages_for(int rows) {
-  return (SMEM_LIMIT - 4 * rows * 128 - 2 * rows * 128) / (2 * K_BYTES) < MAX_STG ? (SMEM_LIMIT - 6 * rows * 128) / (2 * K_BYTES) : MAX_STG;
+constexpr int HD = 256, NQH = 8, KCH = 128, THREADS = 320, SOFTMAX = 256;
+constexpr int UNIT = 32 * 1024;                               // ring unit: 128 keys x 128 dims of K or 64 keys x 256 dims of V
+constexpr int SEG = KCH * 128;                                // one 64-dim block of a K unit
+constexpr int MASK_WORDS = 136;                               // validity bits of up to 4096 prefix tokens + the suffix
+constexpr float RESCALE = 7.5f, RESCALE_LOG = 5.0f;           // of exponents to the base 2 / e: 5 log2 e < 7.5, a moved reference satisfies the bound
+// Shared memory of a tile of N query rows: Q as four 64-dim blocks [N x 128 B], P as [128 keys x 64 query rows] segments, the ring.
+__host__ __device__ constexpr int p_bytes(int n) { return (n > 64 ? 2 : 1) * KCH * 128; }
+__host__ __device__ constexpr int units_for(int n) {
+  return (226 * 1024 - 512 * n - p_bytes(n)) / UNIT < 6 ? (226 * 1024 - 512 * n - p_bytes(n)) / UNIT : 6;
 }
-__host__ __device__ constexpr int smem_for(int rows) { return 6 * rows * 128 + 2 * stages_for(rows) * K_BYTES + 1024; }
-static_assert(stages_for(128) == 2 && smem_for(128) + 2048 <= 227 * 1024 && stages_for(40) == 3, "attention shared memory");
+__host__ __device__ constexpr int smem_for(int n) { return 512 * n + p_bytes(n) + units_for(n) * UNIT + 1024; }
+static_assert(units_for(16) == 6 && units_for(64) == 5 && units_for(112) == 4 && smem_for(32) + 2048 <= 227 * 1024 && smem_for(112) + 4096 <= 227 * 1024, "attention shared memory");
+// FP32 words that a CTA of a split tile leaves behind.
+__host__ __device__ constexpr int part_floats(int n) { return n * (HD + 2); }
+
 struct Args {
-  CUtensorMap q;                           // [tokens x 8 rows, 256 dims], box {64, 8 x tok_tile}
-  CUtensorMap pk, pk_tail, pv, pv_tail;    // prefix keys / values {64 dims, page tokens, 4, layers, pages}, box {64, 64, 4, 1, 1}
-  CUtensorMap o;                           // the output as [observations][rows per observation][256], box {64, rows, 1}
-  CUtensorMap sk, sv;                      // suffix keys / values {64, tokens, 4, observations}, box {64, 64, 4, 1}
+  CUtensorMap q;                           // [tokens x 8 rows, 256 dims], box {64, N}
+  CUtensorMap pk, pk_tail, pv, pv_tail;    // prefix keys / values {64 dims, page tokens, 4, layers, pages}; K: box {64, k_rows, k_rows / 64,
+                                           // 1, 1}, V: box {64, 64, 4, 1, 1}; *_tail: the same, cut at the last valid token of a last page
+  CUtensorMap sk, sv;                      // suffix keys / values {64, tokens, 4, 1, observations}, box {64, 128, 2, 1, 1} and {64, 64, 4, 1, 1}
+  CUtensorMap o;                           // the output as [observations][rows per observation][256], box {64, N, 1}
   const int* page_table;                   // [observation][pages_per_obs], or null: page = observation
   const uint8_t* valid;                    // [observation][prefix]
   __nv_bfloat16* out;                      // [tokens, 2048]
-  float* merge;                            // splits > 1: [tile][split][MERGE_COLS][rows]
-  int pages_per_obs, page_tokens, prefix, suffix;      // suffix: keys behind the prefix (0: none)
-  int obs_tokens, tok_tile, tiles, splits, layer, early, stages;
+  float* merge;                            // splits > 1: [tile][split][part_floats]
+  int pages_per_obs, page_tokens, prefix, suffix;      // suffix: keys behind the prefix (0: none; up to 64)
+  int k_rows;                              // 128: 128 keys of a chunk are one copy; 64: pages of 64 tokens
+  int obs_tokens, tok_tile, tiles, splits, layer, early;
   unsigned int* status;
   long long limit;
 };
@@ -69,149 +73,201 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 __device__ __forceinline__ float lo16(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi16(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// Maximum over the warp.
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
 
-template <int = 0>   // a template, so that only the file that launches it holds its code
+template <int N>     // query rows of a tile
 __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_constant__ Args p) {
+  constexpr int R = N / 2;                                    // query rows per softmax thread
+  constexpr int UNITS = units_for(N), QBLK = N * 128;
+  constexpr int TM_S = 0, TM_O = 2 * N, TM_COLS = N <= 16 ? 64 : N <= 32 ? 128 : N <= 64 ? 256 : 512;    // two S^T buffers, two halves of O^T
+  constexpr float LOG2E = 1.4426950408889634f, SCALE_LOG2E = 0.0625f * LOG2E;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // barriers: q, k_full[3], k_empty[3], v_full[3], v_empty[3], s_full[2], s_empty[2], p_full[2], p_empty[2], o_full
-  __shared__ uint64_t bars[22];
+  // barriers: q, full[6], empty[6], s_full[2], s_empty[2], p_full, p_empty, o_full
+  __shared__ uint64_t bars[20];
   __shared__ uint32_t s_tmem;
   __shared__ uint32_t s_mask[MASK_WORDS];
-  // one value per row exchanged between threads: maxima [chunk parity][half][row] (BF16) during the loop, then sums
-  // [half][row]
-  __shared__ __align__(8) uint8_t s_row[128 * 8];
-  __nv_bfloat16 (*s_max)[2][128] = reinterpret_cast<__nv_bfloat16 (*)[2][128]>(s_row);
-  float (*s_sum)[128] = reinterpret_cast<float (*)[128]>(s_row);
+  __shared__ float s_red[4][N];            // what the four warps of a half exchange: maxima, at the end sums
+  __shared__ __align__(16) float s_m[N], s_mneg[N], s_f[N];   // reference of a row, the same as an exponent's summand, factor of a move / of the result
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x % p.splits, unit = blockIdx.x / p.splits;
   const int ob = unit / p.tiles, tile = unit % p.tiles;
   const int npc = (p.prefix + KCH - 1) / KCH, total = npc + (p.suffix > 0 ? 1 : 0);
   const int cbeg = total * split / p.splits, n = total * (split + 1) / p.splits - cbeg;    // n >= 1: splits <= total
-  const int rows = p.tok_tile * NQH;
   const uint32_t b0 = ptx::smem_u32(bars);
-  const uint32_t q_full = b0, k_full = b0 + 8, k_empty = b0 + 32, v_full = b0 + 56, v_empty = b0 + 80;
-  const uint32_t s_full = b0 + 104, s_empty = b0 + 120, p_full = b0 + 136, p_empty = b0 + 152, o_full = b0 + 168;
-  const uint32_t q_base = ptx::smem_u32(smem), blk = rows * 128;            // one 64-dim block of Q, one P buffer
-  const int stg = p.stages, off_k = 6 * rows * 128;
-  const uint32_t p_base = q_base + 4 * blk, k_base = q_base + off_k, v_base = k_base + stg * K_BYTES;
+  const uint32_t q_full = b0, full = b0 + 8, empty = b0 + 56, s_full = b0 + 104, s_empty = b0 + 120, p_full = b0 + 136, p_empty = b0 + 144,
+                 o_full = b0 + 152;
+  const uint32_t q_base = ptx::smem_u32(smem), p_base = q_base + 4 * QBLK, ring = p_base + p_bytes(N);
   const bool leader = ptx::elect_one();
+
+  // Units of V of this CTA's chunk i, and where its units stand in the ring's order K0 | K1 V0 | K2 V1 | .. | V(n-1).  A suffix
+  // at the end goes behind the values of the chunk before it, which do not depend on the kernel before this one.
+  auto nv = [&](int i) { const int c = cbeg + i; return c < npc ? (p.prefix - c * KCH > 64 ? 2 : 1) : 1; };
+  const bool swapped = n >= 2 && cbeg + n > npc;
+  auto pos_k = [&](int i) { return i == 0 ? 0 : swapped && i == n - 1 ? 4 * i - 2 + nv(i - 1) : 4 * i - 2; };
+  auto pos_v = [&](int i) {
+    if (n == 1) return 2;
+    if (swapped) return i == n - 1 ? pos_k(i) + 2 : i == n - 2 ? 4 * i + 2 : 4 * i + 4;
+    return i == n - 1 ? 4 * i + 2 : 4 * i + 4;
+  };
 
   if (tid == 0) {
     ptx::mbar_init(q_full, 1);
-    for (int i = 0; i < stg; ++i) {
-      ptx::mbar_init(k_full + 8 * i, 1); ptx::mbar_init(k_empty + 8 * i, 1);
-      ptx::mbar_init(v_full + 8 * i, 1); ptx::mbar_init(v_empty + 8 * i, 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(s_full + 8 * i, 1); ptx::mbar_init(s_empty + 8 * i, 256);
-      ptx::mbar_init(p_full + 8 * i, 256); ptx::mbar_init(p_empty + 8 * i, 1);
-    }
+    for (int i = 0; i < UNITS; ++i) { ptx::mbar_init(full + 8 * i, 1); ptx::mbar_init(empty + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { ptx::mbar_init(s_full + 8 * i, 1); ptx::mbar_init(s_empty + 8 * i, SOFTMAX); }
+    ptx::mbar_init(p_full, SOFTMAX);
+    ptx::mbar_init(p_empty, 1);
     ptx::mbar_init(o_full, 1);
     ptx::fence_mbar_init();
     ptx::fence_proxy_async_shared();
   }
   __syncwarp();
-  // one chunk of keys (isv = 0) or values (isv = 1) into its stage
-  auto load_chunk = [&](int i, int slot, int isv) {
-    const int c = cbeg + i;
-    const uint32_t bar = (isv ? v_full : k_full) + 8 * slot, dst = (isv ? v_base : k_base) + slot * K_BYTES;
-    ptx::mbar_expect_tx(bar, K_BYTES);
-    if (c < npc) {
-      // logical page of the chunk -> page of the pool; the last page goes through the map that ends at the last valid row
-      const int lp = p.pages_per_obs == 1 ? 0 : c * KCH / p.page_tokens, row = c * KCH - lp * p.page_tokens;
-      const int page = p.page_table ? __ldg(p.page_table + ob * p.pages_per_obs + lp) : ob;
-      const bool tail = lp == (p.prefix - 1) / p.page_tokens;
-      ptx::tma_load_5d(dst, tail ? (isv ? &p.pv_tail : &p.pk_tail) : (isv ? &p.pv : &p.pk), bar, 0, row, 0, p.layer, page);
-    } else {
-      ptx::tma_load_4d(dst, isv ? &p.sv : &p.sk, bar, 0, 0, 0, ob);
-    }
-  };
-  int early = 0;                           // chunks requested before the dependency is waited for
-  if (warp == 0) {
-    if (p.early) {
-      for (; early < stg && early < n && cbeg + early < npc; ++early)
-        if (leader) { load_chunk(early, early, 0); load_chunk(early, early, 1); }
-    }
-    if (leader) { ptx::prefetch_tensormap(&p.q); ptx::prefetch_tensormap(&p.sk); ptx::prefetch_tensormap(&p.sv); }
-  } else if (warp == 1) {
-    ptx::tmem_alloc(ptx::smem_u32(&s_tmem), TM_COLS);
-    ptx::tmem_relinquish();
-    ptx::grid_dep_launch();                // after the allocation: a later kernel cannot take the columns first
-  } else {
-    // validity bits of this CTA's keys (an input, not an output of the kernel before)
-    for (int w = warp - 2; w < 2 * n; w += 8) {
-      const int t = (cbeg * 2 + w) * 32 + lane, s = t - npc * KCH;
-      const bool ok = s < 0 ? t < p.prefix && p.valid[(size_t)ob * p.prefix + t] != 0 : s < p.suffix;
-      const unsigned bits = __ballot_sync(0xffffffffu, ok);
-      if (lane == 0) s_mask[w] = bits;
-    }
-  }
-  ptx::tc_fence_before();
-  __syncthreads();
-  ptx::tc_fence_after();
-  const uint32_t tmem = s_tmem;
-  ptx::grid_dep_wait();
 
-  // softmax threads: TMEM lanes 32 (warp % 4) .., key half (warps 2..5: keys 0..31 of a chunk, warps 6..9: keys 32..63)
-  const int quad = warp & 3, row = quad * 32 + lane, half = warp >= 6 ? 1 : 0;
-  const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
-  const bool busy = warp >= 2 && quad * 32 < rows;        // a warp whose rows are all beyond the tile only keeps the barriers going
+  // softmax threads: key 32 (warp % 4) + lane of a chunk, query rows [half R, half R + R)
+  const int quad = warp & 3, half = warp >= 6 ? 1 : 0;
   bool ok = true;
-  float m = -1e30f, l = 0.f;
-  constexpr float LOG2E = 1.4426950408889634f;
 
   if (warp == 0) {
     // ---- producer
-    if (leader) {
-      ptx::mbar_expect_tx(q_full, 4 * blk);
-      for (int kb = 0; kb < 4; ++kb)
-        ptx::tma_load_2d(q_base + kb * blk, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
-    }
-    for (int i = early, slot = early % stg, par = (early / stg & 1) ^ 1; i < n; ++i) {
-      if (!ptx::wait_bar(p.status, p.limit, k_empty + 8 * slot, par, 1)) break;
-      if (leader) load_chunk(i, slot, 0);
-      if (!ptx::wait_bar(p.status, p.limit, v_empty + 8 * slot, par, 2)) break;
-      if (leader) load_chunk(i, slot, 1);
-      if (++slot == stg) { slot = 0; par ^= 1; }
-    }
-  } else if (warp == 1) {
-    // ---- MMA issuer
-    const uint32_t idesc_s = ptx::umma_idesc_bf16(128, KCH), idesc_o = ptx::umma_idesc_bf16(128, HD) | ptx::UMMA_B_MN_MAJOR;
-    const uint64_t qdesc = ptx::umma_smem_desc(q_base), kdesc = ptx::umma_smem_desc(k_base);
-    const uint64_t pdesc = ptx::umma_smem_desc(p_base);
-    const uint64_t vdesc = ptx::umma_smem_desc_mn(v_base, KCH * 128);
-    bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, 3);
-    int ks = 0, kpar = 0, vs = 0, vpar = 0;
-    auto issue_s = [&](int i) -> bool {
-      const int slot = i & 1;
-      if (!ptx::wait_bar(p.status, p.limit, k_full + 8 * ks, kpar, 4)) return false;
-      if (!ptx::wait_bar(p.status, p.limit, s_empty + 8 * slot, ((i >> 1) & 1) ^ 1, 5)) return false;
-      ptx::tc_fence_after();
-      if (leader) {
-#pragma unroll
-        for (int kb = 0; kb < 4; ++kb)
-          ptx::umma_bf16_k64(tmem + TM_S + slot * KCH, qdesc + (uint64_t)((kb * blk) >> 4),
-                             kdesc + (uint64_t)((ks * K_BYTES + kb * (KCH * 128)) >> 4), idesc_s, kb ? 1u : 0u, 2, 2);
-        ptx::umma_commit(s_full + 8 * slot);
-        ptx::umma_commit(k_empty + 8 * ks);
+    ptx::bar_arrive(2, THREADS);           // nobody waits for the requests below
+    bool waited = false;
+    int j = 0, slot = 0;                   // unit in the ring's order
+    uint32_t par = 1;
+    auto page_of = [&](int key, int& row, bool& tail) {      // key: first of 64 or 128 keys of a page; beyond the prefix: rows that read as zeros
+      const int last = (p.prefix - 1) / p.page_tokens;
+      int lp = p.pages_per_obs == 1 ? 0 : key / p.page_tokens;
+      row = key - lp * p.page_tokens;
+      if (lp > last) { lp = last; row = p.page_tokens; }
+      tail = lp == last;
+      return p.page_table ? __ldg(p.page_table + ob * p.pages_per_obs + lp) : ob;
+    };
+    auto emit = [&](int i, int isv, int u) {
+      const int c = cbeg + i;
+      if (!waited && (!p.early || j >= UNITS || c >= npc)) {
+        ptx::grid_dep_wait();
+        if (leader) {
+          ptx::mbar_expect_tx(q_full, 4 * QBLK);
+          for (int kb = 0; kb < 4; ++kb)
+            ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
+        }
+        __syncwarp();
+        waited = true;
       }
-      if (++ks == stg) { ks = 0; kpar ^= 1; }
+      if (ok && j >= UNITS) ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1);
+      if (ok && leader) {
+        const uint32_t bar = full + 8 * slot, dst = ring + slot * UNIT;
+        ptx::mbar_expect_tx(bar, UNIT);
+        int row;
+        bool tail;
+        if (c >= npc) {
+          ptx::tma_load_5d(dst, isv ? &p.sv : &p.sk, bar, 0, 0, isv ? 0 : 2 * u, 0, ob);
+        } else if (isv) {
+          const int page = page_of(c * KCH + 64 * u, row, tail);
+          ptx::tma_load_5d(dst, tail ? &p.pv_tail : &p.pv, bar, 0, row, 0, p.layer, page);
+        } else if (p.k_rows == KCH) {
+          const int page = page_of(c * KCH, row, tail);
+          ptx::tma_load_5d(dst, tail ? &p.pk_tail : &p.pk, bar, 0, row, 2 * u, p.layer, page);
+        } else {
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            const int page = page_of(c * KCH + 64 * h, row, tail);
+            ptx::tma_load_5d(dst + h * 64 * 128, tail ? &p.pk_tail : &p.pk, bar, 0, row, 2 * u, p.layer, page);
+            ptx::tma_load_5d(dst + SEG + h * 64 * 128, tail ? &p.pk_tail : &p.pk, bar, 0, row, 2 * u + 1, p.layer, page);
+          }
+        }
+      }
+      __syncwarp();
+      ++j;
+      if (++slot == UNITS) { slot = 0; par ^= 1; }
+    };
+    // groups of units: K0, then (K_i, V_(i-1)) or, a suffix, (V_(i-1), K_i), then V_(n-1)
+#pragma unroll 1
+    for (int g = 0; g < 2 * n; ++g) {
+      const int i = (g + 1) >> 1;                             // groups 2 i - 1 and 2 i are chunk i's keys and the values before it
+      const bool isv = i == n || (g > 0 && ((g & 1) == 0) != (swapped && i == n - 1));
+      const int ch = isv ? i - 1 : i;
+      const int units = isv ? nv(ch) : 2;
+      for (int u = 0; u < units; ++u) emit(ch, isv ? 1 : 0, u);
+    }
+    if (!waited) {                                            // everything fitted the ring
+      ptx::grid_dep_wait();
+      if (leader) {
+        ptx::mbar_expect_tx(q_full, 4 * QBLK);
+        for (int kb = 0; kb < 4; ++kb)
+          ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
+      }
+      __syncwarp();
+    }
+  } else {
+    if (warp == 1) {
+      ptx::tmem_alloc(ptx::smem_u32(&s_tmem), TM_COLS);
+      ptx::tmem_relinquish();
+      ptx::grid_dep_launch();              // after the allocation: a later kernel cannot take the columns first
+      if (leader) { ptx::prefetch_tensormap(&p.q); ptx::prefetch_tensormap(&p.sk); ptx::prefetch_tensormap(&p.sv); }
+    } else {
+      // validity bits of this CTA's keys (an input, not an output of the kernel before)
+      for (int w = warp - 2; w < 4 * n; w += 8) {
+        const int t = (cbeg * 4 + w) * 32 + lane, s = t - npc * KCH;
+        const bool good = s < 0 ? t < p.prefix && p.valid[(size_t)ob * p.prefix + t] != 0 : s < p.suffix;
+        const unsigned bits = __ballot_sync(0xffffffffu, good);
+        if (lane == 0) s_mask[w] = bits;
+      }
+    }
+    ptx::tc_fence_before();
+    ptx::named_bar_sync(2, THREADS);
+    ptx::tc_fence_after();
+  }
+  const uint32_t tmem = s_tmem;            // (not for warp 0)
+
+  if (warp == 1) {
+    // ---- MMA issuer
+    const uint32_t idesc_s = ptx::umma_idesc_bf16(KCH, N), idesc_o = ptx::umma_idesc_bf16(128, N) | ptx::UMMA_A_MN_MAJOR | ptx::UMMA_B_MN_MAJOR;
+    const uint64_t qdesc = ptx::umma_smem_desc(q_base), kdesc = ptx::umma_smem_desc(ring);
+    const uint64_t pdesc = ptx::umma_smem_desc_mn(p_base, SEG), vdesc = ptx::umma_smem_desc_mn(ring, 64 * 128);
+    bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, 3);
+    auto issue_s = [&](int i) -> bool {
+      const int buf = i & 1, at = pos_k(i);
+      if (!ptx::wait_bar(p.status, p.limit, s_empty + 8 * buf, ((i >> 1) & 1) ^ 1, 5)) return false;
+#pragma unroll 1
+      for (int u = 0; u < 2; ++u) {
+        const int slot = (at + u) % UNITS;
+        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, ((at + u) / UNITS) & 1, 4)) return false;
+        ptx::tc_fence_after();
+        if (leader) {
+          const uint64_t kd = kdesc + (uint64_t)((slot * UNIT) >> 4), qd = qdesc + (uint64_t)((2 * u * QBLK) >> 4);
+          ptx::umma_bf16_k64(tmem + TM_S + buf * N, kd, qd, idesc_s, u ? 1u : 0u, 2, 2);
+          ptx::umma_bf16_k64(tmem + TM_S + buf * N, kd + (SEG >> 4), qd + (QBLK >> 4), idesc_s, 1u, 2, 2);
+          ptx::umma_commit(empty + 8 * slot);
+          if (u == 1) ptx::umma_commit(s_full + 8 * buf);
+        }
+        __syncwarp();
+      }
       return true;
     };
     auto issue_pv = [&](int i) -> bool {
-      const int slot = i & 1;
-      if (!ptx::wait_bar(p.status, p.limit, v_full + 8 * vs, vpar, 6)) return false;
-      if (!ptx::wait_bar(p.status, p.limit, p_full + 8 * slot, (i >> 1) & 1, 7)) return false;
-      ptx::tc_fence_after();
-      if (leader) {
-        // 16 keys per MMA: 32 bytes further in P's swizzled rows, 16 rows of 128 B further in V
-        ptx::umma_bf16_k64(tmem + TM_O, pdesc + (uint64_t)((slot * blk) >> 4), vdesc + (uint64_t)((vs * K_BYTES) >> 4),
-                           idesc_o, i ? 1u : 0u, 2, 16 * 128 / 16);
-        ptx::umma_commit(p_empty + 8 * slot);
-        ptx::umma_commit(v_empty + 8 * vs);
+      const int at = pos_v(i), units = nv(i);
+      if (!ptx::wait_bar(p.status, p.limit, p_full, i & 1, 7)) return false;
+#pragma unroll 1
+      for (int u = 0; u < units; ++u) {
+        const int slot = (at + u) % UNITS;
+        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, ((at + u) / UNITS) & 1, 6)) return false;
+        ptx::tc_fence_after();
+        if (leader) {
+          // 16 keys per MMA: 16 rows of 128 B further in V and in P
+          const uint64_t vd = vdesc + (uint64_t)((slot * UNIT) >> 4), pd = pdesc + (uint64_t)((u * 64 * 128) >> 4);
+          const uint32_t acc = i || u ? 1u : 0u;
+          ptx::umma_bf16_k64(tmem + TM_O, vd, pd, idesc_o, acc, 128, 128);
+          ptx::umma_bf16_k64(tmem + TM_O + N, vd + ((2 * 64 * 128) >> 4), pd, idesc_o, acc, 128, 128);
+          ptx::umma_commit(empty + 8 * slot);
+          if (u == units - 1) ptx::umma_commit(p_empty);
+        }
+        __syncwarp();
       }
-      if (++vs == stg) { vs = 0; vpar ^= 1; }
       return true;
     };
     for (int i = 0; go && i < n; ++i) {
@@ -220,191 +276,214 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     }
     if (go) go = issue_pv(n - 1);
     if (go && leader) ptx::umma_commit(o_full);
-  } else {
-    // ---- softmax threads.  A wait that gives up does not end the loop: the other warp of the quadrant counts on this one at
-    // their named barrier, and every further wait returns at once
-    constexpr float SCALE_LOG2E = 0.0625f * LOG2E;
-    const uint32_t prow = p_base + row * 128, psw = row & 7;
+    __syncwarp();
+  } else if (warp >= 2) {
+    // ---- softmax threads.  A wait that gives up does not end the loop: the other warps count on this one at their named
+    // barriers, and every further wait returns at once
+    const int et = tid - 64, r0 = half * R;
+    const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + r0;
+    float l[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) l[r] = 0.f;
+#pragma unroll 1
     for (int i = 0; i < n; ++i) {
-      const int slot = i & 1;
-      ok &= ptx::wait_bar(p.status, p.limit, s_full + 8 * slot, (i >> 1) & 1, 8);
+      const int buf = i & 1;
+      ok &= ptx::wait_bar(p.status, p.limit, s_full + 8 * buf, (i >> 1) & 1, 8);
       ptx::tc_fence_after();
-      if (!busy) {
-        ptx::tc_fence_before();
-        ptx::mbar_arrive(s_empty + 8 * slot);
-        ptx::mbar_arrive(p_full + 8 * slot);
-        continue;
-      }
-      // Both passes over the row's 32 scores go eight columns at a time in loops that stay loops (the scores are read from
-      // TMEM twice): an instruction that runs once costs several cycles to fetch.
-      const uint32_t mask = s_mask[2 * i + half], scol = trow + TM_S + slot * KCH + half * 32;
-      // maximum of the raw scores: rounding to BF16 and the scale are monotonic, so they are applied to it once
-      float mine = -INFINITY;
+      const bool key = s_mask[4 * i + quad] >> lane & 1;      // this thread's key counts
+      const uint32_t scol = trow + TM_S + buf * N;
+      // the key's line of P: piece c (8 query rows) at c ^ (key & 7), 64 query rows per segment
+      const uint32_t line = p_base + (quad * 32 + lane) * 128, psw = lane & 7;
 #pragma unroll 1
-      for (int j0 = 0; j0 < 32; j0 += 8) {
-        uint32_t r[8];
-        ptx::tmem_ld_32x8(scol + j0, r);
-        ptx::tmem_wait_ld();
+      for (int tries = i > 0 ? 1 : 0;; ++tries) {             // 0: no reference yet
+        if (tries > 0) {
+          // p = exp(bf16(s) / 16 - m) as one FMA and one ex2 per score; the vote looks at the exponents
+          float t[R], top = -INFINITY;
+          {
+            uint32_t x[R];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (mask >> (j0 + j) & 1) mine = fmaxf(mine, __uint_as_float(r[j]));
-      }
-      s_max[slot][half][row] = __float2bfloat16_rn(mine);
-      ptx::named_bar_sync(1 + quad, 64);                  // the row's other half is in the other warp of this quadrant
-      const float cm = fmaxf(rb(mine), __bfloat162float(s_max[slot][half ^ 1][row])) * 0.0625f;
-      if (i == 0) {
-        m = fmaxf(cm, -1e30f);
-      } else if (__any_sync(0xffffffffu, cm > m + RESCALE)) {
-        // rare (and the same decision in both warps of the quadrant): move the reference of the rows that need it and
-        // rescale this half of what they have accumulated
-        const float mn = cm > m + RESCALE ? cm : m, f = ptx::ex2_approx((m - mn) * LOG2E);
-        m = mn;
-        l *= f;
-        ok &= ptx::wait_bar(p.status, p.limit, p_empty + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1, 9);
-        ptx::tc_fence_after();
+            for (int c = 0; c < R; c += 8) ptx::tmem_ld_32x8(scol + c, *reinterpret_cast<uint32_t(*)[8]>(&x[c]));
+            ptx::tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < R; c += 4) {
+              const float4 mn = *reinterpret_cast<const float4*>(&s_mneg[r0 + c]);
+              const uint32_t x0 = pack2(__uint_as_float(x[c]), __uint_as_float(x[c + 1])), x1 = pack2(__uint_as_float(x[c + 2]), __uint_as_float(x[c + 3]));
+              t[c] = fmaf(lo16(x0), SCALE_LOG2E, mn.x); t[c + 1] = fmaf(hi16(x0), SCALE_LOG2E, mn.y);
+              t[c + 2] = fmaf(lo16(x1), SCALE_LOG2E, mn.z); t[c + 3] = fmaf(hi16(x1), SCALE_LOG2E, mn.w);
+              top = fmaxf(fmaxf(top, fmaxf(t[c], t[c + 1])), fmaxf(t[c + 2], t[c + 3]));
+            }
+          }
+          if (i == 0 || !ptx::named_bar_or(1, SOFTMAX, key && top > RESCALE) || tries > 2) {
+            uint32_t pk[R / 2];
+#pragma unroll
+            for (int r = 0; r < R; r += 2) {
+              const float e0 = key ? ptx::ex2_approx(t[r]) : 0.f, e1 = key ? ptx::ex2_approx(t[r + 1]) : 0.f;
+              l[r] += e0;
+              l[r + 1] += e1;
+              pk[r / 2] = pack2(e0, e1);
+            }
+            // the P buffer is free once the P V of the chunk before has read it
+            if (i > 0) ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, 10);
+#pragma unroll
+            for (int c = 0; c < R; c += 8) {
+              const uint32_t piece = (uint32_t)(r0 + c) >> 3;
+              ptx::st_shared_v4(line + (piece >> 3) * SEG + (((piece & 7) ^ psw) << 4), pk[c / 2], pk[c / 2 + 1], pk[c / 2 + 2], pk[c / 2 + 3]);
+            }
+            break;
+          }
+        }
+        // rare, but for the first chunk: find the maximum (of the raw scores: rounding to BF16 and the scale are monotonic)
 #pragma unroll 1
-        for (int c0 = half * (HD / 2); c0 < (half + 1) * (HD / 2); c0 += 32) {
-          uint32_t o[32];
-          ptx::tmem_ld_32x32(trow + TM_O + c0, o);
+        for (int c = 0; c < R; c += 8) {
+          uint32_t s[8];
+          ptx::tmem_ld_32x8(scol + c, s);
           ptx::tmem_wait_ld();
+          float mx = 0.f;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-          ptx::tmem_st_32x32(trow + TM_O + c0, o);
+          for (int k = 0; k < 8; ++k) {
+            const float v = warp_max(key ? __uint_as_float(s[k]) : -INFINITY);
+            if (lane == k) mx = v;
+          }
+          if (lane < 8) s_red[quad][r0 + c + lane] = mx;
+          __syncwarp();
         }
-        ptx::tmem_wait_st();
-        ptx::tc_fence_before();
-      }
-      // the P buffer is free once the P V of chunk i - 2 has read it
-      ok &= ptx::wait_bar(p.status, p.limit, p_empty + 8 * slot, ((i >> 1) & 1) ^ 1, 10);
-      // p = exp(bf16(s) / 16 - m) as one FMA and one ex2 per score; masked ones are replaced afterwards
-      const float mneg = -m * LOG2E;
-      const uint32_t dst = prow + slot * blk;
+        ptx::named_bar_sync(1, SOFTMAX);
+        if (et < N) {
+          const float cm = rb(fmaxf(fmaxf(s_red[0][et], s_red[1][et]), fmaxf(s_red[2][et], s_red[3][et]))) * 0.0625f;
+          float m = i == 0 ? fmaxf(cm, -1e30f) : s_m[et], f = 1.f;
+          if (i > 0 && cm > m + RESCALE_LOG) { f = ptx::ex2_approx((m - cm) * LOG2E); m = cm; }
+          s_m[et] = m;
+          s_mneg[et] = -m * LOG2E;
+          s_f[et] = f;
+        }
+        ptx::named_bar_sync(1, SOFTMAX);
+        if (i > 0) {
+          // rescale what has been accumulated
+#pragma unroll
+          for (int r = 0; r < R; ++r) l[r] *= s_f[r0 + r];
+          ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, 9);
+          ptx::tc_fence_after();
 #pragma unroll 1
-      for (int j0 = 0; j0 < 32; j0 += 8) {
-        uint32_t r[8], pk[4];
-        ptx::tmem_ld_32x8(scol + j0, r);
-        ptx::tmem_wait_ld();
-        const uint32_t mk = mask >> j0;
-        float ls[2] = {0.f, 0.f};
+          for (int c = 0; c < 2 * R; c += 8) {
+            const int row = c < R ? c : c - R;
+            const uint32_t at = trow + TM_O + (c < R ? 0 : N) + row;
+            uint32_t o[8];
+            ptx::tmem_ld_32x8(at, o);
+            ptx::tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          const uint32_t s0 = pack2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-          float a = ptx::ex2_approx(fmaf(lo16(s0), SCALE_LOG2E, mneg)), b = ptx::ex2_approx(fmaf(hi16(s0), SCALE_LOG2E, mneg));
-          a = mk & (1u << j) ? a : 0.f;
-          b = mk & (2u << j) ? b : 0.f;
-          ls[0] += a;
-          ls[1] += b;
-          pk[j >> 1] = pack2(a, b);
+            for (int k = 0; k < 8; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * s_f[r0 + row + k]);
+            ptx::tmem_st_32x8(at, o);
+          }
+          ptx::tmem_wait_st();
         }
-        l += ls[0] + ls[1];
-        // 16-byte piece c of the row sits at piece c ^ (row & 7) of its 128-byte line
-        if (row < rows) ptx::st_shared_v4(dst + (((uint32_t)(half * 4 + (j0 >> 3)) ^ psw) << 4), pk[0], pk[1], pk[2], pk[3]);
-        __syncwarp();
       }
-      ptx::tc_fence_before();
-      ptx::mbar_arrive(s_empty + 8 * slot);
       __syncwarp();
-      ptx::fence_proxy_async_shared();
       ptx::tc_fence_before();
-      ptx::mbar_arrive(p_full + 8 * slot);
+      ptx::mbar_arrive(s_empty + 8 * buf);
+      ptx::fence_proxy_async_shared();
+      ptx::mbar_arrive(p_full);
     }
+    // the rows' sums over all keys, while the last P V runs
+    ptx::named_bar_sync(1, SOFTMAX);                          // (s_red may still be read)
+#pragma unroll
+    for (int c = 0; c < R; c += 8) {
+      float mine = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float v = l[c + k];
+#pragma unroll
+        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        if (lane == k) mine = v;
+      }
+      if (lane < 8) s_red[quad][r0 + c + lane] = mine;
+    }
+    __syncwarp();
+    ptx::named_bar_sync(1, SOFTMAX);
+    float* part = p.merge + (size_t)(unit * p.splits + split) * part_floats(N);
+    if (et < N) {
+      const float sum = (s_red[0][et] + s_red[1][et]) + (s_red[2][et] + s_red[3][et]);
+      if (p.splits == 1) s_f[et] = 1.0f / sum;
+      else __stcg(reinterpret_cast<float2*>(part + N * HD) + et, make_float2(s_m[et], sum));
+    }
+    ptx::named_bar_sync(1, SOFTMAX);
     ok &= ptx::wait_bar(p.status, p.limit, o_full, 0, 11);
     ptx::tc_fence_after();
-  }
-  __syncthreads();
-  if (warp >= 2) s_sum[half][row] = l;
-  __syncthreads();
-  if (warp >= 2) l += s_sum[half ^ 1][row];               // both halves of the row's sum
-  __syncthreads();
 
-  // ---- O / l -> BF16: row = token_local * 8 + head, so the tile's rows are one contiguous block of [tokens, 2048].  They leave
-  // through shared memory by tiled copies (which clip what lies beyond the observation's tokens)
-  const int left = p.obs_tokens - tile * p.tok_tile, out_rows = (left < p.tok_tile ? left : p.tok_tile) * NQH;
-  uint4* base = reinterpret_cast<uint4*>(p.out + (size_t)(ob * p.obs_tokens + tile * p.tok_tile) * NQH * HD);
-  const int c_half = half * (HD / 2);
-  if (p.splits == 1) {
-    const uint32_t stage = q_base;                        // four swizzled 64-dim blocks, over Q (every MMA has completed)
-    if (busy) {
-      const float il = 1.0f / l;
+    // ---- O^T / l -> BF16 [row][256] (row = token_local * 8 + head: the tile's rows are one contiguous block of [tokens, 2048]).
+    // They leave through shared memory by tiled copies, which clip what lies beyond the observation's tokens
+    if (p.splits == 1) {
+      // four swizzled 64-dim blocks, over Q (every MMA has completed)
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD / 2; c0 += 16) {
-        uint32_t r[16];
-        ptx::tmem_ld_32x16(trow + TM_O + c_half + c0, r);
+      for (int c = 0; c < 2 * R; c += 8) {
+        const int d = c < R ? 0 : 1, row = r0 + (d ? c - R : c);
+        uint32_t o[8];
+        ptx::tmem_ld_32x8(trow + TM_O + d * N + (row - r0), o);
         ptx::tmem_wait_ld();
-        const int ch = (c_half + c0) >> 3;                // 16-byte piece of the row
-        const uint32_t line = stage + (ch >> 3) * blk + row * 128;
-        if (row < rows)
+        const uint32_t blk = q_base + (2 * d + (quad >> 1)) * QBLK, piece = (quad & 1) * 4 + (lane >> 3);
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
-            ptx::st_shared_v4(line + ((((uint32_t)ch + j) & 7) ^ (row & 7)) * 16,
-                              pack2(__uint_as_float(r[8 * j]) * il, __uint_as_float(r[8 * j + 1]) * il),
-                              pack2(__uint_as_float(r[8 * j + 2]) * il, __uint_as_float(r[8 * j + 3]) * il),
-                              pack2(__uint_as_float(r[8 * j + 4]) * il, __uint_as_float(r[8 * j + 5]) * il),
-                              pack2(__uint_as_float(r[8 * j + 6]) * il, __uint_as_float(r[8 * j + 7]) * il));
-        __syncwarp();
+        for (int k = 0; k < 8; ++k) {
+          const __nv_bfloat16 v = __float2bfloat16_rn(__uint_as_float(o[k]) * s_f[row + k]);
+          // (rows come in groups of eight: row & 7 = k)
+          ptx::st_shared_u16(blk + (row + k) * 128 + ((piece ^ k) << 4) + (lane & 7) * 2, __bfloat16_as_ushort(v));
+        }
       }
       ptx::tc_fence_before();
       ptx::fence_proxy_async_shared();
-    }
-    __syncthreads();
-    if (tid == 64 && ok) {
+      ptx::named_bar_sync(1, SOFTMAX);
+      if (et == 0 && ok) {
 #pragma unroll 1
-      for (int kb = 0; kb < 4; ++kb) ptx::tma_store_3d(&p.o, stage + kb * blk, kb * 64, tile * rows, ob);
-      ptx::bulk_commit();
-      ptx::bulk_wait_read();
-    }
-  } else {
-    const size_t pstride = (size_t)MERGE_COLS * rows;
-    float* parts = p.merge + (size_t)unit * p.splits * pstride;
-    if (busy) {
-      float* mine = parts + split * pstride + row;
-#pragma unroll 1
-      for (int c0 = c_half; c0 < c_half + HD / 2; c0 += 32) {
-        uint32_t r[32];
-        ptx::tmem_ld_32x32(trow + TM_O + c0, r);
-        ptx::tmem_wait_ld();
-        if (row < rows)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) __stcg(mine + (c0 + j) * rows, __uint_as_float(r[j]));
-        __syncwarp();
+        for (int kb = 0; kb < 4; ++kb) ptx::tma_store_3d(&p.o, q_base + kb * QBLK, kb * 64, tile * N, ob);
+        ptx::bulk_commit();
+        ptx::bulk_wait_read();
       }
-      if (row < rows) __stcg(mine + (HD + half) * rows, half ? l : m);
       __syncwarp();
-      ptx::tc_fence_before();
-    }
-    ptx::cluster_sync();                                  // the parts of every CTA of the tile are in memory
-    // this rank's 256 / splits columns (splits is 2, 4 or 8): a thread takes eight columns of a row, a warp 32 rows
-    const int nc = (HD / 8) / p.splits, blocks = (out_rows + 31) >> 5;
+    } else {
 #pragma unroll 1
-    for (int i = warp; i < blocks * nc; i += THREADS / 32) {
-      const int rr = (i / nc) * 32 + lane, c = split * nc + i % nc;
-      if (rr >= out_rows) continue;
-      const float* q = parts + rr;
-      float M = -1e30f, L = 0.f, a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-      for (int s = 0; s < p.splits; s += 2) {             // two parts at a time: 20 loads in flight
-        float v[2][8], pm[2], pl[2];
+      for (int c = 0; c < 2 * R; c += 8) {
+        const int d = c < R ? 0 : 1, row = r0 + (d ? c - R : c);
+        uint32_t o[8];
+        ptx::tmem_ld_32x8(trow + TM_O + d * N + (row - r0), o);
+        ptx::tmem_wait_ld();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float* qs = q + (s + h) * pstride;
-          pm[h] = __ldcg(qs + HD * rows);
-          pl[h] = __ldcg(qs + (HD + 1) * rows);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[h][j] = __ldcg(qs + (c * 8 + j) * rows);
-        }
-        const float mn = fmaxf(M, fmaxf(pm[0], pm[1])), g = ptx::ex2_approx((M - mn) * LOG2E);
-        const float f0 = ptx::ex2_approx((pm[0] - mn) * LOG2E), f1 = ptx::ex2_approx((pm[1] - mn) * LOG2E);
-        M = mn;
-        L = L * g + (pl[0] * f0 + pl[1] * f1);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = a[j] * g + (v[0][j] * f0 + v[1][j] * f1);
+        for (int k = 0; k < 8; ++k) __stcg(part + (row + k) * HD + d * 128 + quad * 32 + lane, __uint_as_float(o[k]));
       }
-      const float il = 1.0f / L;
-      base[rr * (HD / 8) + c] = make_uint4(pack2(a[0] * il, a[1] * il), pack2(a[2] * il, a[3] * il), pack2(a[4] * il, a[5] * il),
-                                           pack2(a[6] * il, a[7] * il));
+      ptx::tc_fence_before();
     }
   }
   __syncthreads();
+  if (p.splits > 1) {
+    ptx::cluster_sync();                                      // the parts of every CTA of the tile are in memory
+    const int left = p.obs_tokens - tile * p.tok_tile, out_rows = (left < p.tok_tile ? left : p.tok_tile) * NQH;
+    uint4* base = reinterpret_cast<uint4*>(p.out + (size_t)(ob * p.obs_tokens + tile * p.tok_tile) * NQH * HD);
+    // a warp takes a row of this rank's, a lane eight dims
+    for (int row = split * (N / p.splits) + warp; row < (split + 1) * (N / p.splits) && row < out_rows; row += THREADS / 32) {
+      const float* q = p.merge + (size_t)unit * p.splits * part_floats(N);
+      float M = -1e30f, L = 0.f, a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int s = 0; s < p.splits; s += 2) {                 // two parts at a time
+        float4 x[2], y[2];
+        float2 ml[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float* qs = q + (s + h) * part_floats(N);
+          ml[h] = __ldcg(reinterpret_cast<const float2*>(qs + N * HD) + row);
+          x[h] = __ldcg(reinterpret_cast<const float4*>(qs + row * HD + lane * 8));
+          y[h] = __ldcg(reinterpret_cast<const float4*>(qs + row * HD + lane * 8) + 1);
+        }
+        const float mn = fmaxf(M, fmaxf(ml[0].x, ml[1].x)), g = ptx::ex2_approx((M - mn) * LOG2E);
+        const float f0 = ptx::ex2_approx((ml[0].x - mn) * LOG2E), f1 = ptx::ex2_approx((ml[1].x - mn) * LOG2E);
+        M = mn;
+        L = L * g + (ml[0].y * f0 + ml[1].y * f1);
+        a[0] = a[0] * g + (x[0].x * f0 + x[1].x * f1); a[1] = a[1] * g + (x[0].y * f0 + x[1].y * f1);
+        a[2] = a[2] * g + (x[0].z * f0 + x[1].z * f1); a[3] = a[3] * g + (x[0].w * f0 + x[1].w * f1);
+        a[4] = a[4] * g + (y[0].x * f0 + y[1].x * f1); a[5] = a[5] * g + (y[0].y * f0 + y[1].y * f1);
+        a[6] = a[6] * g + (y[0].z * f0 + y[1].z * f1); a[7] = a[7] * g + (y[0].w * f0 + y[1].w * f1);
+      }
+      const float il = 1.0f / L;
+      base[row * (HD / 8) + lane] = make_uint4(pack2(a[0] * il, a[1] * il), pack2(a[2] * il, a[3] * il), pack2(a[4] * il, a[5] * il),
+                                               pack2(a[6] * il, a[7] * il));
+    }
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, TM_COLS);

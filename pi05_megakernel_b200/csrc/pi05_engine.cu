@@ -127,7 +127,8 @@ struct pi05_engine {
   int batch = 1;
   int row_groups = 1;
   int key_groups = 1;
-  int pages_per_obs = 1, page_tokens = 1;
+  int pages_per_obs = 1, page_tokens = 1, num_pages = 1;
+  long long kv_strides[3] = {0, 0, 0};      // prefix cache: tokens, layers, pages
   bool clustered = false;        // launched as clusters of two CTAs: consecutive blocks share a TPC
   bool bound = false;
   const void* inputs[PI05_NUM_INPUTS] = {};
@@ -520,7 +521,7 @@ bool uses_graphs(const pi05_engine* h) {
   pi05_tuning d;
   default_tuning(&d);
   d.poll_ns = h->tune.poll_ns;
-  return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0 && (h->batch > 1 || h->prefix <= 192 || h->prefix > 384);
+  return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0 && (h->batch > 1 || h->prefix <= 192 || h->prefix > 384 || getenv("PI05_G"));
 }
 
 int build_graphs(pi05_engine* h, int n_steps, int n_layers) {
@@ -537,7 +538,8 @@ int build_graphs(pi05_engine* h, int n_steps, int n_layers) {
   s.h = region_ptr<__nv_bfloat16>(h, "h"); s.an = region_ptr<__nv_bfloat16>(h, "an_attn");
   s.q = region_ptr<__nv_bfloat16>(h, "q"); s.k = region_ptr<__nv_bfloat16>(h, "k"); s.v = region_ptr<__nv_bfloat16>(h, "v");
   s.attn = region_ptr<__nv_bfloat16>(h, "attn"); s.act = region_ptr<__nv_bfloat16>(h, "act");
-  s.maps = &h->maps;
+  s.pool_k = h->inputs[22]; s.pool_v = h->inputs[23];
+  s.token_stride = h->kv_strides[0]; s.layer_stride = h->kv_strides[1]; s.page_stride = h->kv_strides[2]; s.num_pages = h->num_pages;
   s.page_table = region_ptr<int>(h, "page_table");
   s.pages_per_obs = h->pages_per_obs; s.page_tokens = h->page_tokens;
   s.wait_limit = h->wait_limit;
@@ -731,6 +733,8 @@ int pi05_bind_view(pi05_handle_t h, const void* const inputs[PI05_NUM_INPUTS], c
   h->inputs[22] = kv->k; h->inputs[23] = kv->v;
   h->pages_per_obs = kv->pages_per_obs;
   h->page_tokens = kv->page_tokens;
+  h->num_pages = kv->num_pages;
+  h->kv_strides[0] = kv->token_stride; h->kv_strides[1] = kv->layer_stride; h->kv_strides[2] = kv->page_stride;
   h->actions = actions;
   h->ws = static_cast<uint8_t*>(workspace);
   h->prefix = prefix_len;

@@ -99,12 +99,13 @@ bool map_out(CUtensorMap* m, const void* base, bool f32, uint64_t d0, uint64_t d
              CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers) {
+bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, uint64_t pages, uint64_t token_stride,
+            uint64_t layer_stride, uint64_t page_stride, uint32_t box_tokens, uint32_t box_blocks) {
   EncodeTiledFn enc = encoder();
   if (!enc) return false;
-  cuuint64_t dims[5] = {64, tokens, 4, layers, 1};
-  cuuint64_t strides[4] = {256 * 2, 64 * 2, tokens * 256 * 2, layers * tokens * 256 * 2};
-  cuuint32_t box[5] = {64, 64, 4, 1, 1};
+  cuuint64_t dims[5] = {64, tokens, 4, layers, pages};
+  cuuint64_t strides[4] = {token_stride * 2, 64 * 2, layer_stride * 2, page_stride * 2};
+  cuuint32_t box[5] = {64, box_tokens, box_blocks, 1, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -187,10 +188,19 @@ cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream) {
   return launch_chained(cut->kernel, grid, gemm::THREADS_G, g.smem, stream, g.pair ? 2 : 1, p);
 }
 
+namespace {
+typedef void (*AttentionKernel)(const attn::Args);
+struct Tile { int rows; AttentionKernel kernel; };
+const Tile kTiles[] = {{16, attn::attention_kernel<16>}, {32, attn::attention_kernel<32>}, {48, attn::attention_kernel<48>},
+                       {64, attn::attention_kernel<64>}, {112, attn::attention_kernel<112>}};
+}  // namespace
+
 cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream) {
   const int rows = p.tok_tile * NQH;
-  p.stages = attn::stages_for(rows);
-  return launch_chained(attn::attention_kernel<0>, observations * p.tiles * p.splits, attn::THREADS, attn::smem_for(rows), stream, p.splits, p);
+  for (const Tile& t : kTiles)
+    if (t.rows == rows)
+      return launch_chained(t.kernel, observations * p.tiles * p.splits, attn::THREADS, attn::smem_for(rows), stream, p.splits, p);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t chain_opt_in(const void* kernel, int smem) {
@@ -203,7 +213,9 @@ cudaError_t chain_opt_in(const void* kernel, int smem) {
 cudaError_t ops_opt_in(int device) {
   static bool done[64] = {};
   if (device < 64 && done[device]) return cudaSuccess;
-  cudaError_t e = chain_opt_in((const void*)attn::attention_kernel<0>, 225 * 1024);
+  cudaError_t e = cudaSuccess;
+  for (const Tile& t : kTiles)
+    if (e == cudaSuccess) e = chain_opt_in((const void*)t.kernel, attn::smem_for(t.rows));
   for (const Cut& c : kCuts)
     if (e == cudaSuccess) e = chain_opt_in((const void*)c.kernel, 222 * 1024);
   if (e == cudaSuccess && device < 64) done[device] = true;

@@ -41,8 +41,10 @@ bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uin
 // A dense tensor of two (d2 = 0) or three dimensions, innermost first, of BF16 or FP32 elements, box {box_bytes, box_rows, 1} with
 // the swizzle of that many bytes: the destination of a tiled store.
 bool map_out(CUtensorMap* m, const void* base, bool f32, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_bytes, uint32_t box_rows);
-// Keys or values as the attention's tiled copies read them: {64 dims, tokens, 4 segments, layers, 1} of a dense [layers][tokens][256].
-bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers);
+// Keys or values as the attention's tiled copies read them: {64 dims, tokens, 4 blocks, layers, pages} with strides in elements,
+// box {64, box_tokens, box_blocks, 1, 1}; tokens beyond `tokens` read as zeros.
+bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, uint64_t pages, uint64_t token_stride,
+            uint64_t layer_stride, uint64_t page_stride, uint32_t box_tokens, uint32_t box_blocks);
 
 // How one projection of `tokens` x n features over k is cut.
 struct GemmPlan {

@@ -18,6 +18,7 @@
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
+#include <stdlib.h>
 
 #include <algorithm>
 #include <new>
@@ -182,9 +183,10 @@ PrefillPlan plan_prefill(int sms, int tokens) {
   pl.o = plan_gemm(sms, tokens, pf::H, QD, gemm::EPI_PART, pl.pairs);
   pl.gu = plan_gemm(sms, tokens, 2 * pf::FFN, pf::H, gemm::EPI_GEGLU, pl.pairs);
   pl.down = pl.sk_down ? plan_gemm_sk(sms, tokens, pf::H, pf::FFN) : plan_gemm(sms, tokens, pf::H, pf::FFN, gemm::EPI_PART, 1);
-  // Tiles of 5 tokens (40 query rows) keep three key / value stages; beyond that the tile grows until the CTAs fit the SMs, up to
-  // 16 tokens (128 rows): a CTA's time hardly depends on its rows.
-  pl.tok_tile = std::max(5, std::min(16, (tokens + sms - 1) / sms));
+  pl.tok_tile = 14;
+  for (int t : {8, 6, 4, 2})
+    if ((tokens + t - 1) / t <= sms) pl.tok_tile = t;
+  if (getenv("AT")) pl.tok_tile = atoi(getenv("AT"));
   return pl;
 }
 
@@ -318,14 +320,14 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
                   act_map(&a_dn, act, pf::FFN, pl.down) && weight_map(&wq, LQ, pf::H, QD, pl.qkv) && weight_map(&wk, LK, pf::H, HD, pl.qkv) &&
                   weight_map(&wv, LV, pf::H, HD, pl.qkv) && weight_map(&wo, LO, QD, pf::H, pl.o) && weight_map(&wg, LG, pf::H, pf::FFN, pl.gu) &&
                   weight_map(&wu, LU, pf::H, pf::FFN, pl.gu) && weight_map(&wd, LD, pf::FFN, pf::H, pl.down) &&
-                  map_kv(&ap.pk, K, P, L) &&
-                  map_kv(&ap.pv, V, P, L) &&
+                  map_kv(&ap.pk, K, P, L, 1, HD, (uint64_t)P * HD, L * P * HD, attn::KCH, 2) &&
+                  map_kv(&ap.pv, V, P, L, 1, HD, (uint64_t)P * HD, L * P * HD, 64, 4) &&
                   map_2d(&ap.q, q, HD, (uint64_t)P * NQH, pl.tok_tile * NQH) &&
                   map_out(&ap.o, mixed, false, HD, (uint64_t)P * NQH, 1, 128, pl.tok_tile * NQH);
   if (!ok) { h->last_error = "cuTensorMapEncodeTiled failed"; return PI05_ERR_CUDA; }
   ap.pk_tail = ap.pk; ap.pv_tail = ap.pv; ap.sk = ap.pk; ap.sv = ap.pv;
   ap.valid = static_cast<const uint8_t*>(valid); ap.out = mixed;
-  ap.pages_per_obs = 1; ap.page_tokens = P; ap.prefix = P; ap.obs_tokens = P;
+  ap.pages_per_obs = 1; ap.page_tokens = P; ap.k_rows = attn::KCH; ap.prefix = P; ap.obs_tokens = P;
   ap.tok_tile = pl.tok_tile; ap.tiles = (P + pl.tok_tile - 1) / pl.tok_tile; ap.splits = 1;
   ap.status = status; ap.limit = h->wait_limit;
 

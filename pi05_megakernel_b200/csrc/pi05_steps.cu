@@ -13,6 +13,7 @@
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
+#include <stdlib.h>
 
 #include <algorithm>
 #include <string>
@@ -406,9 +407,11 @@ struct AttnPlan { int tok_tile, tiles, splits; };
 
 AttnPlan plan_attention(int sms, int batch, int prefix) {
   AttnPlan a;
-  // (a merge costs about as much as eight chunks of a CTA of 104 rows, or as two of one that finds all its chunks resident)
-  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1, per_cta = batch <= 3 ? 4 : 8;
-  a.tok_tile = batch <= 3 ? 5 : 13;
+  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1, per_cta = getenv("AP") ? atoi(getenv("AP")) : 5;
+  a.tok_tile = 14;
+  for (int t : {8, 6, 4, 2})
+    if (batch * ((T + t - 1) / t) <= sms) a.tok_tile = t;
+  if (getenv("AT")) a.tok_tile = atoi(getenv("AT"));
   a.tiles = (T + a.tok_tile - 1) / a.tok_tile;
   a.splits = 1;
   while (a.splits < 8 && (chunks + a.splits - 1) / a.splits > per_cta && batch * a.tiles * a.splits * 2 <= sms) a.splits *= 2;
@@ -516,18 +519,28 @@ struct Capture {
     ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits;
     ap.merge = s.part;
     const uint64_t L = NL, M = tokens;
+    // full pages, and the last page of an observation cut at its last valid token; 128 keys are one copy where pages allow it
+    const int tail = s.prefix - (s.prefix - 1) / s.page_tokens * s.page_tokens;
+    ap.k_rows = s.pages_per_obs == 1 || s.page_tokens % attn::KCH == 0 ? attn::KCH : 64;
+    auto keys = [&](CUtensorMap* m, int rows) {
+      return map_kv(m, s.pool_k, rows, L, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, ap.k_rows, ap.k_rows / 64);
+    };
+    auto values = [&](CUtensorMap* m, int rows) {
+      return map_kv(m, s.pool_v, rows, L, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, 64, 4);
+    };
     auto weights = [&](CUtensorMap* m, int which, int k, int rows, const GemmPlan& g) { return map_k(m, s.in[which], k, L * rows, g.w_rows, g.w_kb); };
     if (!(map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
           map_k(&a_dn, s.act, FF, M, pd.arows, pd.ks) && weights(&wq, 8, W, QD, pq) && weights(&wk, 9, W, HD, pq) && weights(&wv, 10, W, HD, pq) &&
           weights(&wo, 11, QD, W, po) && weights(&wg, 12, W, FF, pg) && weights(&wu, 13, W, FF, pg) && weights(&wd, 14, FF, W, pd) &&
           map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH) &&
-          map_out(&ap.o, s.attn, false, HD, (uint64_t)T * NQH, s.batch, 128, ap.tok_tile * NQH))) {
+          map_out(&ap.o, s.attn, false, HD, (uint64_t)T * NQH, s.batch, 128, ap.tok_tile * NQH) && keys(&ap.pk, s.page_tokens) &&
+          keys(&ap.pk_tail, tail) && values(&ap.pv, s.page_tokens) && values(&ap.pv_tail, tail) &&
+          map_kv(&ap.sk, s.k, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, attn::KCH, 2) &&
+          map_kv(&ap.sv, s.v, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, 64, 4))) {
       e = cudaErrorUnknown;
       what = "cuTensorMapEncodeTiled failed";
       return;
     }
-    ap.pk = s.maps->pk; ap.pk_tail = s.maps->pk_tail; ap.pv = s.maps->pv; ap.pv_tail = s.maps->pv_tail;
-    ap.sk = s.maps->sk; ap.sv = s.maps->sv;
     ap.page_table = s.page_table; ap.pages_per_obs = s.pages_per_obs; ap.page_tokens = s.page_tokens;
     ap.valid = (const uint8_t*)s.in[24]; ap.out = s.attn; ap.prefix = s.prefix; ap.suffix = T; ap.obs_tokens = T;
     ap.early = 1; ap.status = s.status; ap.limit = s.wait_limit;
@@ -577,7 +590,7 @@ size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   for (int b = 1; b <= max_batch; ++b) {
     for (int k : {QD, FF}) most = std::max(most, (size_t)plan_gemm(sms, T * b, W, k, gemm::EPI_PART).splits * T * b * W);
     const AttnPlan a = plan_attention(sms, b, max_prefix);          // splits grow with the prefix
-    if (a.splits > 1) most = std::max(most, (size_t)b * a.tiles * a.splits * attn::MERGE_COLS * a.tok_tile * NQH);
+    if (a.splits > 1) most = std::max(most, (size_t)b * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
   }
   return most;
 }

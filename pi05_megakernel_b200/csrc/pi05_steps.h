@@ -19,7 +19,9 @@ struct StepSetup {
   float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions (steps_part_floats)
   uint32_t* rope;
   __nv_bfloat16 *h, *an, *q, *k, *v, *attn, *act;
-  const TMaps* maps;                         // prefix and suffix key / value maps
+  const void *pool_k, *pool_v;               // prefix cache; strides in elements
+  long long token_stride, layer_stride, page_stride;
+  int num_pages;
   const int* page_table;
   int pages_per_obs, page_tokens;
   long long wait_limit;
