@@ -227,8 +227,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   if (warp == 1) {
     // ---- MMA issuer
     const uint32_t idesc_s = ptx::umma_idesc_bf16(KCH, N), idesc_o = ptx::umma_idesc_bf16(128, N) | ptx::UMMA_A_MN_MAJOR | ptx::UMMA_B_MN_MAJOR;
-    const uint64_t qdesc = ptx::umma_smem_desc(q_base), kdesc = ptx::umma_smem_desc(ring);
-    const uint64_t pdesc = ptx::umma_smem_desc_mn(p_base, SEG), vdesc = ptx::umma_smem_desc_mn(ring, 64 * 128);
+    // lower words of the descriptors (the upper one is the same for all)
+    const uint32_t qdesc = (uint32_t)ptx::umma_smem_desc(q_base), kdesc = (uint32_t)ptx::umma_smem_desc(ring);
+    const uint32_t pdesc = (uint32_t)ptx::umma_smem_desc_mn(p_base, SEG), vdesc = (uint32_t)ptx::umma_smem_desc_mn(ring, 64 * 128);
+    const uint32_t on = leader ? 1u : 0u;
     bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, 3);
     auto issue_s = [&](int i) -> bool {
       const int buf = i & 1, at = pos_k(i);
@@ -238,10 +240,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
         const int slot = (at + u) % UNITS;
         if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, ((at + u) / UNITS) & 1, 4)) return false;
         ptx::tc_fence_after();
+        const uint32_t kd = kdesc + ((slot * UNIT) >> 4), qd = qdesc + ((2 * u * QBLK) >> 4);
+        ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd, qd, idesc_s, u ? 1u : 0u, on);
+        ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd + (SEG >> 4), qd + (QBLK >> 4), idesc_s, 1u, on);
         if (leader) {
-          const uint64_t kd = kdesc + (uint64_t)((slot * UNIT) >> 4), qd = qdesc + (uint64_t)((2 * u * QBLK) >> 4);
-          ptx::umma_bf16_k64(tmem + TM_S + buf * N, kd, qd, idesc_s, u ? 1u : 0u, 2, 2);
-          ptx::umma_bf16_k64(tmem + TM_S + buf * N, kd + (SEG >> 4), qd + (QBLK >> 4), idesc_s, 1u, 2, 2);
           ptx::umma_commit(empty + 8 * slot);
           if (u == 1) ptx::umma_commit(s_full + 8 * buf);
         }
@@ -257,12 +259,11 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
         const int slot = (at + u) % UNITS;
         if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, ((at + u) / UNITS) & 1, 6)) return false;
         ptx::tc_fence_after();
+        // 16 keys per MMA: 16 rows of 128 B further in V and in P
+        const uint32_t vd = vdesc + ((slot * UNIT) >> 4), pd = pdesc + ((u * 64 * 128) >> 4), acc = i || u ? 1u : 0u;
+        ptx::umma_bf16_k64<128, 128>(tmem + TM_O, vd, pd, idesc_o, acc, on);
+        ptx::umma_bf16_k64<128, 128>(tmem + TM_O + N, vd + ((2 * 64 * 128) >> 4), pd, idesc_o, acc, on);
         if (leader) {
-          // 16 keys per MMA: 16 rows of 128 B further in V and in P
-          const uint64_t vd = vdesc + (uint64_t)((slot * UNIT) >> 4), pd = pdesc + (uint64_t)((u * 64 * 128) >> 4);
-          const uint32_t acc = i || u ? 1u : 0u;
-          ptx::umma_bf16_k64(tmem + TM_O, vd, pd, idesc_o, acc, 128, 128);
-          ptx::umma_bf16_k64(tmem + TM_O + N, vd + ((2 * 64 * 128) >> 4), pd, idesc_o, acc, 128, 128);
           ptx::umma_commit(empty + 8 * slot);
           if (u == units - 1) ptx::umma_commit(p_empty);
         }

@@ -514,14 +514,12 @@ void describe(pi05_engine* h) {
 bool valid_handle(pi05_handle_t h) { return h != nullptr; }
 
 // Whether a launch without debug controls runs as graphs of kernels (pi05_steps.cu).  The persistent kernel stays for
-// tensor parallel, for the static entry point, for debug controls, for callers that set one of its own tuning settings, and
-// for one observation with a prefix of four to six 64-key chunks, where the chain's attention takes as long as what its other
-// kernels save (301 tokens: 5.70 against 5.77 ms; 128 tokens: 5.28 against 5.10, 968: 6.93 against 5.89).
+// tensor parallel, for the static entry point, for debug controls and for callers that set one of its own tuning settings.
 bool uses_graphs(const pi05_engine* h) {
   pi05_tuning d;
   default_tuning(&d);
   d.poll_ns = h->tune.poll_ns;
-  return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0 && (h->batch > 1 || h->prefix <= 192 || h->prefix > 384 || getenv("PI05_G"));
+  return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0;
 }
 
 int build_graphs(pi05_engine* h, int n_steps, int n_layers) {

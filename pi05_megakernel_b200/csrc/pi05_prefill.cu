@@ -18,7 +18,6 @@
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
-#include <stdlib.h>
 
 #include <algorithm>
 #include <new>
@@ -183,10 +182,11 @@ PrefillPlan plan_prefill(int sms, int tokens) {
   pl.o = plan_gemm(sms, tokens, pf::H, QD, gemm::EPI_PART, pl.pairs);
   pl.gu = plan_gemm(sms, tokens, 2 * pf::FFN, pf::H, gemm::EPI_GEGLU, pl.pairs);
   pl.down = pl.sk_down ? plan_gemm_sk(sms, tokens, pf::H, pf::FFN) : plan_gemm(sms, tokens, pf::H, pf::FFN, gemm::EPI_PART, 1);
+  // The widest tile of query tokens that does not cost a second wave of CTAs: 512 tokens 2.23 ms on tiles of 4, 2.37 on 2 and 2.26
+  // on 8; 968 tokens 3.40 on 8 and 3.75 on 4.
   pl.tok_tile = 14;
   for (int t : {8, 6, 4, 2})
     if ((tokens + t - 1) / t <= sms) pl.tok_tile = t;
-  if (getenv("AT")) pl.tok_tile = atoi(getenv("AT"));
   return pl;
 }
 

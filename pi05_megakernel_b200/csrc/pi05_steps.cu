@@ -13,7 +13,6 @@
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
-#include <stdlib.h>
 
 #include <algorithm>
 #include <string>
@@ -400,22 +399,29 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) tail_kernel(const TailArgs p)
 }
 
 // =========================================================================================== host side
-// How the attention of `batch` observations is cut: tiles of 5 tokens (40 query rows, three key / value stages) for a few
-// observations, where the time of one CTA counts, of 13 (104 rows) for more, where the keys that all CTAs read together do; the
-// keys of a tile over as many CTAs of a cluster as leaves each what its stages hold, as long as the CTAs fit the SMs.
+// How the attention of `batch` observations is cut: `tok_tile` query tokens per CTA, the keys of a tile over `splits` CTAs of a
+// cluster.
 struct AttnPlan { int tok_tile, tiles, splits; };
 
 AttnPlan plan_attention(int sms, int batch, int prefix) {
-  AttnPlan a;
-  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1, per_cta = getenv("AP") ? atoi(getenv("AP")) : 5;
-  a.tok_tile = 14;
-  for (int t : {8, 6, 4, 2})
-    if (batch * ((T + t - 1) / t) <= sms) a.tok_tile = t;
-  if (getenv("AT")) a.tok_tile = atoi(getenv("AT"));
-  a.tiles = (T + a.tok_tile - 1) / a.tok_tile;
-  a.splits = 1;
-  while (a.splits < 8 && (chunks + a.splits - 1) / a.splits > per_cta && batch * a.tiles * a.splits * 2 <= sms) a.splits *= 2;
-  return a;
+  AttnPlan best = {};
+  double best_cost = 1e30;
+  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1;
+  for (int t : {2, 4, 6, 8, 14})
+    for (int splits = 1; splits <= 8 && splits <= chunks; splits *= 2) {
+      const int tiles = (T + t - 1) / t, ctas = batch * tiles * splits;
+      const int per_cta = (chunks + splits - 1) / splits;
+      // (a cluster is resident as a whole, and those of eight CTAs leave some SMs without)
+      if (splits > 1 && (per_cta < 2 || ctas > (splits == 8 ? sms * 3 / 4 : sms))) continue;
+      // Measured, in us: a chunk of 128 keys, what a tile costs besides, a merge, and 2 us for a launch on more than half of the
+      // SMs (the next kernel's CTAs then start, and fetch their weights, when this one's leave; the merges of 4 and 8 include it)
+      const double cost = per_cta * (1.75 + 0.03 * t) * ((ctas + sms - 1) / sms) + 0.4 * t + (splits == 1 ? 0.0 : splits == 2 ? 2.2 : splits == 4 ? 4.5 : 4.9) +
+                          (splits <= 2 && ctas * 2 > sms ? 2.0 : 0.0);
+      if (cost >= best_cost) continue;
+      best_cost = cost;
+      best.tok_tile = t; best.tiles = tiles; best.splits = splits;
+    }
+  return best;
 }
 
 typedef void (*NormKernel)(const NormArgs);

@@ -243,20 +243,6 @@ __device__ __forceinline__ void umma_bf16_stage8(uint32_t d_tmem, uint64_t adesc
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(commit_bar),
         "n"((unsigned long long)A_ATOM), "n"((unsigned long long)B_ATOM) : "memory");
 }
-// Four K = 16 MMAs, `astep` / `bstep` descriptor units (16 bytes) apart.
-__device__ __forceinline__ void umma_bf16_k64(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate, uint64_t astep, uint64_t bstep) {
-  asm volatile(
-      "{\n.reg .pred p;\n.reg .b64 a1, a2, a3, b1, b2, b3;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "add.u64 a1, %1, %5;\n add.u64 a2, a1, %5;\n add.u64 a3, a2, %5;\n"
-      "add.u64 b1, %2, %6;\n add.u64 b2, b1, %6;\n add.u64 b3, b2, %6;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "l"(astep), "l"(bstep) : "memory");
-}
 // One pipeline stage of KS 64-k blocks in one piece: 4 KS MMAs of K = 16 (32-byte steps inside the 128-byte swizzle rows of
 // a block, blocks `ablock` / `bblock` descriptor units apart) and the commit that frees the stage, on one CTA or on a pair
 // (whose commit arrives in both CTAs).  `alo`, `blo`: lower words of the descriptors; the upper word is the same for all.
@@ -283,13 +269,25 @@ __device__ __forceinline__ void umma_bf16_stage(uint32_t d_tmem, uint32_t alo, u
     asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "p") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS);
   else
     asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "p") PI05_UMMA_NEXT PI05_UMMA4("1", "t") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS);
-#undef PI05_UMMA1
 #undef PI05_UMMA4
+#undef PI05_UMMA1
 #undef PI05_UMMA_HEAD
 #undef PI05_UMMA_NEXT
 #undef PI05_UMMA_COMMIT1
 #undef PI05_UMMA_COMMIT2
 #undef PI05_UMMA_ARGS
+}
+// Four K = 16 MMAs on one CTA, ASTEP / BSTEP descriptor units (16 bytes) apart, by the lane for which `on` is set; the rest as above.
+template <int ASTEP, int BSTEP>
+__device__ __forceinline__ void umma_bf16_k64(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc, uint32_t accumulate, uint32_t on) {
+#define PI05_UMMA1(P0) "mov.b64 da, {al, %5};\n mov.b64 db, {bl, %5};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, " P0 ";\n"
+#define PI05_UMMA_STEP "add.u32 al, al, %7;\n add.u32 bl, bl, %8;\n"
+  asm volatile("{\n.reg .pred p, q, t;\n.reg .b32 al, bl;\n.reg .b64 da, db;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %6, 0;\nsetp.eq.b32 t, 0, 0;\n"
+               "mov.b32 al, %1;\nmov.b32 bl, %2;\n" PI05_UMMA1("p") PI05_UMMA_STEP PI05_UMMA1("t") PI05_UMMA_STEP PI05_UMMA1("t") PI05_UMMA_STEP
+               PI05_UMMA1("t") "}"
+               ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI), "r"(on), "n"(ASTEP), "n"(BSTEP) : "memory");
+#undef PI05_UMMA1
+#undef PI05_UMMA_STEP
 }
 // One lane of a converged warp (always the same one), for instructions that a single thread must issue while the
 // loop around them stays warp-uniform.
