@@ -36,11 +36,11 @@ struct Cut { int epi, bn, ks; bool pair, sk; GemmKernel kernel; };
 // Every cut that is built.
 #define CUT(E, BN, PAIR, KS, SK) {gemm::E, BN, KS, PAIR, SK, gemm::gemm_kernel<gemm::E, BN, PAIR, KS, SK>}
 const Cut kCuts[] = {
-    CUT(EPI_QKV, 32, false, 2, false), CUT(EPI_QKV, 128, false, 2, false), CUT(EPI_QKV, 64,true, 2, false),
+    CUT(EPI_QKV, 32, false, 2, false), CUT(EPI_QKV, 64, false, 2, false), CUT(EPI_QKV, 128, false, 2, false), CUT(EPI_QKV, 64,true, 2, false),
     CUT(EPI_QKV, 128,true, 2, false), CUT(EPI_QKV, 256,true, 1, false),
     CUT(EPI_GEGLU, 64, false, 2, false), CUT(EPI_GEGLU, 128, false, 2, false), CUT(EPI_GEGLU, 256, false, 1, false),
     CUT(EPI_GEGLU, 128,true, 2, false), CUT(EPI_GEGLU, 256,true, 1, false),
-    CUT(EPI_PART, 32, false, 2, false), CUT(EPI_PART, 64, false, 2, false), CUT(EPI_PART, 64,true, 2, false),
+    CUT(EPI_PART, 32, false, 2, false), CUT(EPI_PART, 64, false, 2, false), CUT(EPI_PART, 128, false, 2, false), CUT(EPI_PART, 64,true, 2, false),
     CUT(EPI_PART, 128,true, 2, false), CUT(EPI_PART, 256,true, 1, false), CUT(EPI_PART, 256, false, 1, true),
 };
 #undef CUT
@@ -113,12 +113,12 @@ bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, 
 }
 
 // The cheapest of the cuts that are built, by a model of the launch's time in SM cycles: rounds x 64-k blocks x the slower of the
-// MMAs (measured per M128 / M256 K16 instruction: 47 cycles up to N = 32, 50 / 65 / 129 at 64 / 128 / 256; M64:
-// 39 and 41 up to N = 64) and the operands' way
-// into shared memory (~67 B per cycle and SM), not less than the weights' way from HBM (3.3 KB per cycle), plus what every
-// launch pays, an epilogue that grows with the tile, and the way of partial sums through L2 (~2 KB per cycle).  Pairs of CTAs
-// (256 tokens) load half of the tile's weight rows each.  K of the projections whose sums meet in the residual kernel is split
-// in powers of two, down to four 64-k blocks.
+// tensor core (N / 2 cycles per K16 instruction) and shared memory (128 B per cycle: the rows of both operands that an
+// instruction reads, 64 or 128 of the activations, and the copies that bring them), not less than the weights' way from HBM
+// (3.3 KB per cycle), plus what every launch pays, an epilogue that grows with the tile, the start of a cluster for pairs
+// of CTAs (measured: a launch on pairs takes 0.4-0.8 us longer than the same on single CTAs) and the way of partial sums through
+// L2 and the row kernel.  Against every cut measured by itself, 50 to 800 tokens, the choice costs at most 1% of a chunk.
+// K of the projections whose sums meet in the residual kernel is split in powers of two, down to four 64-k blocks.
 GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
   GemmPlan best = {};
   double best_cost = 1e30;
@@ -134,10 +134,11 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
       g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
       g.arows = (g.rows + 7) / 8 * 8;
       const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128, ctas = g.m_tiles * (n / g.bn) * splits, rounds = (ctas + sms - 1) / sms;
-      const bool m64 = !g.pair && g.rows <= 64;
-      const double mma = 4 * (g.bn <= 32 ? (m64 ? 39 : 47) : g.bn == 64 ? (m64 ? 41 : 50) : g.bn == 128 ? 65 : 129), ingest = (g.arows * 128 + w_bytes) / 67.0;
-      double cost = std::max(rounds * g.kblocks * std::max(mma, ingest), (double)n * k * 2 / 3300) + 2000 + g.bn * (epi == gemm::EPI_GEGLU ? 12 : 8);
-      if (epi == gemm::EPI_PART && splits > 1) cost += std::max(150.0 * splits, splits * (double)tokens * n * 4 / 2000);
+      // cycles of a 64-k block: the tensor core's, or what its operands take through shared memory
+      const double smem = (4 * ((!g.pair && g.rows <= 64 ? 2048 : 4096) + g.bn * (g.pair ? 16 : 32)) + g.arows * 128 + w_bytes) / 128.0;
+      double cost = std::max(rounds * g.kblocks * (std::max({2.0 * g.bn, 100.0, smem}) + 70.0 / g.ks), (double)n * k * 2 / 3300) + 2000 +
+                    g.bn * (epi == gemm::EPI_GEGLU ? 24 : 8) + (g.pair ? 2400 : 0);
+      if (splits > 1) cost += std::max(500.0 * splits, splits * (double)tokens * n * 4 / 1800);
       if (cost >= best_cost) continue;
       g.units = g.pair ? ctas / 2 : ctas;
       g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
