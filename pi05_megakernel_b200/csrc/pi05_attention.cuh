@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     float* part = p.merge + (size_t)(unit * p.splits + split) * part_floats(N);
     if (et < N) {
       const float sum = (s_red[0][et] + s_red[1][et]) + (s_red[2][et] + s_red[3][et]);
-      if (p.splits == 1) s_f[et] = 1.0f / sum;
+      if (p.splits == 1) s_f[et] = sum > 0.f ? 1.0f / sum : 0.f;     // (no valid key: zeros)
       else __stcg(reinterpret_cast<float2*>(part + N * HD) + et, make_float2(s_m[et], sum));
     }
     ptx::named_bar_sync(1, SOFTMAX);
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
         a[4] = a[4] * g + (y[0].x * f0 + y[1].x * f1); a[5] = a[5] * g + (y[0].y * f0 + y[1].y * f1);
         a[6] = a[6] * g + (y[0].z * f0 + y[1].z * f1); a[7] = a[7] * g + (y[0].w * f0 + y[1].w * f1);
       }
-      const float il = 1.0f / L;
+      const float il = L > 0.f ? 1.0f / L : 0.f;
       base[row * (HD / 8) + lane] = make_uint4(pack2(a[0] * il, a[1] * il), pack2(a[2] * il, a[3] * il), pack2(a[4] * il, a[5] * il),
                                                pack2(a[6] * il, a[7] * il));
     }

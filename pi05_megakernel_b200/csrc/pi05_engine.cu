@@ -497,12 +497,13 @@ void describe(pi05_engine* h) {
   char buf[1280];
   const bool grouped = h->batch >= h->tune.grouped_from && !h->tune.latency_schedule;
   snprintf(buf, sizeof buf,
-           "{\"kernel\": \"pi05_chunk_kernel\", \"arch\": \"sm_100a\", \"launches_per_chunk\": 1, \"grid\": %d, "
+           "{\"kernel\": \"%s\", \"arch\": \"sm_100a\", \"launches_per_chunk\": %d, \"grid\": %d, "
            "\"threads\": %d, \"smem_bytes\": %d, \"gemm_ctas\": %d, \"row_ctas\": %d, \"stages\": %d, "
            "\"stage_bytes\": %d, \"units\": {\"qkv\": %d, \"o\": %d, \"gate_up\": %d, \"down\": %d}, "
            "\"mma\": \"tcgen05 cta_group::1 M128 N%d K16 bf16\", \"sync\": \"device-scope counters, bounded waits\", "
            "\"clusters_of_2\": %s, \"observations_per_mma\": %d, \"tp_rank\": %d, \"tp_size\": %d, \"schedule\": \"%s\"}",
-           h->grid, THREADS, SMEM_BYTES, h->n_gemm, h->grid - h->n_gemm, h->gn == 1 ? NSTG : 3,
+           h->steps.step ? "chain of kernels replayed from graphs (the fields below: the persistent kernel, pi05_chunk_kernel)" : "pi05_chunk_kernel",
+           h->steps.step ? h->steps.kernels_prologue + h->steps.n_steps * h->steps.kernels_step : 1, h->grid, THREADS, SMEM_BYTES, h->n_gemm, h->grid - h->n_gemm, h->gn == 1 ? NSTG : 3,
            W_STAGE_BYTES + h->gn * A_STAGE_BYTES, h->n_units[0], h->n_units[1], h->n_units[2], h->n_units[3], 64 * h->gn,
            h->clustered ? "true" : "false", h->gn, h->tp_rank, h->tp_size,
            !grouped ? "one observation (units serve every observation in turn)"

@@ -144,6 +144,7 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
       g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
       g.bufs = g.grid < ctas ? 2 : 1;
       lay_out(&g, g.bufs > 1 ? gemm::MAX_STAGES : g.kblocks / g.ks);
+      if (g.stages < 2) continue;
       best = g;
       best_cost = cost;
     }

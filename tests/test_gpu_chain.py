@@ -1,0 +1,75 @@
+"""The kernels of the chain (projections, attention, residual + norm) at the sizes where their cuts change, against the oracle
+within the reference harness's band.  Every test needs a B200."""
+import pytest
+import torch
+
+from oracle import pi05_oracle as O
+from pi05_megakernel_b200 import fixture as FX
+
+pytestmark = pytest.mark.gpu
+
+
+# (prefix, batch, mask, steps and layers).  128-key chunks: up to 64 valid keys in the last one and more, one key; the keys of a
+# tile over 1, 2, 4 and 8 CTAs; projections on tiles of up to 64 and up to 128 tokens, on two, three, six and eight of them,
+# on single CTAs and on pairs, persistent or not; attention on tiles of 2, 4 and 6 tokens.
+@pytest.mark.parametrize("prefix,batch,mask,variant", [
+    (1, 1, "full", "b200-s2-l2"), (63, 1, "scatter", "b200-s2-l2"), (128, 2, "pad", "b200-s2-l2"), (129, 3, "scatter", "b200-s2-l2"),
+    (192, 5, "pad", "b200-s1-l2"), (193, 6, "scatter", "b200-s1-l2"), (301, 1, "scatter", "b200-s2-l2"), (968, 1, "pad", "b200-s2-l2"),
+    (1100, 2, "scatter", "b200-s1-l2"), (130, 7, "full", "b200-s1-l2"), (65, 11, "pad", "b200-s1-l2"), (257, 16, "scatter", "b200-s1-l2")])
+def test_chunk_cuts(prefix, batch, mask, variant):
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo, ogeo = FX.Geometry(prefix=prefix), O.Geo(prefix=prefix)
+    stacked, per = FX.make_batch(geo, FX.SEEDS[1], batch, "cpu", [mask] * batch)
+    arm = Pi05Arm(geo, variant, "cuda", batch=batch)
+    arm.bind({k: v.cuda() for k, v in stacked.items()})
+    arm.launch()
+    arm.status()
+    first = arm.outputs()["actions"].cpu()
+    arm.launch()
+    arm.status()
+    assert torch.equal(first, arm.outputs()["actions"].cpu())          # no order of arrival enters the sums
+    for b in {0, batch // 2, batch - 1}:
+        want, exact = (O.chunk(per[b], ogeo, widen, arm.steps, arm.layers) for widen in (False, True))
+        d = O.band(want, first.reshape(batch, 50, 32)[b], exact)
+        assert d["pass"], (b, d)
+    arm.close()
+
+
+@pytest.mark.parametrize("prefix", [300, 968])
+def test_attention_reference_moves(prefix):
+    """Scores that grow from one chunk of keys to the next: the exponent's reference, taken from the first chunk, has to follow,
+    on one CTA per tile and on a cluster."""
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo, ogeo = FX.Geometry(prefix=prefix), O.Geo(prefix=prefix)
+    cpu = FX.make_inputs(geo, FX.SEEDS[2], "cpu", "full")
+    grow = torch.ones(prefix)
+    grow[prefix // 2:] = 12.0
+    grow[-20:] = 30.0
+    cpu["prefix_k"] = (cpu["prefix_k"].float() * grow.view(1, prefix, *[1] * (cpu["prefix_k"].dim() - 2))).to(torch.bfloat16)
+    arm = Pi05Arm(geo, "b200-s1-l3", "cuda")
+    arm.bind({k: v.cuda() for k, v in cpu.items()})
+    arm.launch()
+    arm.status()
+    want, exact = (O.chunk(cpu, ogeo, widen, arm.steps, arm.layers) for widen in (False, True))
+    d = O.band(want, arm.outputs()["actions"].cpu(), exact)
+    assert d["pass"], d
+    arm.close()
+
+
+@pytest.mark.parametrize("tokens", [1, 65, 128, 129, 297, 600, 900, 1200])
+def test_prefill_cuts(tokens):
+    from pi05_megakernel_b200.prefill import Pi05Prefill
+    geo = FX.PrefillGeometry(tokens=tokens)
+    inputs = FX.make_prefill_inputs(geo, 7, "full")
+    dev = {k: v.cuda() for k, v in inputs.items()}
+    pre = Pi05Prefill(geo, "cuda")
+    pre.bind(dev)
+    k, v = pre.run(dev["embeddings"], dev["valid"], 2)
+    pre.status()
+    args = (inputs, inputs["embeddings"], inputs["valid"], geo.q_heads, geo.kv_heads, geo.head_dim)
+    wk, wv = O.prefill(*args, widen=False, layers=2)
+    ek, ev = O.prefill(*args, widen=True, layers=2)
+    for got, want, exact in ((k.cpu()[:2], wk, ek), (v.cpu()[:2], wv, ev)):
+        d = O.band(want.float(), got.float(), exact.float())
+        assert d["pass"], d
+    pre.close()
