@@ -21,7 +21,7 @@ def test_chunk_cuts(prefix, batch, mask, variant):
     geo, ogeo = FX.Geometry(prefix=prefix), O.Geo(prefix=prefix)
     stacked, per = FX.make_batch(geo, FX.SEEDS[1], batch, "cpu", [mask] * batch)
     arm = Pi05Arm(geo, variant, "cuda", batch=batch)
-    arm.bind({k: v.cuda() for k, v in stacked.items()})
+    arm.bind({k: v.cuda() for k, v in (stacked if batch > 1 else per[0]).items()})
     arm.launch()
     arm.status()
     first = arm.outputs()["actions"].cpu()
