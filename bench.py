@@ -708,7 +708,7 @@ def main() -> int:
             "dtype": "bf16", "data": "synthetic",
             "config": {"workload": f"pi0.5 action chunk, B={B} per GPU, prefix {geo.prefix} ({args.mask} mask), 10 Euler steps x 18 "
                                    "Gemma-300M expert layers, BF16 weights and prefix K/V, FP32 time MLP / "
-                                   "modulation; one persistent kernel launch per chunk",
+                                   "modulation; one pi05_launch per chunk (graphs of chained kernels)",
                        "l2": "flushed before every timed chunk (2x L2 zero fill)",
                        "prefix_cache": f"pool of shuffled {args.kv_pages}-token pages read in place" if args.kv_pages else "dense",
                        "parallelism": f"dp{world} (independent observations, replicated weights, no collective)",

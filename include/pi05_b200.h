@@ -200,7 +200,7 @@ int pi05_tp_attach_pointer(pi05_handle_t h, int peer_rank, void* peer_workspace)
 int pi05_schedule_plan_tp(int sms, int batch, int prefix_len, int tp_rank, int tp_size, const pi05_tuning* tuning,
                           int* entries, int capacity, int* count, int info[PI05_PLAN_INFO]);
 
-/* Number of kernel launches issued by this handle since creation (one per pi05_launch). */
+/* Number of pi05_launch calls of this handle since creation; the kernels of one are the configuration's launches_per_chunk. */
 int pi05_launch_count(pi05_handle_t h, unsigned long long* count);
 
 const char* pi05_error_string(int code);
