@@ -116,13 +116,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     return i == n - 1 ? 4 * i + 2 : 4 * i + 4;
   };
 
-  if (tid == 0) {
-    ptx::mbar_init(q_full, 1);
-    for (int i = 0; i < UNITS; ++i) { ptx::mbar_init(full + 8 * i, 1); ptx::mbar_init(empty + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { ptx::mbar_init(s_full + 8 * i, 1); ptx::mbar_init(s_empty + 8 * i, SOFTMAX); }
-    ptx::mbar_init(p_full, SOFTMAX);
-    ptx::mbar_init(p_empty, 1);
-    ptx::mbar_init(o_full, 1);
+  if (warp == 0) {
+    // all 20 (the last of them unused), a lane each: s_empty[2] and p_full are the softmax threads'
+    if (lane < 20) ptx::mbar_init(b0 + 8 * lane, (lane >= 15 && lane <= 17) ? SOFTMAX : 1);
     ptx::fence_mbar_init();
     ptx::fence_proxy_async_shared();
   }

@@ -207,10 +207,11 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
   const int stages = p.stages;
   const int tcols = p.bufs * (BN < 32 ? 32 : BN);
 
-  if (tid == 0) {
-    // a stage is full when both producers' arrivals (weights, activations) and every byte of both have come
-    for (int i = 0; i < stages; ++i) { ptx::mbar_init(full + 8 * i, 2); ptx::mbar_init(empty + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { ptx::mbar_init(t_full + 8 * i, 1); ptx::mbar_init(t_empty + 8 * i, PAIR ? 2 * EPI_THREADS : EPI_THREADS); }
+  if (warp == 0) {
+    // a stage is full when both producers' arrivals (weights, activations) and every byte of both have come; a lane per stage, since
+    // a CTA that starts when the kernel before it leaves pays for every cycle up to here
+    if (lane < stages) { ptx::mbar_init(full + 8 * lane, 2); ptx::mbar_init(empty + 8 * lane, 1); }
+    if (lane < 2) { ptx::mbar_init(t_full + 8 * lane, 1); ptx::mbar_init(t_empty + 8 * lane, PAIR ? 2 * EPI_THREADS : EPI_THREADS); }
     ptx::fence_mbar_init();
     ptx::fence_proxy_async_shared();
   }
