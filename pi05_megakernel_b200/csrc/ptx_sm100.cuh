@@ -261,7 +261,11 @@ __device__ __forceinline__ void umma_bf16_stage(uint32_t d_tmem, uint32_t alo, u
 #define PI05_UMMA_COMMIT1 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n}"
 #define PI05_UMMA_COMMIT2 ".reg .b16 m;\nmov.b16 m, 3;\n@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], m;\n}"
 #define PI05_UMMA_ARGS ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(commit_bar), "r"(ablock), "r"(bblock), "n"(UMMA_DESC_HI), "r"(on) : "memory"
-  if constexpr (PAIR && KS == 1)
+  if constexpr (KS == 4) {
+    static_assert(!PAIR, "four blocks a stage: single CTAs");
+    asm volatile(PI05_UMMA_HEAD PI05_UMMA4("1", "p") PI05_UMMA_NEXT PI05_UMMA4("1", "t") PI05_UMMA_NEXT PI05_UMMA4("1", "t") PI05_UMMA_NEXT
+                 PI05_UMMA4("1", "t") PI05_UMMA_COMMIT1 PI05_UMMA_ARGS);
+  } else if constexpr (PAIR && KS == 1)
     asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "p") PI05_UMMA_COMMIT2 PI05_UMMA_ARGS);
   else if constexpr (PAIR)
     asm volatile(PI05_UMMA_HEAD PI05_UMMA4("2", "p") PI05_UMMA_NEXT PI05_UMMA4("2", "t") PI05_UMMA_COMMIT2 PI05_UMMA_ARGS);
