@@ -10,8 +10,8 @@
 //   * One CTA = one tile of query tokens against a contiguous share of the keys, in chunks of 128 (the suffix is a chunk of its
 //     own; a chunk of up to 64 valid keys skips the other half of V).  `splits` CTAs of a cluster share the keys of a tile
 //     and merge through global memory (below).
-//   * Warp 0 streams Q and the keys and values with TMA into a ring of 32 KB units, in the order in which the MMAs consume them:
-//     K (dims 0-127, dims 128-255) of chunk i + 1, V (keys 0-63, keys 64-127) of chunk i, ..; warp 1 issues S^T of chunk i + 1
+//   * Warp 0 streams the keys and values with TMA into a ring of 32 KB units, in the order in which the MMAs consume them:
+//     K (dims 0-127, dims 128-255) of chunk i + 1, V (keys 0-63, keys 64-127) of chunk i, ..; warp 1 fetches Q and issues S^T of chunk i + 1
 //     before O^T of chunk i; warps 2..9 are the softmax threads: thread = one key and half of the query rows.  V and P are
 //     taken as they lie, as MN-major operands: nothing is ever transposed in memory.
 //   * The keys are passed over once, and after the first chunk without looking for their maximum: the exponent's reference of a
@@ -134,24 +134,22 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     bool waited = false;
     int j = 0, slot = 0;                   // unit in the ring's order
     uint32_t par = 1;
+    const bool paged = p.pages_per_obs > 1;
+    const int last = paged ? (p.prefix - 1) / p.page_tokens : 0, page0 = paged || !p.page_table ? ob : __ldg(p.page_table + ob);
     auto page_of = [&](int key, int& row, bool& tail) {      // key: first of 64 or 128 keys of a page; beyond the prefix: rows that read as zeros
-      const int last = (p.prefix - 1) / p.page_tokens;
-      int lp = p.pages_per_obs == 1 ? 0 : key / p.page_tokens;
+      row = key;
+      tail = true;
+      if (!paged) return page0;
+      int lp = key / p.page_tokens;
       row = key - lp * p.page_tokens;
       if (lp > last) { lp = last; row = p.page_tokens; }
       tail = lp == last;
-      return p.page_table ? __ldg(p.page_table + ob * p.pages_per_obs + lp) : ob;
+      return __ldg(p.page_table + ob * p.pages_per_obs + lp);
     };
     auto emit = [&](int i, int isv, int u) {
       const int c = cbeg + i;
-      if (!waited && (!p.early || j >= UNITS || c >= npc)) {
+      if (!waited && (!p.early || c >= npc)) {
         ptx::grid_dep_wait();
-        if (leader) {
-          ptx::mbar_expect_tx(q_full, 4 * QBLK);
-          for (int kb = 0; kb < 4; ++kb)
-            ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
-        }
-        __syncwarp();
         waited = true;
       }
       if (ok && j >= UNITS) ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1);
@@ -190,21 +188,13 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       const int units = isv ? nv(ch) : 2;
       for (int u = 0; u < units; ++u) emit(ch, isv ? 1 : 0, u);
     }
-    if (!waited) {                                            // everything fitted the ring
-      ptx::grid_dep_wait();
-      if (leader) {
-        ptx::mbar_expect_tx(q_full, 4 * QBLK);
-        for (int kb = 0; kb < 4; ++kb)
-          ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
-      }
-      __syncwarp();
-    }
   } else {
     if (warp == 1) {
       ptx::tmem_alloc(ptx::smem_u32(&s_tmem), TM_COLS);
       ptx::tmem_relinquish();
       ptx::grid_dep_launch();              // after the allocation: a later kernel cannot take the columns first
       if (leader) { ptx::prefetch_tensormap(&p.q); ptx::prefetch_tensormap(&p.sk); ptx::prefetch_tensormap(&p.sv); }
+      __syncwarp();
     } else {
       // validity bits of this CTA's keys (an input, not an output of the kernel before)
       for (int w = warp - 2; w < 4 * n; w += 8) {
@@ -227,6 +217,13 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     const uint32_t qdesc = (uint32_t)ptx::umma_smem_desc(q_base), kdesc = (uint32_t)ptx::umma_smem_desc(ring);
     const uint32_t pdesc = (uint32_t)ptx::umma_smem_desc_mn(p_base, SEG), vdesc = (uint32_t)ptx::umma_smem_desc_mn(ring, 64 * 128);
     const uint32_t on = leader ? 1u : 0u;
+    ptx::grid_dep_wait();                  // Q is this warp's, which is the one that waits for it: warp 0 may still be at the cache
+    if (leader) {
+      ptx::mbar_expect_tx(q_full, 4 * QBLK);
+#pragma unroll
+      for (int kb = 0; kb < 4; ++kb) ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
+    }
+    __syncwarp();
     bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, 3);
     auto issue_s = [&](int i) -> bool {
       const int buf = i & 1, at = pos_k(i);
@@ -472,25 +469,23 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     for (int row = split * (N / p.splits) + warp; row < (split + 1) * (N / p.splits) && row < out_rows; row += THREADS / 32) {
       const float* q = p.merge + (size_t)unit * p.splits * part_floats(N);
       float M = -1e30f, L = 0.f, a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-      for (int s = 0; s < p.splits; s += 2) {                 // two parts at a time
-        float4 x[2], y[2];
-        float2 ml[2];
+      float4 x[8], y[8];                                      // every part is on its way before the first is used
+      float2 ml[8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float* qs = q + (s + h) * part_floats(N);
-          ml[h] = __ldcg(reinterpret_cast<const float2*>(qs + N * HD) + row);
-          x[h] = __ldcg(reinterpret_cast<const float4*>(qs + row * HD + lane * 8));
-          y[h] = __ldcg(reinterpret_cast<const float4*>(qs + row * HD + lane * 8) + 1);
-        }
-        const float mn = fmaxf(M, fmaxf(ml[0].x, ml[1].x)), g = ptx::ex2_approx((M - mn) * LOG2E);
-        const float f0 = ptx::ex2_approx((ml[0].x - mn) * LOG2E), f1 = ptx::ex2_approx((ml[1].x - mn) * LOG2E);
-        M = mn;
-        L = L * g + (ml[0].y * f0 + ml[1].y * f1);
-        a[0] = a[0] * g + (x[0].x * f0 + x[1].x * f1); a[1] = a[1] * g + (x[0].y * f0 + x[1].y * f1);
-        a[2] = a[2] * g + (x[0].z * f0 + x[1].z * f1); a[3] = a[3] * g + (x[0].w * f0 + x[1].w * f1);
-        a[4] = a[4] * g + (y[0].x * f0 + y[1].x * f1); a[5] = a[5] * g + (y[0].y * f0 + y[1].y * f1);
-        a[6] = a[6] * g + (y[0].z * f0 + y[1].z * f1); a[7] = a[7] * g + (y[0].w * f0 + y[1].w * f1);
+      for (int s = 0; s < 8; ++s) {
+        const float* qs = q + (s < p.splits ? s : 0) * part_floats(N);
+        ml[s] = __ldcg(reinterpret_cast<const float2*>(qs + N * HD) + row);
+        x[s] = __ldcg(reinterpret_cast<const float4*>(qs + row * HD + lane * 8));
+        y[s] = __ldcg(reinterpret_cast<const float4*>(qs + row * HD + lane * 8) + 1);
+        if (s >= p.splits) ml[s] = make_float2(-1e30f, 0.f);
+        M = fmaxf(M, ml[s].x);
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float f = s < p.splits ? ptx::ex2_approx((ml[s].x - M) * LOG2E) : 0.f;
+        L += ml[s].y * f;
+        a[0] += x[s].x * f; a[1] += x[s].y * f; a[2] += x[s].z * f; a[3] += x[s].w * f;
+        a[4] += y[s].x * f; a[5] += y[s].y * f; a[6] += y[s].z * f; a[7] += y[s].w * f;
       }
       const float il = L > 0.f ? 1.0f / L : 0.f;
       base[row * (HD / 8) + lane] = make_uint4(pack2(a[0] * il, a[1] * il), pack2(a[2] * il, a[3] * il), pack2(a[4] * il, a[5] * il),
