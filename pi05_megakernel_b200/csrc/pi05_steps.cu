@@ -413,10 +413,9 @@ AttnPlan plan_attention(int sms, int batch, int prefix) {
       const int per_cta = (chunks + splits - 1) / splits;
       // (a cluster is resident as a whole, and those of eight CTAs leave some SMs without)
       if (splits > 1 && (per_cta < 2 || ctas > (splits == 8 ? sms * 3 / 4 : sms))) continue;
-      // Measured, in us: a chunk of 128 keys, what a tile costs besides, a merge, and 2 us for a launch on more than half of the
-      // SMs (the next kernel's CTAs then start, and fetch their weights, when this one's leave; the merges of 4 and 8 include it)
-      const double cost = per_cta * (1.75 + 0.03 * t) * ((ctas + sms - 1) / sms) + 0.3 * t + 0.02 * t * t + (splits == 1 ? 0.0 : splits == 2 ? 2.2 : splits == 4 ? 4.5 : 4.9) +
-                          (splits <= 2 && ctas * 2 > sms ? 2.0 : 0.0);
+      // Fitted to every cut timed by itself at 1 to 16 observations and 128 to 968 tokens, in us: a chunk of 128 keys, what a tile
+      // costs besides (from 48 query rows on its output is staged), a merge.  The choice is within 1% of the best of a chunk.
+      const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.6 * t - 1.4) + (splits > 1 ? 1.5 + 0.2 * t : 0.0);
       if (cost >= best_cost) continue;
       best_cost = cost;
       best.tok_tile = t; best.tiles = tiles; best.splits = splits;
