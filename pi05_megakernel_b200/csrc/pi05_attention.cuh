@@ -54,7 +54,6 @@ struct Args {
   CUtensorMap pk, pk_tail, pv, pv_tail;    // prefix keys / values {64 dims, page tokens, 4, layers, pages}; K: box {64, k_rows, k_rows / 64,
                                            // 1, 1}, V: box {64, 64, 4, 1, 1}; *_tail: the same, cut at the last valid token of a last page
   CUtensorMap sk, sv;                      // suffix keys / values {64, tokens, 4, 1, observations}, box {64, 128, 2, 1, 1} and {64, 64, 4, 1, 1}
-  CUtensorMap o;                           // the output as [observations][rows per observation][256], box {64, N, 1}
   const int* page_table;                   // [observation][pages_per_obs], or null: page = observation
   const uint8_t* valid;                    // [observation][prefix]
   __nv_bfloat16* out;                      // [tokens, 2048]
@@ -402,11 +401,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     ok &= ptx::wait_bar(p.status, p.limit, o_full, 0, 11);
     ptx::tc_fence_after();
 
-    // ---- O^T / l -> BF16 [row][256] (row = token_local * 8 + head: the tile's rows are one contiguous block of [tokens, 2048]).
-    // They leave through shared memory by tiled copies, which clip what lies beyond the observation's tokens
-    if (p.splits == 1 && N <= 32) {
-      // few rows: 64 bytes of a row per warp, straight to memory (through shared memory and tiled copies, with their fence,
-      // barrier and wait, a layer pass at prefix 128 took 0.3 us longer)
+    // ---- O^T / l -> BF16 [row][256] (row = token_local * 8 + head: the tile's rows are one contiguous block of [tokens, 2048])
+    if (p.splits == 1) {
+      // straight to memory, 64 bytes of a row per warp and store: through shared memory and tiled copies, with their fence, barrier
+      // and wait, a layer pass took 0.3 us longer at 16 query rows per tile and 0.8 us at 48
       const int left = p.obs_tokens - tile * p.tok_tile, out_rows = (left < p.tok_tile ? left : p.tok_tile) * NQH;
       __nv_bfloat16* base = p.out + (size_t)(ob * p.obs_tokens + tile * p.tok_tile) * NQH * HD + quad * 32 + lane;
 #pragma unroll 1
@@ -421,32 +419,6 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
         __syncwarp();
       }
       ptx::tc_fence_before();
-    } else if (p.splits == 1) {
-      // four swizzled 64-dim blocks, over Q (every MMA has completed)
-#pragma unroll 1
-      for (int c = 0; c < 2 * R; c += 8) {
-        const int d = c < R ? 0 : 1, row = r0 + (d ? c - R : c);
-        uint32_t o[8];
-        ptx::tmem_ld_32x8(trow + TM_O + d * N + (row - r0), o);
-        ptx::tmem_wait_ld();
-        const uint32_t blk = q_base + (2 * d + (quad >> 1)) * QBLK, piece = (quad & 1) * 4 + (lane >> 3);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const __nv_bfloat16 v = __float2bfloat16_rn(__uint_as_float(o[k]) * s_f[row + k]);
-          // (rows come in groups of eight: row & 7 = k)
-          ptx::st_shared_u16(blk + (row + k) * 128 + ((piece ^ k) << 4) + (lane & 7) * 2, __bfloat16_as_ushort(v));
-        }
-      }
-      ptx::tc_fence_before();
-      ptx::fence_proxy_async_shared();
-      ptx::named_bar_sync(1, SOFTMAX);
-      if (et == 0 && ok) {
-#pragma unroll 1
-        for (int kb = 0; kb < 4; ++kb) ptx::tma_store_3d(&p.o, q_base + kb * QBLK, kb * 64, tile * N, ob);
-        ptx::bulk_commit();
-        ptx::bulk_wait_read();
-      }
-      __syncwarp();
     } else {
 #pragma unroll 1
       for (int c = 0; c < 2 * R; c += 8) {

@@ -414,8 +414,8 @@ AttnPlan plan_attention(int sms, int batch, int prefix) {
       // (a cluster is resident as a whole, and those of eight CTAs leave some SMs without)
       if (splits > 1 && (per_cta < 2 || ctas > (splits == 8 ? sms * 3 / 4 : sms))) continue;
       // Fitted to every cut timed by itself at 1 to 16 observations and 128 to 968 tokens, in us: a chunk of 128 keys, what a tile
-      // costs besides (from 48 query rows on its output is staged), a merge.  The choice is within 1% of the best of a chunk.
-      const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.6 * t - 1.4) + (splits > 1 ? 1.5 + 0.2 * t : 0.0);
+      // costs besides a merge.  The choice is within 1% of the best of a chunk.
+      const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) + (splits > 1 ? 1.5 + 0.2 * t : 0.0);
       if (cost >= best_cost) continue;
       best_cost = cost;
       best.tok_tile = t; best.tiles = tiles; best.splits = splits;
@@ -538,7 +538,7 @@ struct Capture {
           map_k(&a_dn, s.act, FF, M, pd.arows, pd.ks) && weights(&wq, 8, W, QD, pq) && weights(&wk, 9, W, HD, pq) && weights(&wv, 10, W, HD, pq) &&
           weights(&wo, 11, QD, W, po) && weights(&wg, 12, W, FF, pg) && weights(&wu, 13, W, FF, pg) && weights(&wd, 14, FF, W, pd) &&
           map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH) &&
-          map_out(&ap.o, s.attn, false, HD, (uint64_t)T * NQH, s.batch, 128, ap.tok_tile * NQH) && keys(&ap.pk, s.page_tokens) &&
+          keys(&ap.pk, s.page_tokens) &&
           keys(&ap.pk_tail, tail) && values(&ap.pv, s.page_tokens) && values(&ap.pv_tail, tail) &&
           map_kv(&ap.sk, s.k, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, attn::KCH, 2) &&
           map_kv(&ap.sv, s.v, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, 64, 4))) {
