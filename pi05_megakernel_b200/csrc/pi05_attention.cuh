@@ -104,16 +104,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   const uint32_t q_base = ptx::smem_u32(smem), p_base = q_base + 4 * QBLK, ring = p_base + p_bytes(N);
   const bool leader = ptx::elect_one();
 
-  // Units of V of this CTA's chunk i, and where its units stand in the ring's order K0 | K1 V0 | K2 V1 | .. | V(n-1).  A suffix
-  // at the end goes behind the values of the chunk before it, which do not depend on the kernel before this one.
+  // Units of V of this CTA's chunk i.  The ring's order is K0 | K1 V0 | K2 V1 | .. | V(n-1); a suffix at the end goes behind the values of the chunk before it, which do not depend on the kernel before this one.
   auto nv = [&](int i) { const int c = cbeg + i; return c < npc ? (p.prefix - c * KCH > 64 ? 2 : 1) : 1; };
   const bool swapped = n >= 2 && cbeg + n > npc;
-  auto pos_k = [&](int i) { return i == 0 ? 0 : swapped && i == n - 1 ? 4 * i - 2 + nv(i - 1) : 4 * i - 2; };
-  auto pos_v = [&](int i) {
-    if (n == 1) return 2;
-    if (swapped) return i == n - 1 ? pos_k(i) + 2 : i == n - 2 ? 4 * i + 2 : 4 * i + 4;
-    return i == n - 1 ? 4 * i + 2 : 4 * i + 4;
-  };
 
   if (warp == 0) {
     // all 20 (the last of them unused), a lane each: s_empty[2] and p_full are the softmax threads'
@@ -224,35 +217,41 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     }
     __syncwarp();
     bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, 3);
-    auto issue_s = [&](int i) -> bool {
-      const int buf = i & 1, at = pos_k(i);
-      if (!ptx::wait_bar(p.status, p.limit, s_empty + 8 * buf, ((i >> 1) & 1) ^ 1, 5)) return false;
+    // The units in the ring's order, which is the order of use but for a suffix at the end.  What bounds this loop, next to shared memory,
+    // is the warp's own instructions between two MMAs.
+    int slot = 0;
+    uint32_t par = 0;
+    auto next = [&](int& sl, uint32_t& pr) { if (++sl == UNITS) { sl = 0; pr ^= 1; } };
+    auto issue_s = [&](int i, int& sl, uint32_t& pr) -> bool {
+      const int buf = i & 1;
+      if (i > 1) {
+        if (!ptx::wait_bar(p.status, p.limit, s_empty + 8 * buf, ((i >> 1) & 1) ^ 1, 5)) return false;
+        ptx::tc_fence_after();
+      }
 #pragma unroll 1
       for (int u = 0; u < 2; ++u) {
-        const int slot = (at + u) % UNITS;
-        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, ((at + u) / UNITS) & 1, 4)) return false;
-        ptx::tc_fence_after();
-        const uint32_t kd = kdesc + ((slot * UNIT) >> 4), qd = qdesc + ((2 * u * QBLK) >> 4);
-        ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd, qd, idesc_s, u ? 1u : 0u, on);
+        if (!ptx::wait_bar(p.status, p.limit, full + 8 * sl, pr, 4)) return false;
+        const uint32_t kd = kdesc + sl * (UNIT >> 4), qd = qdesc + u * (2 * QBLK >> 4);
+        ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd, qd, idesc_s, (uint32_t)u, on);
         ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd + (SEG >> 4), qd + (QBLK >> 4), idesc_s, 1u, on);
         if (leader) {
-          ptx::umma_commit(empty + 8 * slot);
+          ptx::umma_commit(empty + 8 * sl);
           if (u == 1) ptx::umma_commit(s_full + 8 * buf);
         }
         __syncwarp();
+        next(sl, pr);
       }
       return true;
     };
     auto issue_pv = [&](int i) -> bool {
-      const int at = pos_v(i), units = nv(i);
+      const int units = nv(i);
       if (!ptx::wait_bar(p.status, p.limit, p_full, i & 1, 7)) return false;
+      ptx::tc_fence_after();
 #pragma unroll 1
       for (int u = 0; u < units; ++u) {
-        const int slot = (at + u) % UNITS;
-        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, ((at + u) / UNITS) & 1, 6)) return false;
-        ptx::tc_fence_after();
+        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, 6)) return false;
         // 16 keys per MMA: 16 rows of 128 B further in V and in P
-        const uint32_t vd = vdesc + ((slot * UNIT) >> 4), pd = pdesc + ((u * 64 * 128) >> 4), acc = i || u ? 1u : 0u;
+        const uint32_t vd = vdesc + slot * (UNIT >> 4), pd = pdesc + u * (64 * 128 >> 4), acc = i || u ? 1u : 0u;
         ptx::umma_bf16_k64<128, 128>(tmem + TM_O, vd, pd, idesc_o, acc, on);
         ptx::umma_bf16_k64<128, 128>(tmem + TM_O + N, vd + ((2 * 64 * 128) >> 4), pd, idesc_o, acc, on);
         if (leader) {
@@ -260,14 +259,22 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
           if (u == units - 1) ptx::umma_commit(p_empty);
         }
         __syncwarp();
+        next(slot, par);
       }
       return true;
     };
-    for (int i = 0; go && i < n; ++i) {
-      go = issue_s(i);
+#pragma unroll 1
+    for (int i = 0; go && i <= n; ++i) {   // S of chunk i, then P V of the one before
+      int sl = slot;
+      uint32_t pr = par;
+      const bool suffix = swapped && i == n - 1;            // its keys stand behind the values of the chunk before it
+      if (suffix)
+        for (int u = nv(i - 1); u > 0; --u) next(sl, pr);
+      if (i < n) go = issue_s(i, sl, pr);
+      if (!suffix) { slot = sl; par = pr; }
       if (go && i >= 1) go = issue_pv(i - 1);
+      if (suffix) { slot = sl; par = pr; }
     }
-    if (go) go = issue_pv(n - 1);
     if (go && leader) ptx::umma_commit(o_full);
     __syncwarp();
   } else if (warp >= 2) {
