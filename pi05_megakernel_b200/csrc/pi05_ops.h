@@ -60,8 +60,10 @@ GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k);
 // Fills in what the plan decides and the destination maps, and launches.  `width` and the pointers have to be set.
 cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream);
 cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream);
-// Shared-memory opt-in of the kernels behind the two calls above, once per device.
-cudaError_t ops_opt_in(int device);
+// Shared-memory opt-in of the kernel behind a plan, before its first launch on a device.  (Only what is used: the first touch loads a
+// kernel's code, and all of them together take 20 ms.)
+cudaError_t opt_in_gemm(const GemmPlan& g, int device);
+cudaError_t opt_in_attention(int tok_tile, int device);
 // One split of L1 and shared memory for all kernels of a chain: an SM that has to change it drains first, which would keep a
 // kernel's CTAs from becoming resident beside the ones of the kernel before.
 cudaError_t chain_opt_in(const void* kernel, int smem);

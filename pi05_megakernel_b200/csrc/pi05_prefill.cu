@@ -201,7 +201,7 @@ size_t part_floats(int sms, int tokens) {
 cudaError_t prefill_opt_in(int device) {
   static bool done[64] = {};
   if (done[device]) return cudaSuccess;
-  cudaError_t e = ops_opt_in(device);
+  cudaError_t e = cudaSuccess;
   const void* all[] = {(const void*)pf::tables_kernel, (const void*)pf::norm_kernel<-1>, (const void*)pf::norm_kernel<0>,
                        (const void*)pf::norm_kernel<1>, (const void*)pf::norm_kernel<2>, (const void*)pf::norm_kernel<4>,
                        (const void*)pf::norm_kernel<8>};
@@ -308,6 +308,10 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
   __nv_bfloat16* K = static_cast<__nv_bfloat16*>(keys);
   __nv_bfloat16* V = static_cast<__nv_bfloat16*>(values);
   const PrefillPlan pl = plan_prefill(h->sms, P);
+  for (const GemmPlan* g : {&pl.qkv, &pl.o, &pl.gu, &pl.down})
+    if (e == cudaSuccess) e = opt_in_gemm(*g, h->device);
+  if (e == cudaSuccess) e = opt_in_attention(pl.tok_tile, h->device);
+  if (e != cudaSuccess) { h->last_error = cudaGetErrorString(e); return PI05_ERR_CUDA; }
 
   // tensor maps: activations (rows = tokens, zero beyond), weights (all layers stacked), keys / values for the attention
   CUtensorMap a_qkv, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;

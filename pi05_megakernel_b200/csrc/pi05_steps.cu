@@ -437,7 +437,7 @@ cudaError_t opt_in(int device) {
       {(const void*)residual_norm_kernel<1>, 0}, {(const void*)residual_norm_kernel<2>, 0},
       {(const void*)residual_norm_kernel<4>, 0}, {(const void*)residual_norm_kernel<8>, 0},
       {(const void*)modulation_kernel, 0}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
-  cudaError_t e = ops_opt_in(device);
+  cudaError_t e = cudaSuccess;
   for (const auto& k : all)
     if (e == cudaSuccess) e = chain_opt_in(k.kernel, k.smem);
   if (e == cudaSuccess && device < 64) done[device] = true;
@@ -604,6 +604,9 @@ int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, st
   steps_free(g);
   Capture c(s, n_steps, n_layers);
   c.e = opt_in(s.device);
+  for (const GemmPlan* g : {&c.pq, &c.po, &c.pg, &c.pd})
+    if (c.e == cudaSuccess) c.e = opt_in_gemm(*g, s.device);
+  if (c.e == cudaSuccess) c.e = opt_in_attention(plan_attention(s.sms, s.batch, s.prefix).tok_tile, s.device);
   if (c.e == cudaSuccess) c.e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
   g->prologue = c.graph([&] { c.prologue(); });
   g->kernels_prologue = c.kernels;
