@@ -271,6 +271,9 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
  * makes the CTA the tile's owner, any other one a contributor of partial sums. */
 #define PI05_PREFILL_PLAN_INFO 6
 int pi05_prefill_plan(int sms, int tokens, int cta, int info[PI05_PREFILL_PLAN_INFO], int* segments, int capacity, int* count);
+/* FP32 words of split-K partial sums that the workspace of a handle for up to max_tokens tokens holds, and that a prefill of
+ * `tokens` of them writes, on a GPU of `sms` SMs; computed on the host (no counterpart in the reference, see above). */
+int pi05_prefill_partials(int sms, int max_tokens, int tokens, size_t* held, size_t* needed);
 /* Synchronises `stream` and reports a bounded device-side wait that gave up (PI05_ERR_DEVICE_TIMEOUT), like pi05_status. */
 int pi05_prefill_status(pi05_prefill_t h, void* stream, int* code, int* where);
 const char* pi05_prefill_last_error(pi05_prefill_t h);

@@ -56,6 +56,24 @@ def test_first_layers_against_the_oracle(tokens, mask, layers):
         assert float(err) < 4e-3, (name, float(err))
 
 
+def test_shorter_prompt_stays_in_the_workspace():
+    """660 tokens on a handle for 968: another cut than the longest prompt's, with more partial sums.  What lies behind the
+    workspace stays as it was, and the keys and values are those of a handle of the prompt's own size."""
+    from pi05_megakernel_b200.prefill import Pi05Prefill
+    inputs = FX.make_prefill_inputs(FX.PrefillGeometry(tokens=660), 31, "pad")
+    want = _run(FX.PrefillGeometry(tokens=660), inputs, 2)
+    dev = {k: v.cuda() for k, v in inputs.items()}
+    pre = Pi05Prefill(FX.PrefillGeometry(tokens=968), "cuda")
+    size = pre.ws.numel()
+    pre.ws = torch.full((size + (4 << 20),), 0xA5, dtype=torch.uint8, device="cuda")
+    pre.bind(dev)
+    k, v = pre.run(dev["embeddings"], dev["valid"], 2)
+    pre.status()
+    assert bool((pre.ws[size:] == 0xA5).all())
+    assert torch.equal(k.cpu()[:2], want[0][:2]) and torch.equal(v.cpu()[:2], want[1][:2])
+    pre.close()
+
+
 def test_full_depth_against_stored_reference_outputs():
     """All 18 layers at 160 tokens (right-padded mask): keys / values of layers 0, 8 and 17 against what the unmodified
     reference and its FP32 dispatch mode produced (tests/golden/prefill_full_p160.npz)."""

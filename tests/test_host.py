@@ -110,6 +110,19 @@ def test_prefill_plan(lib, sms, tokens):
                     end, peer = pb, peer + 1
 
 
+@pytest.mark.parametrize("sms", [132, 148, 152])
+def test_prefill_partials_fit_the_workspace(lib, sms):
+    """A handle for up to max_tokens tokens holds the partial sums of every shorter prompt, whatever cut that one takes."""
+    held, needed = ctypes.c_size_t(), ctypes.c_size_t()
+    need = [0]
+    for tokens in range(1, 4097):
+        assert lib.pi05_prefill_partials(sms, tokens, tokens, ctypes.byref(held), ctypes.byref(needed)) == _lib.OK
+        need.append(max(need[-1], needed.value))
+        assert held.value >= need[tokens], tokens
+    for args in ((1, 64, 64), (sms, 64, 65), (sms, 4097, 1), (sms, 64, 0)):
+        assert lib.pi05_prefill_partials(*args, ctypes.byref(held), ctypes.byref(needed)) == _lib.ERR_ARGUMENT
+
+
 def test_prefill_fixture_is_deterministic():
     geo = FX.PrefillGeometry(tokens=96, layers=1)
     shapes = FX.prefill_shapes(geo)
