@@ -178,6 +178,14 @@ const char* pi05_config_json(pi05_handle_t h);
 int pi05_schedule_plan(int sms, int batch, int prefix_len, const pi05_tuning* tuning, int* entries, int capacity,
                        int* count, int info[PI05_PLAN_INFO]);
 
+/* How the default launch (the chain of kernels) of `batch` observations of prefix_len tokens is cut on a GPU of `sms` SMs, by an
+ * engine created for (max_prefix, max_batch), computed on the host (no counterpart in the reference): info = {query tokens per
+ * CTA of the attention, CTAs that share the keys of a tile, K splits of the O and of the down projection}; the FP32 words of
+ * partial sums that the engine's workspace holds and that this binding writes. */
+#define PI05_CHUNK_PLAN_INFO 4
+int pi05_chunk_plan(int sms, int max_batch, int max_prefix, int batch, int prefix_len, int info[PI05_CHUNK_PLAN_INFO], size_t* held,
+                    size_t* needed);
+
 /* Tensor parallel (no counterpart in the reference, which runs on one GPU only): tp_size engines, one per GPU, each
  * bound to the SAME 25 inputs in its own GPU's memory, compute one chunk together.  Rank r streams only its share of
  * the weights - query heads 8 r / tp_size .. of wq (and the matching columns of wo), MLP columns 4096 r / tp_size ..

@@ -534,6 +534,7 @@ int build_graphs(pi05_engine* h, int n_steps, int n_layers) {
   s.state = region_ptr<int>(h, "state");
   s.temb = region_ptr<float>(h, "temb"); s.hid = region_ptr<float>(h, "hid"); s.cond = region_ptr<float>(h, "cond");
   s.mod = region_ptr<float>(h, "mod"); s.x = region_ptr<float>(h, "x"); s.part = region_ptr<float>(h, "part");
+  s.part_floats = find_region(h, "part")->bytes / 4;
   s.rope = region_ptr<uint32_t>(h, "rope");
   s.h = region_ptr<__nv_bfloat16>(h, "h"); s.an = region_ptr<__nv_bfloat16>(h, "an_attn");
   s.q = region_ptr<__nv_bfloat16>(h, "q"); s.k = region_ptr<__nv_bfloat16>(h, "k"); s.v = region_ptr<__nv_bfloat16>(h, "v");
@@ -978,6 +979,18 @@ int pi05_workspace_region(pi05_handle_t h, const char* name, size_t* offset, siz
 int pi05_schedule_plan(int sms, int batch, int prefix_len, const pi05_tuning* tuning, int* entries, int capacity,
                        int* count, int info[PI05_PLAN_INFO]) {
   return pi05_schedule_plan_tp(sms, batch, prefix_len, 0, 1, tuning, entries, capacity, count, info);
+}
+
+int pi05_chunk_plan(int sms, int max_batch, int max_prefix, int batch, int prefix_len, int info[PI05_CHUNK_PLAN_INFO], size_t* held,
+                    size_t* needed) {
+  if (sms < 2 || sms > 1024 || max_batch < 1 || max_batch > MAXB || max_prefix < 1 || max_prefix > 4096 || batch < 1 || batch > max_batch ||
+      prefix_len < 1 || prefix_len > max_prefix || !info || !held || !needed)
+    return PI05_ERR_ARGUMENT;
+  const StepPlan p = steps_plan(sms, batch, prefix_len);
+  info[0] = p.tok_tile; info[1] = p.splits; info[2] = p.o_splits; info[3] = p.down_splits;
+  *held = steps_part_floats(sms, max_batch, max_prefix);
+  *needed = p.part_floats;
+  return PI05_OK;
 }
 
 int pi05_schedule_plan_tp(int sms, int batch, int prefix_len, int tp_rank, int tp_size, const pi05_tuning* tuning,

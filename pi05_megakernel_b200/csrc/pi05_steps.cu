@@ -590,18 +590,32 @@ struct Capture {
 
 }  // namespace
 
+StepPlan steps_plan(int sms, int batch, int prefix) {
+  const AttnPlan a = plan_attention(sms, batch, prefix);
+  StepPlan p;
+  p.tok_tile = a.tok_tile; p.splits = a.splits;
+  p.o_splits = plan_gemm(sms, T * batch, W, QD, gemm::EPI_PART).splits;
+  p.down_splits = plan_gemm(sms, T * batch, W, FF, gemm::EPI_PART).splits;
+  p.part_floats = (size_t)std::max(p.o_splits, p.down_splits) * T * batch * W;
+  if (a.splits > 1) p.part_floats = std::max(p.part_floats, (size_t)batch * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
+  return p;
+}
+
+// Every number of chunks of every batch is asked: the longest prefix does not need the most (148 SMs, five observations: tiles of 8
+// tokens over four CTAs up to 896 keys, of 4 over two from there on).
 size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   size_t most = 0;
-  for (int b = 1; b <= max_batch; ++b) {
-    for (int k : {QD, FF}) most = std::max(most, (size_t)plan_gemm(sms, T * b, W, k, gemm::EPI_PART).splits * T * b * W);
-    const AttnPlan a = plan_attention(sms, b, max_prefix);          // splits grow with the prefix
-    if (a.splits > 1) most = std::max(most, (size_t)b * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
-  }
+  for (int b = 1; b <= max_batch; ++b)
+    for (int prefix = 1; prefix <= max_prefix; prefix += attn::KCH) most = std::max(most, steps_plan(sms, b, prefix).part_floats);
   return most;
 }
 
 int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, std::string* error) {
   steps_free(g);
+  if (steps_plan(s.sms, s.batch, s.prefix).part_floats > s.part_floats) {
+    *error = "the workspace does not hold the partial sums of this binding";
+    return PI05_ERR_UNSUPPORTED;
+  }
   Capture c(s, n_steps, n_layers);
   c.e = opt_in(s.device);
   for (const GemmPlan* g : {&c.pq, &c.po, &c.pg, &c.pd})

@@ -16,7 +16,8 @@ struct StepSetup {
   float* actions;
   unsigned int* status;
   int* state;                                // {Euler step, finished blocks of the step tail}
-  float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions (steps_part_floats)
+  float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions
+  size_t part_floats;                        // what `part` holds (steps_part_floats)
   uint32_t* rope;
   __nv_bfloat16 *h, *an, *q, *k, *v, *attn, *act;
   const void *pool_k, *pool_v;               // prefix cache; strides in elements
@@ -33,6 +34,13 @@ struct StepGraphs {
   int kernels_prologue = 0, kernels_step = 0;
 };
 
+// How a binding is cut: query tokens per CTA of the attention and CTAs that share the keys of a tile, K splits of the O and down
+// projections, FP32 words of partial sums.
+struct StepPlan {
+  int tok_tile, splits, o_splits, down_splits;
+  size_t part_floats;
+};
+StepPlan steps_plan(int sms, int batch, int prefix);
 // FP32 words of partial sums that up to `max_batch` observations with up to `max_prefix` prefix tokens need.
 size_t steps_part_floats(int sms, int max_batch, int max_prefix);
 // Captures and instantiates the graphs for (n_steps, n_layers); frees what `g` held.

@@ -1,5 +1,7 @@
 """The kernels of the chain (projections, attention, residual + norm) at the sizes where their cuts change, against the oracle
 within the reference harness's band.  Every test needs a B200."""
+import ctypes
+
 import pytest
 import torch
 
@@ -33,6 +35,35 @@ def test_chunk_cuts(prefix, batch, mask, variant):
         d = O.band(want, first.reshape(batch, 50, 32)[b], exact)
         assert d["pass"], (b, d)
     arm.close()
+
+
+def test_smaller_binding_stays_in_the_workspace():
+    """Five observations of 700 tokens on an engine made for 968: an attention cut with more partial sums than the longest prefix's.
+    What lies behind the workspace stays as it was, and the actions are those of an engine of the binding's own size."""
+    from pi05_megakernel_b200 import _lib
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo, batch = FX.Geometry(prefix=700), 5
+    stacked, _ = FX.make_batch(geo, FX.SEEDS[0], batch, "cpu", ["pad"] * batch)
+    dev = {k: v.cuda() for k, v in stacked.items()}
+    arm = Pi05Arm(geo, "b200-s1-l2", "cuda", batch=batch)
+    arm.bind(dev)
+    arm.launch()
+    arm.status()
+    want = arm.outputs()["actions"].clone()
+    arm.close()
+    lib, h, n = _lib.load(), ctypes.c_void_p(), ctypes.c_size_t()
+    assert lib.pi05_create(0, 968, batch, 0, 1, ctypes.byref(h)) == _lib.OK
+    assert lib.pi05_workspace_bytes(h, ctypes.byref(n)) == _lib.OK
+    ws = torch.full((n.value + (4 << 20),), 0xA5, dtype=torch.uint8, device="cuda")
+    got = torch.zeros_like(want)
+    ptrs = (ctypes.c_void_p * _lib.NUM_INPUTS)(*[dev[k].data_ptr() for k in FX.ORDER])
+    assert lib.pi05_bind(h, ptrs, geo.prefix, batch, got.data_ptr(), ws.data_ptr(), n.value) == _lib.OK
+    assert lib.pi05_launch(h, 1, 2, torch.cuda.current_stream().cuda_stream, None) == _lib.OK
+    code, where = ctypes.c_int(), ctypes.c_int()
+    assert lib.pi05_status(h, ctypes.byref(code), ctypes.byref(where)) == _lib.OK
+    assert bool((ws[n.value:] == 0xA5).all())
+    assert torch.equal(got, want)
+    assert lib.pi05_destroy(h) == _lib.OK
 
 
 @pytest.mark.parametrize("prefix", [300, 968])

@@ -123,6 +123,25 @@ def test_prefill_partials_fit_the_workspace(lib, sms):
         assert lib.pi05_prefill_partials(*args, ctypes.byref(held), ctypes.byref(needed)) == _lib.ERR_ARGUMENT
 
 
+@pytest.mark.parametrize("sms", [132, 148, 152])
+def test_chunk_partials_fit_the_workspace(lib, sms):
+    """An engine for (max_batch, max_prefix) holds the partial sums of every smaller batch and shorter prefix."""
+    info, held, needed = (ctypes.c_int * 4)(), ctypes.c_size_t(), ctypes.c_size_t()
+
+    def plan(mb, mp, b, p):
+        assert lib.pi05_chunk_plan(sms, mb, mp, b, p, info, ctypes.byref(held), ctypes.byref(needed)) == _lib.OK
+        return held.value, needed.value
+
+    prefixes = sorted({p for c in range(32) for p in (c * 128 + 1, c * 128 + 77, c * 128 + 128)})
+    need = {(b, p): plan(b, p, b, p)[1] for b in range(1, 17) for p in prefixes}
+    for mb in range(1, 17):
+        for mp in prefixes:
+            most = max(n for (b, p), n in need.items() if b <= mb and p <= mp)
+            assert plan(mb, mp, 1, 1)[0] >= most, (mb, mp)
+    for args in ((1, 1, 64, 1, 64), (sms, 17, 64, 1, 64), (sms, 2, 64, 3, 64), (sms, 2, 64, 1, 65), (sms, 1, 4097, 1, 1)):
+        assert lib.pi05_chunk_plan(*args, info, ctypes.byref(held), ctypes.byref(needed)) == _lib.ERR_ARGUMENT
+
+
 def test_prefill_fixture_is_deterministic():
     geo = FX.PrefillGeometry(tokens=96, layers=1)
     shapes = FX.prefill_shapes(geo)
