@@ -123,7 +123,9 @@ int pi05_refresh(pi05_handle_t h);
 
 /* Replaces launch() (mk/pi05_mk.cu:3523-3620): one whole action chunk, asynchronous on `stream` (a cudaStream_t;
  * NULL = default stream).  n_steps <= 10 Euler steps and n_layers <= 18 expert layers are run (dt stays -0.1);
- * the graded chunk is (10, 18).  stamps, if non-NULL, is a device buffer of PI05_NUM_STAMPS uint64 that
+ * the graded chunk is (10, 18).  The call neither waits nor takes device memory, whatever its arguments, and may be made while the
+ * stream is being captured: the chunk's kernels then become part of the capture, whose replays the caller waits for
+ * (pi05_status waits for launches outside captures).  stamps, if non-NULL, is a device buffer of PI05_NUM_STAMPS uint64 that
  * receives globaltimer values at stage boundaries of the first layer passes and, from three GEMM CTAs, at the
  * points of their pipeline in the second pass (the reference's tstamp tensor, mk/pi05_mk.cu:351).  The caller
  * zeroes it. */

@@ -158,7 +158,8 @@ struct pi05_engine {
   bool in_flight = false;        // a launch has been issued since the last pi05_status
   bool can_cluster = false;      // the device takes the whole grid as clusters of two
   bool graphs = true;            // the chunk may run as graphs of kernels (false: the static entry point, which allocates nothing)
-  StepGraphs steps;              // the chunk's kernels, captured for the bound tensors
+  StepSetup setup = {};          // the bound tensors as the chain's kernels take them
+  StepGraphs steps;              // the chain, captured for them
   std::string config;
   std::string last_error;
 };
@@ -503,7 +504,7 @@ void describe(pi05_engine* h) {
            "\"mma\": \"tcgen05 cta_group::1 M128 N%d K16 bf16\", \"sync\": \"device-scope counters, bounded waits\", "
            "\"clusters_of_2\": %s, \"observations_per_mma\": %d, \"tp_rank\": %d, \"tp_size\": %d, \"schedule\": \"%s\"}",
            h->steps.step ? "chain of kernels replayed from graphs (the fields below: the persistent kernel, pi05_chunk_kernel)" : "pi05_chunk_kernel",
-           h->steps.step ? h->steps.kernels_prologue + h->steps.n_steps * h->steps.kernels_step : 1, h->grid, THREADS, SMEM_BYTES, h->n_gemm, h->grid - h->n_gemm, h->gn == 1 ? NSTG : 3,
+           h->steps.step ? h->steps.kernels_prologue + NS * h->steps.kernels_step : 1, h->grid, THREADS, SMEM_BYTES, h->n_gemm, h->grid - h->n_gemm, h->gn == 1 ? NSTG : 3,
            W_STAGE_BYTES + h->gn * A_STAGE_BYTES, h->n_units[0], h->n_units[1], h->n_units[2], h->n_units[3], 64 * h->gn,
            h->clustered ? "true" : "false", h->gn, h->tp_rank, h->tp_size,
            !grouped ? "one observation (units serve every observation in turn)"
@@ -514,7 +515,7 @@ void describe(pi05_engine* h) {
 
 bool valid_handle(pi05_handle_t h) { return h != nullptr; }
 
-// Whether a launch without debug controls runs as graphs of kernels (pi05_steps.cu).  The persistent kernel stays for
+// Whether a launch without debug controls runs as the chain of kernels (pi05_steps.cu).  The persistent kernel stays for
 // tensor parallel, for the static entry point, for debug controls and for callers that set one of its own tuning settings.
 // Persistent against graphs, ms: one observation 5.30 / 4.67 at prefix 128 and 6.66 / 5.06 at 968, sixteen 18.8 / 10.3 and 41.1 / 12.6.
 bool uses_graphs(const pi05_engine* h) {
@@ -524,7 +525,7 @@ bool uses_graphs(const pi05_engine* h) {
   return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0;
 }
 
-int build_graphs(pi05_engine* h, int n_steps, int n_layers) {
+StepSetup step_setup(const pi05_engine* h) {
   StepSetup s;
   memset(&s, 0, sizeof s);
   s.device = h->device; s.sms = h->sms; s.batch = h->batch; s.prefix = h->prefix;
@@ -544,7 +545,7 @@ int build_graphs(pi05_engine* h, int n_steps, int n_layers) {
   s.page_table = region_ptr<int>(h, "page_table");
   s.pages_per_obs = h->pages_per_obs; s.page_tokens = h->page_tokens;
   s.wait_limit = h->wait_limit;
-  return steps_build(s, n_steps, n_layers, &h->steps, &h->last_error);
+  return s;
 }
 
 }  // namespace
@@ -781,7 +782,8 @@ int pi05_bind_view(pi05_handle_t h, const void* const inputs[PI05_NUM_INPUTS], c
                  cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail_cuda(h, "cudaMemcpy(page table)", e);
   steps_free(&h->steps);
-  if (uses_graphs(h) && (rc = build_graphs(h, NS, NL))) return rc;
+  h->setup = step_setup(h);
+  if (uses_graphs(h) && (rc = steps_build(h->setup, &h->steps, &h->last_error))) return rc;
   describe(h);
   e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceSynchronize", e);
@@ -798,10 +800,7 @@ int pi05_debug(pi05_handle_t h, int max_stage, long long wait_limit_cycles, int 
   if (!valid_handle(h) || drop_event >= NEVENTS) return PI05_ERR_ARGUMENT;
   h->drop_event = drop_event < 0 ? -1 : drop_event;
   h->max_stage = max_stage < 0 ? 0x7fffffff : max_stage;
-  if (wait_limit_cycles > 0 && wait_limit_cycles != h->wait_limit) {
-    h->wait_limit = wait_limit_cycles;
-    h->steps.n_steps = 0;          // captured with the old limit: the next launch captures again
-  }
+  if (wait_limit_cycles > 0) h->wait_limit = wait_limit_cycles;
   return PI05_OK;
 }
 
@@ -814,17 +813,14 @@ int pi05_launch(pi05_handle_t h, int n_steps, int n_layers, void* stream, unsign
   // stamps or a debug control wanted: the traced build of the persistent kernel
   const bool debug = stamps != nullptr || h->max_stage != 0x7fffffff || h->drop_event >= 0;
   if (!debug && uses_graphs(h)) {
-    if (h->steps.n_steps != n_steps || h->steps.n_layers != n_layers) {
-      if (h->in_flight) {          // the graphs that are about to be replaced may still be running
-        const cudaError_t e = cudaEventSynchronize(h->done);
-        if (e != cudaSuccess) return fail_cuda(h, "cudaEventSynchronize", e);
-      }
-      const int rc = build_graphs(h, n_steps, n_layers);
-      if (rc != PI05_OK) return rc;
-    }
-    cudaError_t e = steps_launch(h->steps, (cudaStream_t)stream);
-    if (e != cudaSuccess) return fail_cuda(h, "graph launch", e);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing((cudaStream_t)stream, &cap);
+    if (e != cudaSuccess) return fail_cuda(h, "cudaStreamIsCapturing", e);
+    h->setup.wait_limit = h->wait_limit;
+    const int rc = steps_launch(h->steps, h->setup, n_steps, n_layers, cap != cudaStreamCaptureStatusNone, (cudaStream_t)stream, &h->last_error);
+    if (rc != PI05_OK) return rc;
     h->launches++;
+    if (cap != cudaStreamCaptureStatusNone) return PI05_OK;      // (the event would only be recorded into the capture)
     e = cudaEventRecord(h->done, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail_cuda(h, "cudaEventRecord", e);
     h->in_flight = true;

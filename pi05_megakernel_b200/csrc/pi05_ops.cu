@@ -169,7 +169,7 @@ GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k) {
   return g;
 }
 
-cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream) {
+cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream, bool early) {
   const Cut* cut = nullptr;
   for (const Cut& c : kCuts)
     if (c.epi == g.epi && c.bn == g.bn && c.pair == g.pair && c.ks == g.ks && c.sk == g.sk) cut = &c;
@@ -191,7 +191,7 @@ cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream) {
   }
   if (!ok) return cudaErrorInvalidValue;
   const int ctas = g.pair ? 2 * p.units : p.units, grid = g.sk || g.grid < ctas ? g.grid : ctas;
-  return launch_chained(cut->kernel, grid, gemm::THREADS_G, g.smem, stream, g.pair ? 2 : 1, p);
+  return launch_kernel(cut->kernel, grid, gemm::THREADS_G, g.smem, stream, g.pair ? 2 : 1, early, p);
 }
 
 namespace {

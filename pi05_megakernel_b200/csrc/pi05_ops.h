@@ -13,17 +13,19 @@
 namespace pi05 {
 
 // Launch with programmatic stream serialisation (the kernel may become resident and set up while the one before it in the
-// stream runs) and, with `cluster` > 1, as clusters of that many CTAs.
+// stream runs; `early` false: without it) and, with `cluster` > 1, as clusters of that many CTAs.
 template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream, int cluster, bool early, Args&&... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute at[2];
   int n = 0;
-  at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[n].val.programmaticStreamSerializationAllowed = 1;
-  ++n;
+  if (early) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   if (cluster > 1) {
     at[n].id = cudaLaunchAttributeClusterDimension;
     at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
@@ -31,6 +33,10 @@ cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_
   }
   cfg.attrs = at; cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+  return launch_kernel(kernel, grid, block, smem, stream, cluster, true, std::forward<Args>(args)...);
 }
 
 // An operand [rows, K] BF16 row-major as {64 k, rows, K / 64}, box {64, box_rows, blocks}, 128-byte swizzle: one copy brings
@@ -57,8 +63,9 @@ struct GemmPlan {
 GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs = -1);
 // The stream-K cut of a projection with partial sums: 128 x 256 tiles, one equal range of 64-k blocks per CTA.
 GemmPlan plan_gemm_sk(int sms, int tokens, int n, int k);
-// Fills in what the plan decides and the destination maps, and launches.  `width` and the pointers have to be set.
-cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream);
+// Fills in what the plan decides and the destination maps, and launches.  `width` and the pointers have to be set.  `early`: may
+// start while the kernel before it in the stream runs.
+cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream, bool early = true);
 cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream);
 // Shared-memory opt-in of the kernel behind a plan, before its first launch on a device.  (Only what is used: the first touch loads a
 // kernel's code, and all of them together take 20 ms.)

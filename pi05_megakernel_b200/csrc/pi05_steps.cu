@@ -2,8 +2,10 @@
 //
 // A layer pass is seven kernels - QKV projection (+ RoPE), attention, O projection, gated residual + adaRMS, gate / up
 // projection (+ GeGLU), down projection, gated residual + adaRMS - and an Euler step is 18 of them, the last residual being
-// the step tail.  The step's kernels are captured once per binding; the Euler step index lives in device memory, so the
-// same graph is launched ten times.  Every kernel is launched with programmatic stream serialisation: its CTAs become
+// the step tail.  The step's kernels are captured once per binding; the Euler step index and the number of steps live in
+// device memory, so the same graph is launched once per step.  What the graphs do not fit - fewer layers, a stream that is being
+// captured, another wait limit than at bind - is launched kernel by kernel: a launch never builds a graph.  Every kernel but the
+// first of a step is launched with programmatic stream serialisation: its CTAs become
 // resident, set up and request their weights (or cached keys) while the kernel before it runs, and wait for it only
 // before they touch what it wrote.  Measured on B200, a hop along such a chain (last store to first load) costs 1.25 us
 // against 1.75-2.3 us for a device-scope counter of a persistent kernel, and every stage may use all SMs.
@@ -36,11 +38,11 @@ struct TableArgs {
   uint32_t* rope;
   const uint8_t* mask;
   int* state;
-  int prefix;
+  int prefix, n_steps;
 };
 
 // Time embedding (FP64, reference/pi05.py:232-237), RoPE tables of the suffix positions (reference/pi05.py:218-229, they
-// start at the observation's number of valid prefix tokens) and the step counter.  blockIdx.y = observation.
+// start at the observation's number of valid prefix tokens) and the step state.  blockIdx.y = observation.
 __global__ void __launch_bounds__(256) tables_kernel(const TableArgs p) {
   const int b = blockIdx.y, tid = threadIdx.x, gtid = blockIdx.x * 256 + tid, gn = gridDim.x * 256;
   __shared__ int s_cnt;
@@ -68,7 +70,7 @@ __global__ void __launch_bounds__(256) tables_kernel(const TableArgs p) {
       const double phase = (double)p.t_steps[s] * (1.0 / period * 2 * 3.141592653589793);
       p.temb[i] = (float)(j < W / 2 ? sin(phase) : cos(phase));
     }
-    if (gtid < 2) p.state[gtid] = 0;
+    if (gtid < 3) p.state[gtid] = gtid == 2 ? p.n_steps : 0;
   }
 }
 
@@ -217,7 +219,8 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(const NormArgs p) {
   __shared__ float red[2][8];
   const int c0 = threadIdx.x * 4;
   ptx::grid_dep_launch();
-  // the modulation was finished before this graph was launched, and the step counter only moves at the end of a step
+  // the modulation was finished before the step began (its first kernel does not start early), and the step counter only moves at
+  // the end of a step
   const float* mod_s = p.mod + (size_t)__ldcg(p.state) * NNORM * MODW;
   const float4 g = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)p.gate_norm * MODW + 2 * W + c0));
   const float4 sc = __ldcg(reinterpret_cast<const float4*>(mod_s + (size_t)p.next_norm * MODW + c0));
@@ -266,7 +269,7 @@ struct TailArgs {
   float *x, *actions;
   const unsigned int* status;
   float dt;
-  int gate_norm, n_steps, tokens, splits;
+  int gate_norm, tokens, splits;
 };
 
 constexpr int TAIL_THREADS = 256;
@@ -284,8 +287,9 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) tail_kernel(const TailArgs p)
   __shared__ float red[8], s_x[ADIM];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = tid * 4;
   ptx::grid_dep_launch();
-  const int step = INIT ? -1 : __ldcg(p.state);
-  const bool last = !INIT && step + 1 == p.n_steps;
+  const int4 state = INIT ? make_int4(-1, 0, 0, 0) : __ldcg(reinterpret_cast<const int4*>(p.state));
+  const int step = state.x;
+  const bool last = !INIT && step + 1 == state.z;
   float4 wo[4][8];                                          // action_out rows 4 warp .. 4 warp + 3, columns 4 lane + 128 j
   if (!INIT) {
 #pragma unroll
@@ -444,20 +448,31 @@ cudaError_t opt_in(int device) {
   return e;
 }
 
-struct Capture {
+// The kernels of a chunk, launched into `stream`, which may be one that is being captured.
+struct Chain {
   const StepSetup& s;
   int n_steps, n_layers, kernels = 0;
-  cudaStream_t stream = nullptr;
-  cudaError_t e = cudaSuccess;
+  cudaStream_t stream;
+  cudaError_t e;
   std::string what;
   GemmPlan pq, po, pg, pd;
+  CUtensorMap a_qkv, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;
+  attn::Args ap;
 
-  Capture(const StepSetup& setup, int steps, int layers) : s(setup), n_steps(steps), n_layers(layers) {
+  Chain(const StepSetup& setup, int steps, int layers, cudaStream_t into) : s(setup), n_steps(steps), n_layers(layers), stream(into) {
     const int tokens = T * s.batch;
     pq = plan_gemm(s.sms, tokens, QKVW, W, gemm::EPI_QKV);
     po = plan_gemm(s.sms, tokens, W, QD, gemm::EPI_PART);
     pg = plan_gemm(s.sms, tokens, 2 * FF, W, gemm::EPI_GEGLU);
     pd = plan_gemm(s.sms, tokens, W, FF, gemm::EPI_PART);
+    const AttnPlan pa = plan_attention(s.sms, s.batch, s.prefix);
+    memset(&ap, 0, sizeof ap);
+    ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits;
+    e = opt_in(s.device);
+    for (const GemmPlan* g : {&pq, &po, &pg, &pd})
+      if (e == cudaSuccess) e = opt_in_gemm(*g, s.device);
+    if (e == cudaSuccess) e = opt_in_attention(ap.tok_tile, s.device);
+    if (e == cudaSuccess) encode();
   }
 
   template <typename... P, typename... A>
@@ -475,17 +490,17 @@ struct Capture {
     t.ain_w = (const float*)s.in[0]; t.ain_b = (const float*)s.in[1];
     t.aout_w = (const float*)s.in[6]; t.aout_b = (const float*)s.in[7];
     t.x = s.x; t.actions = s.actions; t.status = s.status; t.dt = (float)(-1.0 / NS);
-    t.gate_norm = 2 * (n_layers - 1) + 1; t.n_steps = n_steps; t.tokens = T * s.batch; t.splits = pd.splits;
+    t.gate_norm = 2 * (n_layers - 1) + 1; t.tokens = T * s.batch; t.splits = pd.splits;
     return t;
   }
 
   void prologue() {
+    if (e != cudaSuccess) return;
     TableArgs t;
     const double dt = -1.0 / NS;
     for (int i = 0; i < NS; ++i) t.t_steps[i] = (float)(1.0 + i * dt);
-    t.temb = s.temb; t.rope = s.rope; t.mask = (const uint8_t*)s.in[24]; t.state = s.state; t.prefix = s.prefix;
-    tables_kernel<<<dim3(std::max(8, s.sms / s.batch), s.batch), 256, 0, stream>>>(t);
-    e = cudaGetLastError();
+    t.temb = s.temb; t.rope = s.rope; t.mask = (const uint8_t*)s.in[24]; t.state = s.state; t.prefix = s.prefix; t.n_steps = n_steps;
+    e = launch_kernel(tables_kernel, dim3(std::max(8, s.sms / s.batch), s.batch), 256, 0, stream, 1, false, t);
     ++kernels;
     MatArgs m;
     memset(&m, 0, sizeof m);
@@ -502,7 +517,7 @@ struct Capture {
   }
 
   void project(const GemmPlan& g, const CUtensorMap& a, const CUtensorMap* b0, const CUtensorMap* b1, const CUtensorMap* b2,
-               int width, int layer) {
+               int width, int layer, bool early = true) {
     if (e != cudaSuccess) return;
     gemm::Args p;
     memset(&p, 0, sizeof p);
@@ -511,19 +526,13 @@ struct Capture {
     if (b2) p.b2 = *b2;
     p.tokens = T * s.batch; p.layer = layer; p.width = width; p.status = s.status; p.limit = s.wait_limit;
     p.q = s.q; p.k = s.k; p.v = s.v; p.rope = s.rope; p.act = s.act; p.part = s.part;
-    e = launch_gemm(g, p, stream);
+    e = launch_gemm(g, p, stream, early);
     ++kernels;
   }
 
-  void step() {
-    const int tokens = T * s.batch;
-    CUtensorMap a_qkv, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;
-    attn::Args ap;
-    memset(&ap, 0, sizeof ap);
-    const AttnPlan pa = plan_attention(s.sms, s.batch, s.prefix);
-    ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits;
+  void encode() {
+    const uint64_t L = NL, M = T * s.batch;
     ap.merge = s.part;
-    const uint64_t L = NL, M = tokens;
     // full pages, and the last page of an observation cut at its last valid token; 128 keys are one copy where pages allow it
     const int tail = s.prefix - (s.prefix - 1) / s.page_tokens * s.page_tokens;
     ap.k_rows = s.pages_per_obs == 1 || s.page_tokens % attn::KCH == 0 ? attn::KCH : 64;
@@ -549,10 +558,14 @@ struct Capture {
     ap.page_table = s.page_table; ap.pages_per_obs = s.pages_per_obs; ap.page_tokens = s.page_tokens;
     ap.valid = (const uint8_t*)s.in[24]; ap.out = s.attn; ap.prefix = s.prefix; ap.suffix = T; ap.obs_tokens = T;
     ap.early = 1; ap.status = s.status; ap.limit = s.wait_limit;
+  }
+
+  void step() {
+    const int tokens = T * s.batch;
     NormArgs n;
     n.part = s.part; n.h = s.h; n.out = s.an; n.mod = s.mod; n.state = s.state;
     for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
-      project(pq, a_qkv, &wq, &wk, &wv, 0, l);
+      project(pq, a_qkv, &wq, &wk, &wv, 0, l, l > 0);      // (what a step leaves behind is complete before the next one's first kernel starts)
       ap.layer = l;
       if (e == cudaSuccess) { e = launch_attention(ap, s.batch, stream); ++kernels; }
       project(po, a_o, &wo, nullptr, nullptr, W, l);
@@ -610,17 +623,21 @@ size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   return most;
 }
 
-int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, std::string* error) {
+namespace {
+int failed(const Chain& c, const char* doing, std::string* error) {
+  *error = doing + (": " + (c.what.empty() ? std::string(cudaGetErrorString(c.e)) : c.what));
+  cudaGetLastError();
+  return PI05_ERR_CUDA;
+}
+}  // namespace
+
+int steps_build(const StepSetup& s, StepGraphs* g, std::string* error) {
   steps_free(g);
   if (steps_plan(s.sms, s.batch, s.prefix).part_floats > s.part_floats) {
     *error = "the workspace does not hold the partial sums of this binding";
     return PI05_ERR_UNSUPPORTED;
   }
-  Capture c(s, n_steps, n_layers);
-  c.e = opt_in(s.device);
-  for (const GemmPlan* g : {&c.pq, &c.po, &c.pg, &c.pd})
-    if (c.e == cudaSuccess) c.e = opt_in_gemm(*g, s.device);
-  if (c.e == cudaSuccess) c.e = opt_in_attention(plan_attention(s.sms, s.batch, s.prefix).tok_tile, s.device);
+  Chain c(s, NS, NL, nullptr);
   if (c.e == cudaSuccess) c.e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
   g->prologue = c.graph([&] { c.prologue(); });
   g->kernels_prologue = c.kernels;
@@ -632,20 +649,30 @@ int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, st
     cudaStreamDestroy(c.stream);
   }
   if (c.e != cudaSuccess) {
-    *error = "capture of the chunk's kernels: " + (c.what.empty() ? std::string(cudaGetErrorString(c.e)) : c.what);
-    cudaGetLastError();
     steps_free(g);
-    return PI05_ERR_CUDA;
+    return failed(c, "capture of the chunk's kernels", error);
   }
-  g->n_steps = n_steps;
-  g->n_layers = n_layers;
+  g->wait_limit = s.wait_limit;
   return PI05_OK;
 }
 
-cudaError_t steps_launch(const StepGraphs& g, cudaStream_t stream) {
-  cudaError_t e = cudaGraphLaunch(g.prologue, stream);
-  for (int s = 0; s < g.n_steps && e == cudaSuccess; ++s) e = cudaGraphLaunch(g.step, stream);
-  return e;
+int steps_launch(const StepGraphs& g, const StepSetup& s, int n_steps, int n_layers, bool capturing, cudaStream_t stream, std::string* error) {
+  // a graph cannot be launched into a stream that is being captured
+  const bool graphs = g.step && !capturing && n_layers == NL && s.wait_limit == g.wait_limit;
+  if (graphs && n_steps == NS) {
+    cudaError_t e = cudaGraphLaunch(g.prologue, stream);
+    for (int i = 0; i < n_steps && e == cudaSuccess; ++i) e = cudaGraphLaunch(g.step, stream);
+    if (e == cudaSuccess) return PI05_OK;
+    *error = std::string("graph launch: ") + cudaGetErrorString(e);
+    return PI05_ERR_CUDA;
+  }
+  Chain c(s, n_steps, n_layers, stream);
+  c.prologue();
+  for (int i = 0; i < n_steps && c.e == cudaSuccess; ++i) {
+    if (graphs) c.e = cudaGraphLaunch(g.step, stream);
+    else c.step();
+  }
+  return c.e == cudaSuccess ? PI05_OK : failed(c, "launch of the chunk's kernels", error);
 }
 
 void steps_free(StepGraphs* g) {

@@ -15,7 +15,7 @@ struct StepSetup {
   const void* const* in;                     // the 25 inputs
   float* actions;
   unsigned int* status;
-  int* state;                                // {Euler step, finished blocks of the step tail}
+  int* state;                                // {Euler step, finished blocks of the step tail, Euler steps of this chunk}
   float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions
   size_t part_floats;                        // what `part` holds (steps_part_floats)
   uint32_t* rope;
@@ -28,9 +28,10 @@ struct StepSetup {
   long long wait_limit;
 };
 
+// The prologue for all Euler steps, and one step of all layers.
 struct StepGraphs {
   cudaGraphExec_t prologue = nullptr, step = nullptr;
-  int n_steps = 0, n_layers = 0;             // what the graphs were captured for
+  long long wait_limit = 0;                  // what the graphs were captured with
   int kernels_prologue = 0, kernels_step = 0;
 };
 
@@ -43,10 +44,11 @@ struct StepPlan {
 StepPlan steps_plan(int sms, int batch, int prefix);
 // FP32 words of partial sums that up to `max_batch` observations with up to `max_prefix` prefix tokens need.
 size_t steps_part_floats(int sms, int max_batch, int max_prefix);
-// Captures and instantiates the graphs for (n_steps, n_layers); frees what `g` held.
-int steps_build(const StepSetup& s, int n_steps, int n_layers, StepGraphs* g, std::string* error);
-// Enqueues one chunk.
-cudaError_t steps_launch(const StepGraphs& g, cudaStream_t stream);
+// Captures and instantiates the graphs; frees what `g` held.
+int steps_build(const StepSetup& s, StepGraphs* g, std::string* error);
+// Enqueues one chunk: the graphs where they fit, else kernel by kernel.  Allocates nothing and does not wait.  `capturing`: the stream
+// is being captured.
+int steps_launch(const StepGraphs& g, const StepSetup& s, int n_steps, int n_layers, bool capturing, cudaStream_t stream, std::string* error);
 void steps_free(StepGraphs* g);
 
 }  // namespace pi05

@@ -66,6 +66,62 @@ def test_smaller_binding_stays_in_the_workspace():
     assert lib.pi05_destroy(h) == _lib.OK
 
 
+@pytest.mark.parametrize("batch,variant", [(1, "b200"), (3, "b200-s2-l2")])
+def test_launch_into_a_capture(batch, variant):
+    """A launch may be recorded into a CUDA graph by its caller; a replay is what a launch is, on the inputs of the moment."""
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo = FX.Geometry(prefix=200)
+    stacked, _ = FX.make_batch(geo, FX.SEEDS[0], batch, "cpu", ["pad"] * batch)
+    dev = {k: (v if batch > 1 or k not in FX.OBSERVATION else v[0]).cuda() for k, v in stacked.items()}
+    arm = Pi05Arm(geo, variant, "cuda", batch=batch)
+    arm.bind(dev)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        arm.launch()
+    for scale in (1.0, -0.5):
+        dev["noise"].mul_(scale)
+        arm.outputs()["actions"].zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        replayed = arm.outputs()["actions"].clone()
+        arm.launch()
+        arm.status()
+        assert bool(replayed.abs().max() > 0) and torch.equal(replayed, arm.outputs()["actions"])
+    del graph
+    arm.close()
+
+
+def test_steps_and_layers_may_change_from_launch_to_launch():
+    """Other numbers of steps and layers than at the last call: each the result of an arm of that variant, no device memory taken."""
+    from pi05_megakernel_b200 import _lib
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo = FX.Geometry(prefix=130)
+    dev = {k: v.cuda() for k, v in FX.make_inputs(geo, FX.SEEDS[1], "cpu", "scatter").items()}
+    sizes = [(10, 18), (3, 18), (2, 2), (10, 18), (9, 5), (1, 18)]
+    want = {}
+    for steps, layers in set(sizes):
+        one = Pi05Arm(geo, f"b200-s{steps}-l{layers}", "cuda")
+        one.bind(dev)
+        one.launch()
+        one.status()
+        want[steps, layers] = one.outputs()["actions"].clone()
+        one.close()
+    arm = Pi05Arm(geo, "b200", "cuda")
+    arm.bind(dev)
+    got = [torch.empty_like(arm.outputs()["actions"]) for _ in sizes]
+    stream = torch.cuda.current_stream().cuda_stream
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for out, (steps, layers) in zip(got, sizes):
+        assert arm.lib.pi05_launch(arm.handle, steps, layers, stream, None) == _lib.OK
+        out.copy_(arm.outputs()["actions"])
+    arm.status()
+    assert torch.cuda.mem_get_info()[0] == free
+    for out, size in zip(got, sizes):
+        assert torch.equal(out, want[size]), size
+    arm.close()
+
+
 @pytest.mark.parametrize("prefix", [300, 968])
 def test_attention_reference_moves(prefix):
     """Scores that grow from one chunk of keys to the next: the exponent's reference, taken from the first chunk, has to follow,
