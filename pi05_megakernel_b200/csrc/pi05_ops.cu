@@ -2,7 +2,6 @@
 #include "pi05_ops.h"
 
 #include <algorithm>
-#include <atomic>
 
 namespace pi05 {
 namespace {
@@ -216,29 +215,19 @@ cudaError_t chain_opt_in(const void* kernel, int smem) {
   return e;
 }
 
-namespace {
-// Once per kernel and device; `done`: a bit per device.
-cudaError_t opt_in_once(std::atomic<uint64_t>* done, const void* kernel, int smem, int device) {
-  const uint64_t bit = device < 64 ? 1ull << device : 0;
-  if (done->load() & bit) return cudaSuccess;
-  const cudaError_t e = chain_opt_in(kernel, smem);
-  if (e == cudaSuccess) done->fetch_or(bit);
-  return e;
-}
-}  // namespace
-
 cudaError_t opt_in_gemm(const GemmPlan& g, int device) {
   static std::atomic<uint64_t> done[sizeof kCuts / sizeof kCuts[0]];
   for (const Cut& c : kCuts)
     if (c.epi == g.epi && c.bn == g.bn && c.pair == g.pair && c.ks == g.ks && c.sk == g.sk)
-      return opt_in_once(&done[&c - kCuts], (const void*)c.kernel, 222 * 1024, device);
+      return once_per_device(&done[&c - kCuts], device, [&] { return chain_opt_in((const void*)c.kernel, 222 * 1024); });
   return cudaErrorInvalidValue;
 }
 
 cudaError_t opt_in_attention(int tok_tile, int device) {
   static std::atomic<uint64_t> done[sizeof kTiles / sizeof kTiles[0]];
   for (const Tile& t : kTiles)
-    if (t.rows == tok_tile * NQH) return opt_in_once(&done[&t - kTiles], (const void*)t.kernel, attn::smem_for(t.rows), device);
+    if (t.rows == tok_tile * NQH)
+      return once_per_device(&done[&t - kTiles], device, [&] { return chain_opt_in((const void*)t.kernel, attn::smem_for(t.rows)); });
   return cudaErrorInvalidValue;
 }
 

@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <atomic>
 #include <utility>
 
 #include "pi05_attention.cuh"
@@ -71,6 +72,15 @@ cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t strea
 // kernel's code, and all of them together take 20 ms.)
 cudaError_t opt_in_gemm(const GemmPlan& g, int device);
 cudaError_t opt_in_attention(int tok_tile, int device);
+// Runs `body` (launch settings that may be made twice) once per device, from whichever threads: `done` has a bit per device.
+template <typename F>
+cudaError_t once_per_device(std::atomic<uint64_t>* done, int device, F body) {
+  const uint64_t bit = device < 64 ? 1ull << device : 0;
+  if (done->load() & bit) return cudaSuccess;
+  const cudaError_t e = body();
+  if (e == cudaSuccess) done->fetch_or(bit);
+  return e;
+}
 // One split of L1 and shared memory for all kernels of a chain: an SM that has to change it drains first, which would keep a
 // kernel's CTAs from becoming resident beside the ones of the kernel before.
 cudaError_t chain_opt_in(const void* kernel, int smem);

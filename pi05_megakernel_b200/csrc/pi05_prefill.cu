@@ -207,16 +207,16 @@ size_t most_part_floats(int sms, int max_tokens) {
 }
 
 cudaError_t prefill_opt_in(int device) {
-  static bool done[64] = {};
-  if (done[device]) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-  const void* all[] = {(const void*)pf::tables_kernel, (const void*)pf::norm_kernel<-1>, (const void*)pf::norm_kernel<0>,
-                       (const void*)pf::norm_kernel<1>, (const void*)pf::norm_kernel<2>, (const void*)pf::norm_kernel<4>,
-                       (const void*)pf::norm_kernel<8>};
-  for (const void* k : all)
-    if (e == cudaSuccess) e = chain_opt_in(k, 0);
-  if (e == cudaSuccess) done[device] = true;
-  return e;
+  static std::atomic<uint64_t> done;
+  return once_per_device(&done, device, [] {
+    cudaError_t e = cudaSuccess;
+    const void* all[] = {(const void*)pf::tables_kernel, (const void*)pf::norm_kernel<-1>, (const void*)pf::norm_kernel<0>,
+                         (const void*)pf::norm_kernel<1>, (const void*)pf::norm_kernel<2>, (const void*)pf::norm_kernel<4>,
+                         (const void*)pf::norm_kernel<8>};
+    for (const void* k : all)
+      if (e == cudaSuccess) e = chain_opt_in(k, 0);
+    return e;
+  });
 }
 
 }  // namespace

@@ -434,18 +434,18 @@ NormKernel norm_kernel_for(int splits) {
 
 // Launch settings of the chain's own kernels, once per device.
 cudaError_t opt_in(int device) {
-  static bool done[64] = {};
-  if (device < 64 && done[device]) return cudaSuccess;
-  struct { const void* kernel; int smem; } all[] = {
-      {(const void*)tail_kernel<false>, TAIL_SMEM}, {(const void*)tail_kernel<true>, TAIL_SMEM},
-      {(const void*)residual_norm_kernel<1>, 0}, {(const void*)residual_norm_kernel<2>, 0},
-      {(const void*)residual_norm_kernel<4>, 0}, {(const void*)residual_norm_kernel<8>, 0},
-      {(const void*)modulation_kernel, 0}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
-  cudaError_t e = cudaSuccess;
-  for (const auto& k : all)
-    if (e == cudaSuccess) e = chain_opt_in(k.kernel, k.smem);
-  if (e == cudaSuccess && device < 64) done[device] = true;
-  return e;
+  static std::atomic<uint64_t> done;
+  return once_per_device(&done, device, [] {
+    const struct { const void* kernel; int smem; } all[] = {
+        {(const void*)tail_kernel<false>, TAIL_SMEM}, {(const void*)tail_kernel<true>, TAIL_SMEM},
+        {(const void*)residual_norm_kernel<1>, 0}, {(const void*)residual_norm_kernel<2>, 0},
+        {(const void*)residual_norm_kernel<4>, 0}, {(const void*)residual_norm_kernel<8>, 0},
+        {(const void*)modulation_kernel, 0}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
+    cudaError_t e = cudaSuccess;
+    for (const auto& k : all)
+      if (e == cudaSuccess) e = chain_opt_in(k.kernel, k.smem);
+    return e;
+  });
 }
 
 // The kernels of a chunk, launched into `stream`, which may be one that is being captured.
