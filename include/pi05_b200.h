@@ -147,12 +147,16 @@ int pi05_workspace_region(pi05_handle_t h, const char* name, size_t* offset, siz
 
 /* Debug control: run only the first max_stage stages after the prologue (a stage is one of the seven
  * per-layer steps QKV, attention, O, residual+norm, gate/up, down, residual+norm); negative = run everything.
- * wait_limit_cycles > 0 overrides the bound (in SM clock cycles) of every device-side wait.  drop_event >= 0
+ * wait_limit_cycles > 0 overrides the bound (in SM clock cycles) of every device-side wait (the kernels of a
+ * default launch take none below 2,000,000, 1 ms).  drop_event >= 0
  * makes the row CTAs skip that stage-completion signal (PI05_EVENT_*), so that the waits on it run out: the
  * way to exercise the time-out path without stalling a GPU; negative = signal everything. */
 int pi05_debug(pi05_handle_t h, int max_stage, long long wait_limit_cycles, int drop_event);
 #define PI05_EVENT_ATTENTION_DONE 7
 #define PI05_EVENT_FFN_NORM_READY 9
+/* The same for the chain of kernels that a default launch runs: the QKV projection of layer `layer` (negative: none) gets copies of
+ * fewer bytes than it waits for, so that its waits run out. */
+int pi05_debug_withhold(pi05_handle_t h, int layer);
 /* pi05_status codes: which kind of wait gave up */
 #define PI05_WAIT_WEIGHT_SLOT 1
 #define PI05_WAIT_WEIGHT_DATA 2

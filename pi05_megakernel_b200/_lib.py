@@ -77,6 +77,7 @@ SIGNATURES = {
     "pi05_workspace_region": (_c.c_int, [_c.c_void_p, _c.c_char_p, _c.POINTER(_c.c_size_t),
                                          _c.POINTER(_c.c_size_t)]),
     "pi05_debug": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_longlong, _c.c_int]),
+    "pi05_debug_withhold": (_c.c_int, [_c.c_void_p, _c.c_int]),
     "pi05_config_json": (_c.c_char_p, [_c.c_void_p]),
     "pi05_launch_count": (_c.c_int, [_c.c_void_p, _c.POINTER(_c.c_ulonglong)]),
     "pi05_error_string": (_c.c_char_p, [_c.c_int]),

@@ -212,6 +212,9 @@ class Pi05Arm:
         _lib.check(self.lib, self.handle,
                    self.lib.pi05_debug(self.handle, max_stage, wait_limit_cycles, drop_event))
 
+    def debug_withhold(self, layer: int = -1) -> None:
+        _lib.check(self.lib, self.handle, self.lib.pi05_debug_withhold(self.handle, layer))
+
     def enable_stamps(self, on: bool = True) -> None:
         self.stamps = torch.zeros(_lib.NUM_STAMPS, dtype=torch.int64, device=self.device) if on else None
 

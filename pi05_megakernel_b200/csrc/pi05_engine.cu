@@ -150,6 +150,7 @@ struct pi05_engine {
   int stream_split = 0;          // groups in the first stream (0: one stream)
   int max_stage = 0x7fffffff;
   int drop_event = -1;
+  int withhold = -1;             // the chain: layer whose QKV projection waits for data that never comes
   long long wait_limit = 4000000000ll;    // ~2 s of SM clocks
   unsigned long long launches = 0;
   cudaEvent_t done = nullptr;    // recorded after this handle's last launch, on that launch's stream
@@ -544,7 +545,8 @@ StepSetup step_setup(const pi05_engine* h) {
   s.token_stride = h->kv_strides[0]; s.layer_stride = h->kv_strides[1]; s.page_stride = h->kv_strides[2]; s.num_pages = h->num_pages;
   s.page_table = region_ptr<int>(h, "page_table");
   s.pages_per_obs = h->pages_per_obs; s.page_tokens = h->page_tokens;
-  s.wait_limit = h->wait_limit;
+  s.wait_limit = std::max(h->wait_limit, ptx::SETTLED);
+  s.withhold = -1;
   return s;
 }
 
@@ -804,6 +806,13 @@ int pi05_debug(pi05_handle_t h, int max_stage, long long wait_limit_cycles, int 
   return PI05_OK;
 }
 
+int pi05_debug_withhold(pi05_handle_t h, int layer) {
+  if (!valid_handle(h) || layer >= NL) return PI05_ERR_ARGUMENT;
+  if (layer >= 0 && !uses_graphs(h)) { h->last_error = "this engine's launches do not run the chain of kernels"; return PI05_ERR_UNSUPPORTED; }
+  h->withhold = layer < 0 ? -1 : layer;
+  return PI05_OK;
+}
+
 int pi05_launch(pi05_handle_t h, int n_steps, int n_layers, void* stream, unsigned long long* stamps) {
   if (!valid_handle(h)) return PI05_ERR_ARGUMENT;
   if (!h->bound) return PI05_ERR_NOT_BOUND;
@@ -816,7 +825,8 @@ int pi05_launch(pi05_handle_t h, int n_steps, int n_layers, void* stream, unsign
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing((cudaStream_t)stream, &cap);
     if (e != cudaSuccess) return fail_cuda(h, "cudaStreamIsCapturing", e);
-    h->setup.wait_limit = h->wait_limit;
+    h->setup.wait_limit = std::max(h->wait_limit, ptx::SETTLED);
+    h->setup.withhold = h->withhold;
     const int rc = steps_launch(h->steps, h->setup, n_steps, n_layers, cap != cudaStreamCaptureStatusNone, (cudaStream_t)stream, &h->last_error);
     if (rc != PI05_OK) return rc;
     h->launches++;

@@ -456,7 +456,7 @@ struct Chain {
   cudaError_t e;
   std::string what;
   GemmPlan pq, po, pg, pd;
-  CUtensorMap a_qkv, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;
+  CUtensorMap a_qkv, a_short, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;
   attn::Args ap;
 
   Chain(const StepSetup& setup, int steps, int layers, cudaStream_t into) : s(setup), n_steps(steps), n_layers(layers), stream(into) {
@@ -543,7 +543,7 @@ struct Chain {
       return map_kv(m, s.pool_v, rows, L, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, 64, 4);
     };
     auto weights = [&](CUtensorMap* m, int which, int k, int rows, const GemmPlan& g) { return map_k(m, s.in[which], k, L * rows, g.w_rows, g.w_kb); };
-    if (!(map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
+    if (!(map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_short, s.an, W, M, pq.arows - 8, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
           map_k(&a_dn, s.act, FF, M, pd.arows, pd.ks) && weights(&wq, 8, W, QD, pq) && weights(&wk, 9, W, HD, pq) && weights(&wv, 10, W, HD, pq) &&
           weights(&wo, 11, QD, W, po) && weights(&wg, 12, W, FF, pg) && weights(&wu, 13, W, FF, pg) && weights(&wd, 14, FF, W, pd) &&
           map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH) &&
@@ -565,7 +565,8 @@ struct Chain {
     NormArgs n;
     n.part = s.part; n.h = s.h; n.out = s.an; n.mod = s.mod; n.state = s.state;
     for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
-      project(pq, a_qkv, &wq, &wk, &wv, 0, l, l > 0);      // (what a step leaves behind is complete before the next one's first kernel starts)
+      // (withheld: copies of fewer bytes than their barrier is told to expect)
+      project(pq, l == s.withhold ? a_short : a_qkv, &wq, &wk, &wv, 0, l, l > 0);      // (what a step leaves behind is complete before the next one's first kernel starts)
       ap.layer = l;
       if (e == cudaSuccess) { e = launch_attention(ap, s.batch, stream); ++kernels; }
       project(po, a_o, &wo, nullptr, nullptr, W, l);
@@ -658,7 +659,7 @@ int steps_build(const StepSetup& s, StepGraphs* g, std::string* error) {
 
 int steps_launch(const StepGraphs& g, const StepSetup& s, int n_steps, int n_layers, bool capturing, cudaStream_t stream, std::string* error) {
   // a graph cannot be launched into a stream that is being captured
-  const bool graphs = g.step && !capturing && n_layers == NL && s.wait_limit == g.wait_limit;
+  const bool graphs = g.step && !capturing && n_layers == NL && s.wait_limit == g.wait_limit && s.withhold < 0;
   if (graphs && n_steps == NS) {
     cudaError_t e = cudaGraphLaunch(g.prologue, stream);
     for (int i = 0; i < n_steps && e == cudaSuccess; ++i) e = cudaGraphLaunch(g.step, stream);

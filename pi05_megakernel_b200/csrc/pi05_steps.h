@@ -26,6 +26,7 @@ struct StepSetup {
   const int* page_table;
   int pages_per_obs, page_tokens;
   long long wait_limit;
+  int withhold;                              // debug: the QKV projection of this layer waits for data that never comes; -1: none
 };
 
 // The prologue for all Euler steps, and one step of all layers.

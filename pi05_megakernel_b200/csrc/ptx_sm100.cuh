@@ -400,15 +400,21 @@ __device__ __forceinline__ void bulk_copy_cluster(uint32_t cluster_dst, uint32_t
 }
 
 // Bounded wait on an mbarrier of this CTA, by a whole converged warp: a wait that runs out records (kind, block) in the
-// status words once, and every later wait returns.  The vote keeps the result warp-uniform and the warp converged, which
+// status words once.  The vote keeps the result warp-uniform and the warp converged, which
 // the .aligned tcgen05 instructions behind a wait rely on.  The waiting itself is one function per kernel: the code of a
 // kernel that runs for a few microseconds is fetched once, and what it does not repeat it pays for.
+//   The time counts from the end of the kernel before this one, which every wait of a CTA is behind, and is cut to SETTLED (1 ms) where
+// another wait has run out.  `limit` is not below SETTLED, and a CTA's longest healthy wait is some 10 us, so a wait only gives up where
+// nothing in the CTA has moved for that long: no other warp of it has copies or MMAs in flight or is about to issue any while it
+// frees its tensor memory and leaves.  (A mark or a vote at the end of every role would see to that as well, but costs 2 to 4% of a chunk.)
+constexpr long long SETTLED = 2000000;
 static __device__ __noinline__ bool wait_bar_slow(unsigned int* status, long long limit, uint32_t bar, uint32_t parity, int kind) {
+  grid_dep_wait();
   const long long t0 = clock64();
   for (unsigned i = 0;; ++i) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     if ((i & 63u) == 63u) {
-      bool stop = ld_relaxed(status) != 0u;
+      bool stop = ld_relaxed(status) != 0u && clock64() - t0 > SETTLED;
       if (!stop && clock64() - t0 > limit) {
         if (atomicCAS(status, 0u, (unsigned)kind) == 0u) status[1] = blockIdx.x << 16;
         stop = true;
@@ -416,7 +422,7 @@ static __device__ __noinline__ bool wait_bar_slow(unsigned int* status, long lon
       if (__any_sync(0xffffffffu, stop)) break;
     }
   }
-  // copies and MMAs that this CTA has in flight finish within microseconds: let them land before it tears itself down
+  // what the CTA may still have in flight finishes within microseconds
   const long long t1 = clock64();
   while (clock64() - t1 < 200000) __nanosleep(1000);
   return false;

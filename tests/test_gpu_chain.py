@@ -122,6 +122,36 @@ def test_steps_and_layers_may_change_from_launch_to_launch():
     arm.close()
 
 
+@pytest.mark.parametrize("prefix,batch", [(128, 1), (968, 1), (130, 3), (65, 16)])
+def test_wait_of_the_chain_that_runs_out(prefix, batch):
+    """A projection waits for data that never comes: its waits give up after 10 ms, the kernels behind it return early, the
+    status says so, the actions are NaN, and the next launch, on its graphs again, is what it was.  Projections on single CTAs and on
+    pairs, attention on one CTA per tile and on a cluster."""
+    from pi05_megakernel_b200 import _lib
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo = FX.Geometry(prefix=prefix)
+    stacked, _ = FX.make_batch(geo, FX.SEEDS[0], batch, "cpu", ["pad"] * batch)
+    arm = Pi05Arm(geo, "b200-s1", "cuda", batch=batch)
+    arm.bind({k: (v if batch > 1 or k not in FX.OBSERVATION else v[0]).cuda() for k, v in stacked.items()})
+    arm.launch()
+    arm.status()
+    good = arm.outputs()["actions"].clone()
+    for layer in (0, 16):
+        arm.debug(-1, 20_000_000, -1)
+        arm.debug_withhold(layer)
+        arm.launch()
+        with pytest.raises(_lib.EngineError) as info:
+            arm.status()
+        assert info.value.code == _lib.ERR_DEVICE_TIMEOUT
+        assert bool(torch.isnan(arm.outputs()["actions"]).all())
+        arm.debug_withhold(-1)
+        arm.debug(-1, 4_000_000_000, -1)
+        arm.launch()
+        assert arm.status() == (0, 0)
+        assert torch.equal(arm.outputs()["actions"], good)
+    arm.close()
+
+
 @pytest.mark.parametrize("prefix", [300, 968])
 def test_attention_reference_moves(prefix):
     """Scores that grow from one chunk of keys to the next: the exponent's reference, taken from the first chunk, has to follow,
