@@ -157,7 +157,8 @@ int pi05_debug(pi05_handle_t h, int max_stage, long long wait_limit_cycles, int 
 /* The same for the chain of kernels that a default launch runs: the QKV projection of layer `layer` (negative: none) gets copies of
  * fewer bytes than it waits for, so that its waits run out. */
 int pi05_debug_withhold(pi05_handle_t h, int layer);
-/* pi05_status codes: which kind of wait gave up */
+/* pi05_status codes: which kind of wait gave up.  In the chain of kernels a stage of a projection holds both operands, and its
+ * arrival is WEIGHT_DATA; the codes from KV_SLOT on are the attention's.  `where` carries no stage there. */
 #define PI05_WAIT_WEIGHT_SLOT 1
 #define PI05_WAIT_WEIGHT_DATA 2
 #define PI05_WAIT_ACT_SLOT 3
@@ -166,6 +167,14 @@ int pi05_debug_withhold(pi05_handle_t h, int layer);
 #define PI05_WAIT_TMEM_DATA 6
 #define PI05_WAIT_EVENT 7
 #define PI05_WAIT_DRAIN 8
+#define PI05_WAIT_KV_SLOT 9
+#define PI05_WAIT_KV_DATA 10
+#define PI05_WAIT_QUERIES 11
+#define PI05_WAIT_SCORE_SLOT 12
+#define PI05_WAIT_SCORES 13
+#define PI05_WAIT_PROBS 14
+#define PI05_WAIT_PROBS_SLOT 15
+#define PI05_WAIT_OUTPUT 16
 
 /* Replaces build_config() (mk/pi05_mk.cu:3632-3656): a JSON object describing the build and the schedule. */
 const char* pi05_config_json(pi05_handle_t h);

@@ -65,6 +65,9 @@ struct Args {
   long long limit;
 };
 
+// Wait kinds of the status word, behind those of the projections (pi05::WAIT_*).
+enum { WAIT_KV_EMPTY = 9, WAIT_KV_FULL, WAIT_Q_FULL, WAIT_S_EMPTY, WAIT_S_FULL, WAIT_P_FULL, WAIT_P_EMPTY, WAIT_O_FULL };
+
 __device__ __forceinline__ float rb(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
         ptx::grid_dep_wait();
         waited = true;
       }
-      if (ok && j >= UNITS) ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1);
+      if (ok && j >= UNITS) ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, WAIT_KV_EMPTY);
       if (ok && leader) {
         const uint32_t bar = full + 8 * slot, dst = ring + slot * UNIT;
         ptx::mbar_expect_tx(bar, UNIT);
@@ -216,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       for (int kb = 0; kb < 4; ++kb) ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
     }
     __syncwarp();
-    bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, 3);
+    bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, WAIT_Q_FULL);
     // The units in the ring's order, which is the order of use but for a suffix at the end.  What bounds this loop, next to shared memory,
     // is the warp's own instructions between two MMAs.
     int slot = 0;
@@ -225,12 +228,12 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     auto issue_s = [&](int i, int& sl, uint32_t& pr) -> bool {
       const int buf = i & 1;
       if (i > 1) {
-        if (!ptx::wait_bar(p.status, p.limit, s_empty + 8 * buf, ((i >> 1) & 1) ^ 1, 5)) return false;
+        if (!ptx::wait_bar(p.status, p.limit, s_empty + 8 * buf, ((i >> 1) & 1) ^ 1, WAIT_S_EMPTY)) return false;
         ptx::tc_fence_after();
       }
 #pragma unroll 1
       for (int u = 0; u < 2; ++u) {
-        if (!ptx::wait_bar(p.status, p.limit, full + 8 * sl, pr, 4)) return false;
+        if (!ptx::wait_bar(p.status, p.limit, full + 8 * sl, pr, WAIT_KV_FULL)) return false;
         const uint32_t kd = kdesc + sl * (UNIT >> 4), qd = qdesc + u * (2 * QBLK >> 4);
         ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd, qd, idesc_s, (uint32_t)u, on);
         ptx::umma_bf16_k64<2, 2>(tmem + TM_S + buf * N, kd + (SEG >> 4), qd + (QBLK >> 4), idesc_s, 1u, on);
@@ -245,11 +248,11 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     };
     auto issue_pv = [&](int i) -> bool {
       const int units = nv(i);
-      if (!ptx::wait_bar(p.status, p.limit, p_full, i & 1, 7)) return false;
+      if (!ptx::wait_bar(p.status, p.limit, p_full, i & 1, WAIT_P_FULL)) return false;
       ptx::tc_fence_after();
 #pragma unroll 1
       for (int u = 0; u < units; ++u) {
-        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, 6)) return false;
+        if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, WAIT_KV_FULL)) return false;
         // 16 keys per MMA: 16 rows of 128 B further in V and in P
         const uint32_t vd = vdesc + slot * (UNIT >> 4), pd = pdesc + u * (64 * 128 >> 4), acc = i || u ? 1u : 0u;
         ptx::umma_bf16_k64<128, 128>(tmem + TM_O, vd, pd, idesc_o, acc, on);
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
       const int buf = i & 1;
-      ok &= ptx::wait_bar(p.status, p.limit, s_full + 8 * buf, (i >> 1) & 1, 8);
+      ok &= ptx::wait_bar(p.status, p.limit, s_full + 8 * buf, (i >> 1) & 1, WAIT_S_FULL);
       ptx::tc_fence_after();
       const bool key = s_mask[4 * i + quad] >> lane & 1;      // this thread's key counts
       const uint32_t scol = trow + TM_S + buf * N;
@@ -323,7 +326,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
               pk[r / 2] = pack2(e0, e1);
             }
             // the P buffer is free once the P V of the chunk before has read it
-            if (i > 0) ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, 10);
+            if (i > 0) ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, WAIT_P_EMPTY);
 #pragma unroll
             for (int c = 0; c < R; c += 8) {
               const uint32_t piece = (uint32_t)(r0 + c) >> 3;
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
           // rescale what has been accumulated
 #pragma unroll
           for (int r = 0; r < R; ++r) l[r] *= s_f[r0 + r];
-          ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, 9);
+          ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, WAIT_P_EMPTY);
           ptx::tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < 2 * R; c += 8) {
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       else __stcg(reinterpret_cast<float2*>(part + N * HD) + et, make_float2(s_m[et], sum));
     }
     ptx::named_bar_sync(1, SOFTMAX);
-    ok &= ptx::wait_bar(p.status, p.limit, o_full, 0, 11);
+    ok &= ptx::wait_bar(p.status, p.limit, o_full, 0, WAIT_O_FULL);
     ptx::tc_fence_after();
 
     // ---- O^T / l -> BF16 [row][256] (row = token_local * 8 + head: the tile's rows are one contiguous block of [tokens, 2048])

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       if (PAIR && rank) { m0 = m1; r0 = r1; }
       for (int i = 0; i < w.nst; ++i) {
         const int kb = (w.st0 + i) * KS;
-        if (!(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 2))) break;
+        if (!(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, WAIT_W_EMPTY))) break;
         if (leader) {
           const uint32_t dst = ring + slot * st_stride + w_off;
           if (rank == 0) ptx::mbar_expect_tx(full + 8 * slot, bytes);
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     Work w;
     while (ok && take(at, w))
       for (int i = 0; i < w.nst; ++i) {
-        if (!(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, 1))) break;
+        if (!(ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, WAIT_A_EMPTY))) break;
         if (leader) {
           const uint32_t dst = ring + slot * st_stride;
           if (rank == 0) ptx::mbar_expect_tx(full + 8 * slot, bytes);
@@ -335,13 +335,13 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       Work w;
       for (; ok && take(at, w); ++it) {
         const uint32_t buf = it & 1;
-        if (!(ok = ptx::wait_bar(p.status, p.limit, t_empty + 8 * buf, ((it >> 1) & 1) ^ 1, 6))) break;
+        if (!(ok = ptx::wait_bar(p.status, p.limit, t_empty + 8 * buf, ((it >> 1) & 1) ^ 1, WAIT_T_EMPTY))) break;
         ptx::tc_fence_after();
         const uint32_t d = tmem + buf * BN;
         uint32_t acc = 0;
 #pragma unroll 1
         for (int i = 0; i < w.nst; ++i) {
-          if (!(ok = ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, 3))) break;
+          if (!(ok = ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, WAIT_W_FULL))) break;
           const uint32_t cur = off, bar = empty + 8 * slot;
           off += st_stride >> 4;
           if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; off = 0; }
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     for (; take(at, w); ++it) {
       const uint32_t buf = it & 1;
       const int token = w.mt * p.rows + row;
-      ok &= ptx::wait_bar(p.status, p.limit, t_full + 8 * buf, (it >> 1) & 1, 5);
+      ok &= ptx::wait_bar(p.status, p.limit, t_full + 8 * buf, (it >> 1) & 1, WAIT_T_FULL);
       ptx::tc_fence_after();
       const uint32_t t0 = tmem + buf * BN + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1

@@ -26,6 +26,12 @@
 namespace pi05 {
 namespace {
 
+static_assert(WAIT_W_EMPTY == PI05_WAIT_WEIGHT_SLOT && WAIT_W_FULL == PI05_WAIT_WEIGHT_DATA && WAIT_A_EMPTY == PI05_WAIT_ACT_SLOT &&
+              WAIT_T_EMPTY == PI05_WAIT_TMEM_SLOT && WAIT_T_FULL == PI05_WAIT_TMEM_DATA && WAIT_DRAIN == PI05_WAIT_DRAIN &&
+              attn::WAIT_KV_EMPTY == PI05_WAIT_KV_SLOT && attn::WAIT_KV_FULL == PI05_WAIT_KV_DATA && attn::WAIT_Q_FULL == PI05_WAIT_QUERIES &&
+              attn::WAIT_S_EMPTY == PI05_WAIT_SCORE_SLOT && attn::WAIT_S_FULL == PI05_WAIT_SCORES && attn::WAIT_P_FULL == PI05_WAIT_PROBS &&
+              attn::WAIT_P_EMPTY == PI05_WAIT_PROBS_SLOT && attn::WAIT_O_FULL == PI05_WAIT_OUTPUT, "status codes of the interface");
+
 using gemm::hi16;
 using gemm::lo16;
 using gemm::pack2;

@@ -1,6 +1,7 @@
 """The kernels of the chain (projections, attention, residual + norm) at the sizes where their cuts change, against the oracle
 within the reference harness's band.  Every test needs a B200."""
 import ctypes
+import re
 
 import pytest
 import torch
@@ -143,6 +144,8 @@ def test_wait_of_the_chain_that_runs_out(prefix, batch):
         with pytest.raises(_lib.EngineError) as info:
             arm.status()
         assert info.value.code == _lib.ERR_DEVICE_TIMEOUT
+        # the MMAs and the epilogue wait for what never comes (and the producers for slots): the header's codes of a projection
+        assert int(re.search(r"wait kind (\d+)", str(info.value))[1]) in (1, 2, 3, 6), str(info.value)
         assert bool(torch.isnan(arm.outputs()["actions"]).all())
         arm.debug_withhold(-1)
         arm.debug(-1, 4_000_000_000, -1)
