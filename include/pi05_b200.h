@@ -297,7 +297,8 @@ int pi05_prefill_plan(int sms, int tokens, int cta, int info[PI05_PREFILL_PLAN_I
 /* FP32 words of split-K partial sums that the workspace of a handle for up to max_tokens tokens holds, and that a prefill of
  * `tokens` of them writes, on a GPU of `sms` SMs; computed on the host (no counterpart in the reference, see above). */
 int pi05_prefill_partials(int sms, int max_tokens, int tokens, size_t* held, size_t* needed);
-/* Synchronises `stream` and reports a bounded device-side wait that gave up (PI05_ERR_DEVICE_TIMEOUT), like pi05_status. */
+/* Synchronises `stream` and reports a bounded device-side wait that gave up (PI05_ERR_DEVICE_TIMEOUT), like pi05_status; where = the
+ * block. */
 int pi05_prefill_status(pi05_prefill_t h, void* stream, int* code, int* where);
 const char* pi05_prefill_last_error(pi05_prefill_t h);
 int pi05_prefill_destroy(pi05_prefill_t h);

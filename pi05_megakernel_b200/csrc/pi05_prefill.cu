@@ -427,7 +427,7 @@ int pi05_prefill_status(pi05_prefill_t h, void* stream, int* code, int* where) {
   if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
   if (e != cudaSuccess) { h->last_error = cudaGetErrorString(e); return PI05_ERR_CUDA; }
   *code = (int)st[0];
-  *where = (int)st[1];
+  *where = (int)(st[1] >> 16);               // the block
   return st[0] ? PI05_ERR_DEVICE_TIMEOUT : PI05_OK;
 }
 

@@ -74,6 +74,25 @@ def test_shorter_prompt_stays_in_the_workspace():
     pre.close()
 
 
+def test_status_names_wait_and_block():
+    """What the kernels leave in the status words (kind, block << 16) reaches the caller as kind and block; the next run clears it."""
+    from pi05_megakernel_b200 import _lib
+    from pi05_megakernel_b200.prefill import Pi05Prefill
+    inputs = FX.make_prefill_inputs(FX.PrefillGeometry(tokens=32), 31, "pad")
+    dev = {k: v.cuda() for k, v in inputs.items()}
+    pre = Pi05Prefill(FX.PrefillGeometry(tokens=32), "cuda")
+    pre.bind(dev)
+    pre.run(dev["embeddings"], dev["valid"], 1)
+    pre.status()
+    pre.ws[:8].view(torch.int32).copy_(torch.tensor([2, 5 << 16], dtype=torch.int32))
+    with pytest.raises(_lib.EngineError, match="kind 2 gave up in block 5$") as info:
+        pre.status()
+    assert info.value.code == _lib.ERR_DEVICE_TIMEOUT
+    pre.run(dev["embeddings"], dev["valid"], 1)
+    pre.status()
+    pre.close()
+
+
 def test_full_depth_against_stored_reference_outputs():
     """All 18 layers at 160 tokens (right-padded mask): keys / values of layers 0, 8 and 17 against what the unmodified
     reference and its FP32 dispatch mode produced (tests/golden/prefill_full_p160.npz)."""
