@@ -130,7 +130,9 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
       g.m_tiles = (tokens + 127) / 128;
       if ((g.pair && g.m_tiles < 2) || (pairs >= 0 && (int)g.pair != pairs)) continue;
       if (g.pair) g.m_tiles = (g.m_tiles + 1) / 2 * 2;
-      if (g.kblocks < 4) continue;
+      // K is split where the tiles of a whole K leave SMs idle, and not to even out rounds: prefill of 2700 tokens 10.9 ms, with K of the
+      // down projection over two CTAs 11.3
+      if (g.kblocks < 4 || (splits > 1 && g.m_tiles * (n / g.bn) >= sms)) continue;
       // Stages of four 64-k blocks where a whole K fits the ring that way: 50 tokens 4.66 against 4.69 ms a chunk; the gate / up, O and
       // down projections got slower on them (+1 to 3%), and every one on stages of a single block (+1 to 2%)
       if (c.ks == 4 && tokens > 64) continue;
@@ -147,7 +149,9 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
       g.grid = std::min(ctas, g.pair ? sms / 2 * 2 : sms);
       g.bufs = g.grid < ctas ? 2 : 1;
       lay_out(&g, g.bufs > 1 ? gemm::MAX_STAGES : g.kblocks / g.ks);
-      if (g.stages < 2) continue;
+      // (a ring of two 64-k blocks, beside the staging of 256 features, leaves the tensor core idle half of the time: prefill of 680
+      // tokens 3.32 ms on such a cut, 2.77 on the next best; 1280 tokens 5.55 and 4.90)
+      if (g.stages * g.ks < 3) continue;
       best = g;
       best_cost = cost;
     }

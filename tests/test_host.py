@@ -123,6 +123,14 @@ def test_prefill_partials_fit_the_workspace(lib, sms):
         assert lib.pi05_prefill_partials(*args, ctypes.byref(held), ctypes.byref(needed)) == _lib.ERR_ARGUMENT
 
 
+@pytest.mark.parametrize("tokens", [1200, 1500, 2340, 2700, 3000, 4096])
+def test_prefill_splits_no_k_where_tiles_fill_the_gpu(lib, tokens):
+    """Long prompts leave one slice of partial sums per projection: their whole-K tiles occupy every SM."""
+    held, needed = ctypes.c_size_t(), ctypes.c_size_t()
+    assert lib.pi05_prefill_partials(148, tokens, tokens, ctypes.byref(held), ctypes.byref(needed)) == _lib.OK
+    assert needed.value == tokens * 2048
+
+
 @pytest.mark.parametrize("sms", [132, 148, 152])
 def test_chunk_partials_fit_the_workspace(lib, sms):
     """An engine for (max_batch, max_prefix) holds the partial sums of every smaller batch and shorter prefix."""
