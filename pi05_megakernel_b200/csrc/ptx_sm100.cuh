@@ -43,16 +43,10 @@ __device__ __forceinline__ void fence_proxy_async_global() {
 __device__ __forceinline__ void fence_proxy_async_shared() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-__device__ __forceinline__ void fence_acq_rel_gpu() {
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
-}
 
 // ----------------------------------------------------------------------------- device-scope flags
 __device__ __forceinline__ void red_release_add(unsigned int* addr, unsigned int v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_release(unsigned int* addr, unsigned int v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* addr) {
   unsigned int v;
@@ -72,9 +66,6 @@ __device__ __forceinline__ unsigned int ld_acquire_sys(const unsigned int* addr)
   unsigned int v;
   asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
   return v;
-}
-__device__ __forceinline__ void fence_acq_rel_sys() {
-  asm volatile("fence.acq_rel.sys;" ::: "memory");
 }
 __device__ __forceinline__ void red_add_f32(float* addr, float v) {
   asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
@@ -105,12 +96,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, uint
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
-// Untiled bulk copy global -> this CTA's shared memory (both addresses 16-byte aligned, size a multiple of 16 bytes),
-// completion on an mbarrier of this CTA.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
 // Tiled stores shared memory -> global, as part of the thread's current bulk group; what lies outside the tensor is clipped.
 // The wait returns when the groups committed so far have read their shared memory.
 __device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int c0, int c1) {
@@ -133,15 +118,6 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
-}
-__device__ __forceinline__ uint64_t policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-// Tiled prefetch of a box into L2 only (no shared-memory destination, no completion tracking).
-__device__ __forceinline__ void tma_prefetch_l2_2d(const void* tmap, int c0, int c1) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
@@ -211,14 +187,6 @@ __device__ __forceinline__ uint64_t umma_smem_desc_mn(uint32_t saddr, uint32_t s
   return (uint64_t)((saddr >> 4) & 0x3fffu) | ((uint64_t)(segment >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 constexpr uint32_t UMMA_A_MN_MAJOR = 1u << 15, UMMA_B_MN_MAJOR = 1u << 16;
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // One pipeline stage of the GEMM CTAs in one piece: eight K = 16 MMAs over a 128-k stage (four 32-byte steps in each
 // of the two 64-k operand atoms, which lie a_atom / b_atom descriptor units apart) and the commit that frees the stage.
 template <uint32_t A_ATOM, uint32_t B_ATOM>
@@ -339,13 +307,6 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tmem_ld_32x2(uint32_t taddr, uint32_t (&r)[2]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
-}
-// Vector FP32 reduction into global memory (16 bytes, one L2 operation).
-__device__ __forceinline__ void red_add_v4_f32(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 
 // ----------------------------------------------------------------------------- CTA pairs (cta_group::2)
 // Two CTAs of a cluster (ranks 2 i and 2 i + 1) share one MMA: M = 256 rows, each CTA holding its 128 rows of A, its half
@@ -359,8 +320,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The shared::cluster address of `saddr` (an address in this CTA's shared memory) in the CTA of rank `rank`.
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -392,12 +351,6 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar, unsigned short ma
                ::"r"(bar), "h"(mask) : "memory");
 }
 
-// Bulk copy from this CTA's shared memory into another's of the cluster (both 16-byte aligned, addresses from map_to_rank),
-// completion on an mbarrier there.
-__device__ __forceinline__ void bulk_copy_cluster(uint32_t cluster_dst, uint32_t src, uint32_t bytes, uint32_t cluster_bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(cluster_dst), "r"(src), "r"(bytes), "r"(cluster_bar) : "memory");
-}
 
 // Bounded wait on an mbarrier of this CTA, by a whole converged warp: a wait that runs out records (kind, block) in the
 // status words once.  The vote keeps the result warp-uniform and the warp converged, which
@@ -437,10 +390,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t saddr, uint32_t& a, uint32_
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(saddr) : "memory");
 }
-__device__ __forceinline__ void ldmatrix_x2(uint32_t saddr, uint32_t& a, uint32_t& b) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
-               : "=r"(a), "=r"(b) : "r"(saddr) : "memory");
-}
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t saddr, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(saddr) : "memory");
@@ -453,17 +402,11 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 // 16-byte store to a shared-memory address given in the shared state space (lets the compiler keep global loads
 // of later iterations ahead of it: the two spaces cannot alias).
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
