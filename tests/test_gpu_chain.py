@@ -15,10 +15,16 @@ pytestmark = pytest.mark.gpu
 # (prefix, batch, mask, steps and layers).  128-key chunks: up to 64 valid keys in the last one and more, one key; the keys of a
 # tile over 1, 2, 4 and 8 CTAs; projections on tiles of up to 64 and up to 128 tokens, on two, three, six and eight of them,
 # on single CTAs and on pairs, persistent or not; attention on tiles of 2, 4 and 6 tokens.
-@pytest.mark.parametrize("prefix,batch,mask,variant", [
+CUTS = [
     (1, 1, "full", "b200-s2-l2"), (63, 1, "scatter", "b200-s2-l2"), (128, 2, "pad", "b200-s2-l2"), (129, 3, "scatter", "b200-s2-l2"),
     (192, 5, "pad", "b200-s1-l2"), (193, 6, "scatter", "b200-s1-l2"), (301, 1, "scatter", "b200-s2-l2"), (968, 1, "pad", "b200-s2-l2"),
-    (1100, 2, "scatter", "b200-s1-l2"), (130, 7, "full", "b200-s1-l2"), (65, 11, "pad", "b200-s1-l2"), (257, 16, "scatter", "b200-s1-l2")])
+    (1100, 2, "scatter", "b200-s1-l2"), (130, 7, "full", "b200-s1-l2"), (65, 11, "pad", "b200-s1-l2"), (257, 16, "scatter", "b200-s1-l2")]
+# (prefix, batch, tokens per page).  What is left of the attention's cuts on a B200: tiles of 2, 4, 6, 8 and 14 tokens over two and four
+# CTAs, the widest with a second segment of probabilities and a ring of four units; dense caches and pages of 64 and 128 tokens
+ATTENTION_CUTS = [(512, 1, 64), (600, 5, 0), (700, 6, 128), (700, 3, 64), (896, 9, 0), (896, 5, 64), (1700, 12, 0), (1300, 9, 64)]
+
+
+@pytest.mark.parametrize("prefix,batch,mask,variant", CUTS)
 def test_chunk_cuts(prefix, batch, mask, variant):
     from pi05_megakernel_b200.arm import Pi05Arm
     geo, ogeo = FX.Geometry(prefix=prefix), O.Geo(prefix=prefix)
@@ -34,6 +40,37 @@ def test_chunk_cuts(prefix, batch, mask, variant):
     for b in {0, batch // 2, batch - 1}:
         want, exact = (O.chunk(per[b], ogeo, widen, arm.steps, arm.layers) for widen in (False, True))
         d = O.band(want, first.reshape(batch, 50, 32)[b], exact)
+        assert d["pass"], (b, d)
+    arm.close()
+
+
+@pytest.mark.parametrize("prefix,batch,page", ATTENTION_CUTS)
+def test_attention_cuts(prefix, batch, page):
+    from pi05_megakernel_b200.arm import PagedPrefix, Pi05Arm
+    geo, ogeo = FX.Geometry(prefix=prefix), O.Geo(prefix=prefix)
+    masks = ["scatter" if b % 2 else "pad" for b in range(batch)]
+    stacked, per = FX.make_batch(geo, FX.SEEDS[1], batch, "cpu", masks)
+    dev = {k: v.cuda() for k, v in (stacked if batch > 1 else per[0]).items()}
+    pages = None
+    if page:
+        n = -(-prefix // page)
+        order = torch.randperm(batch * n, generator=torch.Generator().manual_seed(3))
+        pools = []
+        for name in ("prefix_k", "prefix_v"):
+            t = dev[name].view(batch, geo.layers, prefix, 1, 256)
+            t = torch.nn.functional.pad(t, (0, 0, 0, 0, 0, n * page - prefix), value=float("nan"))     # no token behind the prefix is read
+            pool = torch.empty((batch * n, geo.layers, page, 1, 256), dtype=t.dtype, device="cuda")
+            pool[order.cuda()] = t.view(batch, geo.layers, n, page, 1, 256).transpose(1, 2).reshape(pool.shape)
+            pools.append(pool)
+        pages = PagedPrefix(*pools, order.view(batch, n))
+    arm = Pi05Arm(geo, "b200-s1-l2", "cuda", batch=batch)
+    arm.bind(dev, kv_pages=pages)
+    arm.launch()
+    arm.status()
+    got = arm.outputs()["actions"].cpu().reshape(batch, 50, 32)
+    for b in {0, batch - 1}:
+        want, exact = (O.chunk(per[b], ogeo, widen, 1, 2) for widen in (False, True))
+        d = O.band(want, got[b], exact)
         assert d["pass"], (b, d)
     arm.close()
 

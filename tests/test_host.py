@@ -150,6 +150,19 @@ def test_chunk_partials_fit_the_workspace(lib, sms):
         assert lib.pi05_chunk_plan(*args, info, ctypes.byref(held), ctypes.byref(needed)) == _lib.ERR_ARGUMENT
 
 
+def test_every_attention_cut_has_a_gpu_test(lib):
+    """The sizes of the GPU tests reach every (query tokens, CTAs per tile) that a B200 chooses for any prefix and batch."""
+    from tests.test_gpu_chain import ATTENTION_CUTS, CUTS
+    info, held, needed = (ctypes.c_int * 4)(), ctypes.c_size_t(), ctypes.c_size_t()
+
+    def cut(batch, prefix):
+        assert lib.pi05_chunk_plan(148, batch, prefix, batch, prefix, info, ctypes.byref(held), ctypes.byref(needed)) == _lib.OK
+        return tuple(info)[:2]
+
+    chosen = {cut(b, 128 * c) for b in range(1, 17) for c in range(1, 33)}
+    assert chosen == {cut(b, p) for p, b, _mask, _variant in CUTS} | {cut(b, p) for p, b, _page in ATTENTION_CUTS}
+
+
 def test_prefill_fixture_is_deterministic():
     geo = FX.PrefillGeometry(tokens=96, layers=1)
     shapes = FX.prefill_shapes(geo)
