@@ -48,12 +48,13 @@ def measured_peaks() -> tuple[float, str]:
 
 
 def ncu_traffic(batch: int, prefix: int) -> float | None:
-    """DRAM bytes per launch from the committed ncu summary of this workload (None where none was captured)."""
+    """DRAM bytes per launch from the committed ncu captures of this workload on the kernels that a default launch runs (None
+    where there is none)."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(path):
         with open(path) as f:
             for rec in json.load(f).get("captures", []):
-                # a capture of another build of the kernel than the one this run launches is not this run's traffic
+                # a capture of other kernels than the ones this run launches is not this run's traffic
                 if rec.get("batch") == batch and rec.get("prefix") == prefix and rec.get("matches_default_build"):
                     return rec.get("dram_bytes_per_launch")
     return None
@@ -103,8 +104,15 @@ class ClockSampler:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
+def engine_record(arm) -> dict:
+    """The engine's configuration as far as it describes what the timed launches run."""
+    keys = ("kernel", "arch", "launches_per_chunk", "chain", "prefix", "steps", "layers", "batch")
+    return {k: arm.config[k] for k in keys if k in arm.config} if "chain" in arm.config else arm.config
+
+
 def stage_times(arm, flush) -> None:
-    """One stamped chunk: globaltimer values written by the kernel at stage boundaries (row CTA 0) and at the
+    """One stamped chunk of the persistent kernel (stamps select it: the chain of kernels that the timed launches run has none):
+    globaltimer values written at stage boundaries (row CTA 0) and at the
     pipeline points of three GEMM CTAs in the second layer pass; printed as microseconds since kernel start."""
     arm.enable_stamps(True)
     flush.zero_()
@@ -126,6 +134,7 @@ def stage_times(arm, flush) -> None:
                 out[f"{cta}_{gn}_pass1_us"] = {pt: us(x) for pt, x in zip(pts, row)}
     out["row_cta0_attention_pass1_us"] = {n: us(st[224 + i]) for i, n in enumerate(
         ["prefix_landed", "scores_done", "softmax_done", "pv_done", "stored", "signalled"])}
+    out["kernel"] = "pi05_chunk_kernel"
     print("stage_times " + json.dumps(out), file=sys.stderr, flush=True)
     print(stage_table(out, arm.geo.prefix), file=sys.stderr, flush=True)
 
@@ -180,7 +189,7 @@ def stage_table(t: dict, prefix: int) -> str:
         total_b += nbytes
     lines.append(f"| one layer pass | {total_us:.2f} | {int(total_b):,} | {total_b / total_us / 1e3:.0f} | "
                  f"{100 * total_b / total_us / 1e3 / peak_gbs:.1f} % | - | - | - |")
-    return "stage_table\n" + "\n".join(lines)
+    return "stage_table (pi05_chunk_kernel)\n" + "\n".join(lines)
 
 
 def batch_sweep(args, device) -> None:
@@ -214,9 +223,7 @@ def batch_sweep(args, device) -> None:
         arm.status()
         ms = sum(times) / len(times)
         print(json.dumps({"batch": B, "ms_per_launch": round(ms, 3), "ms_per_chunk": round(ms / B, 3),
-                          "chunks_per_s": round(1e3 * B / ms, 1), "schedule": arm.config.get("schedule"),
-                          "observations_per_mma": arm.config.get("observations_per_mma"),
-                          "gemm_ctas": arm.config.get("gemm_ctas")}), flush=True)
+                          "chunks_per_s": round(1e3 * B / ms, 1), "engine": engine_record(arm)}), flush=True)
         arm.close()
 
 
@@ -557,7 +564,8 @@ def main() -> int:
                          "instead of the benchmark line")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--stage-times", action="store_true",
-                    help="also print (stderr) the in-kernel stage timeline of one L2-flushed chunk")
+                    help="also print (stderr) the stage timeline of one L2-flushed chunk of the persistent kernel (the timed "
+                         "launches run the chain of kernels)")
     args = ap.parse_args()
     rank = int(os.environ.get("RANK", "0"))
     local = int(os.environ.get("LOCAL_RANK", "0"))
@@ -712,7 +720,7 @@ def main() -> int:
                        "l2": "flushed before every timed chunk (2x L2 zero fill)",
                        "prefix_cache": f"pool of shuffled {args.kv_pages}-token pages read in place" if args.kv_pages else "dense",
                        "parallelism": f"dp{world} (independent observations, replicated weights, no collective)",
-                       "engine": arm.config},
+                       "engine": engine_record(arm)},
             "ms_per_chunk": ms_step / B, "ms_per_launch_median": statistics.median(samples), "batch_per_gpu": B,
             "ms_per_launch_steady": steady_ms, "parity": parity,
             "reference_gpu": "not part of this command: `bench.py --impl reference-gpu` times the reference's own CUDA arm "

@@ -59,7 +59,10 @@ int pi05_create(int device, int max_prefix, int max_batch, int tp_rank, int tp_s
  * mk/pi05_mk.cu:34-320), as run-time values.  The library reads no environment variable; a host program that wants
  * settings from its environment fills this struct itself.  pi05_tuning_defaults writes the values a fresh handle
  * uses; pi05_tune replaces a handle's settings (values out of range are clamped) and un-binds it: the schedule and
- * the launch shape are chosen by the next pi05_bind. */
+ * the launch shape are chosen by the next pi05_bind.
+ * All settings are the persistent kernel's.  A handle with the defaults launches the chain of kernels instead; any value but
+ * poll_ns that differs from its default, clusters = 0 included, selects the persistent kernel, which takes 1.1 to 1.3 times as long
+ * for one observation and up to 3.3 times for sixteen. */
 typedef struct pi05_tuning {
   int poll_ns;            /* pause between two samples of a stage counter (default 20) */
   int obs_per_mma;        /* observations side by side in one MMA of a batch: 0 = engine's choice, 1, 2 */
@@ -142,7 +145,7 @@ int pi05_status(pi05_handle_t h, int* code, int* where);
 
 /* Replaces layout_offsets() (mk/pi05_mk.cu:3622-3627): byte offset and size of a named workspace buffer
  * ("mod", "cond", "h", "an_attn", "an_ffn", "qkv_acc", "k", "v", "attn", "o_acc", "act", "d_acc", "x", "rope", ...)
- * for stage-by-stage checks. */
+ * for stage-by-stage checks under pi05_debug(max_stage); a launch of the chain leaves "an_ffn", "qkv_acc", "o_acc" and "d_acc" alone. */
 int pi05_workspace_region(pi05_handle_t h, const char* name, size_t* offset, size_t* bytes);
 
 /* Debug control: run only the first max_stage stages after the prologue (a stage is one of the seven
@@ -176,10 +179,13 @@ int pi05_debug_withhold(pi05_handle_t h, int layer);
 #define PI05_WAIT_PROBS_SLOT 15
 #define PI05_WAIT_OUTPUT 16
 
-/* Replaces build_config() (mk/pi05_mk.cu:3632-3656): a JSON object describing the build and the schedule. */
+/* Replaces build_config() (mk/pi05_mk.cu:3632-3656): a JSON object describing the build and the schedule.  Where launches run the
+ * chain of kernels, "chain" holds its cuts and "launches_per_chunk" its kernels for (10, 18); the fields from "arch" on are always
+ * those of the persistent kernel. */
 const char* pi05_config_json(pi05_handle_t h);
 
-/* The work schedule the engine would bind for `batch` observations of `prefix_len` prefix tokens on a GPU of `sms`
+/* The work schedule of the persistent kernel (what the engine binds for tensor parallel, for a tuning other than the default, and
+ * for stamps and debug controls; the default launch's cuts: pi05_chunk_plan) for `batch` observations of `prefix_len` prefix tokens on a GPU of `sms`
  * SMs, computed on the host without touching a device (the reference derives each block's K chunk and
  * tiles from blockIdx inside its GEMM phases, mk/pi05_mk.cu:736-743, and has no such query; this one exists so that the schedule's invariants can be tested
  * without a GPU).  Writes up to `capacity` entries of PI05_PLAN_ENTRY ints, in the order the CTAs execute them:

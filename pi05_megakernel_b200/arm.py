@@ -150,6 +150,9 @@ class Pi05Arm:
         self.tensors = tensors
         # the engine chooses its schedule when it knows the batch: record what it chose
         self.config.update(json.loads(self.lib.pi05_config_json(self.handle).decode()))
+        chain = self.config.get("chain")
+        if chain:
+            self.config["launches_per_chunk"] = chain["prologue_launches"] + self.steps * self.layers * chain["launches_per_layer"]
 
     # ------------------------------------------------------------------ tensor parallel
     def tp_export(self) -> bytes:

@@ -494,28 +494,6 @@ bool plan_batch(pi05_engine* h, int batch, int prefix_len) {
   return build_schedule(h, (batch + h->gn - 1) / h->gn);
 }
 
-// The engine's description for the caller's records: geometry of the launch and the schedule of the bound batch.
-void describe(pi05_engine* h) {
-  char buf[1280];
-  const bool grouped = h->batch >= h->tune.grouped_from && !h->tune.latency_schedule;
-  snprintf(buf, sizeof buf,
-           "{\"kernel\": \"%s\", \"arch\": \"sm_100a\", \"launches_per_chunk\": %d, \"grid\": %d, "
-           "\"threads\": %d, \"smem_bytes\": %d, \"gemm_ctas\": %d, \"row_ctas\": %d, \"stages\": %d, "
-           "\"stage_bytes\": %d, \"units\": {\"qkv\": %d, \"o\": %d, \"gate_up\": %d, \"down\": %d}, "
-           "\"mma\": \"tcgen05 cta_group::1 M128 N%d K16 bf16\", \"sync\": \"device-scope counters, bounded waits\", "
-           "\"clusters_of_2\": %s, \"observations_per_mma\": %d, \"tp_rank\": %d, \"tp_size\": %d, \"schedule\": \"%s\"}",
-           h->steps.step ? "chain of kernels replayed from graphs (the fields below: the persistent kernel, pi05_chunk_kernel)" : "pi05_chunk_kernel",
-           h->steps.step ? h->steps.kernels_prologue + NS * h->steps.kernels_step : 1, h->grid, THREADS, SMEM_BYTES, h->n_gemm, h->grid - h->n_gemm, h->gn == 1 ? NSTG : 3,
-           W_STAGE_BYTES + h->gn * A_STAGE_BYTES, h->n_units[0], h->n_units[1], h->n_units[2], h->n_units[3], 64 * h->gn,
-           h->clustered ? "true" : "false", h->gn, h->tp_rank, h->tp_size,
-           !grouped ? "one observation (units serve every observation in turn)"
-                    : h->stream_split > 0 ? "throughput, two streams of groups half a layer pass apart"
-                                          : "throughput, one stream");
-  h->config = buf;
-}
-
-bool valid_handle(pi05_handle_t h) { return h != nullptr; }
-
 // Whether a launch without debug controls runs as the chain of kernels (pi05_steps.cu).  The persistent kernel stays for
 // tensor parallel, for the static entry point, for debug controls and for callers that set one of its own tuning settings.
 // Persistent against graphs, ms: one observation 5.30 / 4.67 at prefix 128 and 6.66 / 5.06 at 968, sixteen 18.8 / 10.3 and 41.1 / 12.6.
@@ -525,6 +503,34 @@ bool uses_graphs(const pi05_engine* h) {
   d.poll_ns = h->tune.poll_ns;
   return h->graphs && h->tp_size == 1 && memcmp(&d, &h->tune, sizeof d) == 0;
 }
+
+// The engine's description for the caller's records: the chain's cuts where launches run it; the other fields are the persistent
+// kernel's launch and schedule for the bound batch.
+void describe(pi05_engine* h) {
+  char buf[1280];
+  const bool grouped = h->batch >= h->tune.grouped_from && !h->tune.latency_schedule;
+  snprintf(buf, sizeof buf,
+           "\"arch\": \"sm_100a\", \"grid\": %d, "
+           "\"threads\": %d, \"smem_bytes\": %d, \"gemm_ctas\": %d, \"row_ctas\": %d, \"stages\": %d, "
+           "\"stage_bytes\": %d, \"units\": {\"qkv\": %d, \"o\": %d, \"gate_up\": %d, \"down\": %d}, "
+           "\"mma\": \"tcgen05 cta_group::1 M128 N%d K16 bf16\", \"sync\": \"device-scope counters, bounded waits\", "
+           "\"clusters_of_2\": %s, \"observations_per_mma\": %d, \"tp_rank\": %d, \"tp_size\": %d, \"schedule\": \"%s\"}",
+           h->grid, THREADS, SMEM_BYTES, h->n_gemm, h->grid - h->n_gemm, h->gn == 1 ? NSTG : 3,
+           W_STAGE_BYTES + h->gn * A_STAGE_BYTES, h->n_units[0], h->n_units[1], h->n_units[2], h->n_units[3], 64 * h->gn,
+           h->clustered ? "true" : "false", h->gn, h->tp_rank, h->tp_size,
+           !grouped ? "one observation (units serve every observation in turn)"
+                    : h->stream_split > 0 ? "throughput, two streams of groups half a layer pass apart"
+                                          : "throughput, one stream");
+  h->config = "{\"kernel\": \"pi05_chunk_kernel\", \"launches_per_chunk\": 1, ";
+  if (h->steps.step && uses_graphs(h))
+    h->config = "{\"kernel\": \"chain of kernels replayed from graphs\", \"launches_per_chunk\": " +
+                std::to_string(h->steps.kernels_prologue + NS * h->steps.kernels_step) + ", \"chain\": " +
+                steps_describe(h->sms, h->batch, h->prefix, h->steps) +
+                ", \"fields_below\": \"pi05_chunk_kernel, which runs here with stamps or debug controls only\", ";
+  h->config += buf;
+}
+
+bool valid_handle(pi05_handle_t h) { return h != nullptr; }
 
 StepSetup step_setup(const pi05_engine* h) {
   StepSetup s;

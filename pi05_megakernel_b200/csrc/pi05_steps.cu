@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+#include <stdio.h>
 #include <string.h>
 
 #include <algorithm>
@@ -619,6 +620,25 @@ StepPlan steps_plan(int sms, int batch, int prefix) {
   p.part_floats = (size_t)std::max(p.o_splits, p.down_splits) * T * batch * W;
   if (a.splits > 1) p.part_floats = std::max(p.part_floats, (size_t)batch * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
   return p;
+}
+
+std::string steps_describe(int sms, int batch, int prefix, const StepGraphs& g) {
+  const int tokens = T * batch;
+  const AttnPlan a = plan_attention(sms, batch, prefix);
+  const struct { const char* name; GemmPlan plan; } all[] = {{"qkv", plan_gemm(sms, tokens, QKVW, W, gemm::EPI_QKV)},
+                                                              {"o", plan_gemm(sms, tokens, W, QD, gemm::EPI_PART)},
+                                                              {"gate_up", plan_gemm(sms, tokens, 2 * FF, W, gemm::EPI_GEGLU)},
+                                                              {"down", plan_gemm(sms, tokens, W, FF, gemm::EPI_PART)}};
+  char buf[256];
+  snprintf(buf, sizeof buf, "{\"prologue_launches\": %d, \"launches_per_layer\": %d, \"attention\": {\"query_tokens\": %d, \"ctas_per_tile\": %d, \"ctas\": %d}",
+           g.kernels_prologue, g.kernels_step / NL, a.tok_tile, a.splits, batch * a.tiles * a.splits);
+  std::string out = buf;
+  for (const auto& x : all) {
+    snprintf(buf, sizeof buf, ", \"%s\": {\"tile_tokens\": %d, \"tile_features\": %d, \"cta_pairs\": %s, \"k_splits\": %d, \"ctas\": %d, \"stages\": %d}", x.name,
+             x.plan.rows, x.plan.bn, x.plan.pair ? "true" : "false", x.plan.splits, x.plan.grid, x.plan.stages);
+    out += buf;
+  }
+  return out + "}";
 }
 
 // Every number of chunks of every batch is asked: the longest prefix does not need the most (148 SMs, five observations: tiles of 8

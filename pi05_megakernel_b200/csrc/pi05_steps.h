@@ -43,6 +43,8 @@ struct StepPlan {
   size_t part_floats;
 };
 StepPlan steps_plan(int sms, int batch, int prefix);
+// The cuts of a binding, and the kernels of its launch (`g`: of the captured chain), as a JSON object.
+std::string steps_describe(int sms, int batch, int prefix, const StepGraphs& g);
 // FP32 words of partial sums that up to `max_batch` observations with up to `max_prefix` prefix tokens need.
 size_t steps_part_floats(int sms, int max_batch, int max_prefix);
 // Captures and instantiates the graphs; frees what `g` held.

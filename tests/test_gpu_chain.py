@@ -143,6 +143,7 @@ def test_steps_and_layers_may_change_from_launch_to_launch():
         one.launch()
         one.status()
         want[steps, layers] = one.outputs()["actions"].clone()
+        assert one.config["launches_per_chunk"] == 5 + 7 * steps * layers
         one.close()
     arm = Pi05Arm(geo, "b200", "cuda")
     arm.bind(dev)
