@@ -496,7 +496,7 @@ bool plan_batch(pi05_engine* h, int batch, int prefix_len) {
 
 // Whether a launch without debug controls runs as the chain of kernels (pi05_steps.cu).  The persistent kernel stays for
 // tensor parallel, for the static entry point, for debug controls and for callers that set one of its own tuning settings.
-// Persistent against graphs, ms: one observation 5.30 / 4.67 at prefix 128 and 6.66 / 5.06 at 968, sixteen 18.8 / 10.3 and 41.1 / 12.6.
+// Persistent against chain, ms: one observation 5.30 / 4.65 at prefix 128 and 6.67 / 5.14 at 968, sixteen 18.8 / 10.3 and 41.1 / 12.5.
 bool uses_graphs(const pi05_engine* h) {
   pi05_tuning d;
   default_tuning(&d);

@@ -116,7 +116,8 @@ bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, 
 // instruction reads, 64 or 128 of the activations, and the copies that bring them), not less than the weights' way from HBM
 // (3.3 KB per cycle), plus what every launch pays, an epilogue that grows with the tile, the start of a cluster for pairs
 // of CTAs (measured: a launch on pairs takes 0.4-0.8 us longer than the same on single CTAs) and the way of partial sums through
-// L2 and the row kernel.  Against every cut measured by itself, 50 to 800 tokens, the choice costs at most 1% of a chunk.
+// L2 and the row kernel.  Its constants are fitted to cuts that were timed by themselves, 50 to 800 tokens: it knows nothing of the
+// kernel behind, which starts up to 2 us later behind a launch on more than half of the SMs.
 // K of the projections whose sums meet in the residual kernel is split in powers of two, down to four 64-k blocks.
 GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
   GemmPlan best = {};

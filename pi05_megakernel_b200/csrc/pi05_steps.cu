@@ -425,7 +425,7 @@ AttnPlan plan_attention(int sms, int batch, int prefix) {
       // (a cluster is resident as a whole, and those of eight CTAs leave some SMs without)
       if (splits > 1 && (per_cta < 2 || ctas > (splits == 8 ? sms * 3 / 4 : sms))) continue;
       // Fitted to every cut timed by itself at 1 to 16 observations and 128 to 968 tokens, in us: a chunk of 128 keys, what a tile
-      // costs besides, a merge.  The choice is within 1% of the best of a chunk.
+      // costs besides, a merge.  (What a CTA count does to the start of the kernel behind is not in it.)
       const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) + (splits > 1 ? 1.5 + 0.2 * t : 0.0);
       if (cost >= best_cost) continue;
       best_cost = cost;
