@@ -212,9 +212,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     const uint32_t qdesc = (uint32_t)ptx::umma_smem_desc(q_base), kdesc = (uint32_t)ptx::umma_smem_desc(ring);
     const uint32_t pdesc = (uint32_t)ptx::umma_smem_desc_mn(p_base, SEG), vdesc = (uint32_t)ptx::umma_smem_desc_mn(ring, 64 * 128);
     const uint32_t on = leader ? 1u : 0u;
-    ptx::grid_dep_wait();                  // Q is this warp's, which is the one that waits for it: warp 0 may still be at the cache
     if (leader) {
       ptx::mbar_expect_tx(q_full, 4 * QBLK);
+      ptx::grid_dep_wait();                // Q is this warp's, which is the one that waits for it: warp 0 may still be at the cache
 #pragma unroll
       for (int kb = 0; kb < 4; ++kb) ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
     }

@@ -37,9 +37,9 @@
 namespace gemm {
 using namespace pi05;
 
-constexpr int THREADS_G = 352;     // warp 0 weight producer, warp 1 MMA issuer, warps 2..9 epilogue (two per TMEM lane quadrant), warp 10
-                                   // activation producer
-constexpr int EPI_THREADS = 256;
+// Warp 0 weight producer, warp 1 MMA issuer, the next eight epilogue (two per TMEM lane quadrant; four of them are no faster), the last one activation
+// producer.
+constexpr int EPI_THREADS = 256, THREADS_G = 96 + EPI_THREADS, WARP_A = THREADS_G / 32 - 1;
 constexpr int BK = 64;             // k per stage (one 128-byte swizzle row)
 constexpr int MAX_STAGES = 16;
 
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       if (PAIR) { ptx::tmem_alloc_pair(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish_pair(); }
       else { ptx::tmem_alloc(ptx::smem_u32(&s_tmem), tcols); ptx::tmem_relinquish(); }
       ptx::grid_dep_launch();              // after the allocation: a later kernel cannot take the columns first
-    } else if (warp == 10 && leader) {
+    } else if (warp == WARP_A && leader) {
       ptx::prefetch_tensormap(&p.a);
     }
     ptx::tc_fence_before();
@@ -305,9 +305,9 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
   }
   const uint32_t tmem = s_tmem;
 
-  if (warp == 10) {
-    // ---- activation producer
-    ptx::grid_dep_wait();
+  if (warp == WARP_A) {
+    // ---- activation producer.  It waits for the kernel before this one right before its first copy, when everything that copy takes is computed
+    bool waited = false;
     const uint32_t bytes = (PAIR ? 2 : 1) * KS * a_stride;
     uint32_t slot = 0, par = 1;
     bool ok = true;
@@ -319,9 +319,11 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
         if (leader) {
           const uint32_t dst = ring + slot * st_stride;
           if (rank == 0) ptx::mbar_expect_tx(full + 8 * slot, bytes);
+          if (!waited) ptx::grid_dep_wait();
           if (PAIR) ptx::tma_load_3d_pair(dst, &p.a, ptx::map_to_rank(full + 8 * slot, 0), 0, w.mt * p.rows, (w.st0 + i) * KS);
           else ptx::tma_load_3d(dst, &p.a, full + 8 * slot, 0, w.mt * p.rows, (w.st0 + i) * KS);
         }
+        waited = true;
         if (++slot == (uint32_t)stages) { slot = 0; par ^= 1; }
       }
   } else if (warp == 1) {
