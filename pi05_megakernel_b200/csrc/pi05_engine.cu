@@ -543,7 +543,7 @@ StepSetup step_setup(const pi05_engine* h) {
   s.temb = region_ptr<float>(h, "temb"); s.hid = region_ptr<float>(h, "hid"); s.cond = region_ptr<float>(h, "cond");
   s.mod = region_ptr<float>(h, "mod"); s.x = region_ptr<float>(h, "x"); s.part = region_ptr<float>(h, "part");
   s.part_floats = find_region(h, "part")->bytes / 4;
-  s.rope = region_ptr<uint32_t>(h, "rope");
+  s.rope = region_ptr<uint32_t>(h, "rope"); s.rope4 = region_ptr<uint32_t>(h, "rope2");
   s.h = region_ptr<__nv_bfloat16>(h, "h"); s.an = region_ptr<__nv_bfloat16>(h, "an_attn");
   s.q = region_ptr<__nv_bfloat16>(h, "q"); s.k = region_ptr<__nv_bfloat16>(h, "k"); s.v = region_ptr<__nv_bfloat16>(h, "v");
   s.attn = region_ptr<__nv_bfloat16>(h, "attn"); s.act = region_ptr<__nv_bfloat16>(h, "act");

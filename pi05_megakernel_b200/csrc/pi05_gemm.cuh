@@ -54,10 +54,14 @@ struct Args {
   unsigned int* status;
   long long limit;
   __nv_bfloat16 *q, *k, *v;        // EPI_QKV: [tokens, 2048], [tokens, 256], [tokens, 256]
-  const uint32_t* rope;            // [tokens][128]: cos BF16 | sin BF16 << 16
+  const uint32_t* rope;            // [128 / 4][tokens][4]: cos BF16 | sin BF16 << 16 (rope_at)
   __nv_bfloat16* act;              // EPI_GEGLU: [tokens, width]
   float* part;                     // EPI_PART: [splits][tokens, width]; SK: [slots][128][BN]
 };
+
+// Word of the rotary table: four dims of a token together, tokens next to each other, so that the 32 tokens of an epilogue warp read whole lines.
+// With a token's 128 words in a row, a warp's load touched 32 lines, which the load unit takes one at a time: 2 us of a QKV epilogue of 128 features.
+__host__ __device__ __forceinline__ size_t rope_at(int tokens, int token, int dim) { return ((size_t)(dim >> 2) * tokens + token) * 4 + (dim & 3); }
 
 __device__ __forceinline__ float rb(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
@@ -89,18 +93,21 @@ struct Staging {
   }
 };
 
-// This thread's token row of the accumulator (TMEM lanes of its warp, BN columns from t0); `half` is the half of the columns
+// This thread's token row of the accumulator (TMEM lanes of its warp, BN columns from t0); `part` of PARTS is the share of the columns
 // (of each half of the tile for QKV and GEGLU) that its warp handles.  `out` is the staging buffer; PART fills `boxes` boxes of
 // it from column 32 box0 on.
 // Eight columns at a time in loops that stay loops: an instruction that runs once costs several cycles to fetch.
 template <int EPI, int BN>
-__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int row, int token, bool live, bool mine, int half, uint32_t out,
+__device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt, int split, int row, int token, bool live, bool mine, int part, uint32_t out,
                                              int box0, int boxes) {
   using St = Staging<EPI, BN>;
   constexpr bool STAGED = St::COUNT > 0;
+  constexpr int PARTS = EPI_THREADS / 128;
+  constexpr bool EVEN = BN / 2 / PARTS % 8 == 0;            // else the warps take eight columns in turn
+  constexpr int FIRST = EVEN ? BN / 2 / PARTS : 8;
   const int tok = live ? token : 0;
   if constexpr (EPI == EPI_PART) {
-    const int cols = STAGED ? boxes * 16 : BN / 2, c0 = (STAGED ? box0 * 32 : 0) + half * cols;
+    const int cols = (STAGED ? boxes * 32 : BN) / PARTS, c0 = (STAGED ? box0 * 32 : 0) + part * cols;
     uint4* g = reinterpret_cast<uint4*>(p.part + ((size_t)split * p.tokens + tok) * p.width + nt * BN + c0);
 #pragma unroll 1
     for (int c = 0; c < cols; c += 16) {
@@ -109,7 +116,7 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
       ptx::tmem_wait_ld();
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, (half * cols + c) / 4 + j), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]); }
+        if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, (part * cols + c) / 4 + j), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]); }
         else if (live) g[c / 4 + j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
       }
     }
@@ -117,16 +124,16 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
     // QKV and GEGLU need columns c and c + BN / 2 of the tile together (rotary partner, gate with up)
     constexpr int PER = HD / BN;                            // QKV: tiles per head
     const int head = nt / PER, dim0 = (nt % PER) * (BN / 2);
-    const uint4* cs4 = reinterpret_cast<const uint4*>(p.rope + (size_t)tok * 128 + dim0);
+    const uint4* cs4 = reinterpret_cast<const uint4*>(p.rope) + (size_t)(dim0 / 4) * p.tokens + tok;
     __nv_bfloat16* g = EPI == EPI_GEGLU ? p.act + (size_t)tok * p.width + nt * (BN / 2)
                        : (head < NQH ? p.q + (size_t)tok * QD + head * HD : (head == NQH ? p.k : p.v) + (size_t)tok * HD) + dim0;
 #pragma unroll 1
-    for (int c = half * (BN / 4); c < (half + 1) * (BN / 4); c += 8) {
+    for (int c = part * FIRST; c < (EVEN ? (part + 1) * FIRST : BN / 2); c += EVEN ? 8 : 8 * PARTS) {
       uint32_t r1[8], r2[8], o1[4], o2[4];
       ptx::tmem_ld_32x8(t0 + c, r1);
       ptx::tmem_ld_32x8(t0 + BN / 2 + c, r2);
       uint4 wa, wb;
-      if (EPI == EPI_QKV) { wa = __ldg(cs4 + c / 4); wb = __ldg(cs4 + c / 4 + 1); }
+      if (EPI == EPI_QKV) { wa = __ldg(cs4 + (c / 4) * p.tokens); wb = __ldg(cs4 + (c / 4 + 1) * p.tokens); }
       ptx::tmem_wait_ld();
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -357,11 +364,11 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       }
     }
   } else if (warp >= 2) {
-    // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) ..; thread = token row of the tile, half of its columns.  A wait that
+    // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) ..; thread = token row of the tile, a share of its columns.  A wait that
     // gives up does not end the loop: the other epilogue warps count on this one at their barriers
     // (a tile of up to 64 rows is an MMA of 64, whose rows lie in the first 16 lanes of every warp)
     const bool m64 = !PAIR && p.rows <= 64;
-    const int quad = warp & 3, qrow = m64 ? quad * 16 : quad * 32, row = qrow + lane, half = warp >= 6 ? 1 : 0;
+    const int quad = warp & 3, qrow = m64 ? quad * 16 : quad * 32, row = qrow + lane, part = (warp - 2) >> 2;
     const uint32_t release = PAIR ? ptx::map_to_rank(t_empty, 0) : 0u;
     uint32_t it = 0;
     bool ok = true;
@@ -372,6 +379,15 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     for (; take(at, w); ++it) {
       const uint32_t buf = it & 1;
       const int token = w.mt * p.rows + row;
+      if (EPI == EPI_QKV && BN >= 64) {    // the rotary words of this tile into L1 while the MMAs run: from L2 they cost a round trip per eight columns
+        ptx::grid_dep_wait();
+        constexpr int PARTS = EPI_THREADS / 128;
+        const uint4* cs4 = reinterpret_cast<const uint4*>(p.rope) + (size_t)(w.nt % (HD / BN) * (BN / 8) + part * (BN / 8 / PARTS)) * p.tokens;
+        if (row < p.rows && token < p.tokens)
+#pragma unroll 4
+          for (int c = 0; c < BN / 8 / PARTS; ++c) ptx::touch(cs4 + (size_t)c * p.tokens + token);
+        __syncwarp();
+      }
       ok &= ptx::wait_bar(p.status, p.limit, t_full + 8 * buf, (it >> 1) & 1, WAIT_T_FULL);
       ptx::tc_fence_after();
       const uint32_t t0 = tmem + buf * BN + ((uint32_t)(quad * 32) << 16);
@@ -382,7 +398,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
           ptx::named_bar_sync(1, EPI_THREADS);
         }
         if (qrow < p.rows)
-          epilogue_row<EPI, BN>(p, t0, w.nt, w.split, row, token, ok && row < p.rows && token < p.tokens && (!m64 || lane < 16), !m64 || lane < 16, half, stage, box0, BOXES);
+          epilogue_row<EPI, BN>(p, t0, w.nt, w.split, row, token, ok && row < p.rows && token < p.tokens && (!m64 || lane < 16), !m64 || lane < 16, part, stage, box0, BOXES);
         if (!SK || box0 + BOXES >= Staging<EPI, BN>::COUNT) {   // the accumulator has been read
           ptx::tc_fence_before();
           if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);

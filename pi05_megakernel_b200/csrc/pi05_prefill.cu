@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) tables_kernel(const uint8_t* __restrict__
     const int t = t0 + (i >> 7);
     if (t >= tokens) break;
     const float phase = (float)s_pos[i >> 7] * s_inv[i & 127];
-    rope[(size_t)t * 128 + (i & 127)] = pack2((float)cos((double)phase), (float)sin((double)phase));
+    rope[gemm::rope_at(tokens, t, i & 127)] = pack2((float)cos((double)phase), (float)sin((double)phase));
   }
 }
 

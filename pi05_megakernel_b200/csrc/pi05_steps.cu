@@ -42,7 +42,7 @@ using gemm::rb;
 struct TableArgs {
   float t_steps[NS];
   float* temb;
-  uint32_t* rope;
+  uint32_t *rope, *rope4;                    // [token][128], and in the order in which the QKV epilogue reads it
   const uint8_t* mask;
   int* state;
   int prefix, n_steps;
@@ -66,7 +66,9 @@ __global__ void __launch_bounds__(256) tables_kernel(const TableArgs p) {
     const float e = (float)(2 * j) / (float)HD;
     const float inv = 1.0f / (float)pow(10000.0, (double)e);
     const float phase = (float)(nvalid + t) * inv;
-    p.rope[(size_t)b * T * (HD / 2) + i] = pack2((float)cos((double)phase), (float)sin((double)phase));
+    const uint32_t cs = pack2((float)cos((double)phase), (float)sin((double)phase));
+    p.rope[(size_t)b * T * (HD / 2) + i] = cs;
+    p.rope4[gemm::rope_at(gridDim.y * T, b * T + t, j)] = cs;
   }
   if (b == 0) {
     for (int i = gtid; i < NS * W; i += gn) {
@@ -506,7 +508,7 @@ struct Chain {
     TableArgs t;
     const double dt = -1.0 / NS;
     for (int i = 0; i < NS; ++i) t.t_steps[i] = (float)(1.0 + i * dt);
-    t.temb = s.temb; t.rope = s.rope; t.mask = (const uint8_t*)s.in[24]; t.state = s.state; t.prefix = s.prefix; t.n_steps = n_steps;
+    t.temb = s.temb; t.rope = s.rope; t.rope4 = s.rope4; t.mask = (const uint8_t*)s.in[24]; t.state = s.state; t.prefix = s.prefix; t.n_steps = n_steps;
     e = launch_kernel(tables_kernel, dim3(std::max(8, s.sms / s.batch), s.batch), 256, 0, stream, 1, false, t);
     ++kernels;
     MatArgs m;
@@ -532,7 +534,7 @@ struct Chain {
     if (b1) p.b1 = *b1;
     if (b2) p.b2 = *b2;
     p.tokens = T * s.batch; p.layer = layer; p.width = width; p.status = s.status; p.limit = s.wait_limit;
-    p.q = s.q; p.k = s.k; p.v = s.v; p.rope = s.rope; p.act = s.act; p.part = s.part;
+    p.q = s.q; p.k = s.k; p.v = s.v; p.rope = s.rope4; p.act = s.act; p.part = s.part;
     e = launch_gemm(g, p, stream, early);
     ++kernels;
   }

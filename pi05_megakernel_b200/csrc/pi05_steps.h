@@ -18,7 +18,7 @@ struct StepSetup {
   int* state;                                // {Euler step, finished blocks of the step tail, Euler steps of this chunk}
   float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions
   size_t part_floats;                        // what `part` holds (steps_part_floats)
-  uint32_t* rope;
+  uint32_t *rope, *rope4;
   __nv_bfloat16 *h, *an, *q, *k, *v, *attn, *act;
   const void *pool_k, *pool_v;               // prefix cache; strides in elements
   long long token_stride, layer_stride, page_stride;

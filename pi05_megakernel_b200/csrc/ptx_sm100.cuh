@@ -130,6 +130,16 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 16 bytes of a read-only table into L1.
+__device__ __forceinline__ void touch(const uint4* p) {
+  uint32_t a, b, c, d;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "l"(p));
+}
 // Two FP32 fused multiply-adds in one instruction.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   unsigned long long ra, rb, rc, rd;
