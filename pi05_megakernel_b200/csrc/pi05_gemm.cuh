@@ -18,8 +18,9 @@
 //     sums to a slice of its own and a row kernel adds the slices (atomics made the end of the kernel ~1 us later; folding the
 //     row kernel's normalisation into the projections around it and adding the splits within a cluster made a layer pass
 //     slower, since the row kernel is what the weights of the next projection arrive under);
-//   * results of all but the smallest tiles leave through shared memory by tiled copies (a thread per row stores 16 bytes to
-//     32 different lines, which the LSU takes one at a time: 2 us at 128 features per thread; a bulk copy per row: 1.5 us);
+//   * results of all but the smallest tiles leave through shared memory, from where all epilogue threads store whole lines (a thread per row
+//     stores 16 bytes to 32 different lines, which the LSU takes one at a time: 2 us at 128 features per thread; a bulk copy per row: 1.5 us;
+//     tiled copies by one thread: 1.3 us for 115 rows of 128 FP32 sums, 30 B per cycle, against 0.5);
 //   * SK ("stream-K"): tiles x 64-k blocks, taken as one sequence, are cut into one contiguous, equal range per CTA, so that a
 //     long K with few tiles keeps every SM busy for the same time.  A range that begins inside a tile (a contributor's) leaves
 //     its partial sums in the slot of its CTA, one that begins with a tile (the owner's) in the slot of the tile; the residual
@@ -47,7 +48,6 @@ enum { EPI_QKV = 0, EPI_GEGLU = 1, EPI_PART = 2 };
 struct Args {
   CUtensorMap a;                   // activations as {64 k, rows, K / 64}, box {64, arows, KS}
   CUtensorMap b0, b1, b2;          // weights likewise, box {64, rows of a load, 64-k blocks of a load}.  QKV: wq, wk, wv; GEGLU: gate, up
-  CUtensorMap o0, o1, o2;          // staged results, box {128 or 64 bytes, rows}.  QKV: q, k, v; GEGLU: act; PART: part (3-D)
   int tokens, rows, arows, m_groups, splits, kblocks, units, layer, stages, bufs, off_out;   // kblocks: 64-k blocks per unit
   int width;                       // GEGLU: MLP width; PART: features of the output (rows of a layer's weights)
   int unit0;                       // first unit of the launch (QKV of a last layer: keys and values only)
@@ -74,7 +74,7 @@ __device__ __forceinline__ float hi16(uint32_t v) { return __uint_as_float(v & 0
 // cancellation for negative x.  The constants carry the factor -2 log2 e.
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float e = ptx::ex2_approx(x * fmaf(x * x, -0.10294324f, -2.3022082f));
-  return __fdividef(x, 1.0f + e);
+  return x * ptx::rcp_approx(1.0f + e);
 }
 
 // Staging of a tile's results: boxes of 128 rows x BOX bytes (swizzled as the tiled copy expects), COUNT of them; 0: the tile
@@ -141,7 +141,9 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
         const uint32_t y = pack2(__uint_as_float(r2[2 * j]), __uint_as_float(r2[2 * j + 1]));
         if (EPI == EPI_GEGLU) {
           const uint32_t z = pack2(gelu_tanh(lo16(x)), gelu_tanh(hi16(x)));
-          o1[j] = pack2(lo16(z) * lo16(y), hi16(z) * hi16(y));
+          // (a product of two BF16 is exact in FP32: one rounding either way)
+          const __nv_bfloat162 a = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&z), *reinterpret_cast<const __nv_bfloat162*>(&y));
+          o1[j] = *reinterpret_cast<const uint32_t*>(&a);
         } else {
           // RoPE (reference/pi05.py:218-229 on BF16 tensors): x cos + rotate_half(x) sin, every product and the sum rounded
           // to BF16; dim d pairs with dim d + 128.  A table word holds cos | sin << 16 of one dim.
@@ -165,25 +167,34 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
   }
 }
 
-// The staged tile (PART: boxes box0 .. box0 + boxes - 1 of it) to its place in memory: one thread, a tiled copy per box (rows
-// beyond the tokens are clipped).
+// The staged tile (PART: boxes box0 .. box0 + boxes - 1 of it) to its place in memory: 16 bytes per thread, whole lines per warp.
+// (Tiled copies, a thread issuing one per box, moved 30 B per cycle: 1.3 us for 115 rows of 128 FP32 sums.)
 template <int EPI, int BN, bool SK>
-__device__ __forceinline__ void copy_out(const Args& p, uint32_t stage, int nt, int split, int token0, int box0, int boxes) {
+__device__ __forceinline__ void copy_out(const Args& p, uint32_t stage, int nt, int split, int token0, int box0, int tid) {
   using St = Staging<EPI, BN>;
+  constexpr int PER = EPI == EPI_PART ? (SK ? 16 : BN / 4) : EPI == EPI_GEGLU ? BN / 16 : BN / 8;      // 16-byte pieces of a row
+  const int left = p.tokens - token0, rows = left < p.rows ? left : p.rows;
+  uint4* g;
+  int pitch, jump = 0;                                      // of a row; QKV: from the first half of the pieces to the second
   if constexpr (EPI == EPI_PART) {
-#pragma unroll 1
-    for (int b = 0; b < boxes; ++b)
-      ptx::tma_store_3d(&p.o0, stage + b * 128 * St::BOX, (SK ? 0 : nt * BN) + (box0 + b) * 32, SK ? 0 : token0, split);
+    pitch = (SK ? BN : p.width) / 4;
+    g = reinterpret_cast<uint4*>(p.part) + (SK ? (size_t)split * 128 * pitch : ((size_t)split * p.tokens + token0) * pitch + nt * (BN / 4)) + box0 * 8;
   } else if constexpr (EPI == EPI_GEGLU) {
-#pragma unroll
-    for (int b = 0; b < St::COUNT; ++b) ptx::tma_store_2d(&p.o0, stage + b * 128 * St::BOX, nt * (BN / 2) + b * 64, token0);
+    pitch = p.width / 8;
+    g = reinterpret_cast<uint4*>(p.act) + (size_t)token0 * pitch + nt * (BN / 16);
   } else {
-    constexpr int PER = HD / BN, HB = St::COUNT / 2;
-    const int head = nt / PER, c0 = (head < NQH ? head * HD : 0) + (nt % PER) * (BN / 2);
-    const CUtensorMap* m = head < NQH ? &p.o0 : head == NQH ? &p.o1 : &p.o2;
-#pragma unroll
-    for (int b = 0; b < St::COUNT; ++b)
-      ptx::tma_store_2d(m, stage + b * 128 * St::BOX, c0 + (b / (HB ? HB : 1)) * 128 + (b % (HB ? HB : 1)) * 64, token0);
+    constexpr int HEAD = HD / BN;
+    const int head = nt / HEAD;
+    pitch = (head < NQH ? QD : HD) / 8;
+    g = reinterpret_cast<uint4*>(head < NQH ? p.q + head * HD : head == NQH ? p.k : p.v) + (size_t)token0 * pitch + (nt % HEAD) * (BN / 16);
+    jump = 128 / 8 - PER / 2;
+  }
+  constexpr int UNROLL = BN >= 128 ? 4 : 2;
+#pragma unroll UNROLL
+  for (int i = tid; i < rows * PER; i += EPI_THREADS) {
+    const int row = i / PER, c = i % PER;
+    if (EPI == EPI_GEGLU && BN == 224 && nt * 14 + c >= pitch) continue;      // (the last tile of a width that 112 does not divide)
+    g[(size_t)row * pitch + c + (EPI == EPI_QKV && c >= PER / 2 ? jump : 0)] = ptx::ld_shared_v4(stage + St::at(row, c));
   }
 }
 
@@ -218,7 +229,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
     // a stage is full when both producers' arrivals (weights, activations) and every byte of both have come; a lane per stage, since
     // a CTA that starts when the kernel before it leaves pays for every cycle up to here
     if (lane < stages) { ptx::mbar_init(full + 8 * lane, 2); ptx::mbar_init(empty + 8 * lane, 1); }
-    if (lane < 2) { ptx::mbar_init(t_full + 8 * lane, 1); ptx::mbar_init(t_empty + 8 * lane, PAIR ? 2 * EPI_THREADS : EPI_THREADS); }
+    if (lane < 2) { ptx::mbar_init(t_full + 8 * lane, 1); ptx::mbar_init(t_empty + 8 * lane, OUT == 0 ? EPI_THREADS : (PAIR ? 2 : 1) * EPI_THREADS / 32); }
     ptx::fence_mbar_init();
     ptx::fence_proxy_async_shared();
   }
@@ -393,28 +404,27 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
       const uint32_t t0 = tmem + buf * BN + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
       for (int box0 = 0; box0 < (SK ? Staging<EPI, BN>::COUNT : 1); box0 += SK ? BOXES : 1) {
-        if (OUT > 0 && (it > 0 || box0 > 0)) {                       // what was staged before has left the buffer
-          if (tid == 64) ptx::bulk_wait_read();
-          ptx::named_bar_sync(1, EPI_THREADS);
-        }
+        if (OUT > 0 && (it > 0 || box0 > 0)) ptx::named_bar_sync(1, EPI_THREADS);     // what was staged before has left the buffer
         if (qrow < p.rows)
           epilogue_row<EPI, BN>(p, t0, w.nt, w.split, row, token, ok && row < p.rows && token < p.tokens && (!m64 || lane < 16), !m64 || lane < 16, part, stage, box0, BOXES);
         if (!SK || box0 + BOXES >= Staging<EPI, BN>::COUNT) {   // the accumulator has been read
           ptx::tc_fence_before();
-          if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);
-          else ptx::mbar_arrive(t_empty + 8 * buf);
+          if constexpr (OUT == 0) {
+            ptx::mbar_arrive(t_empty + 8 * buf);
+          } else {                         // by warps, since the stores are still to come: 256 arrivals on a barrier go one after the other
+            __syncwarp();
+            if (lane == 0) {
+              if (PAIR) ptx::mbar_arrive_cluster(release + 8 * buf);
+              else ptx::mbar_arrive(t_empty + 8 * buf);
+            }
+          }
         }
         if constexpr (OUT > 0) {
-          ptx::fence_proxy_async_shared();
           ptx::named_bar_sync(1, EPI_THREADS);
-          if (tid == 64) {
-            if (ok) copy_out<EPI, BN, SK>(p, stage, w.nt, w.split, w.mt * p.rows, box0, BOXES);
-            ptx::bulk_commit();
-          }
+          if (ok) copy_out<EPI, BN, SK>(p, stage, w.nt, w.split, w.mt * p.rows, box0, tid - 64);
         }
       }
     }
-    if (OUT > 0 && tid == 64) ptx::bulk_wait_read();
   }
   __syncthreads();
   if (PAIR) ptx::cluster_sync();           // neither CTA leaves (or frees tensor memory) while the other may still use what is in it

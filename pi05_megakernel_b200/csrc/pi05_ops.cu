@@ -87,17 +87,6 @@ bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uin
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool map_out(CUtensorMap* m, const void* base, bool f32, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_bytes, uint32_t box_rows) {
-  EncodeTiledFn enc = encoder();
-  if (!enc) return false;
-  const uint32_t es = f32 ? 4 : 2;
-  cuuint64_t dims[3] = {d0, d1, d2}, strides[2] = {d0 * es, d0 * d1 * es};
-  cuuint32_t box[3] = {box_bytes / es, box_rows, 1}, estr[3] = {1, 1, 1};
-  return enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d2 ? 3 : 2, const_cast<void*>(base), dims, strides,
-             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, uint64_t pages, uint64_t token_stride,
             uint64_t layer_stride, uint64_t page_stride, uint32_t box_tokens, uint32_t box_blocks) {
   EncodeTiledFn enc = encoder();
@@ -181,18 +170,6 @@ cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream, b
   p.m_groups = g.pair ? g.m_tiles / 2 : g.m_tiles; p.splits = g.splits; p.kblocks = g.kblocks;
   p.stages = g.stages; p.bufs = g.bufs; p.off_out = g.off_out;
   p.units = g.units - p.unit0;
-  const uint64_t M = p.tokens;
-  bool ok =true;
-  if (g.sk) ok = map_out(&p.o0, p.part,true, g.bn, 128, g.grid + g.units, 128, g.rows);
-  else if (!staging_bytes(g.epi, g.bn)) ok =true;
-  else if (g.epi == gemm::EPI_PART) ok = map_out(&p.o0, p.part,true, p.width, M, g.splits, 128, g.rows);
-  else if (g.epi == gemm::EPI_GEGLU) ok = map_out(&p.o0, p.act, false, p.width, M, 0, 128, g.rows);
-  else {
-    const int box = g.bn == 64 ? 64 : 128;
-    ok = map_out(&p.o0, p.q, false, QD, M, 0, box, g.rows) && map_out(&p.o1, p.k, false, HD, M, 0, box, g.rows) &&
-         map_out(&p.o2, p.v, false, HD, M, 0, box, g.rows);
-  }
-  if (!ok) return cudaErrorInvalidValue;
   const int ctas = g.pair ? 2 * p.units : p.units, grid = g.sk || g.grid < ctas ? g.grid : ctas;
   return launch_kernel(cut->kernel, grid, gemm::THREADS_G, g.smem, stream, g.pair ? 2 : 1, early, p);
 }

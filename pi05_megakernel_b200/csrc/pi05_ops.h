@@ -45,9 +45,6 @@ cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_
 bool map_k(CUtensorMap* m, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t blocks);
 // {inner, rows} BF16 row-major, box {64, box_rows}, 128-byte swizzle.
 bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows);
-// A dense tensor of two (d2 = 0) or three dimensions, innermost first, of BF16 or FP32 elements, box {box_bytes, box_rows, 1} with
-// the swizzle of that many bytes: the destination of a tiled store.
-bool map_out(CUtensorMap* m, const void* base, bool f32, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_bytes, uint32_t box_rows);
 // Keys or values as the attention's tiled copies read them: {64 dims, tokens, 4 blocks, layers, pages} with strides in elements,
 // box {64, box_tokens, box_blocks, 1, 1}; tokens beyond `tokens` read as zeros.
 bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, uint64_t pages, uint64_t token_stride,

@@ -96,17 +96,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, uint
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
-// Tiled stores shared memory -> global, as part of the thread's current bulk group; what lies outside the tensor is clipped.
-// The wait returns when the groups committed so far have read their shared memory.
-__device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap), "r"(src), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void tma_store_3d(const void* tmap, uint32_t src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(tmap), "r"(src), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1,
                                                  uint64_t policy) {
   asm volatile(
@@ -416,6 +405,20 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 // of later iterations ahead of it: the two spaces cannot alias).
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d));
+}
+
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t saddr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr) : "memory");
+  return v;
+}
+// 16 bytes from each of four places through L2, all on their way before the first is used.
+__device__ __forceinline__ void ld_l2_f4x4(float4 (&v)[4], const float4* p, size_t step) {
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%16];\n ld.global.cg.v4.f32 {%4, %5, %6, %7}, [%17];\n"
+               "ld.global.cg.v4.f32 {%8, %9, %10, %11}, [%18];\n ld.global.cg.v4.f32 {%12, %13, %14, %15}, [%19];"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z), "=f"(v[1].w),
+                 "=f"(v[2].x), "=f"(v[2].y), "=f"(v[2].z), "=f"(v[2].w), "=f"(v[3].x), "=f"(v[3].y), "=f"(v[3].z), "=f"(v[3].w)
+               : "l"(p), "l"(p + step), "l"(p + 2 * step), "l"(p + 3 * step) : "memory");
 }
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
