@@ -77,18 +77,18 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return x * ptx::rcp_approx(1.0f + e);
 }
 
-// Staging of a tile's results: boxes of 128 rows x BOX bytes (swizzled as the tiled copy expects), COUNT of them; 0: the tile
-// is small and its rows are stored directly.  PART: 32 FP32 columns a box; GEGLU and QKV: 64 BF16 (QKV of 64
-// features: 32, each half of the tile a box).
+// Staging of a tile's results: boxes of 128 rows x BOX bytes (swizzled, so that neither its writers nor its readers meet in a bank), COUNT of them; 0: the
+// tile is small and its rows are stored directly.  PART: 32 FP32 columns a box; GEGLU and QKV: 64 BF16 (QKV of 64
+// features: 32, each half of the tile a box; GEGLU of 224: 16, which 112 results are a multiple of).
 template <int EPI, int BN>
 struct Staging {
-  static constexpr int COUNT = EPI == EPI_PART ? (BN >= 64 ? BN / 32 : 0) : EPI == EPI_GEGLU ? BN / 128 : (BN == 256 ? 4 : BN >= 64 ? 2 : 0);
-  static constexpr int BOX = EPI == EPI_QKV && BN == 64 ? 64 : 128;
+  static constexpr int COUNT = EPI == EPI_PART ? (BN >= 64 ? BN / 32 : 0) : EPI == EPI_GEGLU ? (BN == 224 ? 7 : BN == 112 ? 0 : BN / 128) : (BN == 256 ? 4 : BN >= 64 ? 2 : 0);
+  static constexpr int BOX = EPI == EPI_QKV && BN == 64 ? 64 : EPI == EPI_GEGLU && BN == 224 ? 32 : 128;
   static constexpr int BYTES = COUNT * 128 * BOX;
   // 16-byte piece `c` (counted over the whole row of BN results) of row `row`
   static __device__ __forceinline__ uint32_t at(int row, int c) {
     constexpr int PER = BOX / 16;
-    const uint32_t sw = BOX == 128 ? (row & 7) : ((row >> 1) & 3);
+    const uint32_t sw = BOX == 128 ? (row & 7) : BOX == 64 ? ((row >> 1) & 3) : ((row >> 2) & 1);
     return (uint32_t)(c / PER) * (128 * BOX) + row * BOX + (((c % PER) ^ sw) << 4);
   }
 };
@@ -158,7 +158,7 @@ __device__ __forceinline__ void epilogue_row(const Args& p, uint32_t t0, int nt,
         }
       }
       if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, c / 8), o1[0], o1[1], o1[2], o1[3]); }
-      else if (live) *reinterpret_cast<uint4*>(g + c) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+      else if (live && (BN != 112 || nt * (BN / 2) + c < p.width)) *reinterpret_cast<uint4*>(g + c) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
       if (EPI == EPI_QKV) {
         if (STAGED) { if (mine) ptx::st_shared_v4(out + St::at(row, (BN / 2 + c) / 8), o2[0], o2[1], o2[2], o2[3]); }
         else if (live) *reinterpret_cast<uint4*>(g + 128 + c) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(THREADS_G) gemm_kernel(const __grid_constant__
   const uint32_t full = ptx::smem_u32(bars), empty = full + 8 * MAX_STAGES, t_full = empty + 8 * MAX_STAGES, t_empty = t_full + 16;
   const bool leader = ptx::elect_one();
   const int stages = p.stages;
-  const int tcols = p.bufs * (BN < 32 ? 32 : BN);
+  const int tcols = p.bufs * (BN < 32 ? 32 : BN > 128 ? 256 : BN > 64 ? 128 : BN);      // a power of two
 
   if (warp == 0) {
     // a stage is full when both producers' arrivals (weights, activations) and every byte of both have come; a lane per stage, since

@@ -26,7 +26,7 @@ EncodeTiledFn encoder() {
 int staging_bytes(int epi, int bn) {
   using namespace gemm;
   if (epi == EPI_PART) return bn == 32 ? 0 : bn == 64 ? Staging<EPI_PART, 64>::BYTES : bn == 128 ? Staging<EPI_PART, 128>::BYTES : Staging<EPI_PART, 256>::BYTES;
-  if (epi == EPI_GEGLU) return bn == 64 ? 0 : bn == 128 ? Staging<EPI_GEGLU, 128>::BYTES : Staging<EPI_GEGLU, 256>::BYTES;
+  if (epi == EPI_GEGLU) return bn == 64 || bn == 112 ? 0 : bn == 128 ? Staging<EPI_GEGLU, 128>::BYTES : bn == 224 ? Staging<EPI_GEGLU, 224>::BYTES : Staging<EPI_GEGLU, 256>::BYTES;
   return bn == 32 ? 0 : bn == 64 ? Staging<EPI_QKV, 64>::BYTES : bn == 128 ? Staging<EPI_QKV, 128>::BYTES : Staging<EPI_QKV, 256>::BYTES;
 }
 
@@ -38,7 +38,8 @@ struct Cut { int epi, bn, ks; bool pair, sk; GemmKernel kernel; };
 const Cut kCuts[] = {
     CUT(EPI_QKV, 32, false, 4, false), CUT(EPI_QKV, 32, false, 2, false), CUT(EPI_QKV, 64, false, 2, false), CUT(EPI_QKV, 128, false, 2, false),
     CUT(EPI_QKV, 128, true, 2, false), CUT(EPI_QKV, 256, true, 1, false),
-    CUT(EPI_GEGLU, 64, false, 2, false), CUT(EPI_GEGLU, 128, false, 2, false), CUT(EPI_GEGLU, 128, true, 2, false), CUT(EPI_GEGLU, 256, true, 1, false),
+    CUT(EPI_GEGLU, 64, false, 2, false), CUT(EPI_GEGLU, 128, false, 2, false), CUT(EPI_GEGLU, 128, true, 2, false), CUT(EPI_GEGLU, 112, false, 2, false),
+    CUT(EPI_GEGLU, 224, true, 1, false), CUT(EPI_GEGLU, 256, true, 1, false),
     CUT(EPI_PART, 32, false, 2, false), CUT(EPI_PART, 64, false, 2, false), CUT(EPI_PART, 128, false, 2, false), CUT(EPI_PART, 64, true, 2, false),
     CUT(EPI_PART, 128, true, 2, false), CUT(EPI_PART, 256, true, 1, false), CUT(EPI_PART, 256, false, 1, true),
 };
@@ -121,13 +122,19 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
       if (g.pair) g.m_tiles = (g.m_tiles + 1) / 2 * 2;
       // K is split where the tiles of a whole K leave SMs idle, and not to even out rounds: prefill of 2700 tokens 10.9 ms, with K of the
       // down projection over two CTAs 11.3
-      if (g.kblocks < 4 || (splits > 1 && g.m_tiles * (n / g.bn) >= sms)) continue;
+      const int n_tiles = (n + g.bn - 1) / g.bn;              // (224 features divide no width: what is left of the last tile is computed and clipped)
+      if (g.kblocks < 4 || (splits > 1 && g.m_tiles * n_tiles >= sms)) continue;
       // Stages of four 64-k blocks where a whole K fits the ring that way: 50 tokens 4.66 against 4.69 ms a chunk; the gate / up, O and
       // down projections got slower on them (+1 to 3%), and every one on stages of a single block (+1 to 2%)
       if (c.ks == 4 && tokens > 64) continue;
       g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
       g.arows = (g.rows + 7) / 8 * 8;
-      const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128, ctas = g.m_tiles * (n / g.bn) * splits, rounds = (ctas + sms - 1) / sms;
+      // 112 and 224 features (56 and 112 of gate and of up) are for widths that they cut into whole rounds: 4096 in two rounds of 74 pairs beside 1.73 of
+      // 256 (sixteen observations 10.30 -> 10.13 ms, prefill of 256 tokens 1.52 -> 1.48), 16384 in two rounds of 148 CTAs beside 3.5 of 64 (prefill of 128 tokens
+      // 1.32 -> 1.26).  In a single round either way they only pay where the MMAs take long: 5 observations (tiles of 125 tokens) 6.32 -> 6.21, 9 (113) 8.06 -> 7.96,
+      // but 7 (88) 7.11 -> 7.28: the narrower tile occupies 148 SMs, not 128, and the next kernel's CTAs start late
+      if ((g.bn == 224 || g.bn == 112) && g.m_tiles * n_tiles <= sms && (tokens + g.m_tiles - 1) / g.m_tiles <= 96) continue;
+      const int w_bytes = (g.pair ? g.bn / 2 : g.bn) * 128, ctas = g.m_tiles * n_tiles * splits, rounds = (ctas + sms - 1) / sms;
       // cycles of a 64-k block: the tensor core's, or what its operands take through shared memory
       const double smem = (4 * ((!g.pair && g.rows <= 64 ? 2048 : 4096) + g.bn * (g.pair ? 16 : 32)) + g.arows * 128 + w_bytes) / 128.0;
       double cost = std::max(rounds * g.kblocks * (std::max({2.0 * g.bn, 100.0, smem}) + 70.0 / g.ks), (double)n * k * 2 / 3300) + 2000 +
