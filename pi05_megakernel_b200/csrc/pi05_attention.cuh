@@ -7,8 +7,8 @@
 //     whatever is valid.  With the keys, and the dims of V, as A those rows are always full, and the few query rows are
 //     B, which may be as narrow as it is: 128 keys cost 1.2 us with 16 query rows and 1.7 us with 112, against 2.3 us for
 //     up to 128 rows the other way round.
-//   * One CTA = one tile of query tokens against a contiguous share of the keys, in chunks of 128 (the suffix is a chunk of its
-//     own; a chunk of up to 64 valid keys skips the other half of V).  `splits` CTAs of a cluster share the keys of a tile
+//   * One CTA = one tile of query tokens against a contiguous share of the keys, in chunks of 128.  The suffix joins the last chunk of the
+//     prefix where it fits (up to 72 cached keys there), else it is a chunk of its own; a chunk of up to 64 valid keys skips the other half of V.  `splits` CTAs of a cluster share the keys of a tile
 //     and merge through global memory (below).
 //   * Warp 0 streams the keys and values with TMA into a ring of 32 KB units, in the order in which the MMAs consume them:
 //     K (dims 0-127, dims 128-255) of chunk i + 1, V (keys 0-63, keys 64-127) of chunk i, ..; warp 1 fetches Q and issues S^T of chunk i + 1
@@ -54,12 +54,14 @@ struct Args {
   CUtensorMap pk, pk_tail, pv, pv_tail;    // prefix keys / values {64 dims, page tokens, 4, layers, pages}; K: box {64, k_rows, k_rows / 64,
                                            // 1, 1}, V: box {64, 64, 4, 1, 1}; *_tail: the same, cut at the last valid token of a last page
   CUtensorMap sk, sv;                      // suffix keys / values {64, tokens, 4, 1, observations}, box {64, 128, 2, 1, 1} and {64, 64, 4, 1, 1}
+  CUtensorMap jk, jv, jsk, jsv;            // a last chunk that the suffix joins, a 64-dim segment a copy: m_rows cached keys, then m_suf rows of the suffix
   const int* page_table;                   // [observation][pages_per_obs], or null: page = observation
   const uint8_t* valid;                    // [observation][prefix]
   __nv_bfloat16* out;                      // [tokens, 2048]
   float* merge;                            // splits > 1: [tile][split][part_floats]
   int pages_per_obs, page_tokens, prefix, suffix;      // suffix: keys behind the prefix (0: none; up to 64)
   int k_rows;                              // 128: 128 keys of a chunk are one copy; 64: pages of 64 tokens
+  int m_rows, m_suf;                       // 0, or the cached keys of the joined chunk padded to 8 and what the suffix is padded to (16 rows together)
   int obs_tokens, tok_tile, tiles, splits, layer, early;
   unsigned int* status;
   long long limit;
@@ -82,7 +84,7 @@ __device__ __forceinline__ float warp_max(float v) {
   return r;
 }
 
-template <int N>     // query rows of a tile
+template <int N, bool JOIN>     // query rows of a tile; the suffix joins the last chunk of the prefix
 __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_constant__ Args p) {
   constexpr int R = N / 2;                                    // query rows per softmax thread
   constexpr int UNITS = units_for(N), QBLK = N * 128;
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x % p.splits, unit = blockIdx.x / p.splits;
   const int ob = unit / p.tiles, tile = unit % p.tiles;
-  const int npc = (p.prefix + KCH - 1) / KCH, total = npc + (p.suffix > 0 ? 1 : 0);
+  const int npc = (p.prefix + KCH - 1) / KCH, late = JOIN ? npc - 1 : npc, total = npc + (!JOIN && p.suffix > 0 ? 1 : 0);    // late: the chunk with suffix keys
   const int cbeg = total * split / p.splits, n = total * (split + 1) / p.splits - cbeg;    // n >= 1: splits <= total
   const uint32_t b0 = ptx::smem_u32(bars);
   const uint32_t q_full = b0, full = b0 + 8, empty = b0 + 56, s_full = b0 + 104, s_empty = b0 + 120, p_full = b0 + 136, p_empty = b0 + 144,
@@ -107,9 +109,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   const uint32_t q_base = ptx::smem_u32(smem), p_base = q_base + 4 * QBLK, ring = p_base + p_bytes(N);
   const bool leader = ptx::elect_one();
 
-  // Units of V of this CTA's chunk i.  The ring's order is K0 | K1 V0 | K2 V1 | .. | V(n-1); a suffix at the end goes behind the values of the chunk before it, which do not depend on the kernel before this one.
-  auto nv = [&](int i) { const int c = cbeg + i; return c < npc ? (p.prefix - c * KCH > 64 ? 2 : 1) : 1; };
-  const bool swapped = n >= 2 && cbeg + n > npc;
+  // Units of V of this CTA's chunk i (of a joined chunk: halves of the dims, laid out like K; else halves of the keys).  The ring's order is K0 | K1 V0 | K2 V1 | .. | V(n-1); a suffix at the end goes behind the values of the chunk before it, which do not depend on the kernel before this one.
+  auto nv = [&](int i) { const int c = cbeg + i; return c < late ? (p.prefix - c * KCH > 64 ? 2 : 1) : JOIN ? 2 : 1; };
+  const bool swapped = n >= 2 && cbeg + n > late;
 
   if (warp == 0) {
     // all 20 (the last of them unused), a lane each: s_empty[2] and p_full are the softmax threads'
@@ -141,8 +143,37 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       tail = lp == last;
       return __ldg(p.page_table + ob * p.pages_per_obs + lp);
     };
+    // half of the joined chunk's keys or values (dims 128 u ..): 1: the cached rows, 2: the suffix
+    auto joined = [&](int isv, int u, int sl, int what) {
+      const uint32_t bar = full + 8 * sl, dst = ring + sl * UNIT;
+      if (what & 1) {
+        int row;
+        bool tail;
+        const int page = page_of(late * KCH, row, tail);
+        if (leader) {
+          ptx::mbar_expect_tx(bar, 2 * (p.m_rows + p.m_suf) * 128);
+#pragma unroll 1
+          for (int s = 0; s < 2; ++s) ptx::tma_load_5d(dst + s * SEG, isv ? &p.jv : &p.jk, bar, 0, row, 2 * u + s, p.layer, page);
+        }
+        __syncwarp();
+      }
+      if (what & 2) {
+        if (!waited) { ptx::grid_dep_wait(); waited = true; }
+        if (leader)
+#pragma unroll 1
+          for (int s = 0; s < 2; ++s) ptx::tma_load_5d(dst + s * SEG + p.m_rows * 128, isv ? &p.jsv : &p.jsk, bar, 0, 0, 2 * u + s, 0, ob);
+        __syncwarp();
+      }
+    };
     auto emit = [&](int i, int isv, int u) {
       const int c = cbeg + i;
+      if (JOIN && c == late) {
+        if (ok && j >= UNITS) ok = ptx::wait_bar(p.status, p.limit, empty + 8 * slot, par, WAIT_KV_EMPTY);
+        if (ok) joined(isv, u, slot, 3);
+        ++j;
+        if (++slot == UNITS) { slot = 0; par ^= 1; }
+        return;
+      }
       if (!waited && (!p.early || c >= npc)) {
         ptx::grid_dep_wait();
         waited = true;
@@ -175,6 +206,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       if (++slot == UNITS) { slot = 0; par ^= 1; }
     };
     // groups of units: K0, then (K_i, V_(i-1)) or, a suffix, (V_(i-1), K_i), then V_(n-1)
+    if (JOIN && n == 1 && cbeg == late) {                 // the joined chunk alone: all of its cached rows before the wait
+#pragma unroll 1
+      for (int g = 0; g < 8; ++g) joined(g >> 1 & 1, g & 1, g & 3, g < 4 ? 1 : 2);
+    } else
 #pragma unroll 1
     for (int g = 0; g < 2 * n; ++g) {
       const int i = (g + 1) >> 1;                             // groups 2 i - 1 and 2 i are chunk i's keys and the values before it
@@ -193,8 +228,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     } else {
       // validity bits of this CTA's keys (an input, not an output of the kernel before)
       for (int w = warp - 2; w < 4 * n; w += 8) {
-        const int t = (cbeg * 4 + w) * 32 + lane, s = t - npc * KCH;
-        const bool good = s < 0 ? t < p.prefix && p.valid[(size_t)ob * p.prefix + t] != 0 : s < p.suffix;
+        const int t = (cbeg * 4 + w) * 32 + lane, s = t - late * KCH - (JOIN ? p.m_rows : 0);
+        const bool good = t < p.prefix ? p.valid[(size_t)ob * p.prefix + t] != 0 : s >= 0 && s < p.suffix;
         const unsigned bits = __ballot_sync(0xffffffffu, good);
         if (lane == 0) s_mask[w] = bits;
       }
@@ -250,6 +285,26 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       const int units = nv(i);
       if (!ptx::wait_bar(p.status, p.limit, p_full, i & 1, WAIT_P_FULL)) return false;
       ptx::tc_fence_after();
+      if (JOIN && cbeg + i == late) {
+        const int steps = (p.m_rows + p.m_suf) / 16;
+#pragma unroll 1
+        for (int u = 0; u < 2; ++u) {
+          if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, WAIT_KV_FULL)) return false;
+          const uint32_t vd = vdesc + ((SEG - 64 * 128) << 12) + slot * (UNIT >> 4), od = tmem + TM_O + u * N;      // (segments 128 keys apart)
+          int s = 0;
+#pragma unroll 1
+          for (; s + 4 <= steps; s += 4) ptx::umma_bf16_k64<128, 128>(od, vd + s * 128, pdesc + s * 128, idesc_o, i || s ? 1u : 0u, on);
+#pragma unroll 1
+          for (; s < steps; ++s) ptx::umma_bf16_k16(od, vd + s * 128, pdesc + s * 128, idesc_o, i || s ? 1u : 0u, on);
+          if (leader) {
+            ptx::umma_commit(empty + 8 * slot);
+            if (u == 1) ptx::umma_commit(p_empty);
+          }
+          __syncwarp();
+          next(slot, par);
+        }
+        return true;
+      }
 #pragma unroll 1
       for (int u = 0; u < units; ++u) {
         if (!ptx::wait_bar(p.status, p.limit, full + 8 * slot, par, WAIT_KV_FULL)) return false;

@@ -525,7 +525,7 @@ void describe(pi05_engine* h) {
   if (h->steps.step && uses_graphs(h))
     h->config = "{\"kernel\": \"chain of kernels replayed from graphs\", \"launches_per_chunk\": " +
                 std::to_string(h->steps.kernels_prologue + NS * h->steps.kernels_step) + ", \"chain\": " +
-                steps_describe(h->sms, h->batch, h->prefix, h->steps) +
+                steps_describe(h->sms, h->batch, h->prefix, h->page_tokens, h->steps) +
                 ", \"fields_below\": \"pi05_chunk_kernel, which runs here with stamps or debug controls only\", ";
   h->config += buf;
 }
@@ -998,7 +998,7 @@ int pi05_chunk_plan(int sms, int max_batch, int max_prefix, int batch, int prefi
   if (sms < 2 || sms > 1024 || max_batch < 1 || max_batch > MAXB || max_prefix < 1 || max_prefix > 4096 || batch < 1 || batch > max_batch ||
       prefix_len < 1 || prefix_len > max_prefix || !info || !held || !needed)
     return PI05_ERR_ARGUMENT;
-  const StepPlan p = steps_plan(sms, batch, prefix_len);
+  const StepPlan p = steps_plan(sms, batch, prefix_len, prefix_len);
   info[0] = p.tok_tile; info[1] = p.splits; info[2] = p.o_splits; info[3] = p.down_splits;
   *held = steps_part_floats(sms, max_batch, max_prefix);
   *needed = p.part_floats;

@@ -183,15 +183,16 @@ cudaError_t launch_gemm(const GemmPlan& g, gemm::Args& p, cudaStream_t stream, b
 
 namespace {
 typedef void (*AttentionKernel)(const attn::Args);
-struct Tile { int rows; AttentionKernel kernel; };
-const Tile kTiles[] = {{16, attn::attention_kernel<16>}, {32, attn::attention_kernel<32>}, {48, attn::attention_kernel<48>},
-                       {64, attn::attention_kernel<64>}, {112, attn::attention_kernel<112>}};
+struct Tile { int rows; bool join; AttentionKernel kernel; };
+#define TILE(ROWS) {ROWS, false, attn::attention_kernel<ROWS, false>}, {ROWS, true, attn::attention_kernel<ROWS, true>}
+const Tile kTiles[] = {TILE(16), TILE(32), TILE(48), TILE(64), TILE(112)};
+#undef TILE
 }  // namespace
 
 cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t stream) {
   const int rows = p.tok_tile * NQH;
   for (const Tile& t : kTiles)
-    if (t.rows == rows)
+    if (t.rows == rows && t.join == (p.m_rows > 0))
       return launch_chained(t.kernel, observations * p.tiles * p.splits, attn::THREADS, attn::smem_for(rows), stream, p.splits, p);
   return cudaErrorInvalidValue;
 }
@@ -211,12 +212,21 @@ cudaError_t opt_in_gemm(const GemmPlan& g, int device) {
   return cudaErrorInvalidValue;
 }
 
-cudaError_t opt_in_attention(int tok_tile, int device) {
+cudaError_t opt_in_attention(int tok_tile, bool join, int device) {
   static std::atomic<uint64_t> done[sizeof kTiles / sizeof kTiles[0]];
   for (const Tile& t : kTiles)
-    if (t.rows == tok_tile * NQH)
+    if (t.rows == tok_tile * NQH && t.join == join)
       return once_per_device(&done[&t - kTiles], device, [&] { return chain_opt_in((const void*)t.kernel, attn::smem_for(t.rows)); });
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_attention_o(const attno::Args& p, int observations, int smem, cudaStream_t stream) {
+  return launch_chained(attno::attention_o_kernel<attno::NTHREADS>, observations * NQH * attno::GROUPS, attno::NTHREADS, smem, stream, 1, p);
+}
+
+cudaError_t opt_in_attention_o(int device) {
+  static std::atomic<uint64_t> done;
+  return once_per_device(&done, device, [] { return chain_opt_in((const void*)attno::attention_o_kernel<attno::NTHREADS>, 222 * 1024); });
 }
 
 }  // namespace pi05

@@ -9,6 +9,7 @@
 #include <utility>
 
 #include "pi05_attention.cuh"
+#include "pi05_attention_o.cuh"
 #include "pi05_gemm.cuh"
 
 namespace pi05 {
@@ -68,7 +69,10 @@ cudaError_t launch_attention(attn::Args& p, int observations, cudaStream_t strea
 // Shared-memory opt-in of the kernel behind a plan, before its first launch on a device.  (Only what is used: the first touch loads a
 // kernel's code, and all of them together take 20 ms.)
 cudaError_t opt_in_gemm(const GemmPlan& g, int device);
-cudaError_t opt_in_attention(int tok_tile, int device);
+cudaError_t opt_in_attention(int tok_tile, bool join, int device);
+// Attention and O projection in one kernel (prefixes of up to attno::MAX_PREFIX tokens).
+cudaError_t launch_attention_o(const attno::Args& p, int observations, int smem, cudaStream_t stream);
+cudaError_t opt_in_attention_o(int device);
 // Runs `body` (launch settings that may be made twice) once per device, from whichever threads: `done` has a bit per device.
 template <typename F>
 cudaError_t once_per_device(std::atomic<uint64_t>* done, int device, F body) {

@@ -315,7 +315,7 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
   if (part_floats(pl, P) > h->part_floats) { h->last_error = "the workspace does not hold the partial sums of this prompt"; return PI05_ERR_UNSUPPORTED; }
   for (const GemmPlan* g : {&pl.qkv, &pl.o, &pl.gu, &pl.down})
     if (e == cudaSuccess) e = opt_in_gemm(*g, h->device);
-  if (e == cudaSuccess) e = opt_in_attention(pl.tok_tile, h->device);
+  if (e == cudaSuccess) e = opt_in_attention(pl.tok_tile, false, h->device);
   if (e != cudaSuccess) { h->last_error = cudaGetErrorString(e); return PI05_ERR_CUDA; }
 
   // tensor maps: activations (rows = tokens, zero beyond), weights (all layers stacked), keys / values for the attention

@@ -244,8 +244,13 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(const NormArgs p) {
   for (int pass = 0; pass < 2; ++pass) {
     if (pass) ptx::grid_dep_wait();
     float4 a[S];
+    if constexpr (S == 8) {
+      ptx::ld_l2_f4x4(reinterpret_cast<float4(&)[4]>(a[0]), a4, slice);
+      ptx::ld_l2_f4x4(reinterpret_cast<float4(&)[4]>(a[4]), a4 + 4 * slice, slice);
+    } else {
 #pragma unroll
-    for (int s = 0; s < S; ++s) a[s] = __ldcg(a4 + s * slice);
+      for (int s = 0; s < S; ++s) a[s] = __ldcg(a4 + s * slice);
+    }
     const uint2 hv = __ldcg(reinterpret_cast<const uint2*>(p.h + at));
 #pragma unroll
     for (int s = 1; s < S; ++s) { a[0].x += a[s].x; a[0].y += a[s].y; a[0].z += a[s].z; a[0].w += a[s].w; }
@@ -413,27 +418,48 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) tail_kernel(const TailArgs p)
 
 // =========================================================================================== host side
 // How the attention of `batch` observations is cut: `tok_tile` query tokens per CTA, the keys of a tile over `splits` CTAs of a
-// cluster.
-struct AttnPlan { int tok_tile, tiles, splits; };
+// cluster, the suffix in the last chunk of the prefix (`join`) or in one of its own.
+struct AttnPlan { int tok_tile, tiles, splits; bool join; };
 
-AttnPlan plan_attention(int sms, int batch, int prefix) {
+// Whether attention and O projection run as one kernel: where all keys fit into shared memory and a CTA per head and 128 output features is at most one
+// round.  Prefix 128: 4.66 -> 4.36 ms, 40: 4.61 -> 4.22, two observations at 100: 5.01 -> 4.97; three would be two rounds.
+bool with_o(int sms, int batch, int prefix) {
+  return prefix <= attno::MAX_PREFIX && batch * NQH * attno::GROUPS <= sms;
+}
+
+// Whether the suffix joins the last chunk of the prefix: cached keys there, padded to 8, and the 50 of the suffix are at most 128, and the cached ones
+// are one copy (a page holds them).  968 tokens: eight chunks instead of nine.
+bool joins(int prefix, int page_tokens) {
+  const int rows = (prefix - (prefix - 1) / attn::KCH * attn::KCH + 7) / 8 * 8;
+  return rows <= 72 && (rows <= 64 || prefix <= page_tokens || page_tokens % attn::KCH == 0);
+}
+
+// `prefix_chunks` chunks of 128 cached tokens; `may_join`: the suffix fits into the last of them.  The times behind the cost, in us, were fitted to every cut
+// timed by itself at 1 to 16 observations and 128 to 968 tokens, and then to whole chunks: a chunk of 128 keys, what a tile costs besides, a merge (dearer
+// with several observations, whose next kernels' CTAs wait for the clusters to leave), the copies of a joined chunk.  One chunk per CTA on a cluster of four:
+// 300 tokens 4.84 -> 4.64 ms (apart, 2 tokens x 4 CTAs, against joined on one), 384 4.86 -> 4.62; joined: 968 tokens 5.05 -> 4.85, two observations 5.99 -> 5.87.
+AttnPlan plan_attention(int sms, int batch, int prefix_chunks, bool may_join) {
   AttnPlan best = {};
   double best_cost = 1e30;
-  const int chunks = (prefix + attn::KCH - 1) / attn::KCH + 1;
-  for (int t : {2, 4, 6, 8, 14})
-    for (int splits = 1; splits <= 8 && splits <= chunks; splits *= 2) {
-      const int tiles = (T + t - 1) / t, ctas = batch * tiles * splits;
-      const int per_cta = (chunks + splits - 1) / splits;
-      // (a cluster is resident as a whole, and those of eight CTAs leave some SMs without)
-      if (splits > 1 && (per_cta < 2 || ctas > (splits == 8 ? sms * 3 / 4 : sms))) continue;
-      // Fitted to every cut timed by itself at 1 to 16 observations and 128 to 968 tokens, in us: a chunk of 128 keys, what a tile
-      // costs besides, a merge.  (What a CTA count does to the start of the kernel behind is not in it.)
-      const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) + (splits > 1 ? 1.5 + 0.2 * t : 0.0);
-      if (cost >= best_cost) continue;
-      best_cost = cost;
-      best.tok_tile = t; best.tiles = tiles; best.splits = splits;
-    }
+  for (int i = 0; i < 40; ++i) {
+    static const int kTokens[] = {2, 4, 6, 8, 14};
+    const int join = 1 - i / 20, t = kTokens[i / 4 % 5], splits = 1 << i % 4;
+    const int chunks = prefix_chunks + (join ? 0 : 1), tiles = (T + t - 1) / t, ctas = batch * tiles * splits;
+    if (splits > chunks || (join && !may_join)) continue;
+    const int per_cta = (chunks + splits - 1) / splits;
+    // (a cluster is resident as a whole, and those of four and eight CTAs leave some SMs without: four observations of 968 tokens on 144 CTAs in
+    // clusters of four 8.4 ms, on 112 7.0)
+    if (splits > 1 && ctas > (splits == 8 ? sms * 3 / 4 : splits == 4 ? sms * 7 / 8 : sms)) continue;
+    const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) +
+                        (splits > 1 ? 1.5 + 0.2 * t + (batch > 1 ? 0.9 : 0.0) : 0.0) + (join ? 0.8 : 0.0);
+    if (cost >= best_cost) continue;
+    best_cost = cost;
+    best.tok_tile = t; best.tiles = tiles; best.splits = splits; best.join = join != 0;
+  }
   return best;
+}
+AttnPlan plan_attention_for(int sms, int batch, int prefix, int page_tokens) {
+  return plan_attention(sms, batch, (prefix + attn::KCH - 1) / attn::KCH, joins(prefix, page_tokens));
 }
 
 typedef void (*NormKernel)(const NormArgs);
@@ -460,13 +486,15 @@ cudaError_t opt_in(int device) {
 // The kernels of a chunk, launched into `stream`, which may be one that is being captured.
 struct Chain {
   const StepSetup& s;
-  int n_steps, n_layers, kernels = 0;
+  int n_steps, n_layers, kernels = 0, fused_smem = 0;
   cudaStream_t stream;
   cudaError_t e;
   std::string what;
   GemmPlan pq, po, pg, pd;
   CUtensorMap a_qkv, a_short, a_o, a_gu, a_dn, wq, wk, wv, wo, wg, wu, wd;
   attn::Args ap;
+  attno::Args fp;
+  bool join, fused;                                // attention and O projection as one kernel
 
   Chain(const StepSetup& setup, int steps, int layers, cudaStream_t into) : s(setup), n_steps(steps), n_layers(layers), stream(into) {
     const int tokens = T * s.batch;
@@ -474,13 +502,16 @@ struct Chain {
     po = plan_gemm(s.sms, tokens, W, QD, gemm::EPI_PART);
     pg = plan_gemm(s.sms, tokens, 2 * FF, W, gemm::EPI_GEGLU);
     pd = plan_gemm(s.sms, tokens, W, FF, gemm::EPI_PART);
-    const AttnPlan pa = plan_attention(s.sms, s.batch, s.prefix);
+    const AttnPlan pa = plan_attention_for(s.sms, s.batch, s.prefix, s.page_tokens);
+    join = pa.join;
     memset(&ap, 0, sizeof ap);
     ap.tok_tile = pa.tok_tile; ap.tiles = pa.tiles; ap.splits = pa.splits;
     e = opt_in(s.device);
     for (const GemmPlan* g : {&pq, &po, &pg, &pd})
-      if (e == cudaSuccess) e = opt_in_gemm(*g, s.device);
-    if (e == cudaSuccess) e = opt_in_attention(ap.tok_tile, s.device);
+      if (e == cudaSuccess && !(g == &po && with_o(s.sms, s.batch, s.prefix))) e = opt_in_gemm(*g, s.device);
+    fused = with_o(s.sms, s.batch, s.prefix);
+    if (fused) po.splits = NQH;
+    if (e == cudaSuccess) e = fused ? opt_in_attention_o(s.device) : opt_in_attention(ap.tok_tile, join, s.device);
     if (e == cudaSuccess) encode();
   }
 
@@ -552,7 +583,13 @@ struct Chain {
       return map_kv(m, s.pool_v, rows, L, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, 64, 4);
     };
     auto weights = [&](CUtensorMap* m, int which, int k, int rows, const GemmPlan& g) { return map_k(m, s.in[which], k, L * rows, g.w_rows, g.w_kb); };
-    if (!(map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_short, s.an, W, M, pq.arows - 8, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
+    if (join) {
+      ap.m_rows = (s.prefix - (s.prefix - 1) / attn::KCH * attn::KCH + 7) / 8 * 8;
+      ap.m_suf = 56 + (ap.m_rows % 16 == 0 ? 8 : 0);
+    }
+    auto joined = [&](CUtensorMap* m, const void* pool) { return !ap.m_rows || map_kv(m, pool, tail, L, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, ap.m_rows, 1); };
+    auto joined_suffix = [&](CUtensorMap* m, const void* kv) { return !ap.m_rows || map_kv(m, kv, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, ap.m_suf, 1); };
+    if (!(joined(&ap.jk, s.pool_k) && joined(&ap.jv, s.pool_v) && joined_suffix(&ap.jsk, s.k) && joined_suffix(&ap.jsv, s.v) && map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_short, s.an, W, M, pq.arows - 8, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
           map_k(&a_dn, s.act, FF, M, pd.arows, pd.ks) && weights(&wq, 8, W, QD, pq) && weights(&wk, 9, W, HD, pq) && weights(&wv, 10, W, HD, pq) &&
           weights(&wo, 11, QD, W, po) && weights(&wg, 12, W, FF, pg) && weights(&wu, 13, W, FF, pg) && weights(&wd, 14, FF, W, pd) &&
           map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH) &&
@@ -567,6 +604,33 @@ struct Chain {
     ap.page_table = s.page_table; ap.pages_per_obs = s.pages_per_obs; ap.page_tokens = s.page_tokens;
     ap.valid = (const uint8_t*)s.in[24]; ap.out = s.attn; ap.prefix = s.prefix; ap.suffix = T; ap.obs_tokens = T;
     ap.early = 1; ap.status = s.status; ap.limit = s.wait_limit;
+    if (fused) encode_fused(tail);
+  }
+
+  // Attention with the O projection: the prefix in its first page, or (pages of 64 tokens) in two.
+  void encode_fused(int tail) {
+    const uint64_t M = T * s.batch;
+    const attno::Layout l = attno::layout(s.prefix);
+    memset(&fp, 0, sizeof fp);
+    const bool two = s.prefix > s.page_tokens;
+    fp.rows0 = two ? s.page_tokens : l.rows - attno::SUF;
+    fp.rows1 = l.rows - attno::SUF - fp.rows0;
+    auto cache = [&](CUtensorMap* m, const void* pool, int tokens, int box) {
+      return map_kv(m, pool, tokens, NL, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, box, 1);
+    };
+    auto suffix = [&](CUtensorMap* m, const void* kv) { return map_kv(m, kv, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, attno::SUF, 1); };
+    if (!(map_2d(&fp.q, s.q, QD, M, T) && cache(&fp.pk0, s.pool_k, two ? s.page_tokens : tail, fp.rows0) && cache(&fp.pv0, s.pool_v, two ? s.page_tokens : tail, fp.rows0) &&
+          (!two || (cache(&fp.pk1, s.pool_k, tail, fp.rows1) && cache(&fp.pv1, s.pool_v, tail, fp.rows1))) && suffix(&fp.sk, s.k) && suffix(&fp.sv, s.v) &&
+          map_k(&fp.wo, s.in[11], QD, (uint64_t)NL * W, attno::FEAT, HD / 64))) {
+      e = cudaErrorUnknown;
+      what = "cuTensorMapEncodeTiled failed";
+      return;
+    }
+    fp.wo_base = (const __nv_bfloat16*)s.in[11];
+    fp.page_table = s.page_table; fp.valid = (const uint8_t*)s.in[24]; fp.part = s.part;
+    fp.pages_per_obs = s.pages_per_obs; fp.prefix = s.prefix; fp.tokens = T * s.batch;
+    fp.off_v = l.off_v; fp.off_q = l.off_q; fp.off_wo = l.off_wo; fp.wo_early = l.wo_early; fused_smem = l.smem;
+    fp.status = s.status; fp.limit = s.wait_limit;
   }
 
   void step() {
@@ -576,9 +640,14 @@ struct Chain {
     for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
       // (withheld: copies of fewer bytes than their barrier is told to expect)
       project(pq, l == s.withhold ? a_short : a_qkv, &wq, &wk, &wv, 0, l, l > 0);      // (what a step leaves behind is complete before the next one's first kernel starts)
-      ap.layer = l;
-      if (e == cudaSuccess) { e = launch_attention(ap, s.batch, stream); ++kernels; }
-      project(po, a_o, &wo, nullptr, nullptr, W, l);
+      if (fused) {
+        fp.layer = l;
+        if (e == cudaSuccess) { e = launch_attention_o(fp, s.batch, fused_smem, stream); ++kernels; }
+      } else {
+        ap.layer = l;
+        if (e == cudaSuccess) { e = launch_attention(ap, s.batch, stream); ++kernels; }
+        project(po, a_o, &wo, nullptr, nullptr, W, l);
+      }
       n.gate_norm = 2 * l; n.next_norm = 2 * l + 1;
       put(norm_kernel_for(po.splits), tokens, 256, 0, 1, n);
       project(pg, a_gu, &wg, &wu, nullptr, FF, l);
@@ -613,29 +682,40 @@ struct Chain {
 
 }  // namespace
 
-StepPlan steps_plan(int sms, int batch, int prefix) {
-  const AttnPlan a = plan_attention(sms, batch, prefix);
+namespace {
+StepPlan steps_plan_of(int sms, int batch, const AttnPlan& a, bool o) {
   StepPlan p;
-  p.tok_tile = a.tok_tile; p.splits = a.splits;
-  p.o_splits = plan_gemm(sms, T * batch, W, QD, gemm::EPI_PART).splits;
+  p.tok_tile = o ? T : a.tok_tile; p.splits = o ? 1 : a.splits;
+  p.o_splits = o ? NQH : plan_gemm(sms, T * batch, W, QD, gemm::EPI_PART).splits;
   p.down_splits = plan_gemm(sms, T * batch, W, FF, gemm::EPI_PART).splits;
   p.part_floats = (size_t)std::max(p.o_splits, p.down_splits) * T * batch * W;
-  if (a.splits > 1) p.part_floats = std::max(p.part_floats, (size_t)batch * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
+  if (p.splits > 1) p.part_floats = std::max(p.part_floats, (size_t)batch * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
   return p;
 }
+}  // namespace
 
-std::string steps_describe(int sms, int batch, int prefix, const StepGraphs& g) {
+StepPlan steps_plan(int sms, int batch, int prefix, int page_tokens) {
+  return steps_plan_of(sms, batch, plan_attention_for(sms, batch, prefix, page_tokens), with_o(sms, batch, prefix));
+}
+
+std::string steps_describe(int sms, int batch, int prefix, int page_tokens, const StepGraphs& g) {
   const int tokens = T * batch;
-  const AttnPlan a = plan_attention(sms, batch, prefix);
+  const AttnPlan a = plan_attention_for(sms, batch, prefix, page_tokens);
+  const bool o = with_o(sms, batch, prefix);
   const struct { const char* name; GemmPlan plan; } all[] = {{"qkv", plan_gemm(sms, tokens, QKVW, W, gemm::EPI_QKV)},
                                                               {"o", plan_gemm(sms, tokens, W, QD, gemm::EPI_PART)},
                                                               {"gate_up", plan_gemm(sms, tokens, 2 * FF, W, gemm::EPI_GEGLU)},
                                                               {"down", plan_gemm(sms, tokens, W, FF, gemm::EPI_PART)}};
   char buf[256];
   snprintf(buf, sizeof buf, "{\"prologue_launches\": %d, \"launches_per_layer\": %d, \"attention\": {\"query_tokens\": %d, \"ctas_per_tile\": %d, \"ctas\": %d}",
-           g.kernels_prologue, g.kernels_step / NL, a.tok_tile, a.splits, batch * a.tiles * a.splits);
+           g.kernels_prologue, g.kernels_step / NL, o ? T : a.tok_tile, o ? 1 : a.splits, o ? batch * NQH * attno::GROUPS : batch * a.tiles * a.splits);
   std::string out = buf;
   for (const auto& x : all) {
+    if (o && x.plan.epi == gemm::EPI_PART && x.plan.kblocks * x.plan.splits == QD / gemm::BK) {      // part of the attention
+      snprintf(buf, sizeof buf, ", \"o\": {\"within\": \"attention\", \"features_per_cta\": %d, \"k_splits\": %d}", attno::FEAT, NQH);
+      out += buf;
+      continue;
+    }
     snprintf(buf, sizeof buf, ", \"%s\": {\"tile_tokens\": %d, \"tile_features\": %d, \"cta_pairs\": %s, \"k_splits\": %d, \"ctas\": %d, \"stages\": %d}", x.name,
              x.plan.rows, x.plan.bn, x.plan.pair ? "true" : "false", x.plan.splits, x.plan.grid, x.plan.stages);
     out += buf;
@@ -648,7 +728,9 @@ std::string steps_describe(int sms, int batch, int prefix, const StepGraphs& g) 
 size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   size_t most = 0;
   for (int b = 1; b <= max_batch; ++b)
-    for (int prefix = 1; prefix <= max_prefix; prefix += attn::KCH) most = std::max(most, steps_plan(sms, b, prefix).part_floats);
+    for (int chunks = 1; chunks <= (max_prefix + attn::KCH - 1) / attn::KCH; ++chunks)
+      for (bool join : {false, true})
+        for (bool o : {false, true}) most = std::max(most, steps_plan_of(sms, b, plan_attention(sms, b, chunks, join), o && with_o(sms, b, 1)).part_floats);
   return most;
 }
 
@@ -662,7 +744,7 @@ int failed(const Chain& c, const char* doing, std::string* error) {
 
 int steps_build(const StepSetup& s, StepGraphs* g, std::string* error) {
   steps_free(g);
-  if (steps_plan(s.sms, s.batch, s.prefix).part_floats > s.part_floats) {
+  if (steps_plan(s.sms, s.batch, s.prefix, s.page_tokens).part_floats > s.part_floats) {
     *error = "the workspace does not hold the partial sums of this binding";
     return PI05_ERR_UNSUPPORTED;
   }

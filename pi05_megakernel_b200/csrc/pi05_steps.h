@@ -42,9 +42,9 @@ struct StepPlan {
   int tok_tile, splits, o_splits, down_splits;
   size_t part_floats;
 };
-StepPlan steps_plan(int sms, int batch, int prefix);
+StepPlan steps_plan(int sms, int batch, int prefix, int page_tokens);
 // The cuts of a binding, and the kernels of its launch (`g`: of the captured chain), as a JSON object.
-std::string steps_describe(int sms, int batch, int prefix, const StepGraphs& g);
+std::string steps_describe(int sms, int batch, int prefix, int page_tokens, const StepGraphs& g);
 // FP32 words of partial sums that up to `max_batch` observations with up to `max_prefix` prefix tokens need.
 size_t steps_part_floats(int sms, int max_batch, int max_prefix);
 // Captures and instantiates the graphs; frees what `g` held.

@@ -260,6 +260,12 @@ __device__ __forceinline__ void umma_bf16_k64(uint32_t d_tmem, uint32_t alo, uin
 #undef PI05_UMMA1
 #undef PI05_UMMA_STEP
 }
+// One of them.
+__device__ __forceinline__ void umma_bf16_k16(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc, uint32_t accumulate, uint32_t on) {
+  asm volatile("{\n.reg .pred p, q;\n.reg .b64 da, db;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %6, 0;\nmov.b64 da, {%1, %5};\n mov.b64 db, {%2, %5};\n"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}"
+               ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI), "r"(on) : "memory");
+}
 // One lane of a converged warp (always the same one), for instructions that a single thread must issue while the
 // loop around them stays warp-uniform.
 __device__ __forceinline__ bool elect_one() {

@@ -21,7 +21,13 @@ CUTS = [
     (1100, 2, "scatter", "b200-s1-l2"), (130, 7, "full", "b200-s1-l2"), (65, 11, "pad", "b200-s1-l2"), (257, 16, "scatter", "b200-s1-l2")]
 # (prefix, batch, tokens per page).  What is left of the attention's cuts on a B200: tiles of 2, 4, 6, 8 and 14 tokens over two and four
 # CTAs, the widest with a second segment of probabilities and a ring of four units; dense caches and pages of 64 and 128 tokens
-ATTENTION_CUTS = [(512, 1, 64), (600, 5, 0), (700, 6, 128), (700, 3, 64), (896, 9, 0), (896, 5, 64), (1700, 12, 0), (1300, 9, 64)]
+ATTENTION_CUTS = [(512, 1, 64), (600, 5, 0), (700, 6, 128), (700, 3, 64), (896, 9, 0), (896, 5, 64), (1700, 12, 0), (1300, 9, 64),
+                  (440, 1, 64), (456, 1, 64), (900, 6, 0), (768, 4, 0), (840, 4, 128), (2176, 11, 0), (2177, 11, 64), (2816, 5, 0)]
+# The suffix in the last chunk of the prefix: 8 cached keys there (16 rows with the suffix's padding), 56, 64 and 72, the widest and the narrowest tile,
+# pages of 64 and 128 tokens; 72 keys on pages of 64 stay apart
+# Attention with the O projection (up to 128 cached tokens, up to two observations): 1, 8 and 9 keys, the last with a place of its own for Wo and the first without,
+# 72 and 73 (suffix within the first 128 rows and across them), 120 and 128 (an odd and an even number of eights), one page and two
+ATTENTION_O = [(8, 1, 0), (9, 2, 64), (64, 1, 64), (65, 1, 64), (65, 2, 0), (72, 1, 128), (73, 2, 64), (120, 1, 0), (127, 2, 64), (128, 1, 64), (128, 2, 128)]
 
 
 @pytest.mark.parametrize("prefix,batch,mask,variant", CUTS)
@@ -73,6 +79,11 @@ def test_attention_cuts(prefix, batch, page):
         d = O.band(want, got[b], exact)
         assert d["pass"], (b, d)
     arm.close()
+
+
+@pytest.mark.parametrize("prefix,batch,page", ATTENTION_O)
+def test_attention_with_o_projection(prefix, batch, page):
+    test_attention_cuts(prefix, batch, page)
 
 
 def test_smaller_binding_stays_in_the_workspace():
