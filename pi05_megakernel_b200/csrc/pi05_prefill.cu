@@ -81,8 +81,8 @@ struct NormArgs {
 
 // x = bf16(src + bf16(sum of the parts)); out = Gemma RMSNorm of x (the reference's rms(x, weight, gemma=True),
 // reference/pi05.py:178, 192): FP32 normalisation, scale by (1 + weight), one rounding to BF16.  One token per block, four
-// columns per thread.  S: slices of partial sums ([S][tokens][2048]); 0: no projection before (the embeddings); -1: the slots
-// of a stream-K launch ([slot][128][256]).
+// columns per thread.  S: slices of partial sums ([S][tokens][2048]); 0: no projection before (the embeddings); -1 and -2: the slots
+// of a stream-K launch ([slot][128][256]), -2 with registers for 20 of them, which only a launch of a block per SM at most can afford (256 tokens 1.44 ms, on -2 1.45).
 template <int S>
 __global__ void __launch_bounds__(512) norm_kernel(const __grid_constant__ NormArgs p) {
   __shared__ float red[16];
@@ -105,10 +105,24 @@ __global__ void __launch_bounds__(512) norm_kernel(const __grid_constant__ NormA
     const float* q = p.part + (size_t)(blockIdx.x & 127) * 256 + (c0 & 255);
     a = __ldcg(reinterpret_cast<const float4*>(q + (size_t)(p.owner0 + tile) * 32768));
     const int first = p.first[tile], count = p.count[tile];
+    const float4* q4 = reinterpret_cast<const float4*>(q + (size_t)first * 32768);
+    int s = 0;
+    if constexpr (S == -2) {
+      // up to 20 slots, all on their way before the first is added: in eights, 19 of them took three trips to L2 (61 tokens: 3.6 us of a kernel of 5; prefill of
+      // 128 tokens 1.20 -> 1.18 ms).  What is read beyond the last contributor's is another slot
+      float4 v[20];
+#pragma unroll
+      for (int k = 0; k < 20; k += 4)
+        if (k < count) ptx::ld_l2_f4x4(reinterpret_cast<float4(&)[4]>(v[k]), q4 + (size_t)k * 8192, 8192);
+#pragma unroll
+      for (int k = 0; k < 20; ++k)
+        if (k < count) { a.x += v[k].x; a.y += v[k].y; a.z += v[k].z; a.w += v[k].w; }
+      s = 20;
+    }
 #pragma unroll 8
-    for (int s = 0; s < count; ++s) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(q + (size_t)(first + s) * 32768));
-      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    for (; s < count; ++s) {
+      const float4 w = __ldcg(q4 + (size_t)s * 8192);
+      a.x += w.x; a.y += w.y; a.z += w.z; a.w += w.w;
     }
   }
   float v[4] = {lo16(xv.x), hi16(xv.x), lo16(xv.y), hi16(xv.y)};
@@ -210,7 +224,7 @@ cudaError_t prefill_opt_in(int device) {
   static std::atomic<uint64_t> done;
   return once_per_device(&done, device, [] {
     cudaError_t e = cudaSuccess;
-    const void* all[] = {(const void*)pf::tables_kernel, (const void*)pf::norm_kernel<-1>, (const void*)pf::norm_kernel<0>,
+    const void* all[] = {(const void*)pf::tables_kernel, (const void*)pf::norm_kernel<-2>, (const void*)pf::norm_kernel<-1>, (const void*)pf::norm_kernel<0>,
                          (const void*)pf::norm_kernel<1>, (const void*)pf::norm_kernel<2>, (const void*)pf::norm_kernel<4>,
                          (const void*)pf::norm_kernel<8>};
     for (const void* k : all)
@@ -382,7 +396,7 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
     norm(pf::norm_kernel_for(pl.o.splits), x, w[LN2] + (size_t)l * pf::H);
     project(pl.gu, a_gu, wg, &wu, nullptr, pf::FFN, l);
     project(pl.down, a_dn, wd, nullptr, nullptr, pf::H, l);
-    norm(pl.sk_down ? pf::norm_kernel<-1> : pf::norm_kernel_for(pl.down.splits), x, w[LN1] + (size_t)(l + 1) * pf::H);
+    norm(pl.sk_down ? (P <= h->sms ? pf::norm_kernel<-2> : pf::norm_kernel<-1>) : pf::norm_kernel_for(pl.down.splits), x, w[LN1] + (size_t)(l + 1) * pf::H);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { h->last_error = std::string("kernel launch: ") + cudaGetErrorString(e); return PI05_ERR_CUDA; }
