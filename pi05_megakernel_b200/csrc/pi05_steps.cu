@@ -683,19 +683,18 @@ struct Chain {
 }  // namespace
 
 namespace {
-StepPlan steps_plan_of(int sms, int batch, const AttnPlan& a, bool o) {
+size_t attention_floats(int batch, const AttnPlan& a) { return a.splits > 1 ? (size_t)batch * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH) : 0; }
+}  // namespace
+
+StepPlan steps_plan(int sms, int batch, int prefix, int page_tokens) {
+  const AttnPlan a = plan_attention_for(sms, batch, prefix, page_tokens);
+  const bool o = with_o(sms, batch, prefix);
   StepPlan p;
   p.tok_tile = o ? T : a.tok_tile; p.splits = o ? 1 : a.splits;
   p.o_splits = o ? NQH : plan_gemm(sms, T * batch, W, QD, gemm::EPI_PART).splits;
   p.down_splits = plan_gemm(sms, T * batch, W, FF, gemm::EPI_PART).splits;
-  p.part_floats = (size_t)std::max(p.o_splits, p.down_splits) * T * batch * W;
-  if (p.splits > 1) p.part_floats = std::max(p.part_floats, (size_t)batch * a.tiles * a.splits * attn::part_floats(a.tok_tile * NQH));
+  p.part_floats = std::max((size_t)std::max(p.o_splits, p.down_splits) * T * batch * W, o ? 0 : attention_floats(batch, a));
   return p;
-}
-}  // namespace
-
-StepPlan steps_plan(int sms, int batch, int prefix, int page_tokens) {
-  return steps_plan_of(sms, batch, plan_attention_for(sms, batch, prefix, page_tokens), with_o(sms, batch, prefix));
 }
 
 std::string steps_describe(int sms, int batch, int prefix, int page_tokens, const StepGraphs& g) {
@@ -727,10 +726,12 @@ std::string steps_describe(int sms, int batch, int prefix, int page_tokens, cons
 // tokens over four CTAs up to 896 keys, of 4 over two from there on).
 size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   size_t most = 0;
-  for (int b = 1; b <= max_batch; ++b)
+  for (int b = 1; b <= max_batch; ++b) {
+    const int splits = std::max(plan_gemm(sms, T * b, W, QD, gemm::EPI_PART).splits, plan_gemm(sms, T * b, W, FF, gemm::EPI_PART).splits);
+    most = std::max(most, (size_t)std::max(splits, with_o(sms, b, 1) ? NQH : 0) * T * b * W);
     for (int chunks = 1; chunks <= (max_prefix + attn::KCH - 1) / attn::KCH; ++chunks)
-      for (bool join : {false, true})
-        for (bool o : {false, true}) most = std::max(most, steps_plan_of(sms, b, plan_attention(sms, b, chunks, join), o && with_o(sms, b, 1)).part_floats);
+      for (bool join : {false, true}) most = std::max(most, attention_floats(b, plan_attention(sms, b, chunks, join)));
+  }
   return most;
 }
 
