@@ -45,12 +45,12 @@ __host__ __device__ constexpr int units_for(int n) {
   return (226 * 1024 - 512 * n - p_bytes(n)) / UNIT < 6 ? (226 * 1024 - 512 * n - p_bytes(n)) / UNIT : 6;
 }
 __host__ __device__ constexpr int smem_for(int n) { return 512 * n + p_bytes(n) + units_for(n) * UNIT + 1024; }
-static_assert(units_for(16) == 6 && units_for(64) == 5 && units_for(112) == 4 && smem_for(32) + 2048 <= 227 * 1024 && smem_for(112) + 4096 <= 227 * 1024, "attention shared memory");
+static_assert(units_for(16) == 6 && units_for(64) == 5 && units_for(112) == 4 && smem_for(32) + 2048 <= 227 * 1024 && smem_for(112) + 5120 <= 227 * 1024, "attention shared memory");
 // FP32 words that a CTA of a split tile leaves behind.
 __host__ __device__ constexpr int part_floats(int n) { return n * (HD + 2); }
 
 struct Args {
-  CUtensorMap q;                           // [tokens x 8 rows, 256 dims], box {64, N}
+  CUtensorMap q;                           // [tokens x 8 rows, 256 dims] as {64, rows, 4}, box {64, N, 4}
   CUtensorMap pk, pk_tail, pv, pv_tail;    // prefix keys / values {64 dims, page tokens, 4, layers, pages}; K: box {64, k_rows, k_rows / 64,
                                            // 1, 1}, V: box {64, 64, 4, 1, 1}; *_tail: the same, cut at the last valid token of a last page
   CUtensorMap sk, sv;                      // suffix keys / values {64, tokens, 4, 1, observations}, box {64, 128, 2, 1, 1} and {64, 64, 4, 1, 1}
@@ -97,7 +97,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   __shared__ uint32_t s_tmem;
   __shared__ uint32_t s_mask[MASK_WORDS];
   __shared__ float s_red[4][N];            // what the four warps of a half exchange: maxima, at the end sums
-  __shared__ __align__(16) float s_m[N], s_mneg[N], s_f[N];   // reference of a row, the same as an exponent's summand, factor of a move / of the result
+  // a warp's own, of its half's rows: factor of a move, summand of the exponents, at the end factor of the result.  Every warp works out what it needs:
+  // one barrier less than by a thread per row
+  __shared__ __align__(16) float s_row[4][N];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x % p.splits, unit = blockIdx.x / p.splits;
   const int ob = unit / p.tiles, tile = unit % p.tiles;
@@ -250,8 +252,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     if (leader) {
       ptx::mbar_expect_tx(q_full, 4 * QBLK);
       ptx::grid_dep_wait();                // Q is this warp's, which is the one that waits for it: warp 0 may still be at the cache
-#pragma unroll
-      for (int kb = 0; kb < 4; ++kb) ptx::tma_load_2d(q_base + kb * QBLK, &p.q, q_full, kb * 64, (ob * p.obs_tokens + tile * p.tok_tile) * NQH);
+      ptx::tma_load_3d(q_base, &p.q, q_full, 0, (ob * p.obs_tokens + tile * p.tok_tile) * NQH, 0);
     }
     __syncwarp();
     bool go = ptx::wait_bar(p.status, p.limit, q_full, 0, WAIT_Q_FULL);
@@ -338,11 +339,13 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   } else if (warp >= 2) {
     // ---- softmax threads.  A wait that gives up does not end the loop: the other warps count on this one at their named
     // barriers, and every further wait returns at once
-    const int et = tid - 64, r0 = half * R;
+    const int r0 = half * R;
     const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + r0;
     float l[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) l[r] = 0.f;
+    constexpr int ROWS = (R + 31) / 32;                       // rows of the half per lane, with their references
+    float m[ROWS];
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
       const int buf = i & 1;
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
             ptx::tmem_wait_ld();
 #pragma unroll
             for (int c = 0; c < R; c += 4) {
-              const float4 mn = *reinterpret_cast<const float4*>(&s_mneg[r0 + c]);
+              const float4 mn = *reinterpret_cast<const float4*>(&s_row[quad][r0 + c]);
               const uint32_t x0 = pack2(__uint_as_float(x[c]), __uint_as_float(x[c + 1])), x1 = pack2(__uint_as_float(x[c + 2]), __uint_as_float(x[c + 3]));
               t[c] = fmaf(lo16(x0), SCALE_LOG2E, mn.x); t[c + 1] = fmaf(hi16(x0), SCALE_LOG2E, mn.y);
               t[c + 2] = fmaf(lo16(x1), SCALE_LOG2E, mn.z); t[c + 3] = fmaf(hi16(x1), SCALE_LOG2E, mn.w);
@@ -406,19 +409,22 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
           __syncwarp();
         }
         ptx::named_bar_sync(1, SOFTMAX);
-        if (et < N) {
-          const float cm = rb(fmaxf(fmaxf(s_red[0][et], s_red[1][et]), fmaxf(s_red[2][et], s_red[3][et]))) * 0.0625f;
-          float m = i == 0 ? fmaxf(cm, -1e30f) : s_m[et], f = 1.f;
-          if (i > 0 && cm > m + RESCALE_LOG) { f = ptx::ex2_approx((m - cm) * LOG2E); m = cm; }
-          s_m[et] = m;
-          s_mneg[et] = -m * LOG2E;
-          s_f[et] = f;
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+          const int k = r0 + lane + 32 * j;
+          if (k < r0 + R) {
+            const float cm = rb(fmaxf(fmaxf(s_red[0][k], s_red[1][k]), fmaxf(s_red[2][k], s_red[3][k]))) * 0.0625f;
+            float f = 1.f;
+            if (i == 0) m[j] = fmaxf(cm, -1e30f);
+            else if (cm > m[j] + RESCALE_LOG) { f = ptx::ex2_approx((m[j] - cm) * LOG2E); m[j] = cm; }
+            s_row[quad][k] = i == 0 ? -m[j] * LOG2E : f;
+          }
         }
-        ptx::named_bar_sync(1, SOFTMAX);
+        __syncwarp();
         if (i > 0) {
           // rescale what has been accumulated
 #pragma unroll
-          for (int r = 0; r < R; ++r) l[r] *= s_f[r0 + r];
+          for (int r = 0; r < R; ++r) l[r] *= s_row[quad][r0 + r];
           ok &= ptx::wait_bar(p.status, p.limit, p_empty, (i - 1) & 1, WAIT_P_EMPTY);
           ptx::tc_fence_after();
 #pragma unroll 1
@@ -429,10 +435,15 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
             ptx::tmem_ld_32x8(at, o);
             ptx::tmem_wait_ld();
 #pragma unroll
-            for (int k = 0; k < 8; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * s_f[r0 + row + k]);
+            for (int k = 0; k < 8; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * s_row[quad][r0 + row + k]);
             ptx::tmem_st_32x8(at, o);
           }
           ptx::tmem_wait_st();
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < ROWS; ++j)
+            if (lane + 32 * j < R) s_row[quad][r0 + lane + 32 * j] = -m[j] * LOG2E;
+          __syncwarp();
         }
       }
       __syncwarp();
@@ -442,6 +453,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
       ptx::mbar_arrive(p_full);
     }
     // the rows' sums over all keys, while the last P V runs
+    if (n == 1) ptx::named_bar_sync(1, SOFTMAX);              // (with more chunks their votes lie between the maxima's readers and this)
 #pragma unroll
     for (int c = 0; c < R; c += 8) {
       float mine = 0.f;
@@ -457,12 +469,16 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
     __syncwarp();
     ptx::named_bar_sync(1, SOFTMAX);
     float* part = p.merge + (size_t)(unit * p.splits + split) * part_floats(N);
-    if (et < N) {
-      const float sum = (s_red[0][et] + s_red[1][et]) + (s_red[2][et] + s_red[3][et]);
-      if (p.splits == 1) s_f[et] = sum > 0.f ? 1.0f / sum : 0.f;     // (no valid key: zeros)
-      else __stcg(reinterpret_cast<float2*>(part + N * HD) + et, make_float2(s_m[et], sum));
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      const int k = r0 + lane + 32 * j;
+      if (k < r0 + R) {
+        const float sum = (s_red[0][k] + s_red[1][k]) + (s_red[2][k] + s_red[3][k]);
+        if (p.splits == 1) s_row[quad][k] = sum > 0.f ? 1.0f / sum : 0.f;     // (no valid key: zeros)
+        else if (quad == 0) __stcg(reinterpret_cast<float2*>(part + N * HD) + k, make_float2(m[j], sum));
+      }
     }
-    ptx::named_bar_sync(1, SOFTMAX);
+    __syncwarp();
     ok &= ptx::wait_bar(p.status, p.limit, o_full, 0, WAIT_O_FULL);
     ptx::tc_fence_after();
 
@@ -480,7 +496,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
         ptx::tmem_wait_ld();
         if (row < out_rows && ok)
 #pragma unroll
-          for (int k = 0; k < 8; ++k) base[(row + k) * HD + d * 128] = __float2bfloat16_rn(__uint_as_float(o[k]) * s_f[row + k]);
+          for (int k = 0; k < 8; ++k) base[(row + k) * HD + d * 128] = __float2bfloat16_rn(__uint_as_float(o[k]) * s_row[quad][row + k]);
         __syncwarp();
       }
       ptx::tc_fence_before();

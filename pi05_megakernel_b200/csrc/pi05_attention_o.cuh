@@ -25,9 +25,11 @@ using attn::pack2;
 
 constexpr int NTHREADS = 576, SOFTMAX = 512, N = 64, R = 32, TOK = pi05::T, SUF = 56, QROWS = 56, FEAT = 128, GROUPS = pi05::W / FEAT;
 constexpr int MAX_PREFIX = 128, WO_BYTES = FEAT * HD * 2, OT_BYTES = HD * 128;
+constexpr int MAX_SMEM = 221 * 1024;       // of `layout`, and 5 KB of static shared memory
+static_assert(MAX_SMEM + 5632 <= 227 * 1024, "shared memory");
 
 struct Args {
-  CUtensorMap q;                           // {2048 dims, tokens}, box {64, 50}
+  CUtensorMap q;                           // {64 dims, tokens, 32}, box {64, 56, 4}
   CUtensorMap pk0, pk1, pv0, pv1;          // cached keys / values {64 dims, page tokens, 4, layers, pages}, boxes of rows0 and rows1 tokens; cut at the last valid token
   CUtensorMap sk, sv;                      // suffix keys / values {64, 50, 4, 1, observations}, box {64, 56, 1, 1, 1}
   CUtensorMap wo;                          // {64 k, layers x 1024 features, 32}, box {64, 128, 4}
@@ -48,7 +50,7 @@ inline Layout layout(int prefix) {
   Layout l;
   l.rows = (prefix + 7) / 8 * 8 + SUF;
   const int kv = l.rows * 512, p = (l.rows + 15) / 16 * 16 * 128;
-  l.wo_early = 2 * kv + OT_BYTES + WO_BYTES <= 220 * 1024;
+  l.wo_early = 2 * kv + OT_BYTES + WO_BYTES <= MAX_SMEM - 1024;
   l.off_v = l.wo_early || kv > p + WO_BYTES ? kv : p + WO_BYTES;
   l.off_q = l.off_v + kv;
   l.off_wo = l.wo_early ? l.off_q + OT_BYTES : p;
@@ -156,10 +158,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_o_kernel(const __grid_co
                    odesc = (uint32_t)ptx::umma_smem_desc_mn(q_base, 16384);
     const uint32_t on = leader ? 1u : 0u;
     if (leader) {
-      ptx::mbar_expect_tx(q_full, 4 * TOK * 128);
+      ptx::mbar_expect_tx(q_full, 4 * QROWS * 128);
       ptx::grid_dep_wait();
-#pragma unroll
-      for (int kb = 0; kb < 4; ++kb) ptx::tma_load_2d(q_base + kb * QROWS * 128, &p.q, q_full, head * HD + kb * 64, ob * TOK);
+      ptx::tma_load_3d(q_base, &p.q, q_full, 0, ob * TOK, head * 4);
     }
     __syncwarp();
     bool go = ptx::wait_bar(p.status, p.limit, k_full, 0, attn::WAIT_KV_FULL);

@@ -76,18 +76,6 @@ bool map_k(CUtensorMap* m, const void* base, uint64_t k, uint64_t rows, uint32_t
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
-  EncodeTiledFn enc = encoder();
-  if (!enc) return false;
-  cuuint64_t dims[2] = {inner, rows};
-  cuuint64_t strides[1] = {inner * 2};
-  cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, uint64_t pages, uint64_t token_stride,
             uint64_t layer_stride, uint64_t page_stride, uint32_t box_tokens, uint32_t box_blocks) {
   EncodeTiledFn enc = encoder();
@@ -226,7 +214,7 @@ cudaError_t launch_attention_o(const attno::Args& p, int observations, int smem,
 
 cudaError_t opt_in_attention_o(int device) {
   static std::atomic<uint64_t> done;
-  return once_per_device(&done, device, [] { return chain_opt_in((const void*)attno::attention_o_kernel<attno::NTHREADS>, 222 * 1024); });
+  return once_per_device(&done, device, [] { return chain_opt_in((const void*)attno::attention_o_kernel<attno::NTHREADS>, attno::MAX_SMEM); });
 }
 
 }  // namespace pi05

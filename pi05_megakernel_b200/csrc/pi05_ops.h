@@ -44,8 +44,6 @@ cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, size_
 // An operand [rows, K] BF16 row-major as {64 k, rows, K / 64}, box {64, box_rows, blocks}, 128-byte swizzle: one copy brings
 // `blocks` 64-k blocks of box_rows rows.  Rows beyond `rows` read as zeros.
 bool map_k(CUtensorMap* m, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t blocks);
-// {inner, rows} BF16 row-major, box {64, box_rows}, 128-byte swizzle.
-bool map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_rows);
 // Keys or values as the attention's tiled copies read them: {64 dims, tokens, 4 blocks, layers, pages} with strides in elements,
 // box {64, box_tokens, box_blocks, 1, 1}; tokens beyond `tokens` read as zeros.
 bool map_kv(CUtensorMap* m, const void* base, uint64_t tokens, uint64_t layers, uint64_t pages, uint64_t token_stride,

@@ -345,7 +345,7 @@ int pi05_prefill_run(pi05_prefill_t h, const void* embeddings, const void* valid
                   weight_map(&wu, LU, pf::H, pf::FFN, pl.gu) && weight_map(&wd, LD, pf::FFN, pf::H, pl.down) &&
                   map_kv(&ap.pk, K, P, L, 1, HD, (uint64_t)P * HD, L * P * HD, attn::KCH, 2) &&
                   map_kv(&ap.pv, V, P, L, 1, HD, (uint64_t)P * HD, L * P * HD, 64, 4) &&
-                  map_2d(&ap.q, q, HD, (uint64_t)P * NQH, pl.tok_tile * NQH);
+                  map_k(&ap.q, q, HD, (uint64_t)P * NQH, pl.tok_tile * NQH, HD / 64);
   if (!ok) { h->last_error = "cuTensorMapEncodeTiled failed"; return PI05_ERR_CUDA; }
   ap.pk_tail = ap.pk; ap.pv_tail = ap.pv; ap.sk = ap.pk; ap.sv = ap.pv;
   ap.valid = static_cast<const uint8_t*>(valid); ap.out = mixed;

@@ -592,7 +592,7 @@ struct Chain {
     if (!(joined(&ap.jk, s.pool_k) && joined(&ap.jv, s.pool_v) && joined_suffix(&ap.jsk, s.k) && joined_suffix(&ap.jsv, s.v) && map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_short, s.an, W, M, pq.arows - 8, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
           map_k(&a_dn, s.act, FF, M, pd.arows, pd.ks) && weights(&wq, 8, W, QD, pq) && weights(&wk, 9, W, HD, pq) && weights(&wv, 10, W, HD, pq) &&
           weights(&wo, 11, QD, W, po) && weights(&wg, 12, W, FF, pg) && weights(&wu, 13, W, FF, pg) && weights(&wd, 14, FF, W, pd) &&
-          map_2d(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH) &&
+          map_k(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH, HD / 64) &&
           keys(&ap.pk, s.page_tokens) &&
           keys(&ap.pk_tail, tail) && values(&ap.pv, s.page_tokens) && values(&ap.pv_tail, tail) &&
           map_kv(&ap.sk, s.k, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, attn::KCH, 2) &&
@@ -619,7 +619,7 @@ struct Chain {
       return map_kv(m, pool, tokens, NL, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, box, 1);
     };
     auto suffix = [&](CUtensorMap* m, const void* kv) { return map_kv(m, kv, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, attno::SUF, 1); };
-    if (!(map_2d(&fp.q, s.q, QD, M, T) && cache(&fp.pk0, s.pool_k, two ? s.page_tokens : tail, fp.rows0) && cache(&fp.pv0, s.pool_v, two ? s.page_tokens : tail, fp.rows0) &&
+    if (!(map_k(&fp.q, s.q, QD, M, attno::QROWS, HD / 64) && cache(&fp.pk0, s.pool_k, two ? s.page_tokens : tail, fp.rows0) && cache(&fp.pv0, s.pool_v, two ? s.page_tokens : tail, fp.rows0) &&
           (!two || (cache(&fp.pk1, s.pool_k, tail, fp.rows1) && cache(&fp.pv1, s.pool_v, tail, fp.rows1))) && suffix(&fp.sk, s.k) && suffix(&fp.sv, s.v) &&
           map_k(&fp.wo, s.in[11], QD, (uint64_t)NL * W, attno::FEAT, HD / 64))) {
       e = cudaErrorUnknown;
