@@ -1,7 +1,7 @@
 // The action chunk as a chain of kernels, one set per layer pass, replayed from CUDA graphs.
 //
 // A layer pass is seven kernels - QKV projection (+ RoPE), attention, O projection, gated residual + adaRMS, gate / up
-// projection (+ GeGLU), down projection, gated residual + adaRMS - and an Euler step is 18 of them, the last residual being
+// projection (+ GeGLU), down projection, gated residual + adaRMS; of short prefixes attention and O projection are one - and an Euler step is 18 of them, the last residual being
 // the step tail.  The step's kernels are captured once per binding; the Euler step index and the number of steps live in
 // device memory, so the same graph is launched once per step.  What the graphs do not fit - fewer layers, a stream that is being
 // captured, another wait limit than at bind - is launched kernel by kernel: a launch never builds a graph.  Every kernel but the
@@ -119,62 +119,66 @@ __global__ void __launch_bounds__(256) time_mlp_kernel(const MatArgs p) {
 
 // The 37 modulation layers for the ten time steps at once: out[s][row] = W[row][:] . in[s][:] + bias[row]; the 474 MB of FP32
 // weights are streamed from HBM exactly once.  A warp takes four rows; lane l covers k = 4 l .. 4 l + 3 of every 128, the
-// ten vectors lie in shared memory, products are accumulated in packed FP32 pairs.
-__global__ void __launch_bounds__(256, 2) modulation_kernel(const MatArgs p) {
-  constexpr int R = 4;
-  __shared__ float4 c[NS][W / 4];
+// ten vectors lie in shared memory, products are accumulated in packed FP32 pairs.  What bounds it is how much is on its way from HBM: a lane copies the
+// 16 bytes of each row that it will use itself into a ring of four stages of 128 columns, 96 KB in flight per SM.  (With the next 128 columns in registers,
+// 32 KB in flight, a chunk took 26 to 38 us longer: 4.223 and 4.196 ms at prefix 128.)
+constexpr int MOD_THREADS = 512, MOD_STAGES = 4, MOD_R = 4;
+constexpr int MOD_SMEM = NS * W * 4 + MOD_THREADS / 32 * MOD_STAGES * MOD_R * 512;
+__global__ void __launch_bounds__(MOD_THREADS, 1) modulation_kernel(const MatArgs p) {
+  constexpr int R = MOD_R;
+  extern __shared__ __align__(16) float s_dyn[];
+  float4* c = reinterpret_cast<float4*>(s_dyn);             // [10][256]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float4* ring = c + NS * W / 4 + warp * (MOD_STAGES * R * 32) + lane;
   ptx::grid_dep_launch();
-  const int nrows = NNORM * MODW;
-  const float* wrow = nullptr;
-  const float* bias = nullptr;
-  auto locate = [&](int row0) {
+  const int nrows = NNORM * MODW, step = gridDim.x * (MOD_THREADS / 32) * R;
+  auto weights = [&](int row0, const float*& bias) -> const float* {
     const int n = row0 / MODW, j = row0 - n * MODW, which = n == NNORM - 1 ? 2 : (n & 1);
     const size_t r = which == 2 ? (size_t)j : (size_t)(n >> 1) * MODW + j;
-    wrow = p.w[which] + r * W;
     bias = p.b[which] + r;
+    return p.w[which] + r * W + lane * 4;
   };
-  int row0 = (blockIdx.x * 8 + warp) * R;
-  float4 w[2][R];
-  if (row0 < nrows) {
-    locate(row0);
+  int row0 = (blockIdx.x * (MOD_THREADS / 32) + warp) * R;
+  const float *wrow = nullptr, *bias = nullptr;
+  if (row0 < nrows) wrow = weights(row0, bias);
+  auto request = [&](const float* w, int j) {
+    if (w)
 #pragma unroll
-    for (int r = 0; r < R; ++r) w[0][r] = ptx::ldg_stream_f4(wrow + (size_t)r * W + lane * 4);
-  }
+      for (int r = 0; r < R; ++r) ptx::copy_async_16(ring + ((j & (MOD_STAGES - 1)) * R + r) * 32, w + (size_t)r * W + j * 128);
+    ptx::copy_async_commit();
+  };
+#pragma unroll
+  for (int j = 0; j < MOD_STAGES - 1; ++j) request(wrow, j);
   ptx::grid_dep_wait();
-  for (int i = tid; i < NS * W / 4; i += 256) (&c[0][0])[i] = __ldcg(reinterpret_cast<const float4*>(p.in) + i);
+  for (int i = tid; i < NS * W / 4; i += MOD_THREADS) c[i] = __ldcg(reinterpret_cast<const float4*>(p.in) + i);
   __syncthreads();
-  for (; row0 < nrows; row0 += gridDim.x * 8 * R) {
+  for (; row0 < nrows; row0 += step) {
     float2 acc[R][NS];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int s = 0; s < NS; ++s) acc[r][s] = make_float2(0.f, 0.f);
-    const float* wcur = wrow;
-    const float* bcur = bias;
-    const int next = row0 + gridDim.x * 8 * R;
-    if (next < nrows) locate(next);
+    const float *bcur = bias, *wnext = nullptr;
+    if (row0 + step < nrows) wnext = weights(row0 + step, bias);
 #pragma unroll
     for (int j = 0; j < W / 128; ++j) {
-      // the loads of the next 128 columns (or of the next rows) are issued before this block's products
-      if (j + 1 < W / 128) {
+      if (j + MOD_STAGES - 1 < W / 128) request(wrow, j + MOD_STAGES - 1);
+      else request(wnext, j + MOD_STAGES - 1 - W / 128);
+      ptx::copy_async_wait<MOD_STAGES - 1>();
+      float4 w[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) w[(j + 1) & 1][r] = ptx::ldg_stream_f4(wcur + (size_t)r * W + (j + 1) * 128 + lane * 4);
-      } else if (next < nrows) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) w[0][r] = ptx::ldg_stream_f4(wrow + (size_t)r * W + lane * 4);
-      }
+      for (int r = 0; r < R; ++r) w[r] = ring[((j & (MOD_STAGES - 1)) * R + r) * 32];
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
-        const float4 v = c[s][j * 32 + lane];
+        const float4 v = c[s * (W / 4) + j * 32 + lane];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          const float4 a = w[j & 1][r];
-          acc[r][s] = ptx::fma2(make_float2(a.x, a.y), make_float2(v.x, v.y), acc[r][s]);
-          acc[r][s] = ptx::fma2(make_float2(a.z, a.w), make_float2(v.z, v.w), acc[r][s]);
+          acc[r][s] = ptx::fma2(make_float2(w[r].x, w[r].y), make_float2(v.x, v.y), acc[r][s]);
+          acc[r][s] = ptx::fma2(make_float2(w[r].z, w[r].w), make_float2(v.z, v.w), acc[r][s]);
         }
       }
     }
+    wrow = wnext;
     // 40 sums over the 32 lanes: fold the lanes' halves together while halving the number of values each lane keeps
     float v[40];
 #pragma unroll
@@ -475,7 +479,7 @@ cudaError_t opt_in(int device) {
         {(const void*)tail_kernel<false>, TAIL_SMEM}, {(const void*)tail_kernel<true>, TAIL_SMEM},
         {(const void*)residual_norm_kernel<1>, 0}, {(const void*)residual_norm_kernel<2>, 0},
         {(const void*)residual_norm_kernel<4>, 0}, {(const void*)residual_norm_kernel<8>, 0},
-        {(const void*)modulation_kernel, 0}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
+        {(const void*)modulation_kernel, MOD_SMEM}, {(const void*)time_mlp_kernel, 0}, {(const void*)tables_kernel, 0}};
     cudaError_t e = cudaSuccess;
     for (const auto& k : all)
       if (e == cudaSuccess) e = chain_opt_in(k.kernel, k.smem);
@@ -552,7 +556,7 @@ struct Chain {
     m.w[0] = (const float*)s.in[15]; m.b[0] = (const float*)s.in[16];
     m.w[1] = (const float*)s.in[17]; m.b[1] = (const float*)s.in[18];
     m.w[2] = (const float*)s.in[19]; m.b[2] = (const float*)s.in[20];
-    put(modulation_kernel, 2 * s.sms, 256, 0, 1, m);
+    put(modulation_kernel, s.sms, MOD_THREADS, MOD_SMEM, 1, m);
     put(tail_kernel<true>, std::min(T * s.batch, s.sms), TAIL_THREADS, TAIL_SMEM, 1, tail_args());
   }
 

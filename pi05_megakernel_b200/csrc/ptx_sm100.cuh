@@ -440,6 +440,13 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
                : "=r"(r) : "r"(id), "r"(nthreads), "r"(pred ? 1 : 0) : "memory");
   return r != 0;
 }
+// 16 bytes from global to shared memory past L1, as part of the thread's current group; the wait returns when all but the last N groups are there.
+__device__ __forceinline__ void copy_async_16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // Streaming 16-byte load that does not allocate in L1.
 __device__ __forceinline__ float4 ldg_stream_f4(const float* p) {
   float4 v;
