@@ -201,7 +201,8 @@ int pi05_schedule_plan(int sms, int batch, int prefix_len, const pi05_tuning* tu
 
 /* How the default launch (the chain of kernels) of `batch` observations of prefix_len tokens is cut on a GPU of `sms` SMs, by an
  * engine created for (max_prefix, max_batch), computed on the host (no counterpart in the reference): info = {query tokens per
- * CTA of the attention, CTAs that share the keys of a tile, K splits of the O and of the down projection}; the FP32 words of
+ * CTA of the attention (all 50: of one head, with the O projection in the same kernel, whose splits are then the heads), CTAs that share the
+ * keys of a tile, K splits of the O and of the down projection} for a dense cache; the FP32 words of
  * partial sums that the engine's workspace holds and that this binding writes. */
 #define PI05_CHUNK_PLAN_INFO 4
 int pi05_chunk_plan(int sms, int max_batch, int max_prefix, int batch, int prefix_len, int info[PI05_CHUNK_PLAN_INFO], size_t* held,

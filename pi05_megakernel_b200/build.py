@@ -11,6 +11,7 @@ SOURCES = [os.path.join(HERE, "csrc", "pi05_engine.cu"), os.path.join(HERE, "csr
            os.path.join(HERE, "csrc", "pi05_steps.cu"), os.path.join(HERE, "csrc", "pi05_ops.cu")]
 HEADERS = [os.path.join(HERE, "csrc", "ptx_sm100.cuh"), os.path.join(HERE, "csrc", "pi05_common.cuh"),
            os.path.join(HERE, "csrc", "pi05_chunk_kernel.cuh"), os.path.join(HERE, "csrc", "pi05_attention.cuh"),
+           os.path.join(HERE, "csrc", "pi05_attention_o.cuh"),
            os.path.join(HERE, "csrc", "pi05_gemm.cuh"), os.path.join(HERE, "csrc", "pi05_steps.h"),
            os.path.join(HERE, "csrc", "pi05_ops.h"),
            os.path.join(os.path.dirname(HERE), "include", "pi05_b200.h")]

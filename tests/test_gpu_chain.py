@@ -23,8 +23,8 @@ CUTS = [
 # CTAs, the widest with a second segment of probabilities and a ring of four units; dense caches and pages of 64 and 128 tokens
 ATTENTION_CUTS = [(512, 1, 64), (600, 5, 0), (700, 6, 128), (700, 3, 64), (896, 9, 0), (896, 5, 64), (1700, 12, 0), (1300, 9, 64),
                   (440, 1, 64), (456, 1, 64), (900, 6, 0), (768, 4, 0), (840, 4, 128), (2176, 11, 0), (2177, 11, 64), (2816, 5, 0)]
-# The suffix in the last chunk of the prefix: 8 cached keys there (16 rows with the suffix's padding), 56, 64 and 72, the widest and the narrowest tile,
-# pages of 64 and 128 tokens; 72 keys on pages of 64 stay apart
+# (among them the suffix in the last chunk of the prefix: 8 cached keys there, 56 and 72, the widest tile, pages of 64 and 128 tokens; 72 keys on pages of
+# 64 stay apart)
 # Attention with the O projection (up to 128 cached tokens, up to two observations): 1, 8 and 9 keys, the last with a place of its own for Wo and the first without,
 # 72 and 73 (suffix within the first 128 rows and across them), 120 and 128 (an odd and an even number of eights), one page and two
 ATTENTION_O = [(8, 1, 0), (9, 2, 64), (64, 1, 64), (65, 1, 64), (65, 2, 0), (72, 1, 128), (73, 2, 64), (120, 1, 0), (127, 2, 64), (128, 1, 64), (128, 2, 128)]
