@@ -207,6 +207,11 @@ int pi05_schedule_plan(int sms, int batch, int prefix_len, const pi05_tuning* tu
 #define PI05_CHUNK_PLAN_INFO 4
 int pi05_chunk_plan(int sms, int max_batch, int max_prefix, int batch, int prefix_len, int info[PI05_CHUNK_PLAN_INFO], size_t* held,
                     size_t* needed);
+/* Its attention, also for a paged cache (pages of page_tokens tokens; prefix_len: a dense one): info = {query tokens per CTA, CTAs that share the
+ * keys of a tile, 1 where the suffix joins the last chunk of cached keys, most chunks of 128 keys that a CTA takes, 1 where the O projection is in the
+ * same kernel: the queries of a head then, all keys at once}.  Several pages hold a multiple of 64 tokens each. */
+#define PI05_CHUNK_ATTENTION_INFO 5
+int pi05_chunk_attention(int sms, int batch, int prefix_len, int page_tokens, int info[PI05_CHUNK_ATTENTION_INFO]);
 
 /* Tensor parallel (no counterpart in the reference, which runs on one GPU only): tp_size engines, one per GPU, each
  * bound to the SAME 25 inputs in its own GPU's memory, compute one chunk together.  Rank r streams only its share of

@@ -89,6 +89,7 @@ SIGNATURES = {
                                          _c.POINTER(_c.c_int), _c.c_int, _c.POINTER(_c.c_int), _c.POINTER(_c.c_int)]),
     "pi05_chunk_plan": (_c.c_int, [_c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_c.c_int), _c.POINTER(_c.c_size_t),
                                    _c.POINTER(_c.c_size_t)]),
+    "pi05_chunk_attention": (_c.c_int, [_c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.POINTER(_c.c_int)]),
     "pi05_tp_export": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_size_t]),
     "pi05_tp_attach": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_void_p]),
     "pi05_tp_attach_pointer": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_void_p]),

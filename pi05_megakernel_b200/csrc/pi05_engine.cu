@@ -1005,6 +1005,15 @@ int pi05_chunk_plan(int sms, int max_batch, int max_prefix, int batch, int prefi
   return PI05_OK;
 }
 
+int pi05_chunk_attention(int sms, int batch, int prefix_len, int page_tokens, int info[PI05_CHUNK_ATTENTION_INFO]) {
+  if (sms < 2 || sms > 1024 || batch < 1 || batch > MAXB || prefix_len < 1 || prefix_len > 4096 || page_tokens < 1 ||
+      (page_tokens < prefix_len && page_tokens % 64) || !info)
+    return PI05_ERR_ARGUMENT;
+  const StepPlan p = steps_plan(sms, batch, prefix_len, page_tokens);
+  info[0] = p.tok_tile; info[1] = p.splits; info[2] = p.join; info[3] = p.chunks; info[4] = p.with_o;
+  return PI05_OK;
+}
+
 int pi05_schedule_plan_tp(int sms, int batch, int prefix_len, int tp_rank, int tp_size, const pi05_tuning* tuning,
                           int* entries, int capacity, int* count, int info[PI05_PLAN_INFO]) {
   if (sms < 1 || sms > 1024 || batch < 1 || batch > MAXB || prefix_len < 1 || capacity < 0 || (capacity > 0 && !entries) ||

@@ -695,6 +695,8 @@ StepPlan steps_plan(int sms, int batch, int prefix, int page_tokens) {
   const bool o = with_o(sms, batch, prefix);
   StepPlan p;
   p.tok_tile = o ? T : a.tok_tile; p.splits = o ? 1 : a.splits;
+  p.with_o = o; p.join = !o && a.join;
+  p.chunks = o ? 1 : ((prefix + attn::KCH - 1) / attn::KCH + (a.join ? 0 : 1) + a.splits - 1) / a.splits;
   p.o_splits = o ? NQH : plan_gemm(sms, T * batch, W, QD, gemm::EPI_PART).splits;
   p.down_splits = plan_gemm(sms, T * batch, W, FF, gemm::EPI_PART).splits;
   p.part_floats = std::max((size_t)std::max(p.o_splits, p.down_splits) * T * batch * W, o ? 0 : attention_floats(batch, a));

@@ -40,6 +40,8 @@ struct StepGraphs {
 // projections, FP32 words of partial sums.
 struct StepPlan {
   int tok_tile, splits, o_splits, down_splits;
+  int chunks;                                // of 128 keys, the most that a CTA of the attention takes
+  bool join, with_o;                         // the suffix in the last chunk of the prefix; attention and O projection in one kernel (all keys at once)
   size_t part_floats;
 };
 StepPlan steps_plan(int sms, int batch, int prefix, int page_tokens);

@@ -151,16 +151,19 @@ def test_chunk_partials_fit_the_workspace(lib, sms):
 
 
 def test_every_attention_cut_has_a_gpu_test(lib):
-    """The sizes of the GPU tests reach every (query tokens, CTAs per tile) that a B200 chooses for any prefix and batch."""
-    from tests.test_gpu_chain import ATTENTION_CUTS, CUTS
-    info, held, needed = (ctypes.c_int * 4)(), ctypes.c_size_t(), ctypes.c_size_t()
+    """The sizes of the GPU tests reach every (query tokens, CTAs per tile, suffix in the last chunk of the prefix, with the O projection)
+    that a B200 chooses for any batch, any prefix and a dense cache or pages of 64 or 128 tokens."""
+    from tests.test_gpu_chain import ATTENTION_CUTS, ATTENTION_O, CUTS
+    info = (ctypes.c_int * 5)()
 
-    def cut(batch, prefix):
-        assert lib.pi05_chunk_plan(148, batch, prefix, batch, prefix, info, ctypes.byref(held), ctypes.byref(needed)) == _lib.OK
-        return tuple(info)[:2]
+    def cut(batch, prefix, page):
+        assert lib.pi05_chunk_attention(148, batch, prefix, page or prefix, info) == _lib.OK
+        return info[0], info[1], info[2], info[4]
 
-    chosen = {cut(b, 128 * c) for b in range(1, 17) for c in range(1, 33)}
-    assert chosen == {cut(b, p) for p, b, _mask, _variant in CUTS} | {cut(b, p) for p, b, _page in ATTENTION_CUTS}
+    chosen = {cut(b, p, page) for b in range(1, 17) for p in range(1, 4097) for page in (0, 64, 128)}
+    assert chosen == {cut(b, p, 0) for p, b, _mask, _variant in CUTS} | {cut(b, p, page) for p, b, page in ATTENTION_CUTS + ATTENTION_O}
+    for args in ((1, 1, 64, 64), (148, 0, 64, 64), (148, 17, 64, 64), (148, 1, 0, 64), (148, 1, 4097, 4097), (148, 1, 64, 0), (148, 1, 200, 100)):
+        assert lib.pi05_chunk_attention(*args, info) == _lib.ERR_ARGUMENT
 
 
 def test_prefill_fixture_is_deterministic():
