@@ -206,24 +206,30 @@ def test_wait_of_the_chain_that_runs_out(prefix, batch):
     arm.close()
 
 
-@pytest.mark.parametrize("prefix", [300, 968])
-def test_attention_reference_moves(prefix):
-    """Scores that grow from one chunk of keys to the next: the exponent's reference, taken from the first chunk, has to follow,
-    on one CTA per tile and on a cluster."""
+# Two to nine chunks per CTA: the suffix joined and apart, one CTA per tile and a cluster, the widest tile, whose lanes hold two rows.
+@pytest.mark.parametrize("prefix,batch", [(200, 1), (256, 4), (600, 5), (900, 6), (700, 6), (2177, 11)])
+def test_attention_reference_moves(prefix, batch):
+    """Scores that grow from one chunk of keys to the next, by more than the exponents' reference stands: every CTA has to move it, some
+    of them twice.  (The keys of chunk c are scaled by 1 + 3 (c mod 6).)"""
+    from pi05_megakernel_b200 import _lib
     from pi05_megakernel_b200.arm import Pi05Arm
+    info = (ctypes.c_int * 5)()
+    assert _lib.load().pi05_chunk_attention(torch.cuda.get_device_properties(0).multi_processor_count, batch, prefix, prefix, info) == _lib.OK
+    assert info[3] >= 2 and not info[4]                 # a CTA with one chunk never moves
     geo, ogeo = FX.Geometry(prefix=prefix), O.Geo(prefix=prefix)
-    cpu = FX.make_inputs(geo, FX.SEEDS[2], "cpu", "full")
-    grow = torch.ones(prefix)
-    grow[prefix // 2:] = 12.0
-    grow[-20:] = 30.0
-    cpu["prefix_k"] = (cpu["prefix_k"].float() * grow.view(1, prefix, *[1] * (cpu["prefix_k"].dim() - 2))).to(torch.bfloat16)
-    arm = Pi05Arm(geo, "b200-s1-l3", "cuda")
-    arm.bind({k: v.cuda() for k, v in cpu.items()})
+    stacked, per = FX.make_batch(geo, FX.SEEDS[2], batch, "cpu", ["full"] * batch)
+    grow = 1.0 + 3.0 * (torch.arange(prefix) // 128 % 6)
+    for case in (stacked, *per):
+        case["prefix_k"] = (case["prefix_k"].float() * grow.view(prefix, 1, 1)).to(torch.bfloat16)
+    arm = Pi05Arm(geo, "b200-s1-l3", "cuda", batch=batch)
+    arm.bind({k: v.cuda() for k, v in (stacked if batch > 1 else per[0]).items()})
     arm.launch()
     arm.status()
-    want, exact = (O.chunk(cpu, ogeo, widen, arm.steps, arm.layers) for widen in (False, True))
-    d = O.band(want, arm.outputs()["actions"].cpu(), exact)
-    assert d["pass"], d
+    got = arm.outputs()["actions"].cpu().reshape(batch, 50, 32)
+    for b in {0, batch - 1}:
+        want, exact = (O.chunk(per[b], ogeo, widen, arm.steps, arm.layers) for widen in (False, True))
+        d = O.band(want, got[b], exact)
+        assert d["pass"], (b, d)
     arm.close()
 
 
