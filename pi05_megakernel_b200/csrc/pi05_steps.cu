@@ -728,8 +728,8 @@ std::string steps_describe(int sms, int batch, int prefix, int page_tokens, cons
   return out + "}";
 }
 
-// Every number of chunks of every batch is asked: the longest prefix does not need the most (148 SMs, five observations: tiles of 8
-// tokens over four CTAs up to 896 keys, of 4 over two from there on).
+// Every number of chunks of every batch is asked: the longest prefix does not need the most (148 SMs, four observations: tiles of 8
+// tokens over four CTAs at 968 tokens, of 4 over two at 1100).
 size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   size_t most = 0;
   for (int b = 1; b <= max_batch; ++b) {

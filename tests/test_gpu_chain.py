@@ -89,11 +89,16 @@ def test_attention_with_o_projection(prefix, batch, page):
 
 
 def test_smaller_binding_stays_in_the_workspace():
-    """Five observations of 700 tokens on an engine made for 968: an attention cut with more partial sums than the longest prefix's.
+    """Four observations of 968 tokens on an engine made for 1100: an attention cut with more partial sums than the longest prefix's.
     What lies behind the workspace stays as it was, and the actions are those of an engine of the binding's own size."""
     from pi05_megakernel_b200 import _lib
     from pi05_megakernel_b200.arm import Pi05Arm
-    geo, batch = FX.Geometry(prefix=700), 5
+    geo, batch, longest = FX.Geometry(prefix=968), 4, 1100
+    lib, sms = _lib.load(), torch.cuda.get_device_properties(0).multi_processor_count
+    info, held, needed = (ctypes.c_int * 4)(), ctypes.c_size_t(), [ctypes.c_size_t() for _ in range(2)]
+    for p, n in zip((geo.prefix, longest), needed):
+        assert lib.pi05_chunk_plan(sms, batch, longest, batch, p, info, ctypes.byref(held), ctypes.byref(n)) == _lib.OK
+    assert needed[0].value > needed[1].value            # else room for the longest prefix's sums would do
     stacked, _ = FX.make_batch(geo, FX.SEEDS[0], batch, "cpu", ["pad"] * batch)
     dev = {k: v.cuda() for k, v in stacked.items()}
     arm = Pi05Arm(geo, "b200-s1-l2", "cuda", batch=batch)
@@ -102,8 +107,8 @@ def test_smaller_binding_stays_in_the_workspace():
     arm.status()
     want = arm.outputs()["actions"].clone()
     arm.close()
-    lib, h, n = _lib.load(), ctypes.c_void_p(), ctypes.c_size_t()
-    assert lib.pi05_create(0, 968, batch, 0, 1, ctypes.byref(h)) == _lib.OK
+    h, n = ctypes.c_void_p(), ctypes.c_size_t()
+    assert lib.pi05_create(0, longest, batch, 0, 1, ctypes.byref(h)) == _lib.OK
     assert lib.pi05_workspace_bytes(h, ctypes.byref(n)) == _lib.OK
     ws = torch.full((n.value + (4 << 20),), 0xA5, dtype=torch.uint8, device="cuda")
     got = torch.zeros_like(want)
