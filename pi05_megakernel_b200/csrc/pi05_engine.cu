@@ -213,7 +213,7 @@ void build_layout(pi05_engine* h) {
   add("cond", (size_t)NS * W * 4);
   add("mod", (size_t)NS * NNORM * MODW * 4);
   add("rope", B * T * (HD / 2) * 4);
-  add("rope2", B * T * (HD / 2) * 4);
+  add("rope2", B * T * (HD / 2) * 4);         // the layout is that of the launch: gemm::rope_at over all tokens (chain), [T / 2][128][2] per observation (persistent kernel)
   add("x", B * T * ADIM * 4);
   add("state", 256);
   add("h", B * T * W * 2);

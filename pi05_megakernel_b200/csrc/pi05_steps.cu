@@ -42,7 +42,7 @@ using gemm::rb;
 struct TableArgs {
   float t_steps[NS];
   float* temb;
-  uint32_t *rope, *rope4;                    // [token][128], and in the order in which the QKV epilogue reads it
+  uint32_t *rope, *rope4;                    // [token][128] (no kernel of the chain reads it: the region that callers know as "rope"), and as the QKV epilogue reads it
   const uint8_t* mask;
   int* state;
   int prefix, n_steps;

@@ -18,7 +18,7 @@ struct StepSetup {
   int* state;                                // {Euler step, finished blocks of the step tail, Euler steps of this chunk}
   float *temb, *hid, *cond, *mod, *x, *part; // part: partial sums of split projections and attentions
   size_t part_floats;                        // what `part` holds (steps_part_floats)
-  uint32_t *rope, *rope4;
+  uint32_t *rope, *rope4;                    // [token][128]; the same words as gemm::rope_at orders them
   __nv_bfloat16 *h, *an, *q, *k, *v, *attn, *act;
   const void *pool_k, *pool_v;               // prefix cache; strides in elements
   long long token_stride, layer_stride, page_stride;

@@ -88,6 +88,26 @@ def test_attention_with_o_projection(prefix, batch, page):
     test_attention_cuts(prefix, batch, page)
 
 
+def test_rotary_tables_of_the_chain():
+    """What a launch of the chain leaves in its two rotary tables: cos | sin of dim j of token t, [token][128] as the workspace's "rope"
+    has been, and in groups of four dims, tokens of all observations next to each other, as the QKV projection reads them."""
+    from pi05_megakernel_b200.arm import Pi05Arm
+    geo, batch = FX.Geometry(prefix=77), 3
+    stacked, per = FX.make_batch(geo, FX.SEEDS[0], batch, "cpu", ["pad", "scatter", "full"])
+    arm = Pi05Arm(geo, "b200-s1-l1", "cuda", batch=batch)
+    arm.bind({k: v.cuda() for k, v in stacked.items()})
+    arm.launch()
+    arm.status()
+    rows = arm.region("rope", torch.bfloat16, (batch * 50, 128, 2)).cpu()
+    grouped = arm.region("rope2", torch.bfloat16, (32, batch * 50, 4, 2)).cpu()
+    assert torch.equal(grouped.permute(1, 0, 2, 3).reshape(batch * 50, 128, 2), rows)
+    inv = 1.0 / (O.ROPE_THETA ** (torch.arange(0, 256, 2, dtype=torch.int64).float() / 256))
+    phase = torch.cat([O.suffix_layout(v["prefix_mask"], 50)[0] for v in per]).float()[:, None] * inv[None]
+    # (values up to 1: a rounding to BF16 apart where the FP32 phase differs in its last bit)
+    assert float((rows.float() - torch.stack((phase.cos(), phase.sin()), -1).to(torch.bfloat16).float()).abs().max()) <= 2 ** -7
+    arm.close()
+
+
 def test_smaller_binding_stays_in_the_workspace():
     """Four observations of 968 tokens on an engine made for 1100: an attention cut with more partial sums than the longest prefix's.
     What lies behind the workspace stays as it was, and the actions are those of an engine of the binding's own size."""
