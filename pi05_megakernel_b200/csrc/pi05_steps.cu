@@ -438,11 +438,16 @@ bool joins(int prefix, int page_tokens) {
   return rows <= 72 && (rows <= 64 || prefix <= page_tokens || page_tokens % attn::KCH == 0);
 }
 
-// `prefix_chunks` chunks of 128 cached tokens; `may_join`: the suffix fits into the last of them.  The times behind the cost, in us, were fitted to every cut
+// `prefix_chunks` chunks of 128 cached tokens; `may_join`: the suffix fits into the last of them; `pages`: 0 where an observation's keys lie in one page, else 64 or
+// 128, the tokens that one copy brings of several pages.  The times behind the cost, in us, were fitted to every cut
 // timed by itself at 1 to 16 observations and 128 to 968 tokens, and then to whole chunks: a chunk of 128 keys, what a tile costs besides, a merge (dearer
 // with several observations, whose next kernels' CTAs wait for the clusters to leave), the copies of a joined chunk.  One chunk per CTA on a cluster of four:
 // 300 tokens 4.84 -> 4.64 ms (apart, 2 tokens x 4 CTAs, against joined on one), 384 4.86 -> 4.62; joined: 968 tokens 5.05 -> 4.85, two observations 5.99 -> 5.87.
-AttnPlan plan_attention(int sms, int batch, int prefix_chunks, bool may_join) {
+// Over several pages (fitted to all cuts at 1 to 16 observations, 129 to 1024 tokens) a chunk of cached keys costs 0.15 us more, on pages of 64 0.45, the half of it
+// where few CTAs fetch them, and joining the suffix saves the less the more chunks a CTA takes, behind which its own chunk would hide. Without these terms three
+// observations of 552 tokens on pages of 64 took 7.29 ms on joined tiles of 2 tokens, against 6.72 on 6 tokens x 4 CTAs, sixteen of 959 on pages of 128 12.76 against
+// 12.63 apart.
+AttnPlan plan_attention(int sms, int batch, int prefix_chunks, bool may_join, int pages) {
   AttnPlan best = {};
   double best_cost = 1e30;
   for (int i = 0; i < 40; ++i) {
@@ -454,8 +459,11 @@ AttnPlan plan_attention(int sms, int batch, int prefix_chunks, bool may_join) {
     // (a cluster is resident as a whole, and those of four and eight CTAs leave some SMs without: four observations of 968 tokens on 144 CTAs in
     // clusters of four 8.4 ms, on 112 7.0)
     if (splits > 1 && ctas > (splits == 8 ? sms * 3 / 4 : splits == 4 ? sms * 7 / 8 : sms)) continue;
-    const double cost = per_cta * (1.28 + 0.03 * t) * ((ctas + sms - 1) / sms) + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) +
-                        (splits > 1 ? 1.5 + 0.2 * t + (batch > 1 ? 0.9 : 0.0) : 0.0) + (join ? 0.8 : 0.0);
+    const int rounds = (ctas + sms - 1) / sms;
+    const double joined = pages ? 0.18 * per_cta + (pages == attn::KCH ? 0.3 : 0.0) : 0.8;
+    const double paged = (pages == 0 ? 0.0 : pages == attn::KCH ? 0.15 : 0.45) * (0.5 + 0.5 * std::min(ctas, sms) / sms) * (per_cta - (join || splits > 1 ? 0 : 1));
+    const double cost = (per_cta * (1.28 + 0.03 * t) + paged + (join ? joined : 0.0)) * rounds + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) +
+                        (splits > 1 ? 1.5 + 0.2 * t + (batch > 1 ? 0.9 : 0.0) : 0.0);
     if (cost >= best_cost) continue;
     best_cost = cost;
     best.tok_tile = t; best.tiles = tiles; best.splits = splits; best.join = join != 0;
@@ -463,7 +471,7 @@ AttnPlan plan_attention(int sms, int batch, int prefix_chunks, bool may_join) {
   return best;
 }
 AttnPlan plan_attention_for(int sms, int batch, int prefix, int page_tokens) {
-  return plan_attention(sms, batch, (prefix + attn::KCH - 1) / attn::KCH, joins(prefix, page_tokens));
+  return plan_attention(sms, batch, (prefix + attn::KCH - 1) / attn::KCH, joins(prefix, page_tokens), prefix <= page_tokens ? 0 : page_tokens % attn::KCH ? 64 : attn::KCH);
 }
 
 typedef void (*NormKernel)(const NormArgs);
@@ -736,7 +744,8 @@ size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
     const int splits = std::max(plan_gemm(sms, T * b, W, QD, gemm::EPI_PART).splits, plan_gemm(sms, T * b, W, FF, gemm::EPI_PART).splits);
     most = std::max(most, (size_t)std::max(splits, with_o(sms, b, 1) ? NQH : 0) * T * b * W);
     for (int chunks = 1; chunks <= (max_prefix + attn::KCH - 1) / attn::KCH; ++chunks)
-      for (bool join : {false, true}) most = std::max(most, attention_floats(b, plan_attention(sms, b, chunks, join)));
+      for (int pages : {0, 64, attn::KCH})
+        for (bool join : {false, true}) most = std::max(most, attention_floats(b, plan_attention(sms, b, chunks, join, pages)));
   }
   return most;
 }

@@ -20,11 +20,12 @@ CUTS = [
     (192, 5, "pad", "b200-s1-l2"), (193, 6, "scatter", "b200-s1-l2"), (301, 1, "scatter", "b200-s2-l2"), (968, 1, "pad", "b200-s2-l2"),
     (1100, 2, "scatter", "b200-s1-l2"), (130, 7, "full", "b200-s1-l2"), (65, 11, "pad", "b200-s1-l2"), (257, 16, "scatter", "b200-s1-l2")]
 # (prefix, batch, tokens per page).  What is left of the attention's cuts on a B200: tiles of 2, 4, 6, 8 and 14 tokens over one to eight
-# CTAs, the widest with a second segment of probabilities and a ring of four units; dense caches and pages of 64 and 128 tokens
+# CTAs, the widest with a second segment of probabilities and a ring of four units, also over eight CTAs; dense caches and pages of 64 and 128 tokens
 ATTENTION_CUTS = [(512, 1, 64), (600, 5, 0), (700, 6, 128), (700, 3, 64), (896, 9, 0), (896, 5, 64), (1700, 12, 0), (1300, 9, 64),
                   (440, 1, 64), (456, 1, 64), (900, 6, 0), (768, 4, 0), (840, 4, 128), (2176, 11, 0), (2177, 11, 64), (2816, 5, 0),
-                  (834, 1, 64), (250, 4, 128), (968, 2, 128), (960, 3, 64), (968, 4, 0), (700, 5, 0), (800, 7, 64), (250, 12, 64), (1160, 9, 0), (2950, 5, 0)]
-# (The suffix joins the last chunk of the prefix with 1, 4, 6 and 8 cached keys there (2177, 900, 2950, 1160), 36, 56 and 60 (1700, 440, 700) and
+                  (834, 1, 64), (250, 4, 128), (968, 2, 128), (960, 3, 64), (968, 4, 0), (700, 5, 0), (800, 7, 64), (250, 12, 64), (1160, 9, 0), (2950, 5, 0), (3457, 3, 64),
+                  (2945, 3, 64)]
+# (The suffix joins the last chunk of the prefix with 1, 4, 6 and 8 cached keys there (2177 and 2945, 900, 2950, 1160), 36, 56 and 60 (1700, 440, 700) and
 # with as many as there is room for: 64 on pages of 64 (960), 72 on pages of 128 and dense (968).  72 keys on pages of 64 stay apart (456), and where that is
 # no chunk more (840).)
 # Attention with the O projection (up to 128 cached tokens, up to two observations): 1, 8 and 9 keys, the last with a place of its own for Wo and the first without,

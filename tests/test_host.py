@@ -166,6 +166,50 @@ def test_every_attention_cut_has_a_gpu_test(lib):
         assert lib.pi05_chunk_attention(*args, info) == _lib.ERR_ARGUMENT
 
 
+# ms of an action chunk on a B200 by attention cut (query tokens, CTAs per tile, suffix joined), several cuts in turn in one process; (batch, prefix, page)
+TIMED_CUTS = {
+    (3, 552, 64): {(6, 4, 0): 6.72, (6, 4, 1): 6.79, (8, 4, 1): 6.87, (2, 1, 1): 7.29},
+    (9, 960, 64): {(8, 2, 1): 10.50, (8, 2, 0): 10.62, (4, 1, 0): 11.05, (4, 1, 1): 11.08},
+    (5, 574, 64): {(4, 1, 1): 7.53, (4, 2, 0): 7.55, (4, 2, 1): 7.68, (2, 1, 1): 7.86},
+    (6, 768, 64): {(6, 2, 0): 8.91, (14, 4, 0): 9.17, (4, 1, 0): 9.26},
+    (7, 703, 64): {(6, 2, 1): 8.90, (6, 2, 0): 9.02, (8, 2, 1): 9.17, (4, 1, 1): 9.31},
+    (3, 576, 128): {(6, 4, 0): 6.72, (4, 2, 0): 6.78, (8, 4, 0): 6.89, (2, 1, 1): 6.98},
+    (16, 959, 128): {(6, 1, 0): 12.62, (8, 1, 0): 12.75, (6, 1, 1): 12.76},
+    (11, 958, 128): {(4, 1, 0): 11.11, (4, 1, 1): 11.22, (6, 1, 0): 11.37},
+    (2, 259, 64): {(2, 1, 1): 5.30, (4, 1, 1): 5.32, (2, 1, 0): 5.45},
+    (1, 191, 64): {(2, 1, 1): 4.54, (2, 1, 0): 4.63, (4, 1, 1): 4.65},
+    (14, 190, 64): {(6, 1, 1): 10.02, (8, 1, 1): 10.15, (6, 1, 0): 10.20},
+    (4, 808, 0): {(4, 2, 0): 7.04, (8, 4, 0): 7.06, (8, 4, 1): 7.15},
+    (2, 680, 0): {(4, 4, 1): 5.65, (4, 4, 0): 5.67, (2, 2, 0): 5.86},
+}
+
+
+@pytest.mark.parametrize("batch,prefix,page", TIMED_CUTS)
+def test_attention_cut_is_one_of_the_fastest_timed(lib, batch, prefix, page):
+    """The cost model picks a cut within 0.8 % of the fastest one (runs of one cut differ by up to 0.4 %)."""
+    info = (ctypes.c_int * 5)()
+    assert lib.pi05_chunk_attention(148, batch, prefix, page or prefix, info) == _lib.OK
+    timed = TIMED_CUTS[batch, prefix, page]
+    assert timed.get(tuple(info)[:3], 1e9) <= 1.008 * min(timed.values())
+
+
+@pytest.mark.parametrize("sms", [132, 148, 152])
+def test_partials_of_paged_caches_fit_the_workspace(lib, sms):
+    """The parts of a split attention over several pages, whose cuts are not those of a dense cache."""
+    info, held, needed = (ctypes.c_int * 5)(), ctypes.c_size_t(), ctypes.c_size_t()
+    plan = (ctypes.c_int * 4)()
+    for batch in range(1, 17):
+        most = 0
+        for prefix in sorted({p for c in range(32) for p in (c * 128 + 1, c * 128 + 64, c * 128 + 72, c * 128 + 128)}):
+            for page in (64, 128):
+                assert lib.pi05_chunk_attention(sms, batch, prefix, page, info) == _lib.OK
+                tokens, splits = info[0], info[1]
+                if splits > 1:                              # a part: 8 rows per token, 256 dims, reference and sum
+                    most = max(most, batch * -(-50 // tokens) * splits * tokens * 8 * 258)
+            assert lib.pi05_chunk_plan(sms, batch, prefix, batch, prefix, plan, ctypes.byref(held), ctypes.byref(needed)) == _lib.OK
+            assert held.value >= most, (batch, prefix)
+
+
 def test_prefill_fixture_is_deterministic():
     geo = FX.PrefillGeometry(tokens=96, layers=1)
     shapes = FX.prefill_shapes(geo)
