@@ -438,6 +438,30 @@ bool joins(int prefix, int page_tokens) {
   return rows <= 72 && (rows <= 64 || prefix <= page_tokens || page_tokens % attn::KCH == 0);
 }
 
+// The cuts of `batch` observations and the part of their cost (in us, below) that does not depend on the keys: per chunk, `fixed`; `share`: of the
+// fetches of cached keys that contend.
+struct AttnCuts {
+  struct Cut { int tok_tile, tiles, splits, shift, rounds; double chunk, fixed, share; } cut[20];
+  int n;
+};
+AttnCuts attention_cuts(int sms, int batch) {
+  AttnCuts a;
+  a.n = 0;
+  for (int t : {2, 4, 6, 8, 14})
+    for (int shift = 0; shift < 4; ++shift) {
+      const int splits = 1 << shift, tiles = (T + t - 1) / t, ctas = batch * tiles * splits;
+      // (a cluster is resident as a whole, and those of four and eight CTAs leave some SMs without: four observations of 968 tokens on 144 CTAs in
+      // clusters of four 8.4 ms, on 112 7.0)
+      if (splits > 1 && ctas > (splits == 8 ? sms * 3 / 4 : splits == 4 ? sms * 7 / 8 : sms)) continue;
+      AttnCuts::Cut& c = a.cut[a.n++];
+      c.tok_tile = t; c.tiles = tiles; c.splits = splits; c.shift = shift; c.rounds = (ctas + sms - 1) / sms;
+      c.chunk = 1.28 + 0.03 * t;
+      c.fixed = (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) + (splits > 1 ? 1.5 + 0.2 * t + (batch > 1 ? 0.9 : 0.0) : 0.0);
+      c.share = 0.5 + 0.5 * std::min(ctas, sms) / sms;
+    }
+  return a;
+}
+
 // `prefix_chunks` chunks of 128 cached tokens; `may_join`: the suffix fits into the last of them; `pages`: 0 where an observation's keys lie in one page, else 64 or
 // 128, the tokens that one copy brings of several pages.  The times behind the cost, in us, were fitted to every cut
 // timed by itself at 1 to 16 observations and 128 to 968 tokens, and then to whole chunks: a chunk of 128 keys, what a tile costs besides, a merge (dearer
@@ -447,31 +471,26 @@ bool joins(int prefix, int page_tokens) {
 // where few CTAs fetch them, and joining the suffix saves the less the more chunks a CTA takes, behind which its own chunk would hide. Without these terms three
 // observations of 552 tokens on pages of 64 took 7.29 ms on joined tiles of 2 tokens, against 6.72 on 6 tokens x 4 CTAs, sixteen of 959 on pages of 128 12.76 against
 // 12.63 apart.
-AttnPlan plan_attention(int sms, int batch, int prefix_chunks, bool may_join, int pages) {
+AttnPlan plan_attention(const AttnCuts& cuts, int prefix_chunks, bool may_join, int pages) {
   AttnPlan best = {};
   double best_cost = 1e30;
-  for (int i = 0; i < 40; ++i) {
-    static const int kTokens[] = {2, 4, 6, 8, 14};
-    const int join = 1 - i / 20, t = kTokens[i / 4 % 5], splits = 1 << i % 4;
-    const int chunks = prefix_chunks + (join ? 0 : 1), tiles = (T + t - 1) / t, ctas = batch * tiles * splits;
-    if (splits > chunks || (join && !may_join)) continue;
-    const int per_cta = (chunks + splits - 1) / splits;
-    // (a cluster is resident as a whole, and those of four and eight CTAs leave some SMs without: four observations of 968 tokens on 144 CTAs in
-    // clusters of four 8.4 ms, on 112 7.0)
-    if (splits > 1 && ctas > (splits == 8 ? sms * 3 / 4 : splits == 4 ? sms * 7 / 8 : sms)) continue;
-    const int rounds = (ctas + sms - 1) / sms;
-    const double joined = pages ? 0.18 * per_cta + (pages == attn::KCH ? 0.3 : 0.0) : 0.8;
-    const double paged = (pages == 0 ? 0.0 : pages == attn::KCH ? 0.15 : 0.45) * (0.5 + 0.5 * std::min(ctas, sms) / sms) * (per_cta - (join || splits > 1 ? 0 : 1));
-    const double cost = (per_cta * (1.28 + 0.03 * t) + paged + (join ? joined : 0.0)) * rounds + (t <= 4 ? 0.28 * (t - 2) : 0.42 * t - 1.1) +
-                        (splits > 1 ? 1.5 + 0.2 * t + (batch > 1 ? 0.9 : 0.0) : 0.0);
-    if (cost >= best_cost) continue;
-    best_cost = cost;
-    best.tok_tile = t; best.tiles = tiles; best.splits = splits; best.join = join != 0;
-  }
+  const double page_cost = pages == 0 ? 0.0 : pages == attn::KCH ? 0.15 : 0.45;
+  for (int join = may_join ? 1 : 0; join >= 0; --join)
+    for (int i = 0; i < cuts.n; ++i) {
+      const AttnCuts::Cut& c = cuts.cut[i];
+      const int chunks = prefix_chunks + (join ? 0 : 1), per_cta = (chunks + c.splits - 1) >> c.shift;
+      if (c.splits > chunks) continue;
+      const double joined = !join ? 0.0 : pages ? 0.18 * per_cta + (pages == attn::KCH ? 0.3 : 0.0) : 0.8;
+      const double paged = page_cost * c.share * (per_cta - (join || c.splits > 1 ? 0 : 1));
+      const double cost = (per_cta * c.chunk + paged + joined) * c.rounds + c.fixed;
+      if (cost >= best_cost) continue;
+      best_cost = cost;
+      best.tok_tile = c.tok_tile; best.tiles = c.tiles; best.splits = c.splits; best.join = join != 0;
+    }
   return best;
 }
 AttnPlan plan_attention_for(int sms, int batch, int prefix, int page_tokens) {
-  return plan_attention(sms, batch, (prefix + attn::KCH - 1) / attn::KCH, joins(prefix, page_tokens), prefix <= page_tokens ? 0 : page_tokens % attn::KCH ? 64 : attn::KCH);
+  return plan_attention(attention_cuts(sms, batch), (prefix + attn::KCH - 1) / attn::KCH, joins(prefix, page_tokens), prefix <= page_tokens ? 0 : page_tokens % attn::KCH ? 64 : attn::KCH);
 }
 
 typedef void (*NormKernel)(const NormArgs);
@@ -743,9 +762,10 @@ size_t steps_part_floats(int sms, int max_batch, int max_prefix) {
   for (int b = 1; b <= max_batch; ++b) {
     const int splits = std::max(plan_gemm(sms, T * b, W, QD, gemm::EPI_PART).splits, plan_gemm(sms, T * b, W, FF, gemm::EPI_PART).splits);
     most = std::max(most, (size_t)std::max(splits, with_o(sms, b, 1) ? NQH : 0) * T * b * W);
+    const AttnCuts cuts = attention_cuts(sms, b);
     for (int chunks = 1; chunks <= (max_prefix + attn::KCH - 1) / attn::KCH; ++chunks)
       for (int pages : {0, 64, attn::KCH})
-        for (bool join : {false, true}) most = std::max(most, attention_floats(b, plan_attention(sms, b, chunks, join, pages)));
+        for (bool join : {false, true}) most = std::max(most, attention_floats(b, plan_attention(cuts, chunks, join, pages)));
   }
   return most;
 }
