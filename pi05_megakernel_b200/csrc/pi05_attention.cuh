@@ -111,7 +111,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_kernel(const __grid_cons
   const uint32_t q_base = ptx::smem_u32(smem), p_base = q_base + 4 * QBLK, ring = p_base + p_bytes(N);
   const bool leader = ptx::elect_one();
 
-  // Units of V of this CTA's chunk i (of a joined chunk: halves of the dims, laid out like K; else halves of the keys).  The ring's order is K0 | K1 V0 | K2 V1 | .. | V(n-1); a suffix at the end goes behind the values of the chunk before it, which do not depend on the kernel before this one.
+  // Units of V of this CTA's chunk i (of a joined chunk: halves of the dims, laid out like K; else halves of the keys).  The ring's order is
+  // K0 | K1 V0 | K2 V1 | .. | V(n-1); a suffix at the end goes behind the values of the chunk before it, which do not depend on the kernel
+  // before this one.
   auto nv = [&](int i) { const int c = cbeg + i; return c < late ? (p.prefix - c * KCH > 64 ? 2 : 1) : JOIN ? 2 : 1; };
   const bool swapped = n >= 2 && cbeg + n > late;
 

@@ -63,6 +63,7 @@ __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
   return *reinterpret_cast<const uint32_t*>(&m);
 }
 
+// (A template so that every file that includes this one may, and only the one that launches the kernel compiles it.)
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) attention_o_kernel(const __grid_constant__ Args p) {
   constexpr int TM_S = 0, TM_O = 128, TM_D = 0, TM_COLS = 256;       // two S^T, two halves of O^T; D takes the place of S^T

@@ -70,7 +70,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 __device__ __forceinline__ float lo16(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi16(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
-// 0.5 x (1 + tanh z) = x / (1 + exp(-2 z)) with z = 0.79788 (x + 0.044715 x^3): one exponential and one division, no
+// 0.5 x (1 + tanh z) = x / (1 + exp(-2 z)) with z = 0.79788 (x + 0.044715 x^3): one exponential and one reciprocal, no
 // cancellation for negative x.  The constants carry the factor -2 log2 e.
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float e = ptx::ex2_approx(x * fmaf(x * x, -0.10294324f, -2.3022082f));
@@ -79,7 +79,8 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 
 // Staging of a tile's results: boxes of 128 rows x BOX bytes (swizzled, so that neither its writers nor its readers meet in a bank), COUNT of them; 0: the
 // tile is small and its rows are stored directly.  PART: 32 FP32 columns a box; GEGLU and QKV: 64 BF16 (QKV of 64
-// features: 32, each half of the tile a box; GEGLU of 224: 16, which 112 results are a multiple of).
+// features: 32, each half of the tile a box; GEGLU of 224: 16, which 112 results are a multiple of; GEGLU of 112 is stored directly, 56 results a row, like the 64 of
+// which it is a wider form: staged it was not tried).
 template <int EPI, int BN>
 struct Staging {
   static constexpr int COUNT = EPI == EPI_PART ? (BN >= 64 ? BN / 32 : 0) : EPI == EPI_GEGLU ? (BN == 224 ? 7 : BN == 112 ? 0 : BN / 128) : (BN == 256 ? 4 : BN >= 64 ? 2 : 0);

@@ -620,7 +620,9 @@ struct Chain {
     }
     auto joined = [&](CUtensorMap* m, const void* pool) { return !ap.m_rows || map_kv(m, pool, tail, L, s.num_pages, s.token_stride, s.layer_stride, s.page_stride, ap.m_rows, 1); };
     auto joined_suffix = [&](CUtensorMap* m, const void* kv) { return !ap.m_rows || map_kv(m, kv, T, 1, s.batch, HD, (uint64_t)T * HD, (uint64_t)T * HD, ap.m_suf, 1); };
-    if (!(joined(&ap.jk, s.pool_k) && joined(&ap.jv, s.pool_v) && joined_suffix(&ap.jsk, s.k) && joined_suffix(&ap.jsv, s.v) && map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_short, s.an, W, M, pq.arows - 8, pq.ks) && map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
+    if (!(joined(&ap.jk, s.pool_k) && joined(&ap.jv, s.pool_v) && joined_suffix(&ap.jsk, s.k) && joined_suffix(&ap.jsv, s.v) &&
+          map_k(&a_qkv, s.an, W, M, pq.arows, pq.ks) && map_k(&a_short, s.an, W, M, pq.arows - 8, pq.ks) &&
+          map_k(&a_o, s.attn, QD, M, po.arows, po.ks) && map_k(&a_gu, s.an, W, M, pg.arows, pg.ks) &&
           map_k(&a_dn, s.act, FF, M, pd.arows, pd.ks) && weights(&wq, 8, W, QD, pq) && weights(&wk, 9, W, HD, pq) && weights(&wv, 10, W, HD, pq) &&
           weights(&wo, 11, QD, W, po) && weights(&wg, 12, W, FF, pg) && weights(&wu, 13, W, FF, pg) && weights(&wd, 14, FF, W, pd) &&
           map_k(&ap.q, s.q, HD, M * NQH, ap.tok_tile * NQH, HD / 64) &&

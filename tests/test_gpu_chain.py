@@ -28,9 +28,9 @@ ATTENTION_CUTS = [(512, 1, 64), (600, 5, 0), (700, 6, 128), (700, 3, 64), (896, 
 # (The suffix joins the last chunk of the prefix with 1, 4, 6 and 8 cached keys there (2177 and 2945, 900, 2950, 1160), 36, 56 and 60 (1700, 440, 700) and
 # with as many as there is room for: 64 on pages of 64 (960), 72 on pages of 128 and dense (968).  72 keys on pages of 64 stay apart (456), and where that is
 # no chunk more (840).)
-# Attention with the O projection (up to 128 cached tokens, up to two observations): 1, 8 and 9 keys, the last with a place of its own for Wo and the first without,
+# Attention with the O projection (up to 128 cached tokens, up to two observations): 1, 8 and 9 keys, 64 and 65 (Wo in a place of its own and in that of the keys),
 # 72 and 73 (suffix within the first 128 rows and across them), 120 and 128 (an odd and an even number of eights), one page and two
-ATTENTION_O = [(8, 1, 0), (9, 2, 64), (64, 1, 64), (65, 1, 64), (65, 2, 0), (72, 1, 128), (73, 2, 64), (120, 1, 0), (127, 2, 64), (128, 1, 64), (128, 2, 128)]
+ATTENTION_O = [(1, 1, 0), (1, 2, 64), (8, 1, 0), (9, 2, 64), (64, 1, 64), (65, 1, 64), (65, 2, 0), (72, 1, 128), (73, 2, 64), (120, 1, 0), (127, 2, 64), (128, 1, 64), (128, 2, 128)]
 
 
 @pytest.mark.parametrize("prefix,batch,mask,variant", CUTS)
