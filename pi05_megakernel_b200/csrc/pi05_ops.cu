@@ -118,7 +118,7 @@ GemmPlan plan_gemm(int sms, int tokens, int n, int k, int epi, int pairs) {
       g.rows = (tokens + g.m_tiles - 1) / g.m_tiles;
       g.arows = (g.rows + 7) / 8 * 8;
       // 112 and 224 features (56 and 112 of gate and of up) are for widths that they cut into whole rounds: 4096 in two rounds of 74 pairs beside 1.73 of
-      // 256 (sixteen observations 10.30 -> 10.13 ms, prefill of 256 tokens 1.52 -> 1.48), 16384 in two rounds of 148 CTAs beside 3.5 of 64 (prefill of 128 tokens
+      // 256 (both widths in turn in one process: sixteen observations of 128 tokens 10.32 -> 10.20 ms, of 600 11.51 -> 11.42; prefill of 256 tokens 1.52 -> 1.48), 16384 in two rounds of 148 CTAs beside 3.5 of 64 (prefill of 128 tokens
       // 1.32 -> 1.26).  In a single round either way they only pay where the MMAs take long: 5 observations (tiles of 125 tokens) 6.32 -> 6.21, 9 (113) 8.06 -> 7.96,
       // but 7 (88) 7.11 -> 7.28: the narrower tile occupies 148 SMs, not 128, and the next kernel's CTAs start late
       if ((g.bn == 224 || g.bn == 112) && g.m_tiles * n_tiles <= sms && (tokens + g.m_tiles - 1) / g.m_tiles <= 96) continue;
