@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 # (prefix, batch, mask, steps and layers).  128-key chunks: up to 64 valid keys in the last one and more, one key; the keys of a
-# tile over 1, 2, 4 and 8 CTAs; projections on tiles of up to 64 and up to 128 tokens, on two, three, six and eight of them,
+# tile over 1, 4 and 8 CTAs; projections on tiles of up to 64 and up to 128 tokens, on two, three, six and eight of them,
 # on single CTAs and on pairs, persistent or not; attention on tiles of 2, 4 and 6 tokens.
 CUTS = [
     (1, 1, "full", "b200-s2-l2"), (63, 1, "scatter", "b200-s2-l2"), (128, 2, "pad", "b200-s2-l2"), (129, 3, "scatter", "b200-s2-l2"),
@@ -259,7 +259,8 @@ def test_attention_reference_moves(prefix, batch):
     arm.close()
 
 
-@pytest.mark.parametrize("tokens", [1, 65, 128, 129, 297, 600, 900, 1200])
+# (800: QKV on single CTAs of 128 features; 2400: QKV and O on persistent pairs)
+@pytest.mark.parametrize("tokens", [1, 65, 128, 129, 297, 600, 800, 900, 1200, 2400])
 def test_prefill_cuts(tokens):
     from pi05_megakernel_b200.prefill import Pi05Prefill
     geo = FX.PrefillGeometry(tokens=tokens)
