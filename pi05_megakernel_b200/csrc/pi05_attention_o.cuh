@@ -181,6 +181,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_o_kernel(const __grid_co
     go = go && ptx::wait_bar(p.status, p.limit, p_full, 0, attn::WAIT_P_FULL);
     if (go) {
       ptx::tc_fence_after();
+      // (where the rows are an odd number of eights, the last 16 keys reach into the next segment's values, behind the last one into Q, and into O^T while its
+      // first half is being written there: finite values times the zeros that P has in those rows)
 #pragma unroll 1
       for (int d = 0; d < 2; ++d) {
         const uint32_t vd = vdesc + (d * 2 * seg >> 4), od = tmem + TM_O + d * N;
